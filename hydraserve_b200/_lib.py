@@ -68,6 +68,11 @@ EXPORTS = {
     "hs_greedy_noalloc_error": (C.c_char_p, []),
     "hs_sample_host": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int, C.c_int,
                                  C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint32, C.c_void_p]),
+    "hs_step_block": (C.c_int, [C.c_void_p, C.c_size_t, C.POINTER(C.c_void_p)]),
+    "hs_step": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int, C.c_int, C.c_void_p,
+                          C.POINTER(C.c_void_p), C.c_void_p]),
+    "hs_step_greedy": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int, C.c_int,
+                                 C.POINTER(C.c_void_p), C.c_void_p]),
     "hs_sharded_partial": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int, C.c_int, C.c_int,
                                      C.c_void_p, C.c_void_p, C.c_void_p]),
     "hs_sharded_merge": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p,
@@ -95,6 +100,21 @@ def load() -> C.CDLL:
             fn.argtypes = argtypes
         _lib = lib
     return _lib
+
+
+def load_host():
+    """The native host side (a Python extension next to this file).  It needs no GPU and no CUDA
+    library; when its sources are there and it is not, it is compiled first."""
+    import importlib
+
+    try:
+        return importlib.import_module("hydraserve_b200._host")
+    except ImportError:
+        from . import build
+
+        build.build_host()
+        importlib.invalidate_caches()
+        return importlib.import_module("hydraserve_b200._host")
 
 
 class SamplerError(RuntimeError):

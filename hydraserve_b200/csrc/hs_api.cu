@@ -25,7 +25,6 @@ namespace {
 
 using hs::u64;
 
-constexpr int kGreedyMaxChunks = 64;
 constexpr int kMaxSplit = 4;  // CTAs per row on the candidate path
 constexpr int kSideCapMax = 16384;  // side-list entries a CTA can keep in global scratch
 
@@ -85,7 +84,8 @@ struct hs_sampler {
   int side_cap = 0;
   unsigned long long* phase_clocks = nullptr;  // HS_CREATE_PHASE_CLOCKS: per-row phase timestamps
   hs::Pool pool{};
-  u64* greedy_partials = nullptr;
+  u64* greedy_best = nullptr;   // [batch_max] best element of a row so far (0 between calls)
+  int* greedy_ticket = nullptr;  // [batch_max] its chunks that have arrived (0 between calls)
   float* gstage = nullptr;  // global stand-in for the on-chip row copy (very wide rows only)
   size_t gstage_elems = 0;
   // device + pinned staging for the host-buffer call
@@ -99,6 +99,13 @@ struct hs_sampler {
   int32_t* d_slots = nullptr;
   hs_row_params* h_params = nullptr;  // pinned
   int32_t* h_small = nullptr;         // pinned: offsets[batch_max+1] then slots[batch_max]
+  // hs_step: the pinned block its caller fills, its copy on the device, and pinned results
+  unsigned char* h_block = nullptr;
+  size_t h_block_bytes = 0;
+  unsigned char* d_block = nullptr;
+  size_t d_block_bytes = 0;
+  hs_row_out* h_out = nullptr;    // [batch_max]
+  int32_t* h_tokens = nullptr;    // [batch_max]
   std::mutex mu;         // the staging buffers of hs_sample_host
   // Every launching call takes launch_mu, and work of one call is ordered after the previous
   // call's on the GPU (an event when the stream changed), because all calls share the
@@ -185,9 +192,44 @@ int check_common(hs_sampler* h, const void* logits, int dtype, int batch, int vo
   return HS_OK;
 }
 
+// Launch attributes: `cluster` CTAs per cluster; `behind` = the kernel may get ready while the one
+// launched before it on the stream is still running (it waits for that one's end by itself).
+struct LaunchAttrs {
+  cudaLaunchAttribute a[2];
+  unsigned n = 0;
+  LaunchAttrs(int cluster, bool behind) {
+    if (cluster > 0) {
+      a[n].id = cudaLaunchAttributeClusterDimension;
+      a[n].val.clusterDim.x = (unsigned)cluster; a[n].val.clusterDim.y = 1; a[n].val.clusterDim.z = 1;
+      ++n;
+    }
+    if (behind) {
+      a[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      a[n].val.programmaticStreamSerializationAllowed = 1;
+      ++n;
+    }
+  }
+};
+template <class... Params, class... Args>
+cudaError_t launch(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, LaunchAttrs attrs,
+                   Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attrs.a;
+  cfg.numAttrs = attrs.n;
+  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
+const hs::InlineRows kNoInlineRows{};  // (stands in when the parameters are in device memory)
+
+// `params` in device memory, or null with the rows' parameters in `inl`; `behind`: the launch before
+// this one on the stream is one of this sampler's histogram kernels.
 int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
-                const hs_row_params* params, hs_row_out* out, const float* noise, float* scores_out,
-                int32_t* tokens_out, uint32_t flags, cudaStream_t stream) {
+                const hs_row_params* params, const hs::InlineRows& inl, hs_row_out* out, const float* noise,
+                float* scores_out, int32_t* tokens_out, uint32_t flags, bool behind, cudaStream_t stream) {
   Plan plan;
   hs::RowKernelArgs a{};
   a.logits = logits; a.dtype = dtype; a.row_stride = row_stride; a.vocab = vocab; a.slice = 0;
@@ -214,8 +256,7 @@ int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride
                      csplit, h->ctab, h->crare, h->crare_n, h->count_ticket,
                      split, h->split_lists, h->split_n, h->split_ticket, batch};
     const unsigned grid = (unsigned)batch * (unsigned)(csplit + split);
-    hs::row_kernel_bf16<<<grid, hs::kThreads, hs::bf16_kernel_smem(), stream>>>(a3);
-    HS_CUDA(h, cudaGetLastError());
+    HS_CUDA(h, launch(hs::row_kernel_bf16, dim3(grid), hs::kThreads, hs::bf16_kernel_smem(), stream, LaunchAttrs(0, behind), a3, inl));
     h->launches += 1;
     return HS_OK;
   }
@@ -226,8 +267,9 @@ int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride
   if (dtype == HS_DTYPE_F32 && !h->force_general && !(flags & HS_SAMPLE_GENERAL_KERNEL)) {
     a.skip_candidate_rows = 1;
     hs::F32TopkArgs f{a, h->phase_clocks};
-    hs::row_kernel_f32_topk<<<(unsigned)batch, hs::kThreads, hs::layout_cand().total, stream>>>(f);
-    HS_CUDA(h, cudaGetLastError());
+    HS_CUDA(h, launch(hs::row_kernel_f32_topk, dim3((unsigned)batch), hs::kThreads, hs::layout_cand().total, stream,
+                      LaunchAttrs(0, behind), f, inl));
+    behind = false;
     h->launches += 1;
   }
   if (plan.global_stage) {
@@ -237,35 +279,25 @@ int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride
   a.slice = plan.slice;
   a.gstage = plan.global_stage ? h->gstage : nullptr;
 
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)plan.cluster, (unsigned)batch, 1);
-  cfg.blockDim = dim3(hs::kThreads, 1, 1);
-  cfg.dynamicSmemBytes = plan.smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)plan.cluster;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  HS_CUDA(h, cudaLaunchKernelEx(&cfg, hs::row_kernel, a));
+  HS_CUDA(h, launch(hs::row_kernel, dim3((unsigned)plan.cluster, (unsigned)batch), hs::kThreads, plan.smem, stream,
+                    LaunchAttrs(plan.cluster, behind), a, inl));
   h->launches += 1;
   return HS_OK;
 }
 
 int launch_greedy(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
                   int32_t* tokens_out, cudaStream_t stream) {
-  int chunks = (2 * h->sm_count + batch - 1) / batch;
-  chunks = std::max(1, std::min(chunks, kGreedyMaxChunks));
+  // enough CTAs to fill the SMs four times over (eight fit, but a shorter chunk than one load per
+  // thread gains nothing)
+  int chunks = (4 * h->sm_count + batch - 1) / batch;
+  const int per = hs::kGreedyThreads * (dtype == HS_DTYPE_BF16 ? 8 : 4);
+  chunks = std::max(1, std::min(chunks, (vocab + per - 1) / per));
   int chunk = ((vocab + chunks - 1) / chunks + 7) & ~7;
   chunks = (vocab + chunk - 1) / chunk;
-  hs::greedy_partial_kernel<<<dim3((unsigned)chunks, (unsigned)batch), hs::kGreedyThreads, 0, stream>>>(
-      logits, dtype, row_stride, vocab, chunk, h->greedy_partials);
+  hs::greedy_kernel<<<dim3((unsigned)chunks, (unsigned)batch), hs::kGreedyThreads, 0, stream>>>(
+      logits, dtype, row_stride, vocab, chunk, h->greedy_best, h->greedy_ticket, tokens_out);
   HS_CUDA(h, cudaGetLastError());
-  hs::greedy_final_kernel<<<(batch + 127) / 128, 128, 0, stream>>>(h->greedy_partials, chunks, batch, tokens_out);
-  HS_CUDA(h, cudaGetLastError());
-  h->launches += 2;
+  h->launches += 1;
   return HS_OK;
 }
 
@@ -292,10 +324,13 @@ void release(hs_sampler* h) {
   cudaFree(h->split_lists); cudaFree(h->split_n); cudaFree(h->split_ticket);
   if (h->ev_done) cudaEventDestroy(h->ev_done);
   cudaFree(h->phase_clocks);
-  cudaFree(h->pool.error); cudaFree(h->greedy_partials); cudaFree(h->gstage); cudaFree(h->d_logits);
+  cudaFree(h->pool.error); cudaFree(h->greedy_best); cudaFree(h->greedy_ticket); cudaFree(h->d_block); cudaFree(h->gstage); cudaFree(h->d_logits);
   cudaFree(h->d_params); cudaFree(h->d_out); cudaFree(h->d_hist); cudaFree(h->d_offsets); cudaFree(h->d_slots);
   if (h->h_params) cudaFreeHost(h->h_params);
   if (h->h_small) cudaFreeHost(h->h_small);
+  if (h->h_block) cudaFreeHost(h->h_block);
+  if (h->h_out) cudaFreeHost(h->h_out);
+  if (h->h_tokens) cudaFreeHost(h->h_tokens);
 }
 
 }  // namespace
@@ -450,7 +485,8 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
   ok = ok && dmalloc(h, &h->pool.cls, st * (size_t)h->pool.cls_stride * sizeof(uint32_t));
   ok = ok && dmalloc(h, &h->pool.pos, st * (size_t)vocab_max * sizeof(int32_t));
   ok = ok && dmalloc(h, &h->pool.error, sizeof(int32_t));
-  ok = ok && dmalloc(h, &h->greedy_partials, (size_t)batch_max * kGreedyMaxChunks * sizeof(u64));
+  ok = ok && dmalloc(h, &h->greedy_best, (size_t)batch_max * sizeof(u64));
+  ok = ok && dmalloc(h, &h->greedy_ticket, (size_t)batch_max * sizeof(int));
   ok = ok && dmalloc(h, &h->d_params, (size_t)batch_max * sizeof(hs_row_params));
   ok = ok && dmalloc(h, &h->d_out, (size_t)batch_max * sizeof(hs_row_out));
   ok = ok && dmalloc(h, &h->d_offsets, ((size_t)batch_max + 1) * sizeof(int32_t));
@@ -471,6 +507,8 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
   ok = ok && dmalloc(h, &h->split_n, (size_t)batch_max * kMaxSplit * sizeof(int));
   ok = ok && dmalloc(h, &h->split_ticket, (size_t)batch_max * sizeof(int));
   ok = ok && cudaMallocHost(&h->h_params, (size_t)batch_max * sizeof(hs_row_params)) == cudaSuccess;
+  ok = ok && cudaMallocHost(&h->h_out, (size_t)batch_max * sizeof(hs_row_out)) == cudaSuccess;
+  ok = ok && cudaMallocHost(&h->h_tokens, (size_t)batch_max * sizeof(int32_t)) == cudaSuccess;
   ok = ok && cudaMallocHost(&h->h_small, (2 * (size_t)batch_max + 1) * sizeof(int32_t)) == cudaSuccess;
   if (flags & HS_CREATE_PHASE_CLOCKS) {
     const size_t bytes = (size_t)batch_max * hs::kV3PhaseSlots * sizeof(unsigned long long);
@@ -479,6 +517,8 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
   }
   if (!ok) return bail(HS_ERR_CUDA);
   ok = ok && cudaMemset(h->split_ticket, 0, (size_t)batch_max * sizeof(int)) == cudaSuccess;
+  ok = ok && cudaMemset(h->greedy_best, 0, (size_t)batch_max * sizeof(u64)) == cudaSuccess;
+  ok = ok && cudaMemset(h->greedy_ticket, 0, (size_t)batch_max * sizeof(int)) == cudaSuccess;
   ok = ok && cudaMemset(h->scratch_busy, 0, (size_t)h->resident_bf16 * sizeof(int)) == cudaSuccess;
   ok = ok && cudaMemset(h->count_ticket, 0, (size_t)batch_max * sizeof(int)) == cudaSuccess;
   ok = ok && cudaMemset(h->pool.n, 0, st * sizeof(int32_t)) == cudaSuccess;
@@ -566,8 +606,8 @@ int hs_sample_ex(hs_sampler* h, const void* logits, int dtype, int64_t row_strid
   DeviceGuard guard(h->device);
   Serial serial(h, (cudaStream_t)stream);
   HS_CUDA(h, serial.status);
-  rc = launch_rows(h, logits, dtype, row_stride, batch, vocab, params, out, noise, scores_out, tokens_out,
-                   flags, (cudaStream_t)stream);
+  rc = launch_rows(h, logits, dtype, row_stride, batch, vocab, params, kNoInlineRows, out, noise, scores_out,
+                   tokens_out, flags, false, (cudaStream_t)stream);
   if (rc != HS_OK) return rc;
   HS_CUDA(h, serial.done());
   return HS_OK;
@@ -672,11 +712,134 @@ int hs_sample_host(hs_sampler* h, const void* logits, int dtype, int64_t row_str
     if (rc != HS_OK) return rc;
   }
   HS_CUDA(h, cudaMemcpyAsync(h->d_params, h->h_params, (size_t)batch * sizeof(hs_row_params), cudaMemcpyHostToDevice, stream));
-  rc = launch_rows(h, h->d_logits, dtype, vocab, batch, vocab, h->d_params, h->d_out, nullptr, nullptr, nullptr, flags, stream);
+  rc = launch_rows(h, h->d_logits, dtype, vocab, batch, vocab, h->d_params, kNoInlineRows, h->d_out, nullptr, nullptr,
+                   nullptr, flags, false, stream);
   if (rc != HS_OK) return rc;
   HS_CUDA(h, cudaMemcpyAsync(out, h->d_out, (size_t)batch * sizeof(hs_row_out), cudaMemcpyDeviceToHost, stream));
   HS_CUDA(h, serial.done());
   HS_CUDA(h, cudaStreamSynchronize(stream));
+  return HS_OK;
+}
+
+int hs_step_block(hs_sampler* h, size_t bytes, void** block) {
+  if (!h || !block) return HS_ERR_INVALID;
+  *block = nullptr;
+  if (bytes > h->h_block_bytes) {
+    DeviceGuard guard(h->device);
+    const size_t want = std::max<size_t>(bytes + bytes / 2, 64 << 10);
+    if (h->h_block) cudaFreeHost(h->h_block);
+    h->h_block = nullptr;
+    h->h_block_bytes = 0;
+    HS_CUDA(h, cudaMallocHost(&h->h_block, want));
+    h->h_block_bytes = want;
+  }
+  *block = h->h_block;
+  return HS_OK;
+}
+
+int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
+            const hs_step_desc* d, const hs_row_out** out, void* stream_) {
+  int rc = check_common(h, logits, dtype, batch, vocab);
+  if (rc != HS_OK) return rc;
+  if (!d || !out) return fail(h, HS_ERR_INVALID, "desc / out is null");
+  *out = h->h_out;
+  if (batch == 0) return HS_OK;
+  if (row_stride < vocab) return fail(h, HS_ERR_INVALID, "row_stride smaller than vocab");
+  if (d->n_resets < 0 || d->n_appends < 0 || d->n_appends > 65535 || d->n_resets > 65535)
+    return fail(h, HS_ERR_CAPACITY, "too many slots in one call");
+  if (d->bytes > h->h_block_bytes || d->bytes < (size_t)batch * sizeof(hs_row_params) ||
+      d->resets_at + (size_t)d->n_resets * 4 > d->bytes || d->slots_at + (size_t)d->n_appends * 4 > d->bytes ||
+      (d->n_appends && d->offsets_at + ((size_t)d->n_appends + 1) * 4 > d->bytes) || d->tokens_at > d->bytes)
+    return fail(h, HS_ERR_INVALID, "the step's description does not fit its block");
+  cudaStream_t stream = (cudaStream_t)stream_;
+  DeviceGuard guard(h->device);
+  Serial serial(h, stream);
+  HS_CUDA(h, serial.status);
+
+  // What a small step brings along goes into the launches themselves: 64 rows' parameters (3 KB)
+  // and 256 (slot, token) pairs (2 KB) are cheaper there than one copy ahead of the kernel
+  // (about 3 us of host and GPU time); anything larger is copied in one piece.
+  const auto* params = reinterpret_cast<const hs_row_params*>(h->h_block);
+  const bool counting = d->n_resets > 0 || d->n_appends > 0;
+  const bool singles = d->n_resets == 0 && d->n_appends > 0 && d->max_tokens == 1 && !d->repeats;
+  const bool rows_inline = batch <= hs::kInlineRows;
+  const bool appends_inline = singles && d->n_appends <= hs::kInlineAppends;
+  if (!rows_inline || (counting && !appends_inline)) {
+    const size_t bytes = counting && !appends_inline ? d->bytes : (size_t)batch * sizeof(hs_row_params);
+    if (bytes > h->d_block_bytes) {
+      HS_CUDA(h, cudaStreamSynchronize(stream));
+      cudaFree(h->d_block);
+      h->d_block = nullptr;
+      h->d_block_bytes = 0;
+      const size_t want = std::max<size_t>(bytes + bytes / 2, 64 << 10);
+      HS_CUDA(h, cudaMalloc(&h->d_block, want));
+      h->d_block_bytes = want;
+    }
+    HS_CUDA(h, cudaMemcpyAsync(h->d_block, h->h_block, bytes, cudaMemcpyHostToDevice, stream));
+  }
+  bool behind = false;
+  const auto* h_slots = reinterpret_cast<const int32_t*>(h->h_block + d->slots_at);
+  const auto* h_offsets = reinterpret_cast<const int32_t*>(h->h_block + d->offsets_at);
+  const auto* h_tokens = reinterpret_cast<const int32_t*>(h->h_block + d->tokens_at);
+  const auto* d_slots = reinterpret_cast<const int32_t*>(h->d_block + d->slots_at);
+  const auto* d_offsets = reinterpret_cast<const int32_t*>(h->d_block + d->offsets_at);
+  const auto* d_tokens = reinterpret_cast<const int32_t*>(h->d_block + d->tokens_at);
+  if (appends_inline) {
+    hs::InlineAppends in;
+    in.n = d->n_appends;
+    for (int i = 0; i < d->n_appends; ++i) { in.slot[i] = h_slots[i]; in.token[i] = h_tokens[h_offsets[i]]; }
+    hs::slots_append_inline_kernel<<<(d->n_appends + 31) / 32, 32, 0, stream>>>(h->pool, in, vocab);
+    HS_CUDA(h, cudaGetLastError());
+    h->launches += 1;
+    behind = true;
+  } else if (singles) {
+    hs::slots_append_single_kernel<<<(d->n_appends + 31) / 32, 32, 0, stream>>>(h->pool, d_tokens, d_offsets, d_slots,
+                                                                               d->n_appends, vocab);
+    HS_CUDA(h, cudaGetLastError());
+    h->launches += 1;
+    behind = true;
+  } else {
+    if (d->n_resets) {
+      hs::slots_reset_kernel<<<d->n_resets, 256, 0, stream>>>(
+          h->pool, reinterpret_cast<const int32_t*>(h->d_block + d->resets_at), d->n_resets);
+      HS_CUDA(h, cudaGetLastError());
+      h->launches += 1;
+    }
+    rc = launch_append(h, d_tokens, d_offsets, d_slots, d->n_appends, vocab, d->max_tokens, stream);
+    if (rc != HS_OK) return rc;
+  }
+  hs::InlineRows inl;
+  if (rows_inline) std::memcpy(inl.p, params, (size_t)batch * sizeof(hs_row_params));
+  // bf16 rows' records go straight to pinned memory (one burst per row, see write_record); the
+  // general kernel's CTAs put a row's record together in device memory
+  const bool direct = dtype == HS_DTYPE_BF16 && !h->force_general;
+  rc = launch_rows(h, logits, dtype, row_stride, batch, vocab,
+                   rows_inline ? nullptr : reinterpret_cast<const hs_row_params*>(h->d_block), rows_inline ? inl : kNoInlineRows,
+                   direct ? h->h_out : h->d_out, nullptr, nullptr, nullptr, 0u, behind, stream);
+  if (rc != HS_OK) return rc;
+  if (!direct)
+    HS_CUDA(h, cudaMemcpyAsync(h->h_out, h->d_out, (size_t)batch * sizeof(hs_row_out), cudaMemcpyDeviceToHost, stream));
+  HS_CUDA(h, cudaStreamSynchronize(stream));
+  h->have_last = false;  // everything enqueued so far has been waited for
+  return HS_OK;
+}
+
+int hs_step_greedy(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
+                   const int32_t** tokens, void* stream_) {
+  int rc = check_common(h, logits, dtype, batch, vocab);
+  if (rc != HS_OK) return rc;
+  if (!tokens) return fail(h, HS_ERR_INVALID, "tokens is null");
+  *tokens = h->h_tokens;
+  if (batch == 0) return HS_OK;
+  if (row_stride < vocab) return fail(h, HS_ERR_INVALID, "row_stride smaller than vocab");
+  cudaStream_t stream = (cudaStream_t)stream_;
+  DeviceGuard guard(h->device);
+  Serial serial(h, stream);
+  HS_CUDA(h, serial.status);
+  rc = launch_greedy(h, logits, dtype, row_stride, batch, vocab, h->h_tokens, stream);
+  if (rc != HS_OK) return rc;
+  HS_CUDA(h, cudaStreamSynchronize(stream));
+  h->have_last = false;
   return HS_OK;
 }
 

@@ -37,7 +37,8 @@ __device__ __noinline__ void count_chunk_slow(uint32_t* tab, int* rare_n, int2* 
 // this CTA counts the whole row.  part >= 0: the row's tokens are counted by args.csplit CTAs,
 // each a contiguous range; every part leaves its count table and rare list in global scratch,
 // and the part that arrives last (a ticket) adds the others' to its own and goes on alone.
-__device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* smem_raw, int row_index, int part) {
+__device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* smem_raw, const hs_row_params& P,
+                                          hs_row_out* out, int row_index, int part) {
   const RowKernelArgs& a = args.base;
   const LayoutV3 lay = layout_v3();
   Ctx3 c;
@@ -60,8 +61,6 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
   c.vocab = a.vocab;
   c.logits = reinterpret_cast<const unsigned short*>(a.logits) + (long long)c.row * a.row_stride;
   c.vec = (reinterpret_cast<uintptr_t>(c.logits) & 15u) == 0;
-  const hs_row_params P = a.params[c.row];
-  hs_row_out* out = a.out + c.row;
   c.greedy = P.temperature == 0.0f;
   c.T = P.temperature;
   c.rp = P.repetition_penalty;
@@ -108,7 +107,7 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
       float* dst = a.scores_out + (size_t)c.row * a.vocab;
       for (int id = tid; id < c.vocab; id += kThreads) dst[id] = canonical(__uint_as_float((uint32_t)c.logits[id] << 16));
     }
-    if (tid == 0) {
+    if (tid == 0) {  // (`out` is this CTA's record in shared memory)
       out->token = (int)(~(uint32_t)(best & 0xffffffffu));
       if (a.tokens_out) a.tokens_out[c.row] = out->token;
       out->logprob = 0.f; out->n_top = 0; out->status = status;
@@ -116,6 +115,8 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
       out->cut_bits = 0xff800000u; out->n_cut_ties = -1;
       out->row_max = score_of((uint32_t)(best >> 32)); out->log_z = 0.f;
     }
+    __syncthreads();
+    if (tid < 32) write_record(a.out + c.row, *out, false);
     return;
   }
 
@@ -332,6 +333,8 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
   const int scratch = small[15];
   if (scratch < 0) {  // cannot happen while n_scratch covers the resident CTAs; fail the row, do not wait
     if (tid == 0) { out->token = 0; out->status = 128; out->n_top = 0; out->n_kept = 0; }
+    __syncthreads();
+    if (tid < 32) write_record(a.out + c.row, *out, false);
     return;
   }
   auto release_scratch = [&]() {
@@ -863,7 +866,8 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
     }
   }
   (void)cut_group_cnt;
-  release_scratch();
+  release_scratch();  // (a barrier first: the record is complete)
+  if (tid < 32) write_record(a.out + c.row, *out, P.n_logprobs >= 0);
   mark(9);
 }
 
@@ -876,7 +880,8 @@ __device__ __forceinline__ bool is_candidate_row(const hs_row_params& P, int voc
 // One part of a candidate row (a contiguous range of its tokens).  The CTA that brings in the
 // row's last part finishes the row.  Returns true when the row's candidate list overflowed
 // and the caller (the finishing CTA) has to count the row after all.
-__device__ __forceinline__ bool cand_part(const RowV3Args& args, unsigned char* smem_raw, int row_index, int part) {
+__device__ __forceinline__ bool cand_part(const RowV3Args& args, unsigned char* smem_raw, const hs_row_params& P,
+                                          hs_row_out* out, int row_index, int part) {
   const RowKernelArgs& a = args.base;
   const LayoutCand lay = layout_cand();
   Ctx3 c;
@@ -887,7 +892,6 @@ __device__ __forceinline__ bool cand_part(const RowV3Args& args, unsigned char* 
   const int tid = threadIdx.x;
   c.row = row_index;
   c.vocab = a.vocab;
-  const hs_row_params P = a.params[c.row];
   c.greedy = false;
   // the row is streamed by args.split CTAs, each taking a contiguous range of tokens
   const int split = args.split;
@@ -896,7 +900,6 @@ __device__ __forceinline__ bool cand_part(const RowV3Args& args, unsigned char* 
   c.hi = min(c.lo + width, a.vocab);
   c.logits = reinterpret_cast<const unsigned short*>(a.logits) + (long long)c.row * a.row_stride;
   c.vec = (reinterpret_cast<uintptr_t>(c.logits) & 15u) == 0;
-  hs_row_out* out = a.out + c.row;
   c.T = P.temperature; c.rp = P.repetition_penalty; c.pp = P.presence_penalty; c.fp = P.frequency_penalty;
   c.pool = a.pool;
   c.slot = P.slot;
@@ -989,6 +992,8 @@ __device__ __forceinline__ bool cand_part(const RowV3Args& args, unsigned char* 
       if (!slot_append_one(a.pool, P.slot, r.token)) out->status = r.status | 2;
     }
   }
+  __syncthreads();
+  if (tid < 32) write_record(a.out + c.row, *out, P.n_logprobs >= 0);
   mark(8);
   return false;
 }
@@ -1003,15 +1008,23 @@ __host__ __device__ inline size_t bf16_kernel_smem() {
 // order, long ones first: batch * csplit items = part p of row r on the counting path (a CTA
 // whose row is not a counting row leaves at once), then batch * split items = part p of row r
 // on the candidate path (likewise).  No CTA waits for another.
-__global__ void __launch_bounds__(kThreads, 2) row_kernel_bf16(const RowV3Args args) {
+__global__ void __launch_bounds__(kThreads, 2) row_kernel_bf16(const __grid_constant__ RowV3Args args,
+                                                               const __grid_constant__ InlineRows inl) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ hs_row_out record;
   const int item = blockIdx.x;
   const int n_count = args.batch * args.csplit;
   bool count = item < n_count;
   // counting items are laid out part-major, so that the parts of one row start on different SMs
   int row = count ? item % args.batch : (item - n_count) / args.split;
   int part = count ? item / args.batch : (item - n_count) % args.split;
-  if (is_candidate_row(args.base.params[row], args.base.vocab) == count) return;  // the other path's row
+  __shared__ hs_row_params P;  // (shared: its twelve words would be spilled)
+  if (threadIdx.x == 0) P = row_params(args.base, inl, row);
+  __syncthreads();
+  if (is_candidate_row(P, args.base.vocab) == count) return;  // the other path's row
+  cudaGridDependencySynchronize();  // (the histograms are up to date from here on)
+  if (threadIdx.x < sizeof(hs_row_out) / 4) reinterpret_cast<uint32_t*>(&record)[threadIdx.x] = 0u;
+  __syncthreads();
   // (tuning aid: when each item started and ended, in ns of the global timer, slots 48.. of its row)
   unsigned long long* when = nullptr;
   if (args.phase_clocks && threadIdx.x == 0) {
@@ -1019,7 +1032,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel_bf16(const RowV3Args a
     when[0] = global_timer_ns();
   }
   if (!count) {
-    if (!cand_part(args, smem_raw, row, part)) {
+    if (!cand_part(args, smem_raw, P, &record, row, part)) {
       if (when) when[1] = global_timer_ns();
       return;
     }
@@ -1028,7 +1041,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel_bf16(const RowV3Args a
   } else if (args.csplit == 1) {
     part = -1;
   }
-  count_row(args, smem_raw, row, part);
+  count_row(args, smem_raw, P, &record, row, part);
   if (when) when[1] = global_timer_ns();
 }
 

@@ -61,11 +61,16 @@ struct F32TopkArgs {
   unsigned long long* phase_clocks;
 };
 
-__global__ void __launch_bounds__(kThreads, 2) row_kernel_f32_topk(const F32TopkArgs args) {
+__global__ void __launch_bounds__(kThreads, 2) row_kernel_f32_topk(const __grid_constant__ F32TopkArgs args,
+                                                                   const __grid_constant__ InlineRows inl) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const RowKernelArgs& a = args.base;
   const int row = blockIdx.x;
-  const hs_row_params P = a.params[row];
+  __shared__ hs_row_params P;
+  if (threadIdx.x == 0) P = row_params(a, inl, row);
+  __syncthreads();
+  // (before anything returns: the general kernel behind this one counts on the histograms too)
+  cudaGridDependencySynchronize();
   if (!is_candidate_row(P, a.vocab)) return;  // the general kernel's row
   const LayoutCand lay = layout_cand();
   Ctx3 c;

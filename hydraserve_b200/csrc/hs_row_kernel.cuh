@@ -45,6 +45,25 @@ struct RowKernelArgs {
   int token_draw;       // bf16 counting rows draw near-flat rows by rejection on tokens (tuning / test switch)
 };
 
+// Parameters of a small batch travel in the launch itself (args.params is null then): no copy to
+// wait for ahead of the kernel.
+constexpr int kInlineRows = 64;
+struct InlineRows {
+  hs_row_params p[kInlineRows];
+};
+__device__ __forceinline__ hs_row_params row_params(const RowKernelArgs& a, const InlineRows& inl, int row) {
+  return a.params ? a.params[row] : inl.p[row];
+}
+
+// A row's record is put together in shared memory and leaves in one piece: `out` may be pinned
+// host memory, where every store is a transfer of its own.
+__device__ __forceinline__ void write_record(hs_row_out* out, const hs_row_out& rec, bool with_top) {
+  static_assert(sizeof(hs_row_out) == 52 * 4 && offsetof(hs_row_out, top_ids) == 12 * 4, "words of a record");
+  const int n = with_top ? 52 : 12;
+  for (int i = threadIdx.x; i < n; i += 32)
+    reinterpret_cast<uint32_t*>(out)[i] = reinterpret_cast<const uint32_t*>(&rec)[i];
+}
+
 struct RowCtx : ClusterCtx {
   int row;
   int vocab;
@@ -308,14 +327,16 @@ __device__ void write_top_logprobs(RowCtx& c, const KeptSet& kept, uint32_t key_
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 1) row_kernel(const RowKernelArgs a) {
+__global__ void __launch_bounds__(kThreads, 1) row_kernel(const __grid_constant__ RowKernelArgs a,
+                                                          const __grid_constant__ InlineRows inl) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  const hs_row_params P = row_params(a, inl, blockIdx.y);
   if (a.skip_candidate_rows) {
     // fp32 rows with a small top_k are sampled by the candidate kernel launched next to this
     // one (every CTA of the row's cluster sees the same parameters and leaves together)
-    const hs_row_params& p = a.params[blockIdx.y];
-    if (p.temperature != 0.0f && p.top_k > 0 && p.top_k <= kCandidateTopKMax && p.top_k < a.vocab) return;
+    if (P.temperature != 0.0f && P.top_k > 0 && P.top_k <= kCandidateTopKMax && P.top_k < a.vocab) return;
   }
+  cudaGridDependencySynchronize();  // (the histograms are up to date from here on)
   RowCtx c{{cg::this_cluster()}};
   c.rank = c.cluster.block_rank();
   c.nranks = c.cluster.num_blocks();
@@ -343,7 +364,6 @@ __global__ void __launch_bounds__(kThreads, 1) row_kernel(const RowKernelArgs a)
   if (threadIdx.x == 0) c.x->ring_phase = 0;
 
   const int tid = threadIdx.x;
-  const hs_row_params P = a.params[c.row];
   hs_row_out* out = a.out + c.row;
   const bool greedy = P.temperature == 0.0f;
 

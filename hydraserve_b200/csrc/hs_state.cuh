@@ -164,66 +164,155 @@ __device__ __forceinline__ bool slot_append_one(const Pool& p, int s, int token)
   return true;
 }
 
-// ---- plain greedy: arg max per row, lowest id on ties (reference sampling.py:69-73) ---
-constexpr int kGreedyThreads = 512;
+// One new token per listed slot (the common step of a decode loop: every request has gained the
+// token sampled last), each by one thread: no slot is listed twice, so nothing is contended and
+// the three passes above are one.  Up to kInlineAppends pairs travel in the launch's own
+// parameters; without inline pairs they come from device memory as hs_slots_append takes them.
+constexpr int kInlineAppends = 256;
+struct InlineAppends {
+  int n;
+  int slot[kInlineAppends];
+  int token[kInlineAppends];
+};
+__device__ __forceinline__ void append_single(const Pool& p, int s, int t, int vocab) {
+  if (s < 0 || s >= p.slots_total || t < 0 || t >= vocab || t >= p.pos_stride) return;
+  if (!slot_append_one(p, s, t)) *p.error = 1;
+}
+__global__ void slots_append_inline_kernel(const Pool p, const __grid_constant__ InlineAppends in, int vocab) {
+  // (the sampling kernel behind this one may get its CTAs ready meanwhile; it waits for this
+  // grid's end before it looks at a histogram)
+  cudaTriggerProgrammaticLaunchCompletion();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < in.n) append_single(p, in.slot[i], in.token[i], vocab);
+}
+__global__ void slots_append_single_kernel(const Pool p, const int32_t* tokens, const int32_t* offsets,
+                                           const int32_t* slots, int n_slots, int vocab) {
+  cudaTriggerProgrammaticLaunchCompletion();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n_slots && offsets[i + 1] > offsets[i]) append_single(p, slots[i], tokens[offsets[i]], vocab);
+}
 
-// Each CTA scans one chunk of one row and leaves (key << 32 | ~id) of its best element.
+// ---- plain greedy: arg max per row, lowest id on ties (reference sampling.py:69-73) ---
+// Bound by HBM once the row chunks of a call fill the SMs, by latency below that.  A CTA takes
+// one chunk of one row.  Values are compared as integers in their order (two bf16 values per
+// 32-bit word: sign-magnitude to two's complement, which gives -0.0 and +0.0 one value; NaNs of
+// positive sign come out on top, as the fp32 key order has them); a thread keeps its best value
+// and the first 16 bytes it saw it in, and only the chunk's winner looks into those again.
+constexpr int kGreedyThreads = 256;
+constexpr int kGreedyUnroll = 8;  // 128-bit loads in flight per thread
+
+__device__ __forceinline__ int greedy_image_f32(float f) {
+  const uint32_t u = __float_as_uint(f);
+  const int mag = (int)(u & 0x7fffffffu);
+  return (int)u < 0 ? -mag : mag;
+}
+__device__ __forceinline__ int greedy_image_bf16(uint32_t raw) {
+  const int mag = (int)(raw & 0x7fffu);
+  return (raw & 0x8000u) ? -mag : mag;
+}
+// Highest of the eight values of a 16-byte chunk, as an integer image.
+__device__ __forceinline__ int greedy_chunk_bf16(const uint4& w) {
+  uint32_t best = 0x80018001u;  // below every image
+  const uint32_t words[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    uint32_t mask;
+    asm("prmt.b32 %0, %1, 0, 0xBB99;" : "=r"(mask) : "r"(words[k]));  // 0xffff per negative half
+    best = __viaddmax_s16x2((words[k] & 0x7fff7fffu) ^ mask, mask & 0x00010001u, best);
+  }
+  return max((int)(short)(best & 0xffffu), (int)best >> 16);
+}
+__device__ __forceinline__ int greedy_chunk_f32(const uint4& w) {
+  return max(max(greedy_image_f32(__uint_as_float(w.x)), greedy_image_f32(__uint_as_float(w.y))),
+             max(greedy_image_f32(__uint_as_float(w.z)), greedy_image_f32(__uint_as_float(w.w))));
+}
+
+// Best element of tokens [begin, begin + n) of a row, as (order-preserving value, ~id); valid in
+// thread 0.
+template <bool BF16>
+__device__ u64 greedy_chunk_best(const void* logits, long long row_offset, int begin, int n) {
+  __shared__ u64 warp_best[kGreedyThreads / 32];
+  constexpr int kPer = BF16 ? 8 : 4;  // values per 16 bytes
+  const int tid = threadIdx.x;
+  const unsigned char* base = reinterpret_cast<const unsigned char*>(logits) + (row_offset + begin) * (BF16 ? 2 : 4);
+  const bool vec = (reinterpret_cast<uintptr_t>(base) & 15u) == 0;
+  const int n16 = vec ? n / kPer : 0;
+  const uint4* src = reinterpret_cast<const uint4*>(base);
+  auto image = [&](int i) {
+    return BF16 ? greedy_image_bf16(reinterpret_cast<const unsigned short*>(base)[i])
+                : greedy_image_f32(reinterpret_cast<const float*>(base)[i]);
+  };
+  constexpr int kNone = (int)0x80000000;  // below every image (an fp32 image is at least -0x7fffffff)
+  int best = kNone, at = 0;
+  int i = tid;
+  for (; i + (kGreedyUnroll - 1) * kGreedyThreads < n16; i += kGreedyUnroll * kGreedyThreads) {
+    uint4 w[kGreedyUnroll];
+#pragma unroll
+    for (int u = 0; u < kGreedyUnroll; ++u) w[u] = __ldcs(src + i + u * kGreedyThreads);
+#pragma unroll
+    for (int u = 0; u < kGreedyUnroll; ++u) {
+      const int v = BF16 ? greedy_chunk_bf16(w[u]) : greedy_chunk_f32(w[u]);
+      if (v > best) { best = v; at = i + u * kGreedyThreads; }
+    }
+  }
+  if (i < n16) {
+    uint4 w[kGreedyUnroll];
+#pragma unroll
+    for (int u = 0; u < kGreedyUnroll - 1; ++u)
+      if (i + u * kGreedyThreads < n16) w[u] = __ldcs(src + i + u * kGreedyThreads);
+#pragma unroll
+    for (int u = 0; u < kGreedyUnroll - 1; ++u) {
+      if (i + u * kGreedyThreads >= n16) break;
+      const int v = BF16 ? greedy_chunk_bf16(w[u]) : greedy_chunk_f32(w[u]);
+      if (v > best) { best = v; at = i + u * kGreedyThreads; }
+    }
+  }
+  // (value, ~first element of the chunk of 16 bytes it was seen in)
+  u64 mine = best == kNone ? 0ull : ((u64)((uint32_t)best ^ 0x80000000u) << 32) | (uint32_t)(~(uint32_t)(at * kPer));
+  for (int k = n16 * kPer + tid; k < n; k += kGreedyThreads) {
+    const u64 e = ((u64)((uint32_t)image(k) ^ 0x80000000u) << 32) | (uint32_t)(~(uint32_t)k);
+    mine = e > mine ? e : mine;
+  }
+  mine = warp_max_u64(mine);
+  if ((tid & 31) == 0) warp_best[tid >> 5] = mine;
+  __syncthreads();
+  if (tid != 0) return 0;
+#pragma unroll
+  for (int k = 1; k < kGreedyThreads / 32; ++k) mine = warp_best[k] > mine ? warp_best[k] : mine;
+  int id = (int)(~(uint32_t)mine);
+  const int value = (int)((uint32_t)(mine >> 32) ^ 0x80000000u);
+  if (id < n16 * kPer)
+    while (image(id) != value) ++id;  // (one of the chunk's eight or four)
+  return (mine & 0xffffffff00000000ull) | (uint32_t)(~(uint32_t)(begin + id));
+}
+
+// The row's best over its chunks meets in best[row] (0 between calls); the CTA that draws the
+// row's last ticket writes the id and puts both back to 0.
+__global__ void __launch_bounds__(kGreedyThreads) greedy_kernel(
+    const void* logits, int dtype, long long row_stride, int vocab, int chunk, u64* best, int* ticket, int32_t* tokens_out) {
+  const int row = blockIdx.y, begin = blockIdx.x * chunk, n = max(0, min(chunk, vocab - begin));
+  const u64 mine = dtype == HS_DTYPE_BF16 ? greedy_chunk_best<true>(logits, row * row_stride, begin, n)
+                                          : greedy_chunk_best<false>(logits, row * row_stride, begin, n);
+  if (threadIdx.x != 0) return;
+  u64 top = mine;
+  if (gridDim.x > 1) {
+    atomicMax(&best[row], mine);
+    __threadfence();
+    if (atomicAdd(&ticket[row], 1) != (int)gridDim.x - 1) return;
+    __threadfence();
+    top = atomicExch(&best[row], 0ull);
+    ticket[row] = 0;
+  }
+  tokens_out[row] = (int32_t)(~(uint32_t)(top & 0xffffffffu));
+}
+
+// The same in two launches, with nothing that has to hold a value between calls.
 __global__ void __launch_bounds__(kGreedyThreads) greedy_partial_kernel(
     const void* logits, int dtype, long long row_stride, int vocab, int chunk, u64* partials) {
-  __shared__ u64 warp_best[kGreedyThreads / 32];
-  const int row = blockIdx.y;
-  const int begin = blockIdx.x * chunk;
-  const int n = max(0, min(chunk, vocab - begin));
-  const int tid = threadIdx.x;
-  u64 best = 0;
-  auto consider = [&](float f, int gid) {
-    const u64 packed = ((u64)key_of(canonical(f)) << 32) | (uint32_t)(~(uint32_t)gid);
-    best = packed > best ? packed : best;
-  };
-  const long long gofs = (long long)row * row_stride + begin;
-  if (dtype == HS_DTYPE_BF16) {
-    const unsigned short* src = reinterpret_cast<const unsigned short*>(logits) + gofs;
-    const bool vec = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
-    const int nvec = vec ? n / 8 : 0;
-    const uint4* src4 = reinterpret_cast<const uint4*>(src);
-    for (int i = tid; i < nvec; i += kGreedyThreads) {
-      const uint4 w = __ldcs(src4 + i);
-      const int g = begin + 8 * i;
-      consider(__uint_as_float(w.x << 16), g + 0); consider(__uint_as_float(w.x & 0xffff0000u), g + 1);
-      consider(__uint_as_float(w.y << 16), g + 2); consider(__uint_as_float(w.y & 0xffff0000u), g + 3);
-      consider(__uint_as_float(w.z << 16), g + 4); consider(__uint_as_float(w.z & 0xffff0000u), g + 5);
-      consider(__uint_as_float(w.w << 16), g + 6); consider(__uint_as_float(w.w & 0xffff0000u), g + 7);
-    }
-    for (int i = nvec * 8 + tid; i < n; i += kGreedyThreads)
-      consider(__uint_as_float((uint32_t)src[i] << 16), begin + i);
-  } else {
-    const float* src = reinterpret_cast<const float*>(logits) + gofs;
-    const bool vec = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
-    const int nvec = vec ? n / 4 : 0;
-    const float4* src4 = reinterpret_cast<const float4*>(src);
-    for (int i = tid; i < nvec; i += kGreedyThreads) {
-      const float4 w = __ldcs(src4 + i);
-      const int g = begin + 4 * i;
-      consider(w.x, g); consider(w.y, g + 1); consider(w.z, g + 2); consider(w.w, g + 3);
-    }
-    for (int i = nvec * 4 + tid; i < n; i += kGreedyThreads) consider(src[i], begin + i);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const u64 t = __shfl_xor_sync(0xffffffffu, best, o);
-    best = t > best ? t : best;
-  }
-  if ((tid & 31) == 0) warp_best[tid >> 5] = best;
-  __syncthreads();
-  if (tid < 32) {
-    best = tid < kGreedyThreads / 32 ? warp_best[tid] : 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const u64 t = __shfl_xor_sync(0xffffffffu, best, o);
-      best = t > best ? t : best;
-    }
-    if (tid == 0) partials[(size_t)row * gridDim.x + blockIdx.x] = best;
-  }
+  const int row = blockIdx.y, begin = blockIdx.x * chunk, n = max(0, min(chunk, vocab - begin));
+  const u64 mine = dtype == HS_DTYPE_BF16 ? greedy_chunk_best<true>(logits, row * row_stride, begin, n)
+                                          : greedy_chunk_best<false>(logits, row * row_stride, begin, n);
+  if (threadIdx.x == 0) partials[(size_t)row * gridDim.x + blockIdx.x] = mine;
 }
 
 __global__ void greedy_final_kernel(const u64* partials, int chunks, int batch, int32_t* tokens_out) {

@@ -14,19 +14,16 @@ and the process-wide sampler of a GPU is never destroyed while a call is inside 
 from __future__ import annotations
 
 import ctypes as C
-import itertools
 import os
 import threading
-from collections import OrderedDict
 
 import numpy as np
 
 from .. import _lib
-from .sampling import SamplingParams, TokenSample, _has_penalties, _is_plain_greedy, _token_only
+from .sampling import SamplingParams, TokenSample, _has_penalties, _is_plain_greedy  # noqa: F401
 
 SEED_STRIDE = 0x1E3779B97F4A7C15  # reference sampling.py:148
 _NEG_INF = float("-inf")
-_MASK63 = np.uint64(2**63 - 1)
 
 # status bits of hs_row_out.status (include/hs_sampler.h)
 STATUS_FELL_BACK, STATUS_APPEND_FAILED, STATUS_NEEDS_GENERAL = 1, 2, 4
@@ -39,40 +36,6 @@ def mixed_seed(seed: int, step: int) -> int:
     return (int(seed) + (int(step) + 1) * SEED_STRIDE) % (2**63)
 
 
-def _static_row(p: SamplingParams) -> bytes:
-    """The 48 bytes of hs_row_params that depend on the SamplingParams alone (seed and slot
-    are filled in per call)."""
-    rec = np.zeros(1, dtype=_lib.ROW_PARAMS)
-    rec["temperature"] = p.temperature
-    rec["top_p"] = p.top_p
-    rec["min_p"] = p.min_p
-    rec["repetition_penalty"] = p.repetition_penalty
-    rec["presence_penalty"] = p.presence_penalty
-    rec["frequency_penalty"] = p.frequency_penalty
-    rec["top_k"] = min(int(p.top_k), 2**31 - 1)
-    rec["n_logprobs"] = -1 if p.logprobs is None else int(p.logprobs)
-    rec["flags"] = _lib.HS_ROW_PLAIN_GREEDY if _is_plain_greedy(p) else 0
-    rec["slot"] = -1
-    return rec.tobytes()
-
-
-_static_rows: dict = {}  # id(params) -> (params, packed bytes); the object is kept so the id stays its own
-_STATIC_ROWS_MAX = 8192
-_static_batches: dict = {}  # ids of a batch's params -> (the params, packed static part, any unseeded, seeds)
-_STATIC_BATCHES_MAX = 64
-
-
-def _static_row_cached(p: SamplingParams) -> bytes:
-    hit = _static_rows.get(id(p))
-    if hit is not None and hit[0] is p:
-        return hit[1]
-    row = _static_row(p)
-    if len(_static_rows) >= _STATIC_ROWS_MAX:
-        _static_rows.clear()
-    _static_rows[id(p)] = (p, row)
-    return row
-
-
 def draw_unseeded_keys(params):
     """Stream keys for the rows that sample without a seed.  The reference falls back to
     torch's global generator there (sampling.py:145); the keys come from the same place."""
@@ -82,25 +45,30 @@ def draw_unseeded_keys(params):
             if (p.seed is None and p.temperature != 0.0) else None for p in params]
 
 
-def batch_static(params):
-    """What depends on a batch's SamplingParams alone: (the params, packed static part, any
-    unseeded row, seeds, which rows have penalties).  A serving loop passes the same objects
-    step after step, so this is kept per batch (the entry holds the objects: their ids stay
-    theirs while it lives)."""
-    n = len(params)
-    key = tuple(map(id, params))
-    hit = _static_batches.get(key)
-    if hit is None:
-        static = np.frombuffer(b"".join(_static_row_cached(p) for p in params), dtype=_lib.ROW_PARAMS).copy() \
-            if n else np.zeros(0, dtype=_lib.ROW_PARAMS)
-        unseeded = any(p.seed is None and p.temperature != 0.0 for p in params)
-        fixed_seeds = None if unseeded else np.fromiter((p.seed if p.seed is not None else 0 for p in params),
-                                                        dtype=np.uint64, count=n)
-        if len(_static_batches) >= _STATIC_BATCHES_MAX:
-            _static_batches.clear()
-        hit = _static_batches[key] = (tuple(params), static, unseeded, fixed_seeds,
-                                      tuple(_has_penalties(p) for p in params))
-    return hit
+def _as_int64(tokens) -> np.ndarray:
+    """Any sequence of token ids as a flat int64 array (what the native planner asks for when a
+    history is not a plain list or tuple of ints)."""
+    if isinstance(tokens, (np.ndarray, list, tuple)) or not hasattr(tokens, "__iter__"):
+        return np.ascontiguousarray(np.asarray(tokens, dtype=np.int64).reshape(-1))
+    return np.fromiter(tokens, dtype=np.int64)
+
+
+_host = _lib.load_host()
+_host.bind(TokenSample, _as_int64, draw_unseeded_keys)
+
+# What depends on a batch's SamplingParams alone: (the params, packed static part, any unseeded
+# row, seeds, which rows have penalties).  A serving loop passes the same objects step after
+# step, so this is kept per batch (the entry holds the objects: their ids stay theirs while it
+# lives).
+batch_static = _host.batch
+
+# Whether HYDRASERVE_BATCHED_GREEDY (reference sampling.py:69) is anything but "0" right now.
+batched_greedy = _host.batched_greedy
+
+# Which request holds which resident histogram slot, and how much of its history the device has
+# already counted: release(request) and lookup(request, requests of the batch) -> (entry, is
+# new); least recently used requests are evicted first, never one that belongs to the batch.
+SlotBook = _host.SlotBook
 
 
 def pack_params(params, steps, slots=None, unseeded_keys=None) -> np.ndarray:
@@ -108,24 +76,7 @@ def pack_params(params, steps, slots=None, unseeded_keys=None) -> np.ndarray:
 
     unseeded_keys: per row, the stream key of a row whose ``seed`` is None (or None); drawn
     from torch's global generator when not given."""
-    n = len(params)
-    hit = batch_static(params)
-    _, static, unseeded, fixed_seeds, _ = hit
-    rec = static.copy()
-    if unseeded:
-        if unseeded_keys is None:
-            unseeded_keys = draw_unseeded_keys(params)
-        seeds = np.fromiter(
-            ((p.seed if p.seed is not None else ((unseeded_keys[i] if unseeded_keys else None) or 0))
-             for i, p in enumerate(params)), dtype=np.uint64, count=n)
-    else:
-        seeds = fixed_seeds
-    step_arr = (np.asarray(steps, dtype=np.int64) + 1).astype(np.uint64)
-    with np.errstate(over="ignore"):
-        rec["seed"] = (seeds + step_arr * np.uint64(SEED_STRIDE)) & _MASK63  # == mixed_seed, vectorised
-    if slots is not None:
-        rec["slot"] = np.asarray(slots, dtype=np.int32)
-    return rec
+    return np.frombuffer(_host.pack(params, steps, slots, unseeded_keys), dtype=_lib.ROW_PARAMS)
 
 
 def history_array(history, vocab: int) -> np.ndarray:
@@ -149,41 +100,6 @@ def slot_bytes(vocab_max: int, hist_cap: int = 0) -> int:
     return 12 * cap + 4 * int(vocab_max) + 4 * ((int(vocab_max) + 15) // 16 + 4) + 8
 
 
-class SlotBook:
-    """Which request holds which resident histogram slot, and how much of its history the
-    device has already counted.  Pure host bookkeeping (no GPU): least recently used
-    requests are evicted first, never one that belongs to the batch being packed."""
-
-    def __init__(self, n_slots: int):
-        self.n_slots = int(n_slots)
-        self.entries: OrderedDict = OrderedDict()  # request id -> [slot, tokens counted]
-        self.free = list(range(self.n_slots - 1, -1, -1))
-
-    def release(self, request_id) -> bool:
-        entry = self.entries.pop(request_id, None)
-        if entry is None:
-            return False
-        self.free.append(entry[0])
-        return True
-
-    def lookup(self, request_id, in_batch):
-        """(entry, is_new) for the request, or (None, False) when every slot is held by a
-        request of the current batch (the caller then rebuilds that row's histogram in a
-        per-call slot).  ``in_batch``: the ids of all requests of the call."""
-        entry = self.entries.get(request_id)
-        if entry is not None:
-            self.entries.move_to_end(request_id)
-            return entry, False
-        if not self.free:
-            victim = next((rid for rid in self.entries if rid not in in_batch), None)
-            if victim is None:
-                return None, False
-            self.free.append(self.entries.pop(victim)[0])
-        entry = [self.free.pop(), 0]
-        self.entries[request_id] = entry
-        return entry, True
-
-
 class DeviceSampler:
     """One C-ABI sampler handle on one GPU plus the torch buffers around it."""
 
@@ -196,6 +112,8 @@ class DeviceSampler:
         self.torch = torch
         self.lib = _lib.load()
         self.device = torch.device(device)
+        self.index = self.device.index or 0
+        self._dtypes = {torch.bfloat16: _lib.HS_DTYPE_BF16, torch.float32: _lib.HS_DTYPE_F32}
         self.vocab_max = int(vocab_max)
         self.batch_max = int(batch_max)
         self.resident_slots = int(resident_slots)
@@ -211,6 +129,10 @@ class DeviceSampler:
         self.lock = threading.RLock()
         self._pinned = threading.local()
         self.book = SlotBook(self.resident_slots)
+        address = lambda fn: C.cast(fn, C.c_void_p).value  # noqa: E731
+        self.host = _host.Stepper(handle.value, self.book, self.scratch_base, _lib.SamplerError,
+                                  address(self.lib.hs_step_block), address(self.lib.hs_step),
+                                  address(self.lib.hs_step_greedy), address(self.lib.hs_last_error))
         self.users = 0        # calls inside this sampler (guarded by _samplers_lock)
         self.retired = False  # replaced by a larger one: closed when the last user leaves
 
@@ -227,8 +149,11 @@ class DeviceSampler:
             pass
 
     # -- small helpers -------------------------------------------------------------
+    def _raw_stream(self) -> int:
+        return self.torch._C._cuda_getCurrentRawStream(self.index)
+
     def _stream(self):
-        return C.c_void_p(self.torch.cuda.current_stream(self.device).cuda_stream)
+        return C.c_void_p(self._raw_stream())
 
     def _to_device(self, array: np.ndarray):
         """Host array -> device tensor through this thread's pinned arena (no cudaHostAlloc per
@@ -278,16 +203,17 @@ class DeviceSampler:
         _lib.check(self.lib, self.handle, self.lib.hs_debug_set(self.handle, 3, 1 if on else 0), "hs_debug_set")
 
     def prepare_logits(self, logits):
-        torch = self.torch
-        if logits.device != self.device:
+        if logits.get_device() != self.index:
             logits = logits.to(self.device, non_blocking=True)
-        if logits.dtype not in (torch.bfloat16, torch.float32):
-            logits = logits.float()
-        if logits.stride(-1) != 1 or (logits.shape[0] > 1 and logits.stride(0) < logits.shape[1]):
+        code = self._dtypes.get(logits.dtype)
+        if code is None:
+            logits, code = logits.float(), _lib.HS_DTYPE_F32
+        batch, vocab = logits.shape
+        stride, step = logits.stride()
+        if step != 1 or (batch > 1 and stride < vocab):
             logits = logits.contiguous()
-        dtype = _lib.HS_DTYPE_BF16 if logits.dtype == torch.bfloat16 else _lib.HS_DTYPE_F32
-        stride = logits.stride(0) if logits.shape[0] > 1 else logits.shape[1]
-        return logits, dtype, int(stride)
+            stride = vocab
+        return logits, code, stride if batch > 1 else vocab
 
     # -- histograms ----------------------------------------------------------------
     def reset_slots(self, slots) -> None:
@@ -302,15 +228,12 @@ class DeviceSampler:
         Ids outside [0, vocab) are ignored, as in the reference (sampling.py:108)."""
         if len(slots) == 0:
             return
-        lens = [len(a) for a in token_arrays]
+        arrays = [_as_int64(a) for a in token_arrays]
+        lens = [a.size for a in arrays]
         total = sum(lens)
         if total == 0:
             return
-        if all(not isinstance(a, np.ndarray) for a in token_arrays):
-            # short Python sequences (the one token a request gained since its last step): one pass
-            flat = np.fromiter(itertools.chain.from_iterable(token_arrays), dtype=np.int64, count=total)
-        else:
-            flat = np.concatenate([np.asarray(a, dtype=np.int64).reshape(-1) for a in token_arrays])
+        flat = np.concatenate(arrays)
         # the device ignores ids outside [0, vocab); -1 stands for everything that is
         flat = np.where((flat < 0) | (flat >= vocab), -1, flat).astype(np.int32)
         offsets = np.zeros(len(slots) + 1, dtype=np.int32)
@@ -333,25 +256,6 @@ class DeviceSampler:
     def release_request(self, request_id) -> None:
         with self.lock:
             self.book.release(request_id)
-
-    def _slot_for_request(self, request_id, history, vocab, resets, appends, in_batch):
-        """Resident slot of a request, scheduling only the not-yet-counted tail of its
-        history for upload; falls back to a rebuild when the history shrank.  Returns -1
-        when no resident slot can be had (the caller uses a per-call slot)."""
-        entry, is_new = self.book.lookup(request_id, in_batch)
-        if entry is None:
-            return -1
-        n = len(history)
-        if is_new:
-            resets.append(entry[0])
-        elif n < entry[1]:
-            resets.append(entry[0])
-            entry[1] = 0
-        if n > entry[1]:
-            tail = history[entry[1]:] if hasattr(history, "__getitem__") else tuple(history)[entry[1]:]
-            appends.append((entry[0], tail))
-            entry[1] = n
-        return entry[0]
 
     # -- the calls -------------------------------------------------------------------
     def greedy(self, logits):
@@ -400,16 +304,23 @@ class DeviceSampler:
             host.copy_(d_out, non_blocking=True)
             torch.cuda.current_stream(self.device).synchronize()
             records = host.numpy().view(_lib.ROW_OUT).reshape(batch).copy()  # the pinned buffer is reused
-        again = np.nonzero(records["status"] & STATUS_NEEDS_GENERAL)[0]
-        if again.size and not general:
-            idx = torch.from_numpy(again.astype(np.int64)).to(self.device)
-            sub, sub_scores = self.run(
-                logits.index_select(0, idx), rec[again], noise=None if d_noise is None else d_noise.index_select(0, idx),
-                want_scores=want_scores, append_token=append_token, general=True)
-            records[again] = sub
-            if scores is not None:
-                scores[idx] = sub_scores
+        if not general:
+            self._again_general(logits, rec, records, d_noise, scores, append_token)
         return records, scores
+
+    def _again_general(self, logits, rec, records, d_noise=None, scores=None, append_token=False) -> None:
+        """Rows reported with status 4 once more, by the general kernel; ``records`` (and
+        ``scores``) are brought up to date in place."""
+        again = np.nonzero(records["status"] & STATUS_NEEDS_GENERAL)[0]
+        if not again.size:
+            return
+        idx = self.torch.from_numpy(again.astype(np.int64)).to(self.device)
+        sub, sub_scores = self.run(
+            logits.index_select(0, idx), rec[again], noise=None if d_noise is None else d_noise.index_select(0, idx),
+            want_scores=scores is not None, append_token=append_token, general=True)
+        records[again] = sub
+        if scores is not None:
+            scores[idx] = sub_scores
 
     def _pinned_records(self, batch: int):
         """A pinned host buffer for the result records (pinning per call costs more than the copy);
@@ -424,44 +335,43 @@ class DeviceSampler:
     def plan_slots(self, histories, params, vocab: int, request_ids=None):
         """Slot per row plus the histogram resets / appends that bring the device up to date
         (issued here, on the current stream).  Call with the sampler lock held."""
-        batch = len(params)
-        slots = [-1] * batch
-        resets, appends = [], []
-        in_batch = None
-        entries = self.book.entries if request_ids is not None else None
-        for i, penalised in enumerate(batch_static(params)[4]):
-            if not penalised:
-                continue
-            history = histories[i]
-            slot = -1
-            if entries is not None and request_ids[i] is not None:
-                # the common step in line: a known request whose history grew by one token
-                entry = entries.get(request_ids[i])
-                if entry is not None and len(history) == entry[1] + 1 and type(history) in (list, tuple):
-                    entries.move_to_end(request_ids[i])
-                    appends.append((entry[0], history[-1:]))
-                    entry[1] += 1
-                    slots[i] = entry[0]
-                    continue
-                if in_batch is None:
-                    in_batch = {r for r in request_ids if r is not None}
-                slot = self._slot_for_request(request_ids[i], history, vocab, resets, appends, in_batch)
-                if slot >= 0 and len(history) == 0:
-                    # nothing to penalise yet: the row goes without a slot, as it does in a
-                    # stateless call, so that the same kernel path serves it either way (the
-                    # path decides which token a seeded draw lands on); the slot stays the
-                    # request's and is filled from the next step on
-                    continue
-            if slot < 0:
-                if len(history) == 0:
-                    continue
-                slot = self.scratch_base + i
-                resets.append(slot)
-                appends.append((slot, history if isinstance(history, (np.ndarray, list, tuple)) else tuple(history)))
-            slots[i] = slot
+        slots, resets, appends = _host.plan(self.book, self.scratch_base, histories, params, request_ids)
         self.reset_slots(resets)
         self.append_tokens([s for s, _ in appends], [t for _, t in appends], vocab)
         return slots
+
+    def step(self, logits, histories, params, steps, request_ids=None, packed: bool = False):
+        """One step as a serving loop runs it, host to host: the native planner fills one pinned
+        block (parameters, new tokens), the library counts, samples and waits.  Returns a tuple of
+        TokenSample, or (packed) a PackedSamples."""
+        # (a copy of host logits is started first: the bookkeeping runs while they travel)
+        logits, dtype, stride = self.prepare_logits(logits)
+        vocab = logits.shape[1]
+        with self.lock:
+            got = self.host.step(logits.data_ptr(), dtype, stride, vocab, histories, params, steps, request_ids,
+                                 self._raw_stream(), packed)
+            if type(got) is list:  # some row needs more than that
+                records = np.frombuffer(got[0], dtype=_lib.ROW_OUT)
+                self._again_general(logits, np.frombuffer(got[1], dtype=_lib.ROW_PARAMS), records)
+        if type(got) is list:
+            _check_status(records)
+            return PackedSamples(records, _logprob_codes(params), vocab) if packed \
+                else records_to_samples(records, params, vocab)
+        if packed:
+            return PackedSamples(np.frombuffer(got[0], dtype=_lib.ROW_OUT), np.frombuffer(got[1], dtype=np.int8), vocab)
+        return got
+
+    def step_greedy(self, logits, packed: bool = False):
+        """One step of a batch of plain-greedy rows, host to host."""
+        logits, dtype, stride = self.prepare_logits(logits)
+        batch, vocab = logits.shape
+        with self.lock:
+            got = self.host.greedy(logits.data_ptr(), dtype, stride, batch, vocab, self._raw_stream(), packed)
+        if not packed:
+            return got
+        records = np.zeros(batch, _lib.ROW_OUT)
+        records["token"] = np.frombuffer(got, dtype=np.int32)
+        return PackedSamples(records, np.full(batch, -1, np.int8), vocab)
 
     def sample(self, logits, histories, params, steps, request_ids=None, *, noise=None,
                want_scores: bool = False):
@@ -485,6 +395,8 @@ DEFAULT_HIST_CAP = int(os.environ.get("HYDRASERVE_SAMPLER_HIST_CAP", "65536"))
 class _Lease:
     """The process-wide sampler of a GPU for the time of one call."""
 
+    __slots__ = ("sampler",)
+
     def __init__(self, sampler):
         self.sampler = sampler
 
@@ -504,21 +416,24 @@ class _Lease:
 def lease_sampler(device, vocab: int, batch: int, hist_need: int = 0) -> _Lease:
     """The process-wide sampler of a GPU, replaced by a larger one when a call outgrows it.
     The old one is closed only after the last call inside it has returned."""
-    key = str(device)
-    hist_need = min(int(vocab), max(int(hist_need), min(DEFAULT_HIST_CAP, int(vocab))))
+    if isinstance(device, str):
+        device = _cuda_device(device)
+    if hist_need > vocab:
+        hist_need = vocab
     with _samplers_lock:
-        s = _samplers.get(key)
-        if s is None or vocab > s.vocab_max or batch > s.batch_max or hist_need > s.hist_cap:
+        s = _samplers.get(device)
+        if s is None or vocab > s.vocab_max or batch > s.batch_max or \
+                max(hist_need, min(DEFAULT_HIST_CAP, vocab)) > s.hist_cap:
             vocab_max = max(vocab, s.vocab_max if s else 0)
             batch_max = max(batch, s.batch_max if s else 64)
-            hist_cap = min(vocab_max, max(hist_need, s.hist_cap if s else 0))
+            hist_cap = min(vocab_max, max(hist_need, min(DEFAULT_HIST_CAP, vocab), s.hist_cap if s else 0))
             fresh = DeviceSampler(device, vocab_max, batch_max, resident_slots=max(256, batch_max),
                                   hist_cap=hist_cap)
             if s is not None:
                 s.retired = True
                 if s.users == 0:
                     s.close()
-            _samplers[key] = s = fresh
+            _samplers[device] = s = fresh
         s.users += 1
         return _Lease(s)
 
@@ -531,12 +446,12 @@ def sampler_for(device, vocab: int, batch: int, hist_need: int = 0) -> DeviceSam
 
 
 def _target_device(logits):
+    if logits.is_cuda:
+        return logits.device
     import torch
 
     if not torch.cuda.is_available():
         raise RuntimeError("hydraserve_b200 needs a CUDA GPU: there is no CPU sampling path")
-    if logits.is_cuda:
-        return logits.device
     return torch.device("cuda", torch.cuda.current_device())
 
 
@@ -559,12 +474,7 @@ def record_to_sample(rec, logprobs, vocab: int) -> TokenSample:
 
 
 def records_to_samples(records, params, vocab: int):
-    tokens = records["token"].tolist()
-    out = list(map(_token_only, tokens))
-    for i, p in enumerate(params):
-        if p.logprobs is not None:
-            out[i] = record_to_sample(records[i], p.logprobs, vocab)
-    return tuple(out)
+    return _host.samples(np.ascontiguousarray(records).view(np.uint8), params, vocab)
 
 
 class PackedSamples:
@@ -618,41 +528,45 @@ def _unpack_samples(record_bytes: bytes, logprob_bytes: bytes, vocab: int) -> Pa
                          np.frombuffer(logprob_bytes, dtype=np.int8), vocab)
 
 
-def _logprob_codes(params):
-    return [-1 if p.logprobs is None else int(p.logprobs) for p in params]
+def _logprob_codes(params) -> np.ndarray:
+    return np.frombuffer(_host.logprob_codes(params), dtype=np.int8)
 
 
-def sample_batch(logits, histories, params, steps, request_ids, all_plain_greedy: bool = False,
-                 packed: bool = False):
-    device = _target_device(logits)
-    batch, vocab = int(logits.shape[0]), int(logits.shape[1])
-    if batch == 0:
-        return PackedSamples(np.zeros(0, _lib.ROW_OUT), [], vocab) if packed else ()
-    hist_need = 0
-    if not all_plain_greedy:
-        pen = batch_static(params)[4]
-        hist_need = max((len(h) for h, on in zip(histories, pen) if on), default=0)
-    with lease_sampler(device, vocab, batch, hist_need) as sampler:
-        if all_plain_greedy:
-            tokens = sampler.greedy(logits).cpu().numpy()
-            if packed:
-                records = np.zeros(batch, _lib.ROW_OUT)
-                records["token"] = tokens
-                return PackedSamples(records, [-1] * batch, vocab)
-            return tuple(TokenSample(int(t)) for t in tokens.tolist())
-        records, _ = sampler.sample(logits, histories, params, steps, request_ids)
-    bad = records["status"] & (STATUS_APPEND_FAILED | STATUS_NEEDS_GENERAL | STATUS_BAD_SLOT | STATUS_NO_SCRATCH)
+_BAD_STATUS = STATUS_APPEND_FAILED | STATUS_NEEDS_GENERAL | STATUS_BAD_SLOT | STATUS_NO_SCRATCH
+
+
+def _check_status(records) -> None:
+    bad = records["status"] & _BAD_STATUS
     if bad.any():
         raise _lib.SamplerError(f"sampler reported status {int(bad.max())} for row {int(np.argmax(bad != 0))}")
-    if packed:
-        return PackedSamples(records, _logprob_codes(params), vocab)
-    return records_to_samples(records, params, vocab)
+
+
+def sample_batch(logits, histories, params, steps, request_ids, packed: bool = False, fast_greedy: bool = True):
+    """One sampling step on the process-wide sampler of the logits' GPU.  ``fast_greedy``: a batch
+    of plain-greedy rows takes the arg-max kernel."""
+    device = _target_device(logits)
+    batch, vocab = logits.shape
+    if batch == 0:
+        return PackedSamples(np.zeros(0, _lib.ROW_OUT), [], vocab) if packed else ()
+    longest = _host.survey(histories, params)
+    with lease_sampler(device, vocab, batch, longest) as sampler:
+        if longest < 0 and fast_greedy:
+            return sampler.step_greedy(logits, packed)
+        return sampler.step(logits, histories, params, steps, request_ids, packed)
+
+
+def _cuda_device(device):
+    """A device as the process-wide samplers are kept by: with its index."""
+    import torch
+
+    device = torch.device(device)
+    return device if device.index is not None else torch.device(device.type, torch.cuda.current_device())
 
 
 def release_request(request_id, device=None) -> None:
     """Forget a request's resident histogram (call when the request finishes)."""
     with _samplers_lock:
-        targets = list(_samplers.values()) if device is None else [_samplers.get(str(device))]
+        targets = list(_samplers.values()) if device is None else [_samplers.get(_cuda_device(device))]
     for s in targets:
         if s is not None:
             s.release_request(request_id)

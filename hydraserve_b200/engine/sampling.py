@@ -21,7 +21,6 @@ Extensions over the reference, all optional:
 """
 from __future__ import annotations
 
-import os
 from dataclasses import dataclass, replace
 from typing import Iterable, Sequence
 
@@ -82,20 +81,9 @@ class TokenSample:
     top_logprobs: tuple[tuple[int, float], ...] = ()
 
 
-_new_object = object.__new__
-_set_token_id = TokenSample.token_id.__set__
-_set_logprob = TokenSample.logprob.__set__
-_set_top_logprobs = TokenSample.top_logprobs.__set__
-
-
 def _token_only(token_id: int) -> TokenSample:
-    """``TokenSample(token_id)`` without the frozen dataclass's ``__init__`` (which goes through
-    ``object.__setattr__`` per field): the result path builds one per row and step."""
-    sample = _new_object(TokenSample)
-    _set_token_id(sample, token_id)
-    _set_logprob(sample, None)
-    _set_top_logprobs(sample, ())
-    return sample
+    """``TokenSample(token_id)``: a row without log-probabilities."""
+    return TokenSample(token_id)
 
 
 def _has_penalties(params: SamplingParams) -> bool:
@@ -112,18 +100,28 @@ def _is_plain_greedy(params: SamplingParams) -> bool:
     return params.temperature == 0.0 and params.logprobs is None and not _has_penalties(params)
 
 
-def _module():
-    import sys
+_device_module = None
 
-    return sys.modules[__name__]
+
+def _device():
+    """The GPU side, imported at the first call (it imports this module)."""
+    global _device_module
+    if _device_module is None:
+        from . import _device as module
+
+        _device_module = module
+    return _device_module
 
 
 def _checked(logits, histories, params, steps, request_ids):
     if logits.ndim != 2:
         raise ValueError("sampling logits must have shape [batch, vocabulary]")
-    histories = tuple(histories)
-    params = tuple(params)
-    steps = tuple(int(step) for step in steps)
+    if type(histories) not in (list, tuple):
+        histories = tuple(histories)
+    if type(params) not in (list, tuple):
+        params = tuple(params)
+    if type(steps) not in (list, tuple):
+        steps = tuple(steps)
     if not (len(histories) == len(params) == len(steps) == logits.shape[0]):
         raise ValueError("sampling metadata must match the logits batch")
     if request_ids is not None and len(request_ids) != len(params):
@@ -147,21 +145,15 @@ def sample_logits(
     Raises ``ValueError`` for the same shape and length mismatches as the reference.
     """
     histories, params, steps = _checked(logits, histories, params, steps, request_ids)
-    this = _module()
-    from . import _device
-
-    if os.environ.get("HYDRASERVE_BATCHED_GREEDY", "1") != "0" and all(
-        this._is_plain_greedy(config) for config in params
-    ):
-        return _device.sample_batch(logits, None, params, steps, None, all_plain_greedy=True)
-    if os.environ.get("HYDRASERVE_BATCHED_GREEDY", "1") == "0":
+    gpu = _device()
+    if not gpu.batched_greedy():
         # Per-row routing, as the reference does when its batched fast path is disabled
         # (sampling.py:69, :78-83): every row goes through the module-level _sample_row.
         return tuple(
-            this._sample_row(logits[i], histories[i], params[i], steps[i])
+            _sample_row(logits[i], histories[i], params[i], steps[i])
             for i in range(len(params))
         )
-    return _device.sample_batch(logits, histories, params, steps, request_ids)
+    return gpu.sample_batch(logits, histories, params, steps, request_ids)
 
 
 def sample_logits_packed(
@@ -175,24 +167,16 @@ def sample_logits_packed(
     """``sample_logits`` with the result as one ``PackedSamples`` (an array of fixed-size
     records that indexes and iterates like the reference's tuple and pickles as bytes)."""
     histories, params, steps = _checked(logits, histories, params, steps, request_ids)
-    from . import _device
-
-    greedy = all(_is_plain_greedy(config) for config in params)
-    return _device.sample_batch(logits, None if greedy else histories, params, steps,
-                                None if greedy else request_ids, all_plain_greedy=greedy, packed=True)
+    return _device().sample_batch(logits, histories, params, steps, request_ids, packed=True)
 
 
 def release_request(request_id, device=None) -> None:
     """Free the device-resident histogram of a finished request (one that was sampled with
     ``request_ids``); the place of the reference backends' ``release``
     (serving_loop.py:1481-1488).  Unknown ids are ignored."""
-    from . import _device
-
-    _device.release_request(request_id, device)
+    _device().release_request(request_id, device)
 
 
 def _sample_row(logits, history, params: SamplingParams, step: int) -> TokenSample:
     """One row (reference sampling.py:102-163); ``logits`` is a 1-D tensor."""
-    from . import _device
-
-    return _device.sample_batch(logits.reshape(1, -1), (history,), (params,), (int(step),), None)[0]
+    return _device().sample_batch(logits.reshape(1, -1), (history,), (params,), (int(step),), None, fast_greedy=False)[0]
