@@ -507,8 +507,6 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
   ok = ok && dmalloc(h, &h->split_n, (size_t)batch_max * kMaxSplit * sizeof(int));
   ok = ok && dmalloc(h, &h->split_ticket, (size_t)batch_max * sizeof(int));
   ok = ok && cudaMallocHost(&h->h_params, (size_t)batch_max * sizeof(hs_row_params)) == cudaSuccess;
-  ok = ok && cudaMallocHost(&h->h_out, (size_t)batch_max * sizeof(hs_row_out)) == cudaSuccess;
-  ok = ok && cudaMallocHost(&h->h_tokens, (size_t)batch_max * sizeof(int32_t)) == cudaSuccess;
   ok = ok && cudaMallocHost(&h->h_small, (2 * (size_t)batch_max + 1) * sizeof(int32_t)) == cudaSuccess;
   if (flags & HS_CREATE_PHASE_CLOCKS) {
     const size_t bytes = (size_t)batch_max * hs::kV3PhaseSlots * sizeof(unsigned long long);
@@ -737,12 +735,26 @@ int hs_step_block(hs_sampler* h, size_t bytes, void** block) {
   return HS_OK;
 }
 
+}  // extern "C"
+
+namespace {
+// The pinned results of hs_step (records) and hs_step_greedy (ids), made at the first step: a
+// sampler that only ever runs device-chained steps does without.
+template <class T>
+int pinned_results(hs_sampler* h, T** p) {
+  if (!*p) HS_CUDA(h, cudaMallocHost(p, (size_t)h->batch_max * sizeof(T)));
+  return HS_OK;
+}
+}  // namespace
+
+extern "C" {
+
 int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
             const hs_step_desc* d, const hs_row_out** out, void* stream_) {
   int rc = check_common(h, logits, dtype, batch, vocab);
   if (rc != HS_OK) return rc;
   if (!d || !out) return fail(h, HS_ERR_INVALID, "desc / out is null");
-  *out = h->h_out;
+  *out = nullptr;
   if (batch == 0) return HS_OK;
   if (row_stride < vocab) return fail(h, HS_ERR_INVALID, "row_stride smaller than vocab");
   if (d->n_resets < 0 || d->n_appends < 0 || d->n_appends > 65535 || d->n_resets > 65535)
@@ -755,6 +767,9 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
   DeviceGuard guard(h->device);
   Serial serial(h, stream);
   HS_CUDA(h, serial.status);
+
+  if ((rc = pinned_results(h, &h->h_out)) != HS_OK) return rc;
+  *out = h->h_out;
 
   // What a small step brings along goes into the launches themselves: 64 rows' parameters (3 KB)
   // and 256 (slot, token) pairs (2 KB) are cheaper there than one copy ahead of the kernel
@@ -829,13 +844,15 @@ int hs_step_greedy(hs_sampler* h, const void* logits, int dtype, int64_t row_str
   int rc = check_common(h, logits, dtype, batch, vocab);
   if (rc != HS_OK) return rc;
   if (!tokens) return fail(h, HS_ERR_INVALID, "tokens is null");
-  *tokens = h->h_tokens;
+  *tokens = nullptr;
   if (batch == 0) return HS_OK;
   if (row_stride < vocab) return fail(h, HS_ERR_INVALID, "row_stride smaller than vocab");
   cudaStream_t stream = (cudaStream_t)stream_;
   DeviceGuard guard(h->device);
   Serial serial(h, stream);
   HS_CUDA(h, serial.status);
+  if ((rc = pinned_results(h, &h->h_tokens)) != HS_OK) return rc;
+  *tokens = h->h_tokens;
   rc = launch_greedy(h, logits, dtype, row_stride, batch, vocab, h->h_tokens, stream);
   if (rc != HS_OK) return rc;
   HS_CUDA(h, cudaStreamSynchronize(stream));

@@ -16,7 +16,7 @@ namespace hs {
 // One chunk of eight tokens the counting loop could not take in its branch-free form (a
 // value outside the bin window, a token of count class 3): token by token, out of line so
 // that the unrolled loop stays small.
-__device__ __noinline__ void count_chunk_slow(uint32_t* tab, int* rare_n, int2* rare, uint4 w, uint32_t cl, int i) {
+__device__ __noinline__ void count_chunk_slow(uint32_t* tab, int* rare_n, int2* rare, uint4 w, uint32_t cl, int first) {
   const uint32_t words[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll 1
   for (int k = 0; k < 8; ++k) {
@@ -28,7 +28,7 @@ __device__ __noinline__ void count_chunk_slow(uint32_t* tab, int* rare_n, int2* 
       atomicAdd(&tab[cc * kV3Bins + b], 1u);
     } else {
       const int slot = atomicAdd(rare_n, 1);
-      if (slot < kV3RareCap) rare[slot] = make_int2(8 * i + k, (int)(raw | ((uint32_t)cc << 16)));
+      if (slot < kV3RareCap) rare[slot] = make_int2(first + k, (int)(raw | ((uint32_t)cc << 16)));
     }
   }
 }
@@ -59,8 +59,7 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
   const int tid = threadIdx.x;
   c.row = row_index;
   c.vocab = a.vocab;
-  c.logits = reinterpret_cast<const unsigned short*>(a.logits) + (long long)c.row * a.row_stride;
-  c.vec = (reinterpret_cast<uintptr_t>(c.logits) & 15u) == 0;
+  c.set_row(a.logits, a.row_stride);
   c.greedy = P.temperature == 0.0f;
   c.T = P.temperature;
   c.rp = P.repetition_penalty;
@@ -94,14 +93,13 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
       const u64 packed = ((u64)key_of(canonical(__uint_as_float(raw << 16))) << 32) | (uint32_t)(~(uint32_t)id);
       best = packed > best ? packed : best;
     };
-    const int n8 = c.vec ? c.vocab / 8 : 0;
-    for (int i = tid; i < n8; i += kThreads) {
-      uint32_t raw[8], cls16;
-      load_chunk(c, i, raw, cls16);
+    for (int i = tid; i < c.n8(); i += kThreads) {
+      const uint4 w = __ldcg(c.chunks() + i);
+      const uint32_t words[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-      for (int k = 0; k < 8; ++k) consider(raw[k], 8 * i + k);
+      for (int k = 0; k < 8; ++k) consider((words[k >> 1] >> (16 * (k & 1))) & 0xffffu, c.first_of(i) + k);
     }
-    for (int id = n8 * 8 + tid; id < c.vocab; id += kThreads) consider(c.logits[id], id);
+    if (tid < c.n_loose()) consider(c.logits[c.loose(tid)], c.loose(tid));
     best = block_max_u64(*c.x, best);
     if (a.scores_out) {
       float* dst = a.scores_out + (size_t)c.row * a.vocab;
@@ -130,9 +128,9 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
     n_heavy = a.pool.n_heavy[P.slot];
     if (tid < a.pool.unique_cap) hv_q = load_now_s32(a.pool.heavy + (size_t)P.slot * a.pool.unique_cap + tid);
   }
-  // this CTA's range of 8-token chunks [chunk_lo, chunk_hi); the last part also takes the
-  // tokens after the last whole chunk
-  const int n8_row = c.vec ? c.vocab / 8 : 0;
+  // this CTA's range of 8-token chunks [chunk_lo, chunk_hi); the last part also takes the row's
+  // loose tokens
+  const int n8_row = c.n8();
   const int parts = part < 0 ? 1 : args.csplit;
   const int my_part = part < 0 ? 0 : part;
   const int per_part = (n8_row + parts - 1) / parts;
@@ -162,8 +160,8 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
         if (slot < kV3RareCap) rare[slot] = make_int2(id, (int)(raw | ((uint32_t)cc << 16)));
       }
     };
-    const uint4* src4 = reinterpret_cast<const uint4*>(c.logits);
-    const unsigned short* cls16p = reinterpret_cast<const unsigned short*>(c.cls);
+    const uint4* src4 = c.chunks();
+    const bool has_cls = c.cls != nullptr;
     // Eight tokens at a time without a branch per token.  Per 32-bit word (two tokens):
     // |x| + (0x8000 - base) sets bit 15 of a half iff |x| >= base and leaves |x| - base in its
     // low bits; |x| + (0x8000 - top) sets it iff |x| >= top; a byte permute with sign
@@ -218,35 +216,46 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
     // loop runs without bounds checks; what is left over is taken chunk by chunk.
     constexpr int kInFlight = 2;  // 128-bit loads per thread and batch
     constexpr int kStride = kInFlight * kThreads;
-    const int n_full = (chunk_hi - chunk_lo) / kStride;
-    int i0 = chunk_lo + tid;
     if (hv_pair.x >= 0 && hv_pair.x < c.vocab) hv_raw = load_now_u16(c.logits + hv_pair.x);
-    if (n_full > 0) {
-      uint4 w[kInFlight], wn[kInFlight];
-      uint32_t cl[kInFlight], cn[kInFlight];
+    // (one copy of the loop per way to get at the count classes: the question is not asked per chunk)
+    auto count_chunks = [&](auto classes) {
+      const int n_full = (chunk_hi - chunk_lo) / kStride;
+      int i0 = chunk_lo + tid;
+      if (n_full > 0) {
+        uint4 w[kInFlight], wn[kInFlight];
+        uint32_t cl[kInFlight], cn[kInFlight];
 #pragma unroll
-      for (int u = 0; u < kInFlight; ++u) {
-        w[u] = __ldcg(src4 + i0 + u * kThreads);  // past L1: almost all of it is shared memory here
-        cl[u] = cls16p ? (uint32_t)__ldcg(cls16p + i0 + u * kThreads) : 0u;
-        wn[u] = w[u];
-        cn[u] = cl[u];
-      }
-      for (int it = 0; it < n_full; ++it) {
-        if (it + 1 < n_full) {
-#pragma unroll
-          for (int u = 0; u < kInFlight; ++u) {
-            wn[u] = __ldcg(src4 + i0 + kStride + u * kThreads);
-            cn[u] = cls16p ? (uint32_t)__ldcg(cls16p + i0 + kStride + u * kThreads) : 0u;
-          }
+        for (int u = 0; u < kInFlight; ++u) {
+          w[u] = __ldcg(src4 + i0 + u * kThreads);  // past L1: almost all of it is shared memory here
+          cl[u] = classes(i0 + u * kThreads);
+          wn[u] = w[u];
+          cn[u] = cl[u];
         }
+        for (int it = 0; it < n_full; ++it) {
+          if (it + 1 < n_full) {
 #pragma unroll
-        for (int u = 0; u < kInFlight; ++u) take_chunk(w[u], cl[u], i0 + u * kThreads);
+            for (int u = 0; u < kInFlight; ++u) {
+              wn[u] = __ldcg(src4 + i0 + kStride + u * kThreads);
+              cn[u] = classes(i0 + kStride + u * kThreads);
+            }
+          }
 #pragma unroll
-        for (int u = 0; u < kInFlight; ++u) { w[u] = wn[u]; cl[u] = cn[u]; }
-        i0 += kStride;
+          for (int u = 0; u < kInFlight; ++u) take_chunk(w[u], cl[u], i0 + u * kThreads);
+#pragma unroll
+          for (int u = 0; u < kInFlight; ++u) { w[u] = wn[u]; cl[u] = cn[u]; }
+          i0 += kStride;
+        }
       }
+      for (int i = i0; i < chunk_hi; i += kThreads) take_chunk(__ldcg(src4 + i), classes(i), i);
+    };
+    if (!has_cls) {
+      count_chunks([](int) { return 0u; });
+    } else if (c.head() == 0) {
+      const unsigned short* cls16 = reinterpret_cast<const unsigned short*>(c.cls);
+      count_chunks([cls16](int i) { return (uint32_t)__ldcg(cls16 + i); });
+    } else {
+      count_chunks([&c](int i) { return c.chunk_classes(i); });
     }
-    for (int i = i0; i < chunk_hi; i += kThreads) take_chunk(__ldcg(src4 + i), cls16p ? (uint32_t)__ldcg(cls16p + i) : 0u, i);
     // the chunks that were set aside, token by token, one thread per chunk
     __syncthreads();
     {
@@ -254,24 +263,23 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
       if (n_defer <= kV3DeferCap) {
         for (int j = tid; j < n_defer; j += kThreads) {
           const int i = defer[j];
-          count_chunk_slow(c.tab, rare_n, rare, __ldcg(src4 + i), cls16p ? (uint32_t)__ldcg(cls16p + i) : 0u, i);
+          count_chunk_slow(c.tab, rare_n, rare, __ldcg(src4 + i), has_cls ? c.chunk_classes(i) : 0u, c.first_of(i));
         }
       } else {
         // more than the list holds (a row full of values outside the bin window): every chunk of
         // the range is looked at again and those the loop did not take are counted now
         for (int i = chunk_lo + tid; i < chunk_hi; i += kThreads) {
           const uint4 w4 = __ldcg(src4 + i);
-          const uint32_t cl4 = cls16p ? (uint32_t)__ldcg(cls16p + i) : 0u;
+          const uint32_t cl4 = has_cls ? c.chunk_classes(i) : 0u;
           const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
           bool slow = (cl4 & (cl4 >> 1) & 0x5555u) != 0u;
 #pragma unroll
           for (int q = 0; q < 8; ++q) slow = slow || v3_bin_of_raw((words[q >> 1] >> (16 * (q & 1))) & 0xffffu) < 0;
-          if (slow) count_chunk_slow(c.tab, rare_n, rare, w4, cl4, i);
+          if (slow) count_chunk_slow(c.tab, rare_n, rare, w4, cl4, c.first_of(i));
         }
       }
     }
-    if (last_part)
-      for (int id = n8_row * 8 + tid; id < c.vocab; id += kThreads) count_one(c.logits[id], c.class_of(id), id);
+    if (last_part && tid < c.n_loose()) count_one(c.logits[c.loose(tid)], c.class_of(c.loose(tid)), c.loose(tid));
   }
   __syncthreads();
   if (parts > 1) {
@@ -895,11 +903,12 @@ __device__ __forceinline__ bool cand_part(const RowV3Args& args, unsigned char* 
   c.greedy = false;
   // the row is streamed by args.split CTAs, each taking a contiguous range of tokens
   const int split = args.split;
-  const int width = (((a.vocab + split - 1) / split) + 7) & ~7;
-  c.lo = min(part * width, a.vocab);
-  c.hi = min(c.lo + width, a.vocab);
-  c.logits = reinterpret_cast<const unsigned short*>(a.logits) + (long long)c.row * a.row_stride;
-  c.vec = (reinterpret_cast<uintptr_t>(c.logits) & 15u) == 0;
+  c.set_row(a.logits, a.row_stride);
+  const int width = (c.n8() + split - 1) / split;
+  c.chunk_lo = min(part * width, c.n8());
+  c.chunk_hi = min(c.chunk_lo + width, c.n8());
+  c.lo = part == 0 ? 0 : c.first_of(c.chunk_lo);
+  c.hi = part == split - 1 ? a.vocab : c.first_of(c.chunk_hi);
   c.T = P.temperature; c.rp = P.repetition_penalty; c.pp = P.presence_penalty; c.fp = P.frequency_penalty;
   c.pool = a.pool;
   c.slot = P.slot;

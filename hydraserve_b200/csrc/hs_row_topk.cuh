@@ -221,8 +221,8 @@ __device__ void stream_at_or_above(const Ctx3& c, const int* thr, Hit&& hit) {
     const int cc = c.class_of(id);
     if (cc != 3 && t16_of_raw(raw) >= thr[cc]) hit(id, raw, cc);
   };
-  const int n8 = c.vec ? c.vocab / 8 : 0;
-  const uint4* src4 = reinterpret_cast<const uint4*>(c.logits);
+  const int n8 = c.n8();
+  const uint4* src4 = c.chunks();
   constexpr int kInFlight = 8;
   for (int base = 0; base < n8; base += kInFlight * kThreads) {
     uint4 w[kInFlight];
@@ -247,18 +247,19 @@ __device__ void stream_at_or_above(const Ctx3& c, const int* thr, Hit&& hit) {
         const int q = __ffs(hits) - 1;
         hits &= hits - 1;
         const uint32_t word = q < 2 ? w[u].x : (q < 4 ? w[u].y : (q < 6 ? w[u].z : w[u].w));
-        look(8 * i + q, (word >> (16 * (q & 1))) & 0xffffu);
+        look(c.first_of(i) + q, (word >> (16 * (q & 1))) & 0xffffu);
       }
     }
   }
-  for (int id = n8 * 8 + tid; id < c.vocab; id += kThreads) {
-    const uint32_t raw = c.logits[id];
-    if (t16_of_raw(raw) >= t_min) look(id, raw);
+  if (tid < c.n_loose()) {
+    const uint32_t raw = c.logits[c.loose(tid)];
+    if (t16_of_raw(raw) >= t_min) look(c.loose(tid), raw);
   }
 }
 
 // A lower bound (as signed 16-bit image of a raw value) of the k-th highest raw value among
-// the tokens of [begin, end) that the history does not hold, or -32768 when none is found.
+// the tokens of this CTA's first 2,048 chunks that the history does not hold, or -32768 when
+// none is found.
 // The sampled tokens are cut into groups of eight (one 128-bit load); the k highest group
 // maxima are k different tokens, so the k-th highest maximum is such a bound, and with
 // k much smaller than the number of groups it is about as tight as the k-th highest token.
@@ -271,40 +272,29 @@ struct SampleRegs {
   uint32_t cl[kSampleGroups];
 };
 // Starts the loads of the sample (nothing waits for them here).
-__device__ __forceinline__ void sample_fetch(const Ctx3& c, int begin, int end, SampleRegs& r) {
-  const int tid = threadIdx.x;
-  const bool vec = c.vec && (begin & 7) == 0;
-  const int n8 = vec ? (end - begin) / 8 : 0;  // whole 8-token chunks read as 128-bit words
-  const uint4* src4 = reinterpret_cast<const uint4*>(c.logits) + (begin >> 3);
-  const unsigned short* cls16p = c.cls ? reinterpret_cast<const unsigned short*>(c.cls) + (begin >> 3) : nullptr;
+__device__ __forceinline__ void sample_fetch(const Ctx3& c, SampleRegs& r) {
+  const uint4* src4 = c.chunks();
 #pragma unroll
   for (int u = 0; u < kSampleGroups; ++u) {
-    const int i = tid + u * kThreads;
-    if (i < n8) { r.w[u] = src4[i]; r.cl[u] = cls16p ? cls16p[i] : 0u; }
+    const int i = c.chunk_lo + threadIdx.x + u * kThreads;
+    if (i < c.chunk_hi) { r.w[u] = __ldcg(src4 + i); r.cl[u] = c.cls ? c.chunk_classes(i) : 0u; }
   }
 }
-__device__ int sample_kth_t16(const Ctx3& c, CandCtx& L, int begin, int end, int k, const SampleRegs& r) {
+__device__ int sample_kth_t16(const Ctx3& c, CandCtx& L, int k, const SampleRegs& r) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int kGroups = kSampleGroups;
-  const bool vec = c.vec && (begin & 7) == 0;
-  const int n8 = vec ? (end - begin) / 8 : 0;
   int top[kGroups];  // value + 32768 of the group maximum, 0 = no token
   {
 #pragma unroll
     for (int u = 0; u < kGroups; ++u) {
       top[u] = 0;
-      if (tid + u * kThreads >= n8) continue;
+      if (c.chunk_lo + tid + u * kThreads >= c.chunk_hi) continue;
       const uint32_t words[4] = {r.w[u].x, r.w[u].y, r.w[u].z, r.w[u].w};
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         if (((r.cl[u] >> (2 * q)) & 3u) == 0)
           top[u] = max(top[u], t16_of_raw((words[q >> 1] >> (16 * (q & 1))) & 0xffffu) + 32768);
     }
-  }
-  if (!vec) {
-    // a part that is not 16-byte aligned: thread-strided groups over the scalar view
-    for (int id = begin + tid; id < end; id += kThreads)
-      if (c.class_of(id) == 0) top[0] = max(top[0], t16_of_raw(c.logits[id]) + 32768);
   }
   // k-th highest of the positive maxima: bins of L.count, 256 per level
   int prefix = 0, want = k;
@@ -389,14 +379,13 @@ __device__ int topk_candidates(Ctx3& c, CandCtx& L, int k) {
   // The chain heavy -> pairs -> logits is three dependent reads; it is started for list entry
   // `tid` before the sample is fetched and worked off between the sample's steps, so that
   // the waits overlap.
-  const int sample_end = min(c.hi, c.lo + kSample);
   int n_heavy = 0, hv_q = -1;
   if (c.cls) {
     n_heavy = load_now_s32(c.pool.n_heavy + c.slot);
     if (tid < c.pool.unique_cap) hv_q = load_now_s32(c.pool.heavy + (size_t)c.slot * c.pool.unique_cap + tid);
   }
   SampleRegs sample;
-  sample_fetch(c, c.lo, sample_end, sample);
+  sample_fetch(c, sample);
   n_heavy = min(n_heavy, c.pool.unique_cap);
   const int2* pairs = c.pool.pairs + (size_t)c.slot * c.pool.unique_cap;
   int2 hv_pair = make_int2(-1, 0);
@@ -405,7 +394,7 @@ __device__ int topk_candidates(Ctx3& c, CandCtx& L, int k) {
   uint32_t hv_raw = 0;
   if (hv_mine) hv_raw = load_now_u16(c.logits + hv_pair.x);
   // the first bound: from the group maxima of the sampled tokens outside the history
-  const int t_k = sample_kth_t16(c, L, c.lo, sample_end, k, sample);
+  const int t_k = sample_kth_t16(c, L, k, sample);
   if (c.cls) {
     auto add_scored = [&](int id, uint32_t raw, int count) {  // the exact count is at hand
       const int slot = atomicAdd(L.n, 1);
@@ -432,9 +421,8 @@ __device__ int topk_candidates(Ctx3& c, CandCtx& L, int k) {
   int refreshes = 0;
   // 2. the rest of the row: eight tokens per 128-bit load, one native bf16x2 comparison per
   // two tokens against the most permissive class threshold; the rare hit is looked at closely
-  const int first8 = c.lo / 8;  // lo is a multiple of 8
-  const int n8 = c.vec ? c.hi / 8 : first8;
-  const uint4* src4 = reinterpret_cast<const uint4*>(c.logits);
+  const int first8 = c.chunk_lo, n8 = c.chunk_hi;
+  const uint4* src4 = c.chunks();
   constexpr int kBatch = HS_CAND_BATCH;  // two batches of loads: the next is on its way while this one is compared
   int n_scored = n;
   uint4 w[kBatch], wn[kBatch];
@@ -473,7 +461,7 @@ __device__ int topk_candidates(Ctx3& c, CandCtx& L, int k) {
         hits &= hits - 1;
         const uint32_t word = q < 2 ? w[u].x : (q < 4 ? w[u].y : (q < 6 ? w[u].z : w[u].w));
         const uint32_t raw = (word >> (16 * (q & 1))) & 0xffffu;
-        push(8 * i + q, raw, 4);
+        push(c.first_of(i) + q, raw, 4);
       }
     }
 #pragma unroll
@@ -507,11 +495,14 @@ __device__ int topk_candidates(Ctx3& c, CandCtx& L, int k) {
   }
   __syncthreads();
   if (L.dbg && tid == 0) { L.dbg[5] = clock64(); L.dbg[6] = (unsigned long long)refreshes; L.dbg[7] = (unsigned long long)*L.n; }
-  // scalar tail (or the whole remainder of a row that is not 16-byte aligned)
-  for (int id = max(n8 * 8, c.lo) + tid; id < c.hi; id += kThreads) {
-    const uint32_t raw = c.logits[id];
-    const int cc = c.class_of(id);
-    if (cc != 3 && t16_of_raw(raw) >= L.thr[cc]) push(id, raw, cc);
+  // the loose tokens of this CTA's range
+  if (tid < c.n_loose()) {
+    const int id = c.loose(tid);
+    if (id >= c.lo && id < c.hi) {
+      const uint32_t raw = c.logits[id];
+      const int cc = c.class_of(id);
+      if (cc != 3 && t16_of_raw(raw) >= L.thr[cc]) push(id, raw, cc);
+    }
   }
   __syncthreads();
   if (*L.lost) return -1;

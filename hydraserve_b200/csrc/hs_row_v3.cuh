@@ -179,10 +179,32 @@ struct Ctx3 {
   int* step_n = nullptr;  // two counters the early-exit scan alternates between
   int row, vocab;
   unsigned long long* dbg = nullptr;
-  int lo, hi;                    // token range this CTA streams in the candidate path (lo a multiple of 8)
+  int lo, hi;                    // token range this CTA streams in the candidate path ...
+  int chunk_lo, chunk_hi;        // ... and the whole chunks in it
   const unsigned short* logits;  // this row
   const uint32_t* cls;           // this row's 2-bit classes, or null (no penalties)
-  bool vec;                      // row start is 16-byte aligned
+  // The row in 16-byte chunks of eight tokens: a row may start anywhere (an odd vocabulary shifts
+  // every row by another two bytes), so the first `head` tokens (at most seven) lie before the
+  // first 16-byte boundary, n8 whole chunks follow, and the rest lies behind them.  Chunk i holds
+  // tokens head + 8 i to head + 8 i + 7; the up to fourteen others are "loose".
+  // (Worked out from the pointer where it is needed.)
+  __device__ __forceinline__ void set_row(const void* all_logits, long long row_stride) {
+    logits = reinterpret_cast<const unsigned short*>(all_logits) + (long long)row * row_stride;
+  }
+  __device__ __forceinline__ int head() const {
+    return min((int)((0u - (uint32_t)reinterpret_cast<uintptr_t>(logits)) & 15u) >> 1, vocab);
+  }
+  __device__ __forceinline__ int n8() const { return (vocab - head()) >> 3; }
+  __device__ __forceinline__ const uint4* chunks() const { return reinterpret_cast<const uint4*>(logits + head()); }
+  __device__ __forceinline__ int first_of(int chunk) const { return head() + 8 * chunk; }
+  __device__ __forceinline__ int n_loose() const { return vocab - 8 * n8(); }
+  __device__ __forceinline__ int loose(int j) const { return j < head() ? j : j + 8 * n8(); }
+  // the eight 2-bit classes of a chunk (cls is not null); past L1
+  __device__ __forceinline__ uint32_t chunk_classes(int chunk) const {
+    if (head() == 0) return (uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(cls) + chunk);
+    const int id = first_of(chunk);
+    return __funnelshift_r(__ldcg(cls + (id >> 4)), __ldcg(cls + (id >> 4) + 1), (uint32_t)(id & 15) * 2u) & 0xffffu;
+  }
   Pool pool;
   int slot;
   int2* s_pair;
@@ -581,22 +603,15 @@ __device__ __forceinline__ bool in_group(const Ctx3& c, const Group& g, int id, 
   return key_of(c.score_of(raw, c.heavy_count(id))) == g.key;
 }
 
-// Loads chunk i (8 tokens) of the row and its classes.
-__device__ __forceinline__ void load_chunk(const Ctx3& c, int i, uint32_t (&raw)[8], uint32_t& cls16) {
-  const uint4 w = reinterpret_cast<const uint4*>(c.logits)[i];
-  raw[0] = w.x & 0xffffu; raw[1] = w.x >> 16; raw[2] = w.y & 0xffffu; raw[3] = w.y >> 16;
-  raw[4] = w.z & 0xffffu; raw[5] = w.z >> 16; raw[6] = w.w & 0xffffu; raw[7] = w.w >> 16;
-  cls16 = c.cls ? reinterpret_cast<const unsigned short*>(c.cls)[i] : 0u;
-}
-// Bit k set: token 8*i + k belongs to the group.
+// Bit k set: token k of chunk i belongs to the group.
 __device__ __forceinline__ uint32_t chunk_members(const Ctx3& c, const Group& g, int i, const uint4& w,
                                                   uint32_t cls16) {
   const uint32_t words[4] = {w.x, w.y, w.z, w.w};
   uint32_t memb = 0;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    memb |= (in_group(c, g, 8 * i + 2 * k, words[k] & 0xffffu, (cls16 >> (4 * k)) & 3) ? 1u : 0u) << (2 * k);
-    memb |= (in_group(c, g, 8 * i + 2 * k + 1, words[k] >> 16, (cls16 >> (4 * k + 2)) & 3) ? 1u : 0u) << (2 * k + 1);
+    memb |= (in_group(c, g, c.first_of(i) + 2 * k, words[k] & 0xffffu, (cls16 >> (4 * k)) & 3) ? 1u : 0u) << (2 * k);
+    memb |= (in_group(c, g, c.first_of(i) + 2 * k + 1, words[k] >> 16, (cls16 >> (4 * k + 2)) & 3) ? 1u : 0u) << (2 * k + 1);
   }
   return memb;
 }
@@ -604,8 +619,7 @@ __device__ __forceinline__ uint32_t chunk_members(const Ctx3& c, const Group& g,
 // loads in flight per lane.
 __device__ __forceinline__ u64 count_members(const Ctx3& c, const Group& g, int b, int e) {
   const int lane = threadIdx.x & 31;
-  const uint4* src4 = reinterpret_cast<const uint4*>(c.logits);
-  const unsigned short* cls16p = reinterpret_cast<const unsigned short*>(c.cls);
+  const uint4* src4 = c.chunks();
   u64 mine = 0;
   for (int i0 = b + lane; i0 < e; i0 += 4 * 32) {
     uint4 w[4];
@@ -613,7 +627,7 @@ __device__ __forceinline__ u64 count_members(const Ctx3& c, const Group& g, int 
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int i = i0 + 32 * u;
-      if (i < e) { w[u] = src4[i]; cl[u] = cls16p ? cls16p[i] : 0u; }
+      if (i < e) { w[u] = __ldcg(src4 + i); cl[u] = c.cls ? c.chunk_classes(i) : 0u; }
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -630,9 +644,15 @@ __device__ __forceinline__ u64 count_members(const Ctx3& c, const Group& g, int 
 // warp can rank its members with ballots.
 __device__ int nth_in_group(Ctx3& c, const Group& g, u64 n) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
-  const int n8 = c.vec ? c.vocab / 8 : 0;
-  int b = 0, e = n8;
+  int b = 0, e = c.n8();
   u64 before = 0;
+  // the loose tokens ahead of the first chunk, by every warp alike
+  {
+    const bool mbr = lane < c.head() && in_group(c, g, lane, c.logits[lane], c.class_of(lane));
+    const uint32_t ballot = __ballot_sync(0xffffffffu, mbr);
+    if ((u64)__popc(ballot) >= n) return (int)__fns(ballot, 0, (int)n);
+    before = (u64)__popc(ballot);
+  }
   bool in_tail = false;
   int result = 0x7fffffff;
   while (true) {
@@ -656,43 +676,31 @@ __device__ int nth_in_group(Ctx3& c, const Group& g, u64 n) {
   }
   if (tid == 0) c.x->bcast[6] = 0;
   __syncthreads();
-  if (!in_tail && warp == 0) {
-    // at most 128 chunks: rank members with warp scans
-    const uint4* src4 = reinterpret_cast<const uint4*>(c.logits);
-    const unsigned short* cls16p = reinterpret_cast<const unsigned short*>(c.cls);
+  if (warp == 0) {
+    // at most 128 chunks, then the loose tokens behind the last one: rank members with warp scans
+    const uint4* src4 = c.chunks();
     u64 running = before;
-    for (int i0 = b; i0 < e && running < n; i0 += 32) {
+    for (int i0 = b; !in_tail && i0 < e && running < n; i0 += 32) {
       const int i = i0 + lane;
       uint32_t memb = 0;
-      if (i < e) memb = chunk_members(c, g, i, src4[i], cls16p ? cls16p[i] : 0u);
+      if (i < e) memb = chunk_members(c, g, i, __ldcg(src4 + i), c.cls ? c.chunk_classes(i) : 0u);
       const u64 incl = warp_scan_u64((u64)__popc(memb));
       u64 rank = running + incl - __popc(memb);
       for (int k = 0; k < 8; ++k) {
         if (!((memb >> k) & 1u)) continue;
-        if (++rank == n) c.x->bcast[6] = (u64)(8 * i + k) + 1;
+        if (++rank == n) c.x->bcast[6] = (u64)(c.first_of(i) + k) + 1;
       }
       running += shfl_u64(incl, 31);
     }
-    if (running < n) before = running;  // not reached inside the vector part: look in the tail
-    if (lane == 0 && running < n) c.x->bcast[5] = running;
+    if (running < n) {
+      const int id = c.first_of(c.n8()) + lane;
+      const bool mbr = id < c.vocab && in_group(c, g, id, c.logits[id], c.class_of(id));
+      const uint32_t ballot = __ballot_sync(0xffffffffu, mbr);
+      const u64 rank = running + __popc(ballot & ((1u << lane) - 1u)) + 1;
+      if (mbr && rank == n) c.x->bcast[6] = (u64)id + 1;
+    }
   }
   __syncthreads();
-  if (c.x->bcast[6] == 0) {
-    // scalar tail of the row (all of it when the row is not 16-byte aligned)
-    if (!in_tail) before = c.x->bcast[5];
-    if (warp == 0) {
-      u64 running = in_tail ? before : c.x->bcast[5];
-      for (int id0 = n8 * 8; id0 < c.vocab && running < n; id0 += 32) {
-        const int id = id0 + lane;
-        const bool mbr = id < c.vocab && in_group(c, g, id, c.logits[id], c.class_of(id));
-        const uint32_t ballot = __ballot_sync(0xffffffffu, mbr);
-        const u64 rank = running + __popc(ballot & ((1u << lane) - 1u)) + 1;
-        if (mbr && rank == n) c.x->bcast[6] = (u64)id + 1;
-        running += __popc(ballot);
-      }
-    }
-    __syncthreads();
-  }
   const u64 found = c.x->bcast[6];
   __syncthreads();
   if (found) result = (int)(found - 1);
@@ -700,8 +708,7 @@ __device__ int nth_in_group(Ctx3& c, const Group& g, u64 n) {
 }
 
 // Token id of the n-th (1-based, ascending id) of the `members` tokens of ONE class (count
-// class and one-value bin `cell`), for classes of at most kV3ScanCap tokens, or -1 when the row
-// has no 16-byte aligned view.  The row is walked from the end that is nearer to the n-th
+// class and one-value bin `cell`), for classes of at most kV3ScanCap tokens.  The row is walked from the end that is nearer to the n-th
 // member, 16,384 tokens per step, and the walk stops soon after the step that reaches it (it
 // looks every fourth step): members are spread evenly over the row, so on average a third of
 // it is read.  A class is one bf16 bit
@@ -716,7 +723,7 @@ static_assert(kV3ScanCap * sizeof(int) <= 2 * kV3ListCap * sizeof(V3Entry), "sca
 struct ScanArgs {
   const unsigned short* logits;
   const uint32_t* cls;
-  int vocab;
+  int vocab, head, n8;
   int* ids;       // [kV3ScanCap]
   int* slot_n;    // ids used
   int* step_n;    // [2]
@@ -733,9 +740,8 @@ __device__ __noinline__ void scan_small_class(const ScanArgs c, uint32_t raw, in
   if (tid == 0) { *c.slot_n = 0; c.step_n[0] = 0; c.step_n[1] = 0; *c.result = 0; }
   __syncthreads();
   if (c.dbg && tid == 0) c.dbg[40] = clock64();
-  const int n8 = c.vocab / 8;
-  const uint4* src4 = reinterpret_cast<const uint4*>(c.logits);
-  const unsigned short* cls16p = reinterpret_cast<const unsigned short*>(c.cls);
+  const int n8 = c.n8;
+  const uint4* src4 = reinterpret_cast<const uint4*>(c.logits + c.head);
   // Members found are counted in two counters that take turns from one look to the next:
   // after a look's barrier every thread reads that turn's counter, which nobody adds to before
   // the barrier after next, so all threads see the same running total and leave together.
@@ -744,12 +750,13 @@ __device__ __noinline__ void scan_small_class(const ScanArgs c, uint32_t raw, in
     if (slot < kV3ScanCap) ids[slot] = id;
     atomicAdd(c.step_n + parity, 1);
   };
-  // the few tokens after the last whole chunk: first when walking backwards, last otherwise
-  auto tail = [&](int parity) {
-    for (int id = n8 * 8 + tid; id < c.vocab; id += kThreads)
-      if ((uint32_t)c.logits[id] == raw && (c.cls ? (int)((c.cls[id >> 4] >> ((id & 15) * 2)) & 3u) : 0) == cc) note(id, parity);
+  // the loose tokens at the end the walk starts from, and later those at its other end
+  auto loose = [&](int from, int to, int parity) {
+    const int id = from + tid;
+    if (id < to && (uint32_t)c.logits[id] == raw && (c.cls ? (int)((c.cls[id >> 4] >> ((id & 15) * 2)) & 3u) : 0) == cc) note(id, parity);
   };
-  if (!forward) tail(0);
+  const int tail_at = c.head + 8 * n8;
+  if (forward) loose(0, c.head, 0); else loose(tail_at, c.vocab, 0);
   constexpr int kBatch = 4;
   constexpr int kStep = kBatch * kThreads;  // chunks per step
   constexpr int kCheckShift = 2;            // the walk looks whether it may stop every 2^kCheckShift steps
@@ -764,7 +771,15 @@ __device__ __noinline__ void scan_small_class(const ScanArgs c, uint32_t raw, in
       const int i = chunk_of(s, u);
       const bool in = s < n_steps && i < n8;
       dw[u] = in ? __ldcg(src4 + i) : make_uint4(~vv, ~vv, ~vv, ~vv);
-      dc[u] = (in && cls16p) ? (uint32_t)__ldcg(cls16p + i) : 0u;
+      dc[u] = 0u;
+      if (in && c.cls) {
+        if (c.head == 0) {
+          dc[u] = (uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(c.cls) + i);
+        } else {
+          const int id = c.head + 8 * i;
+          dc[u] = __funnelshift_r(__ldcg(c.cls + (id >> 4)), __ldcg(c.cls + (id >> 4) + 1), (uint32_t)(id & 15) * 2u);
+        }
+      }
     }
   };
   fetch(w, cl, 0);
@@ -779,7 +794,7 @@ __device__ __noinline__ void scan_small_class(const ScanArgs c, uint32_t raw, in
       const uint32_t m2 = __heq2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[u].z), vv2);
       const uint32_t m3 = __heq2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[u].w), vv2);
       if (m0 | m1 | m2 | m3) {
-        const int id = 8 * chunk_of(s, u);
+        const int id = c.head + 8 * chunk_of(s, u);
         uint32_t hits = ((m0 & 1u) | ((m0 >> 15) & 2u)) | (((m1 & 1u) | ((m1 >> 15) & 2u)) << 2) |
                         (((m2 & 1u) | ((m2 >> 15) & 2u)) << 4) | (((m3 & 1u) | ((m3 >> 15) & 2u)) << 6);
         while (hits) {
@@ -802,7 +817,7 @@ __device__ __noinline__ void scan_small_class(const ScanArgs c, uint32_t raw, in
 #pragma unroll
     for (int u = 0; u < kBatch; ++u) { w[u] = wn[u]; cl[u] = cn[u]; }
   }
-  if (forward && !reached) tail(0);
+  if (!reached) { if (forward) loose(tail_at, c.vocab, 0); else loose(0, c.head, 0); }
   if (c.dbg && tid == 0) c.dbg[43] = clock64();
   __syncthreads();
   if (c.dbg && tid == 0) c.dbg[41] = clock64();
@@ -819,9 +834,9 @@ __device__ __noinline__ void scan_small_class(const ScanArgs c, uint32_t raw, in
   if (c.dbg && tid == 0) { c.dbg[42] = clock64(); c.dbg[44] = (unsigned long long)found; }
 }
 __device__ __forceinline__ int nth_in_small_class(Ctx3& c, int cell, u64 n, u64 members) {
-  if (!c.vec || members > (u64)kV3ScanCap || n < 1 || n > members) return -1;
+  if (members > (u64)kV3ScanCap || n < 1 || n > members) return -1;
   const int cc = cell / kV3Bins;
-  const ScanArgs sa{c.logits, c.cls, c.vocab, reinterpret_cast<int*>(c.gbuf), c.gbuf_n, c.step_n, &c.x->bcast[6], c.dbg};
+  const ScanArgs sa{c.logits, c.cls, c.vocab, c.head(), c.n8(), reinterpret_cast<int*>(c.gbuf), c.gbuf_n, c.step_n, &c.x->bcast[6], c.dbg};
   scan_small_class(sa, v3_raw_of_bin(cell - cc * kV3Bins), cc, (int)n, (int)members);
   const u64 hit = c.x->bcast[6];
   __syncthreads();
@@ -830,24 +845,24 @@ __device__ __forceinline__ int nth_in_small_class(Ctx3& c, int cell, u64 n, u64 
 
 // Appends to the gather buffer the ids of all group members with id <= id_limit.
 __device__ void emit_group_upto(Ctx3& c, const Group& g, int id_limit) {
-  const int n8 = c.vec ? c.vocab / 8 : 0;
-  const int last = min(n8, id_limit / 8 + 1);
-  const uint4* src4 = reinterpret_cast<const uint4*>(c.logits);
-  const unsigned short* cls16p = reinterpret_cast<const unsigned short*>(c.cls);
+  const int last = min(c.n8(), max(0, id_limit - c.head()) / 8 + 1);
+  const uint4* src4 = c.chunks();
   auto emit = [&](int id) {
     const int slot = atomicAdd(c.gbuf_n, 1);
     if (slot < kV3ListCap) c.gbuf[slot] = V3Entry{g.key, id, 1u, 0u, 0ull};
   };
   for (int i = threadIdx.x; i < last; i += kThreads) {
-    uint32_t memb = chunk_members(c, g, i, src4[i], cls16p ? cls16p[i] : 0u);
+    uint32_t memb = chunk_members(c, g, i, __ldcg(src4 + i), c.cls ? c.chunk_classes(i) : 0u);
     while (memb) {
       const int k = __ffs(memb) - 1;
       memb &= memb - 1;
-      if (8 * i + k <= id_limit) emit(8 * i + k);
+      if (c.first_of(i) + k <= id_limit) emit(c.first_of(i) + k);
     }
   }
-  for (int id = n8 * 8 + threadIdx.x; id < c.vocab && id <= id_limit; id += kThreads)
-    if (in_group(c, g, id, c.logits[id], c.class_of(id))) emit(id);
+  if ((int)threadIdx.x < c.n_loose()) {
+    const int id = c.loose(threadIdx.x);
+    if (id <= id_limit && in_group(c, g, id, c.logits[id], c.class_of(id))) emit(id);
+  }
   __syncthreads();
 }
 

@@ -49,8 +49,9 @@ __global__ void __launch_bounds__(kThreads, 2) shard_partial_kernel(const ShardA
   c.vocab = a.vocab;
   c.lo = 0;
   c.hi = a.vocab;
-  c.logits = reinterpret_cast<const unsigned short*>(a.logits) + (long long)c.row * a.row_stride;
-  c.vec = (reinterpret_cast<uintptr_t>(c.logits) & 15u) == 0;
+  c.set_row(a.logits, a.row_stride);
+  c.chunk_lo = 0;
+  c.chunk_hi = c.n8();
   const hs_row_params P = a.params[c.row];
   c.greedy = P.temperature == 0.0f;
   c.T = P.temperature; c.rp = P.repetition_penalty; c.pp = P.presence_penalty; c.fp = P.frequency_penalty;
@@ -99,24 +100,22 @@ __global__ void __launch_bounds__(kThreads, 2) shard_partial_kernel(const ShardA
                   "the count tables fit in the place of the candidate list, its masses and the counters");
     for (int i = tid; i < kCells; i += kThreads) tab[i] = 0;
     __syncthreads();
-    const int n8 = c.vec ? c.vocab / 8 : 0;
-    const uint4* src4 = reinterpret_cast<const uint4*>(c.logits);
-    const unsigned short* cls16p = reinterpret_cast<const unsigned short*>(c.cls);
+    const uint4* src4 = c.chunks();
     const uint32_t tab_at = (uint32_t)__cvta_generic_to_shared(tab);
     auto take = [&](int id, uint32_t raw, int cc) {
       const int b = cc == 3 ? -1 : v3_bin_of_raw(raw);
       if (b >= 0) asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(tab_at + 4u * (uint32_t)(cc * kV3Bins + b)) : "memory");
       else z += mass_of(c.element_score(id, raw, cc), m);
     };
-    for (int i = tid; i < n8; i += kThreads) {
+    for (int i = tid; i < c.n8(); i += kThreads) {
       const uint4 w = __ldcg(src4 + i);
-      const uint32_t cl = cls16p ? (uint32_t)cls16p[i] : 0u;
+      const uint32_t cl = c.cls ? c.chunk_classes(i) : 0u;
       const uint32_t words[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
       for (int q = 0; q < 8; ++q)
-        take(8 * i + q, (words[q >> 1] >> (16 * (q & 1))) & 0xffffu, (int)((cl >> (2 * q)) & 3u));
+        take(c.first_of(i) + q, (words[q >> 1] >> (16 * (q & 1))) & 0xffffu, (int)((cl >> (2 * q)) & 3u));
     }
-    for (int id = n8 * 8 + tid; id < c.vocab; id += kThreads) take(id, c.logits[id], c.class_of(id));
+    if (tid < c.n_loose()) take(c.loose(tid), c.logits[c.loose(tid)], c.class_of(c.loose(tid)));
     __syncthreads();
     for (int cell = tid; cell < kCells; cell += kThreads) {
       const uint32_t count = tab[cell];
