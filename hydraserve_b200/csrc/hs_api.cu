@@ -14,12 +14,12 @@
 #include "../../include/hs_sampler.h"
 #include "hs_common.cuh"
 #include "hs_state.cuh"
-#include "hs_row_kernel.cuh"
+#include "hs_row_args.cuh"
 #include "hs_row_v3.cuh"
 #include "hs_row_topk.cuh"
 #include "hs_sharded.cuh"
 #include "hs_row_bf16_kernel.cuh"
-#include "hs_row_f32_topk.cuh"
+#include "hs_row_resident.cuh"
 
 namespace {
 
@@ -50,11 +50,17 @@ struct Plan {
 
 inline size_t align16(size_t v) { return (v + 15) & ~size_t(15); }
 
+// Shared memory of the resident kernel next to the slice: a candidate row's finisher takes the
+// slice's place, so that never gets less than kResMerge bytes.
 size_t fixed_smem(int cluster) {
   size_t off = align16(sizeof(hs::Exchange));
   off += sizeof(hs::Hist);
   off += (sizeof(u64) + sizeof(uint32_t)) * (hs::kBins / cluster);
   return align16(off);
+}
+size_t resident_smem(int cluster, int slice, bool global_stage) {
+  const size_t stage = global_stage ? 0 : (size_t)slice * sizeof(float);
+  return fixed_smem(cluster) + std::max(stage, (size_t)hs::kResMerge);
 }
 
 }  // namespace
@@ -163,23 +169,30 @@ bool dmalloc(hs_sampler* h, T** p, size_t bytes) {
   return true;
 }
 
-bool make_plan(const hs_sampler* h, int vocab, Plan& p) {
-  static const int sizes[4] = {1, 2, 4, 8};
-  for (int k = 0; k < 4; ++k) {
-    const int c = sizes[k];
-    if (h->force_cluster && c != h->force_cluster) continue;
+// The resident kernel's geometry.  As many CTAs per row as leave each at least 4,096 tokens (below
+// that a row's time is its barriers), eight at most (the portable cluster size): the row's passes
+// over its slices are what takes time, and eight slices of up to about 19,000 tokens still sit two
+// to an SM.  A batch that would run to more than four waves of two CTAs per SM gets fewer, larger
+// slices (fewer merges per row), down to the smallest cluster whose shared memory holds the row.
+bool make_plan(const hs_sampler* h, int vocab, int batch, Plan& p) {
+  auto plan_of = [&](int c, bool global_stage) {
     const int slice = ((vocab + c - 1) / c + 7) & ~7;
-    const size_t smem = fixed_smem(c) + (size_t)slice * sizeof(float);
-    if (smem <= (size_t)h->smem_optin && slice <= hs::kMaxSliceElems) {
-      p = Plan{c, slice, smem, false};
-      return true;
-    }
+    return Plan{c, slice, resident_smem(c, slice, global_stage), global_stage};
+  };
+  auto fits = [&](int c) {
+    const Plan q = plan_of(c, false);
+    return q.smem <= (size_t)h->smem_optin && q.slice <= hs::kMaxSliceElems;
+  };
+  if (h->force_cluster) {
+    if (fits(h->force_cluster)) { p = plan_of(h->force_cluster, false); return true; }
+  } else {
+    int c = hs::kMaxCluster;
+    while (c > 1 && vocab / c < 4096 && fits(c / 2)) c /= 2;
+    while (c > 1 && (long long)batch * c > 8ll * h->sm_count && fits(c / 2)) c /= 2;
+    if (fits(c)) { p = plan_of(c, false); return true; }
   }
-  const int c = hs::kMaxCluster;
-  const int slice = ((vocab + c - 1) / c + 7) & ~7;
-  if (slice > hs::kMaxSliceElems) return false;
-  p = Plan{c, slice, fixed_smem(c), true};
-  return true;
+  p = plan_of(hs::kMaxCluster, true);
+  return p.slice <= hs::kMaxSliceElems;
 }
 
 int check_common(hs_sampler* h, const void* logits, int dtype, int batch, int vocab) {
@@ -260,18 +273,9 @@ int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride
     h->launches += 1;
     return HS_OK;
   }
-  if (!make_plan(h, vocab, plan)) return fail(h, HS_ERR_CAPACITY, "vocabulary too wide for the row kernel");
-  // fp32 rows with a small top_k: the candidate kernel, one CTA per row (the other rows' CTAs
-  // leave at once); the general kernel below leaves those rows alone
-  a.skip_candidate_rows = 0;
-  if (dtype == HS_DTYPE_F32 && !h->force_general && !(flags & HS_SAMPLE_GENERAL_KERNEL)) {
-    a.skip_candidate_rows = 1;
-    hs::F32TopkArgs f{a, h->phase_clocks};
-    HS_CUDA(h, launch(hs::row_kernel_f32_topk, dim3((unsigned)batch), hs::kThreads, hs::layout_cand().total, stream,
-                      LaunchAttrs(0, behind), f, inl));
-    behind = false;
-    h->launches += 1;
-  }
+  if (!make_plan(h, vocab, batch, plan)) return fail(h, HS_ERR_CAPACITY, "vocabulary too wide for the row kernel");
+  // (bf16 rows that get here, and whatever is asked for by flag, are finished in token order)
+  a.general_order = dtype == HS_DTYPE_BF16 || h->force_general || (flags & HS_SAMPLE_GENERAL_KERNEL) ? 1 : 0;
   if (plan.global_stage) {
     const size_t need = (size_t)batch * plan.slice * plan.cluster;
     if (need > h->gstage_elems) return fail(h, HS_ERR_CAPACITY, "global stage too small for this batch x vocab");
@@ -459,9 +463,9 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
   auto bail = [&](int code) { release(h); delete h; return code; };
   if (cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return bail(HS_ERR_CUDA);
   if (cudaDeviceGetAttribute(&h->smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return bail(HS_ERR_CUDA);
+  h->smem_optin -= 1024;  // (the kernels' static shared memory)
   if (cudaFuncSetAttribute(hs::row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, h->smem_optin) != cudaSuccess) return bail(HS_ERR_CUDA);
   if (cudaFuncSetAttribute(hs::row_kernel_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs::bf16_kernel_smem()) != cudaSuccess) return bail(HS_ERR_CUDA);
-  if (cudaFuncSetAttribute(hs::row_kernel_f32_topk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs::layout_cand().total) != cudaSuccess) return bail(HS_ERR_CUDA);
   if (cudaFuncSetAttribute(hs::shard_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs::layout_cand().total) != cudaSuccess) return bail(HS_ERR_CUDA);
   if (cudaFuncSetAttribute(hs::shard_merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs::layout_cand().total) != cudaSuccess) return bail(HS_ERR_CUDA);
   {
@@ -526,7 +530,7 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
   ok = ok && cudaMemset(h->pool.error, 0, sizeof(int32_t)) == cudaSuccess;
   if (!ok) return bail(HS_ERR_CUDA);
   Plan plan;
-  if (!make_plan(h, vocab_max, plan)) return bail(HS_ERR_CAPACITY);
+  if (!make_plan(h, vocab_max, batch_max, plan)) return bail(HS_ERR_CAPACITY);
   if (plan.global_stage) {
     h->gstage_elems = (size_t)batch_max * plan.slice * plan.cluster;
     if (!dmalloc(h, &h->gstage, h->gstage_elems * sizeof(float))) return bail(HS_ERR_CUDA);
@@ -825,15 +829,11 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
   }
   hs::InlineRows inl;
   if (rows_inline) std::memcpy(inl.p, params, (size_t)batch * sizeof(hs_row_params));
-  // bf16 rows' records go straight to pinned memory (one burst per row, see write_record); the
-  // general kernel's CTAs put a row's record together in device memory
-  const bool direct = dtype == HS_DTYPE_BF16 && !h->force_general;
+  // (the records go straight to pinned memory, one burst per row: see write_record)
   rc = launch_rows(h, logits, dtype, row_stride, batch, vocab,
                    rows_inline ? nullptr : reinterpret_cast<const hs_row_params*>(h->d_block), rows_inline ? inl : kNoInlineRows,
-                   direct ? h->h_out : h->d_out, nullptr, nullptr, nullptr, 0u, behind, stream);
+                   h->h_out, nullptr, nullptr, nullptr, 0u, behind, stream);
   if (rc != HS_OK) return rc;
-  if (!direct)
-    HS_CUDA(h, cudaMemcpyAsync(h->h_out, h->d_out, (size_t)batch * sizeof(hs_row_out), cudaMemcpyDeviceToHost, stream));
   HS_CUDA(h, cudaStreamSynchronize(stream));
   h->have_last = false;  // everything enqueued so far has been waited for
   return HS_OK;
@@ -937,8 +937,8 @@ int hs_query(hs_sampler* h, int what, int vocab, int dtype) {
   Plan plan;
   const bool v3 = dtype == HS_DTYPE_BF16 && !h->force_general;
   switch (what) {
-    case 0: return v3 ? 1 : (make_plan(h, vocab, plan) ? plan.cluster : HS_ERR_CAPACITY);
-    case 1: return v3 ? 0 : (make_plan(h, vocab, plan) ? (plan.global_stage ? 0 : 1) : HS_ERR_CAPACITY);
+    case 0: return v3 ? 1 : (make_plan(h, vocab, 1, plan) ? plan.cluster : HS_ERR_CAPACITY);
+    case 1: return v3 ? 0 : (make_plan(h, vocab, 1, plan) ? (plan.global_stage ? 0 : 1) : HS_ERR_CAPACITY);
     case 4: return v3 ? 1 : 0;
     case 2: return h->sm_count;
     case 3: return (int)(h->launches & 0x7fffffffull);

@@ -880,11 +880,6 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
 }
 
 
-// Rows with 0 < top_k <= kTopKMax take the candidate path.
-__device__ __forceinline__ bool is_candidate_row(const hs_row_params& P, int vocab) {
-  return P.temperature != 0.0f && P.top_k > 0 && P.top_k <= kTopKMax && P.top_k < vocab;
-}
-
 // One part of a candidate row (a contiguous range of its tokens).  The CTA that brings in the
 // row's last part finishes the row.  Returns true when the row's candidate list overflowed
 // and the caller (the finishing CTA) has to count the row after all.

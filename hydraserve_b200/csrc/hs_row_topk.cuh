@@ -30,7 +30,6 @@
 
 namespace hs {
 
-constexpr int kTopKMax = 256;      // largest top_k served by the candidate path
 constexpr int kCandCap = 4096;     // candidate list capacity (shared memory, 8 bytes each)
 constexpr int kCandSoft = 2048;    // raise the bound once the list is this long
 constexpr int kSortAll = 128;      // a merged list this short is sorted whole instead of cut first

@@ -34,7 +34,7 @@
 #include "hs_common.cuh"
 #include "hs_select.cuh"
 #include "hs_state.cuh"
-#include "hs_row_kernel.cuh"
+#include "hs_row_args.cuh"
 #include "../../include/hs_sampler.h"
 
 namespace hs {
