@@ -283,7 +283,7 @@ int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride
   a.slice = plan.slice;
   a.gstage = plan.global_stage ? h->gstage : nullptr;
 
-  HS_CUDA(h, launch(hs::row_kernel, dim3((unsigned)plan.cluster, (unsigned)batch), hs::kThreads, plan.smem, stream,
+  HS_CUDA(h, launch(plan.global_stage ? hs::row_kernel<false> : hs::row_kernel<true>, dim3((unsigned)plan.cluster, (unsigned)batch), hs::kThreads, plan.smem, stream,
                     LaunchAttrs(plan.cluster, behind), a, inl));
   h->launches += 1;
   return HS_OK;
@@ -464,7 +464,8 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
   if (cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return bail(HS_ERR_CUDA);
   if (cudaDeviceGetAttribute(&h->smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return bail(HS_ERR_CUDA);
   h->smem_optin -= 1024;  // (the kernels' static shared memory)
-  if (cudaFuncSetAttribute(hs::row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, h->smem_optin) != cudaSuccess) return bail(HS_ERR_CUDA);
+  if (cudaFuncSetAttribute(hs::row_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, h->smem_optin) != cudaSuccess) return bail(HS_ERR_CUDA);
+  if (cudaFuncSetAttribute(hs::row_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, h->smem_optin) != cudaSuccess) return bail(HS_ERR_CUDA);
   if (cudaFuncSetAttribute(hs::row_kernel_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs::bf16_kernel_smem()) != cudaSuccess) return bail(HS_ERR_CUDA);
   if (cudaFuncSetAttribute(hs::shard_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs::layout_cand().total) != cudaSuccess) return bail(HS_ERR_CUDA);
   if (cudaFuncSetAttribute(hs::shard_merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs::layout_cand().total) != cudaSuccess) return bail(HS_ERR_CUDA);

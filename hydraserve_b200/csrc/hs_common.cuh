@@ -146,7 +146,6 @@ struct Exchange {
   u64 warp_b[kWarps];
   u64 ring[2][4];      // values this CTA publishes to its cluster, double buffered
   u64 bcast[8];        // results broadcast within the CTA
-  uint32_t ring_phase;
 };
 
 // Sum of (a, b) over the CTA; every thread gets the totals.  Two barriers.
@@ -196,78 +195,32 @@ __device__ __forceinline__ void block_warp_prefix2(Exchange& x, u64 wa, u64 wb, 
 }
 
 // ---- cluster primitives --------------------------------------------------------------
-// Every CTA of the cluster publishes up to four 64-bit values; all CTAs read all of
-// them.  ring_publish, then any cluster-wide barrier, then ring_read.  The buffer is
-// double buffered, so no barrier is needed after the read.  `vals` must be CTA-uniform.
+// Every CTA of the cluster publishes up to four 64-bit values (CTA-uniform; thread 0's count);
+// afterwards lane r of EVERY warp holds the values of rank r, lanes beyond the ranks hold zeros: one
+// remote read each, side by side.  The buffer takes turns with a second one, so no barrier is
+// needed after the read; `turn` counts the exchanges, per thread.
 template <int N>
-__device__ __forceinline__ uint32_t ring_publish(Exchange& x, const u64 (&vals)[N]) {
-  static_assert(N <= 4, "ring holds four values");
-  __syncthreads();
-  const uint32_t phase = x.ring_phase & 1u;
+__device__ __forceinline__ void cluster_exchange(cg::cluster_group& cluster, Exchange& x, uint32_t& turn,
+                                                 const u64 (&vals)[N], u64 (&got)[N]) {
+  static_assert(N <= 4, "the ring holds four values");
+  const uint32_t at = turn++ & 1u;
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int i = 0; i < N; ++i) x.ring[phase][i] = vals[i];
+    for (int i = 0; i < N; ++i) x.ring[at][i] = vals[i];
   }
-  __syncthreads();
-  if (threadIdx.x == 0) x.ring_phase = phase ^ 1u;
-  return phase;
-}
-template <int N>
-__device__ __forceinline__ void ring_read(cg::cluster_group& cluster, Exchange& x, uint32_t phase,
-                                          u64 (&out)[kMaxCluster][N]) {
-  const unsigned nranks = cluster.num_blocks();
-  for (unsigned r = 0; r < nranks; ++r) {
-    const Exchange* remote = nranks > 1 ? cluster.map_shared_rank(&x, r) : &x;
+  const unsigned n = cluster.num_blocks(), lane = threadIdx.x & 31u;
+  if (n > 1) cluster.sync(); else __syncthreads();
+  const Exchange* remote = n > 1 ? cluster.map_shared_rank(&x, lane < n ? lane : 0u) : &x;
 #pragma unroll
-    for (int i = 0; i < N; ++i) out[r][i] = remote->ring[phase][i];
-  }
+  for (int i = 0; i < N; ++i) got[i] = lane < n ? remote->ring[at][i] : 0ull;
 }
-// Reductions over the published values of all CTAs, read straight from the ring.
-enum class RingOp { Sum, Max, Min };
-template <RingOp OP>
-__device__ __forceinline__ u64 ring_reduce(cg::cluster_group& cluster, Exchange& x, uint32_t phase, int i) {
-  const unsigned nranks = cluster.num_blocks();
-  u64 acc = OP == RingOp::Min ? ~0ull : 0ull;
-#pragma unroll
-  for (unsigned r = 0; r < (unsigned)kMaxCluster; ++r) {
-    if (r >= nranks) break;
-    const Exchange* remote = nranks > 1 ? cluster.map_shared_rank(&x, r) : &x;
-    const u64 v = remote->ring[phase][i];
-    if (OP == RingOp::Sum) acc += v;
-    else if (OP == RingOp::Max) acc = v > acc ? v : acc;
-    else acc = v < acc ? v : acc;
-  }
-  return acc;
+// Sum over the ranks below `rank` of a value held by lane as above.
+__device__ __forceinline__ u64 ranks_below(u64 v, unsigned rank) {
+  return warp_sum_u64((threadIdx.x & 31u) < rank ? v : 0ull);
 }
-// Sum over the CTAs of rank < my_rank (exclusive prefix in rank order).
-__device__ __forceinline__ u64 ring_prefix(cg::cluster_group& cluster, Exchange& x, uint32_t phase, int i,
-                                           unsigned my_rank) {
-  const unsigned nranks = cluster.num_blocks();
-  u64 acc = 0;
-#pragma unroll
-  for (unsigned r = 0; r < (unsigned)kMaxCluster; ++r) {
-    if (r >= my_rank || r >= nranks) break;
-    const Exchange* remote = nranks > 1 ? cluster.map_shared_rank(&x, r) : &x;
-    acc += remote->ring[phase][i];
-  }
-  return acc;
-}
-// publish + one cluster barrier; returns the ring phase to reduce from.
-template <int N>
-__device__ __forceinline__ uint32_t cluster_publish(cg::cluster_group& cluster, Exchange& x,
-                                                    const u64 (&vals)[N]) {
-  const uint32_t phase = ring_publish<N>(x, vals);
-  if (cluster.num_blocks() > 1) cluster.sync();
-  return phase;
-}
-
-// publish + barrier + read in one call.  out[rank][i].
-template <int N>
-__device__ __forceinline__ void cluster_allgather(cg::cluster_group& cluster, Exchange& x,
-                                                  const u64 (&vals)[N], u64 (&out)[kMaxCluster][N]) {
-  const uint32_t phase = ring_publish<N>(x, vals);
-  if (cluster.num_blocks() > 1) cluster.sync();
-  ring_read<N>(cluster, x, phase, out);
+// Minimum over the first n lanes.
+__device__ __forceinline__ u64 ranks_min(u64 v, unsigned n) {
+  return ~warp_max_u64((threadIdx.x & 31u) < n ? ~v : 0ull);
 }
 
 }  // namespace hs

@@ -48,6 +48,11 @@ struct RowCtx : ClusterCtx {
   int n_local;   // elements in this CTA's slice
   int seg;       // elements per warp in the id-ordered walks (multiple of 32)
   float* stage;  // this CTA's slice: final scores
+  uint32_t turn = 0;  // exchanges so far (see cluster_exchange)
+  template <int N>
+  __device__ __forceinline__ void exchange(const u64 (&vals)[N], u64 (&got)[N]) {
+    cluster_exchange<N>(cluster, *x, turn, vals, got);
+  }
 };
 
 // Every element of the resident fp32 row, for descend_core.
@@ -92,11 +97,10 @@ __device__ void totals_above(RowCtx& c, uint32_t lo_key, float m, bool with_mass
     }
   }
   block_sum2(*c.x, a, b);
-  u64 vals[2] = {a, b};
-  u64 all[kMaxCluster][2];
-  cluster_allgather<2>(c.cluster, *c.x, vals, all);
-  cnt = mass = 0;
-  for (unsigned r = 0; r < c.nranks; ++r) { cnt += all[r][0]; mass += all[r][1]; }
+  u64 vals[2] = {a, b}, got[2];
+  c.exchange<2>(vals, got);
+  cnt = warp_sum_u64(got[0]);
+  mass = warp_sum_u64(got[1]);
 }
 
 // Global id of the t-th (1-based) element, in ascending id order, whose key equals `key`.
@@ -109,14 +113,11 @@ __device__ int find_tth_equal(RowCtx& c, uint32_t key, u64 t) {
   const u64 wtot = warp_sum_u64(mine);
   u64 pre, pre_unused, tot, tot_unused;
   block_warp_prefix2(*c.x, wtot, 0, pre, pre_unused, tot, tot_unused);
-  u64 vals[1] = {tot};
-  u64 all[kMaxCluster][1];
-  cluster_allgather<1>(c.cluster, *c.x, vals, all);
-  u64 cta_pre = 0;
-  for (unsigned r = 0; r < c.rank; ++r) cta_pre += all[r][0];
+  u64 vals[1] = {tot}, got[1];
+  c.exchange<1>(vals, got);
   if (threadIdx.x == 0) c.x->bcast[6] = 0;
   __syncthreads();
-  const u64 before = cta_pre + pre;
+  const u64 before = ranks_below(got[0], c.rank) + pre;
   if (before < t && t <= before + wtot) {  // this warp holds the t-th
     u64 running = before;
     for (int i0 = w0; i0 < w1; i0 += 32) {
@@ -135,11 +136,9 @@ __device__ int find_tth_equal(RowCtx& c, uint32_t key, u64 t) {
   }
   __syncthreads();
   u64 v2[1] = {c.x->bcast[6]};
-  cluster_allgather<1>(c.cluster, *c.x, v2, all);
-  int result = 0x7fffffff;
-  for (unsigned r = 0; r < c.nranks; ++r)
-    if (all[r][0]) result = (int)(all[r][0] - 1);
-  return result;
+  c.exchange<1>(v2, got);
+  const u64 found = warp_max_u64(got[0]);  // (id + 1, on the one rank that has it)
+  return found ? (int)(found - 1) : 0x7fffffff;
 }
 
 // arg max over the kept set of fl(fl(e / z) / noise), lowest id on ties: what
@@ -157,18 +156,18 @@ __device__ int draw_with_noise(RowCtx& c, const KeptSet& kept, float m, float zf
     best = packed > best ? packed : best;
   }
   best = block_max_u64(*c.x, best);
-  u64 vals[1] = {best};
-  u64 all[kMaxCluster][1];
-  cluster_allgather<1>(c.cluster, *c.x, vals, all);
-  for (unsigned r = 0; r < c.nranks; ++r) best = all[r][0] > best ? all[r][0] : best;
+  u64 vals[1] = {best}, got[1];
+  c.exchange<1>(vals, got);
+  best = warp_max_u64(got[0]);
   return (int)(~(uint32_t)(best & 0xffffffffu));
 }
 
 
 // Inverse CDF over the kept set in ascending id order: the first kept element at which the
 // running integer mass exceeds `target` (0 <= target < total kept mass), or -1.  Thread t adds up
-// elements [t, t + 1) * run of the slice (run is odd: the threads' reads fall on different banks),
-// and the warp that owns the run with the target in it looks into it.
+// elements [t, t + 1) * run of the slice (run is odd: the threads' reads fall on different banks);
+// it first marks the kept ones of 32 at a time, so that a warp spends an exponential per kept
+// element and not per element.  The warp that owns the run with the target in it looks into it.
 __device__ int draw_inverse_cdf(RowCtx& c, const KeptSet& kept, float m, u64 target) {
   const int tid = threadIdx.x, lane = tid & 31;
   const int run = ((c.n_local + kThreads - 1) / kThreads) | 1;
@@ -178,17 +177,23 @@ __device__ int draw_inverse_cdf(RowCtx& c, const KeptSet& kept, float m, u64 tar
     return kept.has(key_of(s), c.base + i) ? mass_of(s, m) : 0ull;
   };
   u64 mine = 0;
-  for (int i = r0; i < r1; ++i) mine += mass_at(i);
+  for (int b = r0; b < r1; b += 32) {
+    uint32_t marks = 0;
+    const int n = min(32, r1 - b);
+#pragma unroll 8
+    for (int j = 0; j < n; ++j) marks |= (kept.has(key_of(c.stage[b + j]), c.base + b + j) ? 1u : 0u) << j;
+    while (marks) {
+      const int j = __ffs(marks) - 1;
+      marks &= marks - 1;
+      mine += mass_of(c.stage[b + j], m);
+    }
+  }
   const u64 incl = warp_scan_u64(mine);
   u64 pre, pu, tot, tu;
   block_warp_prefix2(*c.x, shfl_u64(incl, 31), 0, pre, pu, tot, tu);
-  u64 vals[1] = {tot};
-  u64 all[kMaxCluster][1];
-  cluster_allgather<1>(c.cluster, *c.x, vals, all);
-  u64 before = pre + incl - mine;
-#pragma unroll
-  for (unsigned r = 0; r < (unsigned)kMaxCluster; ++r)
-    if (r < c.rank) before += all[r][0];
+  u64 vals[1] = {tot}, got[1];
+  c.exchange<1>(vals, got);
+  const u64 before = ranks_below(got[0], c.rank) + pre + incl - mine;
   if (tid == 0) c.x->bcast[6] = 0;
   __syncthreads();
   const uint32_t votes = __ballot_sync(0xffffffffu, before <= target && target < before + mine);
@@ -209,8 +214,8 @@ __device__ int draw_inverse_cdf(RowCtx& c, const KeptSet& kept, float m, u64 tar
   }
   __syncthreads();
   u64 v2[1] = {c.x->bcast[6]};
-  const uint32_t phase = cluster_publish<1>(c.cluster, *c.x, v2);
-  return (int)ring_reduce<RingOp::Max>(c.cluster, *c.x, phase, 0) - 1;
+  c.exchange<1>(v2, got);
+  return (int)warp_max_u64(got[0]) - 1;
 }
 
 // ---- the one histogram ------------------------------------------------------------------
@@ -225,24 +230,30 @@ struct BucketHit {
   u64 above_cnt, above_mass, bin_cnt, bin_mass;
 };
 // Fills the merged histogram: afterwards rank r holds buckets [r, r + 1) * kResBuckets / nranks
-// in red_cnt / red_mass, and every CTA knows every rank's totals (seg_cnt / seg_mass).
-__device__ void res_histogram(RowCtx& c, const ResHist& rh, float m, u64 (&seg)[kMaxCluster][2]) {
+// in red_cnt / red_mass, and lane r of every warp holds rank r's totals in `seg`.
+__device__ void res_histogram(RowCtx& c, const ResHist& rh, float m, u64 (&seg)[2]) {
   uint32_t* cnt = reinterpret_cast<uint32_t*>(c.hist);
   const int tid = threadIdx.x;
   for (int b = tid; b < 4 * kResBuckets; b += kThreads) cnt[b] = 0;
   __syncthreads();
-#pragma unroll 2
-  for (int i = tid; i < c.n_local; i += kThreads) {
-    const float s = c.stage[i];
+  auto take = [&](float s) {
     const int b = rh.bucket(s);
     atomicAdd(&cnt[b], 1u);
-    if (s - m < -29.0f) continue;  // (rounds to no mass at all)
-    const u64 q = mass_of(s, m);
+    const u64 q = mass_of(s, m);  // (0 from 28.4 below the maximum on)
     const uint32_t a0 = (uint32_t)q & kLimbMask, a1 = (uint32_t)(q >> kLimbBits) & kLimbMask, a2 = (uint32_t)(q >> (2 * kLimbBits));
     if (a0) atomicAdd(&cnt[kResBuckets + b], a0);
     if (a1) atomicAdd(&cnt[2 * kResBuckets + b], a1);
     if (a2) atomicAdd(&cnt[3 * kResBuckets + b], a2);
+  };
+  int i = tid;
+  for (; i + 3 * kThreads < c.n_local; i += 4 * kThreads) {
+    float s[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) s[u] = c.stage[i + u * kThreads];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) take(s[u]);
   }
+  for (; i < c.n_local; i += kThreads) take(c.stage[i]);
   c.sync_all();
   const int per = kResBuckets / (int)c.nranks;
   u64 tc = 0, tm = 0;
@@ -265,45 +276,67 @@ __device__ void res_histogram(RowCtx& c, const ResHist& rh, float m, u64 (&seg)[
   }
   block_sum2(*c.x, tc, tm);
   u64 vals[2] = {tc, tm};
-  cluster_allgather<2>(c.cluster, *c.x, vals, seg);
+  c.exchange<2>(vals, seg);
 }
 // The bucket, from the top, at which the running count (or mass) reaches `want` (>= 1, at most the
 // total).  Every CTA works it out for itself; no barrier between CTAs.
 template <bool BY_MASS>
-__device__ BucketHit res_find(RowCtx& c, const u64 (&seg)[kMaxCluster][2], u64 want) {
-  u64 ac = 0, am = 0;
-  unsigned r = c.nranks - 1;
-#pragma unroll
-  for (int k = kMaxCluster - 1; k > 0; --k) {
-    if ((unsigned)k > r) continue;                              // (ranks from the top down)
-    if (want <= (BY_MASS ? am + seg[k][1] : ac + seg[k][0])) break;
-    ac += seg[k][0];
-    am += seg[k][1];
-    r = (unsigned)k - 1u;
-  }
+__device__ BucketHit res_find(RowCtx& c, const u64 (&seg)[2], u64 want) {
   const int per = kResBuckets / (int)c.nranks, lane = threadIdx.x & 31;
   __syncthreads();
   if (threadIdx.x < 32) {
+    // the rank: what lies above rank r is the total less the ranks up to r
+    const u64 ic = warp_scan_u64(seg[0]), im = warp_scan_u64(seg[1]);
+    const u64 over_c = shfl_u64(ic, 31) - ic, over_m = shfl_u64(im, 31) - im;
+    const u64 over = BY_MASS ? over_m : over_c;
+    const uint32_t here = __ballot_sync(0xffffffffu, over < want && want <= over + seg[BY_MASS ? 1 : 0]);
+    const unsigned r = here ? (unsigned)(__ffs(here) - 1) : 0u;
+    u64 ac = shfl_u64(over_c, (int)r), am = shfl_u64(over_m, (int)r);
     const uint32_t* rc = c.nranks > 1 ? c.cluster.map_shared_rank(c.red_cnt, r) : c.red_cnt;
     const u64* rm = c.nranks > 1 ? c.cluster.map_shared_rank(c.red_mass, r) : c.red_mass;
-    bool found = false;
-    for (int hi = per - 1; hi >= 0 && !found; hi -= 32) {
-      const int b = hi - lane;
-      const u64 n = b >= 0 ? rc[b] : 0ull, q = b >= 0 ? rm[b] : 0ull;
-      const u64 in = warp_scan_u64(n), iq = warp_scan_u64(q);
-      const uint32_t votes = __ballot_sync(0xffffffffu, want <= (BY_MASS ? am + iq : ac + in));
-      if (votes) {
-        found = true;
-        if (lane == __ffs(votes) - 1) {
-          c.x->bcast[0] = (u64)((int)r * per + b);
-          c.x->bcast[1] = ac + in - n;
-          c.x->bcast[2] = am + iq - q;
-          c.x->bcast[3] = n;
-          c.x->bcast[4] = q;
+    // its buckets: lane l owns per / 32 consecutive ones (a multiple of four), the highest lane 0
+    const int mine = per >> 5, first = per - mine * (lane + 1);
+    u64 sn = 0, sq = 0;
+    uint4 n4 = make_uint4(0, 0, 0, 0);
+    ulonglong2 qa = make_ulonglong2(0, 0), qb = qa;
+    for (int u = 0; u < mine; u += 4) {
+      n4 = *reinterpret_cast<const uint4*>(rc + first + u);
+      qa = *reinterpret_cast<const ulonglong2*>(rm + first + u);
+      qb = *reinterpret_cast<const ulonglong2*>(rm + first + u + 2);
+      sn += (u64)n4.x + n4.y + n4.z + n4.w;
+      sq += qa.x + qa.y + qb.x + qb.y;
+    }
+    const u64 in = warp_scan_u64(sn), iq = warp_scan_u64(sq);
+    const uint32_t votes = __ballot_sync(0xffffffffu, want <= (BY_MASS ? am + iq : ac + in));
+    if (lane == __ffs(votes) - 1) {
+      ac += in - sn;
+      am += iq - sq;
+      for (int u = mine - 4; u >= 0; u -= 4) {
+        if (mine > 4) {  // (else the four are at hand)
+          n4 = *reinterpret_cast<const uint4*>(rc + first + u);
+          qa = *reinterpret_cast<const ulonglong2*>(rm + first + u);
+          qb = *reinterpret_cast<const ulonglong2*>(rm + first + u + 2);
         }
+        const uint32_t n[4] = {n4.x, n4.y, n4.z, n4.w};
+        const u64 q[4] = {qa.x, qa.y, qb.x, qb.y};
+        bool done = false;
+#pragma unroll
+        for (int k = 3; k >= 0; --k) {
+          if (done) continue;
+          if (want <= (BY_MASS ? am + q[k] : ac + n[k])) {
+            c.x->bcast[0] = (u64)((int)r * per + first + u + k);
+            c.x->bcast[1] = ac;
+            c.x->bcast[2] = am;
+            c.x->bcast[3] = n[k];
+            c.x->bcast[4] = q[k];
+            done = true;
+          } else {
+            ac += n[k];
+            am += q[k];
+          }
+        }
+        if (done) break;
       }
-      ac += shfl_u64(in, 31);
-      am += shfl_u64(iq, 31);
     }
   }
   __syncthreads();
@@ -311,6 +344,23 @@ __device__ BucketHit res_find(RowCtx& c, const u64 (&seg)[kMaxCluster][2], u64 w
   __syncthreads();
   return h;
 }
+
+// The CTAs' lists (lane r of every warp holds the length of rank r's) one behind the other into
+// dst: one remote read per entry, all side by side.
+__device__ __forceinline__ void res_collect(RowCtx& c, u64* list, u64 len, int total, u64* dst) {
+  for (int i0 = threadIdx.x & ~31; i0 < total; i0 += kThreads) {
+    const int i = i0 + (threadIdx.x & 31);
+    int at = i;
+    unsigned r = 0;
+    for (unsigned k = 0; k + 1 < c.nranks; ++k) {
+      const int n = (int)shfl_u64(len, (int)k);
+      if (r == k && at >= n) { at -= n; r = k + 1; }
+    }
+    if (i < total) dst[i] = (c.nranks > 1 ? c.cluster.map_shared_rank(list, r) : list)[at];
+  }
+}
+// Entries in all lists (a list that ran over counts as very long).
+__device__ __forceinline__ int res_total(u64 len) { return (int)warp_sum_u64(min(len, (u64)1 << 20)); }
 
 // All elements `take(score)` names, from all slices, sorted by (score descending, id ascending), in
 // every CTA's own copy; returns how many, or -1 when they are more than a list holds.  `first` =
@@ -324,30 +374,24 @@ __device__ int res_gather(RowCtx& c, bool& first, Take&& take) {
   first = false;
   if (threadIdx.x == 0) *n_at = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < c.n_local; i += kThreads) {
-    const float s = c.stage[i];
-    if (!take(s, c.base + i)) continue;
-    const int slot = atomicAdd(n_at, 1);
-    if (slot < kResList) list[slot] = cand_pack(key_of(s), c.base + i);
+  for (int i0 = threadIdx.x; i0 < c.n_local; i0 += 4 * kThreads) {
+    float s[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) s[u] = i0 + u * kThreads < c.n_local ? c.stage[i0 + u * kThreads] : 0.f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * kThreads;
+      if (i >= c.n_local || !take(s[u], c.base + i)) continue;
+      const int slot = atomicAdd(n_at, 1);
+      if (slot < kResList) list[slot] = cand_pack(key_of(s[u]), c.base + i);
+    }
   }
   __syncthreads();
-  u64 vals[1] = {(u64)*n_at};
-  u64 all[kMaxCluster][1];
-  cluster_allgather<1>(c.cluster, *c.x, vals, all);
-  int total = 0;
-#pragma unroll
-  for (unsigned r = 0; r < (unsigned)kMaxCluster; ++r)
-    if (r < c.nranks) total += (int)min(all[r][0], (u64)1 << 20);
+  u64 vals[1] = {(u64)*n_at}, len[1];
+  c.exchange<1>(vals, len);
+  const int total = res_total(len[0]);
   if (total > kResList) return -1;
-  int at = 0;
-#pragma unroll
-  for (unsigned r = 0; r < (unsigned)kMaxCluster; ++r) {
-    if (r >= c.nranks) break;
-    const u64* theirs = c.nranks > 1 ? c.cluster.map_shared_rank(list, r) : list;
-    const int n = (int)all[r][0];
-    for (int i = threadIdx.x; i < n; i += kThreads) members[at + i] = theirs[i];
-    at += n;
-  }
+  res_collect(c, list, len[0], total, members);
   __syncthreads();
   CandCtx L{members, nullptr, nullptr, nullptr, nullptr, nullptr};
   cand_sort(L, total);
@@ -432,6 +476,8 @@ __device__ uint32_t slice_bound(RowCtx& c, uint32_t thread_max, int j) {
 }
 
 // ---- the kernel -----------------------------------------------------------------------
+// ON_CHIP: the slices are in shared memory (else in global scratch).
+template <bool ON_CHIP>
 __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant__ RowKernelArgs a,
                                                           const __grid_constant__ InlineRows inl) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -460,8 +506,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
   off += sizeof(uint32_t) * (kBins / c.nranks);
   off = (off + 15) & ~size_t(15);
   unsigned char* on_chip = smem_raw + off;
-  c.stage = a.gstage ? a.gstage + (size_t)c.row * ((size_t)a.slice * c.nranks) + c.base : reinterpret_cast<float*>(on_chip);
-  if (threadIdx.x == 0) c.x->ring_phase = 0;
+  if constexpr (ON_CHIP) c.stage = reinterpret_cast<float*>(on_chip);
+  else c.stage = a.gstage + (size_t)c.row * ((size_t)a.slice * c.nranks) + c.base;
   cudaGridDependencySynchronize();  // (the histograms are up to date from here on)
   __syncthreads();
 
@@ -471,13 +517,17 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
   const bool slot_ok = P.slot >= 0 && P.slot < a.pool.slots_total;
   const bool penalised = slot_ok && (P.repetition_penalty != 1.0f || P.presence_penalty != 0.0f ||
                                      P.frequency_penalty != 0.0f);
+  // (in registers: the compiler cannot know that storing a score leaves P alone)
+  const float rp = P.repetition_penalty, pp = P.presence_penalty, fp = P.frequency_penalty;
+  const float T = P.temperature;
+  const bool divide = !greedy && T != 1.0f;
   auto score = [&](float v, int count) {
     if (count > 0) {
-      v = v < 0.0f ? __fmul_rn(v, P.repetition_penalty) : __fdiv_rn(v, P.repetition_penalty);
-      v = __fsub_rn(v, P.presence_penalty);
-      v = __fsub_rn(v, __fmul_rn(P.frequency_penalty, (float)count));
+      v = v < 0.0f ? __fmul_rn(v, rp) : __fdiv_rn(v, rp);
+      v = __fsub_rn(v, pp);
+      v = __fsub_rn(v, __fmul_rn(fp, (float)count));
     }
-    if (!greedy && P.temperature != 1.0f) v = __fdiv_rn(v, P.temperature);
+    if (divide) v = __fdiv_rn(v, T);
     return canonical(v);
   };
 
@@ -568,11 +618,11 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
   uint32_t bound = 0;
   if (candidate) bound = slice_bound(c, top_key, (P.top_k + (int)c.nranks - 1) / (int)c.nranks);
   {
-    u64 vals[3] = {best, (u64)low_key, (u64)bound};
-    const uint32_t phase = cluster_publish<3>(c.cluster, *c.x, vals);
-    best = ring_reduce<RingOp::Max>(c.cluster, *c.x, phase, 0);
-    low_key = (uint32_t)ring_reduce<RingOp::Min>(c.cluster, *c.x, phase, 1);
-    bound = (uint32_t)ring_reduce<RingOp::Min>(c.cluster, *c.x, phase, 2);
+    u64 vals[3] = {best, (u64)low_key, (u64)bound}, got[3];
+    c.exchange<3>(vals, got);
+    best = warp_max_u64(got[0]);
+    low_key = (uint32_t)ranks_min(got[1], c.nranks);
+    bound = (uint32_t)ranks_min(got[2], c.nranks);
   }
   const uint32_t max_key = (uint32_t)(best >> 32);
   const int argmax_id = (int)(~(uint32_t)(best & 0xffffffffu));
@@ -584,24 +634,27 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
   if (candidate) {
     u64* list = reinterpret_cast<u64*>(c.hist);
     int* n_at = reinterpret_cast<int*>(&c.x->bcast[7]);
-    u64 lens[kMaxCluster][1];
+    u64 len[1];
     int total = 0;
     for (int attempt = 0; attempt < 2; ++attempt) {
       if (tid == 0) *n_at = 0;
       __syncthreads();
-      for (int i = tid; i < c.n_local; i += kThreads) {
-        const uint32_t k = key_of(c.stage[i]);
-        if (k < bound) continue;
-        const int slot = atomicAdd(n_at, 1);
-        if (slot < kCandCap) list[slot] = cand_pack(k, c.base + i);
+      for (int i0 = tid; i0 < c.n_local; i0 += 4 * kThreads) {
+        uint32_t k[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) k[u] = i0 + u * kThreads < c.n_local ? key_of(c.stage[i0 + u * kThreads]) : 0u;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + u * kThreads;
+          if (i >= c.n_local || k[u] < bound) continue;
+          const int slot = atomicAdd(n_at, 1);
+          if (slot < kCandCap) list[slot] = cand_pack(k[u], c.base + i);
+        }
       }
       __syncthreads();
       u64 vals[1] = {(u64)*n_at};
-      cluster_allgather<1>(c.cluster, *c.x, vals, lens);
-      total = 0;
-#pragma unroll
-      for (unsigned r = 0; r < (unsigned)kMaxCluster; ++r)
-        if (r < c.nranks) total += (int)min(lens[r][0], (u64)1 << 20);
+      c.exchange<1>(vals, len);
+      total = res_total(len[0]);
       if (total <= kCandCap || attempt == 1) break;
       // (values that lie unevenly over the slices: once more from the exact k-th highest key)
       const Selection sk = descend<false, false>(c, 0u, (u64)P.top_k, 1.0f, m);
@@ -611,16 +664,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
     if (total <= kCandCap) {
       if (c.rank == 0) {
         u64* merged = reinterpret_cast<u64*>(on_chip);  // (the slice has served)
-        int at = 0;
         __syncthreads();
-#pragma unroll
-        for (unsigned r = 0; r < (unsigned)kMaxCluster; ++r) {
-          if (r >= c.nranks) break;
-          const u64* theirs = c.nranks > 1 ? c.cluster.map_shared_rank(list, r) : list;
-          const int n = (int)lens[r][0];
-          for (int i = tid; i < n; i += kThreads) merged[at + i] = theirs[i];
-          at += n;
-        }
+        res_collect(c, list, len[0], total, merged);
       }
       c.sync_all();  // (the lists have been read: the other CTAs may leave)
       if (c.rank != 0) return;
@@ -676,14 +721,13 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
     const float range = m - rh.lo;
     bool hist_ok = range > 0.f && range < 3.0e38f;
     rh.scale = hist_ok ? __fdiv_rn((float)kResBuckets - 0.5f, range) : 0.f;
-    u64 seg[kMaxCluster][2];
+    u64 seg[2] = {0, 0};
     u64 cnt = 0, mass = 0;
     bool first = true;
     if (hist_ok) {
       res_histogram(c, rh, m, seg);
-#pragma unroll
-      for (unsigned r = 0; r < (unsigned)kMaxCluster; ++r)
-        if (r < c.nranks) { cnt += seg[r][0]; mass += seg[r][1]; }
+      cnt = warp_sum_u64(seg[0]);
+      mass = warp_sum_u64(seg[1]);
     } else {
       totals_above(c, 0u, m, true, cnt, mass);
     }
@@ -762,9 +806,9 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
           if (k >= kept.cut_key && k < lowest && !(__fdiv_rn(expf(s - m), z1) < thr)) lowest = k;
         }
         lowest = ~block_max_u32(*c.x, ~lowest);
-        u64 vals[1] = {(u64)lowest};
-        const uint32_t phase = cluster_publish<1>(c.cluster, *c.x, vals);
-        lowest = (uint32_t)ring_reduce<RingOp::Min>(c.cluster, *c.x, phase, 0);
+        u64 vals[1] = {(u64)lowest}, got[1];
+        c.exchange<1>(vals, got);
+        lowest = (uint32_t)ranks_min(got[0], c.nranks);
         first = true;
         if (lowest != 0xffffffffu && lowest > kept.cut_key) {
           kept.cut_key = lowest;

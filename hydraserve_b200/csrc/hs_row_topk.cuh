@@ -514,14 +514,21 @@ __device__ int topk_candidates(Ctx3& c, CandCtx& L, int k) {
 // A compare-exchange step of stride <= 32 stays inside the 64 entries one warp handles, so
 // only the wider steps (and the changes between the two kinds) need the block barrier.
 __device__ void cand_sort(CandCtx& L, int n) {
-  if (n <= 128) {
-    // short list: every entry counts the entries above it (entries are distinct: they end
-    // in the token id) and moves to that position
+  if (n <= kThreads) {
+    // one entry per thread: every entry counts the entries above it (entries are distinct: they
+    // end in the token id) and moves to that position
     const int i = threadIdx.x;
     const u64 mine = i < n ? L.cand[i] : 0ull;
     int rank = 0;
-    if (i < n)
-      for (int j = 0; j < n; ++j) rank += L.cand[j] > mine ? 1 : 0;
+    if ((i & ~31) < n) {
+      const ulonglong2* two = reinterpret_cast<const ulonglong2*>(L.cand);
+#pragma unroll 4
+      for (int j = 0; j < n / 2; ++j) {
+        const ulonglong2 o = two[j];
+        rank += (o.x > mine) + (o.y > mine);
+      }
+      if (n & 1) rank += L.cand[n - 1] > mine;
+    }
     __syncthreads();
     if (i < n) L.cand[rank] = mine;
     __syncthreads();
