@@ -782,6 +782,20 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
   const auto* params = reinterpret_cast<const hs_row_params*>(h->h_block);
   const bool counting = d->n_resets > 0 || d->n_appends > 0;
   const bool singles = d->n_resets == 0 && d->n_appends > 0 && d->max_tokens == 1 && !d->repeats;
+  // a slot that is emptied and then filled again is one entry of the build (the two lists are in
+  // the same order); what is only emptied stays in the list of resets
+  int n_alone = 0;
+  if (d->n_resets) {
+    auto* resets = reinterpret_cast<int32_t*>(h->h_block + d->resets_at);
+    auto* slots = reinterpret_cast<int32_t*>(h->h_block + d->slots_at);
+    int j = 0;
+    for (int i = 0; i < d->n_resets; ++i) {
+      int k = j;
+      while (!d->repeats && k < d->n_appends && slots[k] != resets[i]) ++k;
+      if (!d->repeats && k < d->n_appends) { slots[k] |= hs::kResetFirst; j = k + 1; }
+      else resets[n_alone++] = resets[i];
+    }
+  }
   const bool rows_inline = batch <= hs::kInlineRows;
   const bool appends_inline = singles && d->n_appends <= hs::kInlineAppends;
   if (!rows_inline || (counting && !appends_inline)) {
@@ -819,14 +833,25 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
     h->launches += 1;
     behind = true;
   } else {
-    if (d->n_resets) {
-      hs::slots_reset_kernel<<<d->n_resets, 256, 0, stream>>>(
-          h->pool, reinterpret_cast<const int32_t*>(h->d_block + d->resets_at), d->n_resets);
+    if (n_alone) {
+      hs::slots_reset_kernel<<<n_alone, 256, 0, stream>>>(
+          h->pool, reinterpret_cast<const int32_t*>(h->d_block + d->resets_at), n_alone);
       HS_CUDA(h, cudaGetLastError());
       h->launches += 1;
     }
-    rc = launch_append(h, d_tokens, d_offsets, d_slots, d->n_appends, vocab, d->max_tokens, stream);
-    if (rc != HS_OK) return rc;
+    if (d->n_appends && d->repeats) {
+      rc = launch_append(h, d_tokens, d_offsets, d_slots, d->n_appends, vocab, d->max_tokens, stream);
+      if (rc != HS_OK) return rc;
+    } else if (d->n_appends) {
+      // one token per thread, as long as the CTAs are few enough to run side by side
+      int c = 1;
+      while (c < hs::kMaxCluster && c * hs::kBuildThreads < d->max_tokens && d->n_appends * c < 2 * h->sm_count) c *= 2;
+      HS_CUDA(h, launch(hs::slots_build_kernel, dim3((unsigned)c, (unsigned)d->n_appends), hs::kBuildThreads, 0, stream,
+                        LaunchAttrs(c, false), h->pool,
+                        reinterpret_cast<int32_t*>(h->d_block + d->tokens_at), d_offsets, d_slots, d->n_appends, vocab));
+      h->launches += 1;
+      behind = true;
+    }
   }
   hs::InlineRows inl;
   if (rows_inline) std::memcpy(inl.p, params, (size_t)batch * sizeof(hs_row_params));

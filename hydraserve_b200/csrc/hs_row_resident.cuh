@@ -225,6 +225,17 @@ struct ResHist {
     return min(max(__float2int_rz((s - lo) * scale), 0), kResBuckets - 1);
   }
 };
+// Scores that can be in buckets [first, last], with a bucket's width to spare on either side: two
+// comparisons instead of a bucket number per element.
+struct ResRange {
+  float from, to;
+  __device__ __forceinline__ ResRange(const ResHist& h, int first, int last) {
+    const float width = __fdiv_rn(1.0f, h.scale);
+    from = first <= 0 ? __int_as_float(0xff800000) : h.lo + ((float)first - 1.0f) * width;
+    to = last >= kResBuckets - 1 ? __int_as_float(0x7f800000) : h.lo + ((float)last + 2.0f) * width;
+  }
+  __device__ __forceinline__ bool near(float s) const { return !(s < from || s > to); }  // (a NaN may be)
+};
 struct BucketHit {
   int bucket;
   u64 above_cnt, above_mass, bin_cnt, bin_mass;
@@ -550,6 +561,25 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
       c.stage[i] = v;
       note(v, i);
     };
+    // four neighbours at once: the common case (none of them in the history, no NaN) without a
+    // branch per token, one 128-bit store
+    auto put4 = [&](const float4& w, uint32_t cl, int i) {
+      if ((cl & 0xffu) == 0u) {
+        const float4 v = make_float4(score(canonical(w.x), 0), score(canonical(w.y), 0), score(canonical(w.z), 0), score(canonical(w.w), 0));
+        const uint32_t k0 = key_of(v.x), k1 = key_of(v.y), k2 = key_of(v.z), k3 = key_of(v.w);
+        const uint32_t hi = max(max(k0, k1), max(k2, k3)), lo = min(min(k0, k1), min(k2, k3));
+        if (hi <= 0xff800000u && lo >= 0x007fffffu) {  // (keys of +inf and -inf)
+          *reinterpret_cast<float4*>(c.stage + i) = v;
+          low_key = min(low_key, lo);
+          if (hi > top_key) {
+            top_key = hi;
+            top_at = i + (k0 == hi ? 0 : (k1 == hi ? 1 : (k2 == hi ? 2 : 3)));
+          }
+          return;
+        }
+      }
+      put(w.x, cl & 3u, i); put(w.y, (cl >> 2) & 3u, i + 1); put(w.z, (cl >> 4) & 3u, i + 2); put(w.w, (cl >> 6) & 3u, i + 3);
+    };
     if (a.dtype == HS_DTYPE_BF16) {
       const unsigned short* src = reinterpret_cast<const unsigned short*>(a.logits) + gofs;
 #pragma unroll 4
@@ -563,7 +593,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
       const bool vec = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
       const int n4 = vec ? c.n_local / 4 : 0;
       const float4* src4 = reinterpret_cast<const float4*>(src);
-      constexpr int kFlight = 4;  // 128-bit loads in flight per thread
+      constexpr int kFlight = 6;  // 128-bit loads in flight per thread
       for (int i0 = tid; i0 < n4; i0 += kFlight * kThreads) {
         float4 w[kFlight];
         uint32_t cl[kFlight];
@@ -581,8 +611,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
         for (int u = 0; u < kFlight; ++u) {
           const int i = i0 + u * kThreads;
           if (i >= n4) break;
-          put(w[u].x, cl[u] & 3u, 4 * i); put(w[u].y, (cl[u] >> 2) & 3u, 4 * i + 1);
-          put(w[u].z, (cl[u] >> 4) & 3u, 4 * i + 2); put(w[u].w, (cl[u] >> 6) & 3u, 4 * i + 3);
+          put4(w[u], cl[u], 4 * i);
         }
       }
 #pragma unroll 8
@@ -741,7 +770,9 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
       if (hist_ok) {
         const BucketHit h = res_find<BY_MASS>(c, seg, want);
         const bool with_top = BY_MASS;  // (the last cut: the top-N come along in the same gather)
+        const ResRange range_of(rh, h.bucket, with_top && top_bucket < kResBuckets ? kResBuckets - 1 : h.bucket);
         const int n = res_gather(c, first, [&](float s, int) {
+          if (!range_of.near(s)) return false;
           const int b = rh.bucket(s);
           return (b == h.bucket && key_of(s) >= lo_key) || (with_top && b >= top_bucket);
         });
@@ -845,7 +876,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
     if (n_want_all > 0 && n_top_list < 0) {
       const int n_want = (int)min((u64)n_want_all, n_kept);
       if (hist_ok) {
-        n_top_list = res_gather(c, first, [&](float s, int) { return rh.bucket(s) >= top_bucket; });
+        const ResRange range_of(rh, top_bucket, kResBuckets - 1);
+        n_top_list = res_gather(c, first, [&](float s, int) { return range_of.near(s) && rh.bucket(s) >= top_bucket; });
       }
       if (n_top_list < 0) {
         hist_ok = false;
