@@ -25,7 +25,8 @@ namespace {
 
 using hs::u64;
 
-constexpr int kMaxSplit = 4;  // CTAs per row on the candidate path
+constexpr int kMaxParts = 16;  // CTAs per counting row
+constexpr int kMaxSplit = 8;   // CTAs per candidate row: the parts' lists, top_k entries and ties each, meet in one list
 constexpr int kSideCapMax = 16384;  // side-list entries a CTA can keep in global scratch
 
 struct DeviceGuard {
@@ -75,16 +76,16 @@ struct hs_sampler {
   int force_split = 0;    // CTAs per candidate row (0 = chosen per call)
   int force_csplit = 0;   // CTAs per counting row (0 = chosen per call)
   int token_draw = 1;     // near-flat counting rows draw by rejection on tokens
-  int ctab_tables = 0;    // count tables the hand-over scratch holds
+  int ctab_tables = 0;    // parts of counting rows the hand-over scratch holds
   uint32_t* ctab = nullptr;   // [ctab_tables, kCells]
   int2* crare = nullptr;      // [ctab_tables, kV3RareCap]
-  int* crare_n = nullptr;     // [ctab_tables]
+  int2* crare_n = nullptr;    // [ctab_tables]
+  int split_tables = 0;   // parts of candidate rows
   int* count_ticket = nullptr;  // [batch_max]
   int resident_bf16 = 0;  // CTAs of the bf16 kernel that can be resident at once: CTAs per SM x SMs
   int2* side_pair = nullptr;  // [resident_bf16, side_cap] side lists too long for shared memory
-  hs::ClassPacked* clist = nullptr;  // [resident_bf16, kCells] class list of the row a CTA works on
   int* scratch_busy = nullptr;  // [resident_bf16] which of those scratch sets are in use
-  unsigned long long* split_lists = nullptr;  // [batch_max, kMaxSplit, kSplitCap]
+  unsigned long long* split_lists = nullptr;  // [split_tables, kSplitCap], a list per part
   int* split_n = nullptr;
   int* split_ticket = nullptr;
   int side_cap = 0;
@@ -236,12 +237,19 @@ cudaError_t launch(void (*kernel)(Params...), dim3 grid, int threads, size_t sme
   return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
 
+int n_count_of(const hs_row_params* params, int batch, int vocab) {
+  int n = 0;
+  for (int r = 0; r < batch; ++r) n += hs::is_candidate_row(params[r], vocab) ? 0 : 1;
+  return n;
+}
+
 const hs::InlineRows kNoInlineRows{};  // (stands in when the parameters are in device memory)
 
-// `params` in device memory, or null with the rows' parameters in `inl`; `behind`: the launch before
+// `params` in device memory, or null with the rows' parameters in `inl`; n_count: how many rows are
+// not candidate rows, or -1 when the host does not know; `behind`: the launch before
 // this one on the stream is one of this sampler's histogram kernels.
 int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
-                const hs_row_params* params, const hs::InlineRows& inl, hs_row_out* out, const float* noise,
+                const hs_row_params* params, const hs::InlineRows& inl, int n_count, hs_row_out* out, const float* noise,
                 float* scores_out, int32_t* tokens_out, uint32_t flags, bool behind, cudaStream_t stream) {
   Plan plan;
   hs::RowKernelArgs a{};
@@ -250,22 +258,33 @@ int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride
   a.pool = h->pool; a.flags = flags & HS_SAMPLE_APPEND_TOKEN; a.tokens_out = tokens_out;
   a.token_draw = h->token_draw;
   if (dtype == HS_DTYPE_BF16 && !h->force_general && !(flags & HS_SAMPLE_GENERAL_KERNEL)) {
-    // One launch: a CTA per counting row and per part of a candidate row, two resident per
-    // SM.  Small batches: several CTAs stream each candidate row so that every SM has work.
-    // (as many CTAs per row as fit in one wave, rounded down: a second, partial wave costs more
-    // than idle SMs in the first)
-    int split = h->force_split ? h->force_split : h->resident_bf16 / batch;
-    split = std::max(1, std::min(split, kMaxSplit));
-    if (vocab < split * 2 * hs::kSample) split = 1;
-    // counting rows: as many CTAs per row as the hand-over scratch allows (the whole batch may
-    // be counting rows), so that a small batch still spreads over the SMs
-    int csplit = 1;
-    if (vocab >= 65536) {
-      if ((long long)batch * 4 <= h->ctab_tables) csplit = 4;
-      else if ((long long)batch * 2 <= h->ctab_tables) csplit = 2;
+    // One launch: the parts of the counting rows, then the parts of the candidate rows, two CTAs
+    // resident per SM.  How many rows take which path is known when the parameters come from the
+    // host (n_count >= 0).  Then counting rows, whose last part has a long chain of selections
+    // ahead of it, are cut into as many parts (up to sixteen) as three quarters of a wave hold, into
+    // two as long as that is one wave; candidate rows into what the wave has left, up to eight
+    // (a second, partial wave costs more than idle SMs in the first).  No part is below 8,192 tokens
+    // (16,384, its bound's sample, for a candidate row): shorter ones end with the hand-over.
+    // When the host does not know, every row may be either: four parts or two, as the hand-over
+    // scratch allows, and a wave of candidate parts.
+    const int resident = h->resident_bf16;
+    const bool known = n_count >= 0;
+    int csplit, split;
+    if (known) {
+      const int n_cand = batch - n_count;
+      csplit = std::max(resident * 3 / 4 / std::max(1, n_count), 2 * n_count <= resident ? 2 : 1);
+      csplit = std::max(1, std::min({csplit, kMaxParts, vocab / 8192}));
+      split = (resident - std::min(resident, n_count * csplit)) / std::max(1, n_cand);
+      split = std::max(1, std::min({split, kMaxSplit, vocab / hs::kSample}));
+    } else {
+      csplit = vocab < 65536 ? 1 : (long long)batch * 4 <= h->ctab_tables ? 4 : 2;
+      split = std::max(1, std::min({resident / batch, 4, vocab / (2 * hs::kSample)}));
     }
-    if (h->force_csplit && (long long)batch * h->force_csplit <= h->ctab_tables) csplit = h->force_csplit;
-    hs::RowV3Args a3{a, h->clist, h->side_pair, h->side_cap, h->resident_bf16, h->scratch_busy, h->phase_clocks,
+    if (h->force_csplit) csplit = h->force_csplit;
+    if (h->force_split) split = vocab < h->force_split * 2 * hs::kSample ? 1 : h->force_split;
+    csplit = std::max(1, std::min(csplit, h->ctab_tables / batch));
+    split = std::max(1, std::min(split, h->split_tables / batch));
+    hs::RowV3Args a3{a, h->side_pair, h->side_cap, h->resident_bf16, h->scratch_busy, h->phase_clocks,
                      csplit, h->ctab, h->crare, h->crare_n, h->count_ticket,
                      split, h->split_lists, h->split_n, h->split_ticket, batch};
     const unsigned grid = (unsigned)batch * (unsigned)(csplit + split);
@@ -323,7 +342,7 @@ int launch_append(hs_sampler* h, const int32_t* tokens, const int32_t* offsets, 
 
 void release(hs_sampler* h) {
   cudaFree(h->pool.pairs); cudaFree(h->pool.cls); cudaFree(h->pool.heavy); cudaFree(h->pool.n_heavy); cudaFree(h->pool.n); cudaFree(h->pool.pos);
-  cudaFree(h->side_pair); cudaFree(h->clist); cudaFree(h->scratch_busy);
+  cudaFree(h->side_pair); cudaFree(h->scratch_busy);
   cudaFree(h->ctab); cudaFree(h->crare); cudaFree(h->crare_n); cudaFree(h->count_ticket);
   cudaFree(h->split_lists); cudaFree(h->split_n); cudaFree(h->split_ticket);
   if (h->ev_done) cudaEventDestroy(h->ev_done);
@@ -499,17 +518,17 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
   // scratch of the bf16 kernel, per resident CTA (not per row of the batch)
   h->side_cap = std::min((vocab_max + 7) & ~7, kSideCapMax);
   ok = ok && dmalloc(h, &h->side_pair, (size_t)h->resident_bf16 * h->side_cap * sizeof(int2));
-  ok = ok && dmalloc(h, &h->clist, (size_t)h->resident_bf16 * hs::kCells * sizeof(hs::ClassPacked));
   ok = ok && dmalloc(h, &h->scratch_busy, (size_t)h->resident_bf16 * sizeof(int));
-  // hand-over scratch of counting rows split over several CTAs: two tables per resident CTA
+  // hand-over scratch of rows split over several CTAs: two parts per resident CTA
   h->ctab_tables = 2 * h->resident_bf16;
+  h->split_tables = std::max(2 * h->resident_bf16, 2 * batch_max);
   ok = ok && dmalloc(h, &h->ctab, (size_t)h->ctab_tables * hs::kCells * sizeof(uint32_t));
   ok = ok && dmalloc(h, &h->crare, (size_t)h->ctab_tables * hs::kV3RareCap * sizeof(int2));
-  ok = ok && dmalloc(h, &h->crare_n, (size_t)h->ctab_tables * sizeof(int));
+  ok = ok && dmalloc(h, &h->crare_n, (size_t)h->ctab_tables * sizeof(int2));
   ok = ok && dmalloc(h, &h->count_ticket, (size_t)batch_max * sizeof(int));
   ok = ok && cudaEventCreateWithFlags(&h->ev_done, cudaEventDisableTiming) == cudaSuccess;
-  ok = ok && dmalloc(h, &h->split_lists, (size_t)batch_max * kMaxSplit * hs::kSplitCap * sizeof(unsigned long long));
-  ok = ok && dmalloc(h, &h->split_n, (size_t)batch_max * kMaxSplit * sizeof(int));
+  ok = ok && dmalloc(h, &h->split_lists, (size_t)h->split_tables * hs::kSplitCap * sizeof(unsigned long long));
+  ok = ok && dmalloc(h, &h->split_n, (size_t)h->split_tables * sizeof(int));
   ok = ok && dmalloc(h, &h->split_ticket, (size_t)batch_max * sizeof(int));
   ok = ok && cudaMallocHost(&h->h_params, (size_t)batch_max * sizeof(hs_row_params)) == cudaSuccess;
   ok = ok && cudaMallocHost(&h->h_small, (2 * (size_t)batch_max + 1) * sizeof(int32_t)) == cudaSuccess;
@@ -609,7 +628,7 @@ int hs_sample_ex(hs_sampler* h, const void* logits, int dtype, int64_t row_strid
   DeviceGuard guard(h->device);
   Serial serial(h, (cudaStream_t)stream);
   HS_CUDA(h, serial.status);
-  rc = launch_rows(h, logits, dtype, row_stride, batch, vocab, params, kNoInlineRows, out, noise, scores_out,
+  rc = launch_rows(h, logits, dtype, row_stride, batch, vocab, params, kNoInlineRows, -1, out, noise, scores_out,
                    tokens_out, flags, false, (cudaStream_t)stream);
   if (rc != HS_OK) return rc;
   HS_CUDA(h, serial.done());
@@ -715,7 +734,7 @@ int hs_sample_host(hs_sampler* h, const void* logits, int dtype, int64_t row_str
     if (rc != HS_OK) return rc;
   }
   HS_CUDA(h, cudaMemcpyAsync(h->d_params, h->h_params, (size_t)batch * sizeof(hs_row_params), cudaMemcpyHostToDevice, stream));
-  rc = launch_rows(h, h->d_logits, dtype, vocab, batch, vocab, h->d_params, kNoInlineRows, h->d_out, nullptr, nullptr,
+  rc = launch_rows(h, h->d_logits, dtype, vocab, batch, vocab, h->d_params, kNoInlineRows, n_count_of(h->h_params, batch, vocab), h->d_out, nullptr, nullptr,
                    nullptr, flags, false, stream);
   if (rc != HS_OK) return rc;
   HS_CUDA(h, cudaMemcpyAsync(out, h->d_out, (size_t)batch * sizeof(hs_row_out), cudaMemcpyDeviceToHost, stream));
@@ -858,7 +877,7 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
   // (the records go straight to pinned memory, one burst per row: see write_record)
   rc = launch_rows(h, logits, dtype, row_stride, batch, vocab,
                    rows_inline ? nullptr : reinterpret_cast<const hs_row_params*>(h->d_block), rows_inline ? inl : kNoInlineRows,
-                   h->h_out, nullptr, nullptr, nullptr, 0u, behind, stream);
+                   n_count_of(params, batch, vocab), h->h_out, nullptr, nullptr, nullptr, 0u, behind, stream);
   if (rc != HS_OK) return rc;
   HS_CUDA(h, cudaStreamSynchronize(stream));
   h->have_last = false;  // everything enqueued so far has been waited for

@@ -194,6 +194,23 @@ __device__ __forceinline__ void block_warp_prefix2(Exchange& x, u64 wa, u64 wb, 
   pre_b = eb;
 }
 
+// Where this thread's n entries go when the CTA's threads put theirs one behind the other; total =
+// all of them.  scratch: kWarps ints.  One barrier, before which scratch must not be in use.
+__device__ __forceinline__ int block_place(int* scratch, int n, int& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = n;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += o;
+  }
+  if (lane == 31) scratch[warp] = incl;
+  __syncthreads();
+  const int w = lane < kWarps ? scratch[lane] : 0;
+  total = __reduce_add_sync(0xffffffffu, w);
+  return incl - n + __reduce_add_sync(0xffffffffu, lane < warp ? w : 0);
+}
+
 // ---- cluster primitives --------------------------------------------------------------
 // Every CTA of the cluster publishes up to four 64-bit values (CTA-uniform; thread 0's count);
 // afterwards lane r of EVERY warp holds the values of rank r, lanes beyond the ranks hold zeros: one

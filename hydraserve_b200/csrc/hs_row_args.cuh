@@ -49,7 +49,7 @@ __device__ __forceinline__ void write_record(hs_row_out* out, const hs_row_out& 
 constexpr int kTopKMax = 256;  // largest top_k served by the candidate paths
 
 // Rows whose candidates (the top_k highest scores and the ties of the last) make a short list.
-__device__ __forceinline__ bool is_candidate_row(const hs_row_params& P, int vocab) {
+__host__ __device__ __forceinline__ bool is_candidate_row(const hs_row_params& P, int vocab) {
   return P.temperature != 0.0f && P.top_k > 0 && P.top_k <= kTopKMax && P.top_k < vocab;
 }
 

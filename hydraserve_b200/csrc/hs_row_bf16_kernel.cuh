@@ -44,14 +44,19 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
   Ctx3 c;
   c.x = reinterpret_cast<Exchange*>(smem_raw + lay.x);
   c.tab = reinterpret_cast<uint32_t*>(smem_raw + lay.tab);
-  c.hist = reinterpret_cast<LocalHist*>(smem_raw + lay.hist);   // in the count table's place, once it has served
-  c.gbuf = reinterpret_cast<V3Entry*>(smem_raw + lay.gbuf);
-  c.list = reinterpret_cast<V3Entry*>(smem_raw + lay.list);
+  c.hist = reinterpret_cast<uint32_t*>(smem_raw + lay.hist);
+  c.members = reinterpret_cast<V3Member*>(smem_raw + lay.members);
+  c.gbuf = reinterpret_cast<V3Entry*>(smem_raw + lay.members);
+  c.list = reinterpret_cast<int*>(smem_raw + lay.list);
+  uint32_t* staged = reinterpret_cast<uint32_t*>(smem_raw + lay.staged);
   int2* side_shared = reinterpret_cast<int2*>(smem_raw + lay.side);
   int2* rare = reinterpret_cast<int2*>(smem_raw + lay.rare);  // (id, raw bits | count class << 16)
   int* small = reinterpret_cast<int*>(smem_raw + lay.small);
   c.gbuf_n = small;
   c.step_n = small + 24;
+  c.span = reinterpret_cast<uint32_t*>(small + 30);
+  c.ends = small + 16;
+  c.range = small + 40;
   int* rare_n = small + 1;
   int* side_n = small + 2;
   int* defer_n = small + 27;
@@ -74,8 +79,6 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
   c.s_pair = nullptr;
   c.s_cap = 0;
   c.n_s = 0;
-  c.cl = nullptr;
-  c.n_cl = 0;
   c.m = 0.f;
   unsigned long long* clocks = args.phase_clocks ? args.phase_clocks + (size_t)c.row * kV3PhaseSlots : nullptr;
   c.dbg = clocks;
@@ -137,7 +140,7 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
   const int chunk_lo = min(my_part * per_part, n8_row), chunk_hi = min(chunk_lo + per_part, n8_row);
   const bool last_part = my_part == parts - 1;
   // small[16..18] / [19..21]: highest (+ 1) / lowest non-empty cell per count class; [22]: lowest side key
-  if (tid < 32) small[tid] = (tid >= 19 && tid <= 22) ? -1 : 0;
+  if (tid < 64) small[tid] = (tid >= 19 && tid <= 22) ? -1 : 0;
   if (tid == 0) c.x->bcast[5] = 0;  // highest side element, (key, ~id)
   __syncthreads();
   for (int i = tid; i < kCells; i += kThreads) c.tab[i] = 0;
@@ -283,16 +286,38 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
   }
   __syncthreads();
   if (parts > 1) {
-    // Hand this part's counts over: table and rare list to global scratch, then a ticket.  The
-    // part that draws the last ticket adds the other parts' to its own and goes on; the
-    // others are done.  Nobody waits for anybody.
+    // Hand this part's counts over, as a list of (class, count), with its rare tokens; then a ticket.
+    // The part that draws the last ticket adds the other parts' lists to its own table and goes on;
+    // the others are done.  Nobody waits for anybody.  (Lists instead of whole tables: about 16 KB a
+    // part instead of 72, so that a lone row can be counted by sixteen CTAs.)
     const size_t mine = (size_t)c.row * parts + my_part;
-    uint32_t* gtab = args.ctab + mine * kCells;
-    for (int i = tid; i < kCells / 4; i += kThreads)
-      reinterpret_cast<uint4*>(gtab)[i] = reinterpret_cast<const uint4*>(c.tab)[i];
     const int nr = *rare_n;
     for (int t = tid; t < min(nr, kV3RareCap); t += kThreads) args.crare[mine * kV3RareCap + t] = rare[t];
-    if (tid == 0) args.crare_n[mine] = nr;
+    {
+      // a count that 17 bits do not hold takes several entries
+      u64 left = 0;
+      int n = 0;
+#pragma unroll 4
+      for (int u = 0; u < kCells / kThreads; ++u) {
+        const uint32_t v = c.tab[tid + u * kThreads];
+        if (v) { left |= 1ull << u; n += 1 + (int)((v - 1u) / kMostHanded); }
+      }
+      int total;
+      int at = block_place(small + 48, n, total);  // (a barrier inside: the rare tokens have left)
+      uint32_t* gtab = args.ctab + mine * kCells;
+      uint32_t* dst = total <= kV3Staged ? staged : gtab;
+      for (; left; left &= left - 1) {
+        const int cell = tid + (__ffsll((long long)left) - 1) * kThreads;
+        uint32_t v = c.tab[cell];
+        for (; v > kMostHanded; v -= kMostHanded) dst[at++] = (uint32_t)cell | (kMostHanded << 15);
+        dst[at++] = (uint32_t)cell | (v << 15);
+      }
+      __syncthreads();
+      if (total <= kV3Staged)
+        for (int i = tid; i < (total + 3) / 4; i += kThreads)
+          reinterpret_cast<uint4*>(gtab)[i] = reinterpret_cast<const uint4*>(staged)[i];
+      if (tid == 0) args.crare_n[mine] = make_int2(total, nr);
+    }
     __threadfence();
     __syncthreads();
     if (tid == 0) small[14] = atomicAdd(&args.count_ticket[c.row], 1);
@@ -300,59 +325,60 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
     if (small[14] != parts - 1) return;
     __threadfence();
     if (tid == 0) args.count_ticket[c.row] = 0;
+    // all parts' lengths, then every warp takes its share of each list, the next list's entries
+    // on their way while this one's are added
+    const int2* lens = args.crare_n + (size_t)c.row * parts;
+    const uint32_t* lists = args.ctab + (size_t)c.row * parts * kCells;
+    int n_rare_all = 0;
     for (int g = 0; g < parts; ++g) {
-      if (g == my_part) continue;
-      const size_t theirs = (size_t)c.row * parts + g;
-      const uint4* src = reinterpret_cast<const uint4*>(args.ctab + theirs * kCells);
-      for (int i = tid; i < kCells / 4; i += kThreads) {
-        const uint4 v = __ldcg(src + i);
-        uint4 t = reinterpret_cast<uint4*>(c.tab)[i];
-        t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
-        reinterpret_cast<uint4*>(c.tab)[i] = t;
+      const int2 len = __ldcg(lens + g);
+      if (g != my_part) {
+        const uint32_t* src = lists + (size_t)g * kCells;
+        constexpr int kFlight = 8;
+        for (int i0 = tid; i0 < len.x; i0 += kFlight * kThreads) {
+          uint32_t v[kFlight];
+#pragma unroll
+          for (int u = 0; u < kFlight; ++u) v[u] = i0 + u * kThreads < len.x ? __ldcg(src + i0 + u * kThreads) : 0u;
+#pragma unroll
+          for (int u = 0; u < kFlight; ++u)
+            if (v[u]) atomicAdd(&c.tab[v[u] & 0x7fffu], v[u] >> 15);
+        }
       }
-      // their rare list goes behind this CTA's (a total beyond the capacity is swept up below)
-      const int ng = ((volatile int*)args.crare_n)[theirs];
-      __syncthreads();
-      const int have = *rare_n;
-      __syncthreads();
-      if (have <= kV3RareCap && ng <= kV3RareCap) {
-        for (int t = tid; t < ng; t += kThreads)
-          if (have + t < kV3RareCap) rare[have + t] = __ldcg(args.crare + theirs * kV3RareCap + t);
-      }
-      if (tid == 0) *rare_n = have + ng;
-      __syncthreads();
+      // (a total beyond the capacity is swept up below)
+      for (int t = tid; t < min(len.y, kV3RareCap); t += kThreads)
+        if (n_rare_all + t < kV3RareCap) rare[n_rare_all + t] = __ldcg(args.crare + ((size_t)c.row * parts + g) * kV3RareCap + t);
+      n_rare_all += len.y;
     }
+    if (tid == 0) *rare_n = n_rare_all;
+    __syncthreads();
   }
   mark(1);
-  // Global scratch (class list, long side lists) is held per RESIDENT CTA: a CTA claims one of
-  // the n_scratch sets (as many as CTAs can be resident, so one is always free), starting its
-  // search at the pair of its SM, and gives it back at the end.
-  if (tid == 0) {
-    unsigned smid;
-    asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-    int got = -1;
-    for (int k = 0; k < 2 * args.n_scratch && got < 0; ++k) {
-      const int at = (int)((2u * smid + (unsigned)k) % (unsigned)args.n_scratch);
-      if (atomicCAS(&args.scratch_busy[at], 0, 1) == 0) got = at;
+  // Global scratch, for the side lists and class lists that shared memory does not hold, is kept per
+  // RESIDENT CTA: a CTA in need claims one of the n_scratch sets (as many as CTAs can be resident,
+  // so one is always free), starting its search at the pair of its SM, and gives it back at the end.
+  int scratch = -1;
+  auto claim_scratch = [&]() -> bool {
+    if (scratch >= 0) return true;
+    __syncthreads();
+    if (tid == 0) {
+      unsigned smid;
+      asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+      int got = -1;
+      for (int k = 0; k < 2 * args.n_scratch && got < 0; ++k) {
+        const int at = (int)((2u * smid + (unsigned)k) % (unsigned)args.n_scratch);
+        if (atomicCAS(&args.scratch_busy[at], 0, 1) == 0) got = at;
+      }
+      small[15] = got;
     }
-    small[15] = got;
-  }
-  __syncthreads();
-  const int scratch = small[15];
-  if (scratch < 0) {  // cannot happen while n_scratch covers the resident CTAs; fail the row, do not wait
+    __syncthreads();
+    scratch = small[15];
+    return scratch >= 0;
+  };
+  auto no_scratch = [&]() {  // cannot happen while n_scratch covers the resident CTAs; fail the row, do not wait
     if (tid == 0) { out->token = 0; out->status = 128; out->n_top = 0; out->n_kept = 0; }
     __syncthreads();
     if (tid < 32) write_record(a.out + c.row, *out, false);
-    return;
-  }
-  auto release_scratch = [&]() {
-    __syncthreads();
-    if (tid == 0) { __threadfence(); atomicExch(&args.scratch_busy[scratch], 0); }
   };
-  c.s_pair = args.s_pair + (size_t)scratch * args.s_cap;
-  c.s_cap = args.s_cap;
-  c.cl = args.clist + (size_t)scratch * kCells;
-
 
   // ---- B. the side list: tokens with history count >= 3, and values outside the bin window
   // It is walked by every selection, so it lives in shared memory when it fits.
@@ -362,6 +388,10 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
   if (n_rare <= kV3RareCap && n_heavy + kV3RareCap <= kV3SideShared) {
     c.s_pair = side_shared;
     c.s_cap = kV3SideShared;
+  } else {
+    if (!claim_scratch()) { no_scratch(); return; }
+    c.s_pair = args.s_pair + (size_t)scratch * args.s_cap;
+    c.s_cap = args.s_cap;
   }
   {
     auto put = [&](int slot, int id, float s) {
@@ -410,27 +440,20 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
     }
   }
   if (clocks && tid == 0) clocks[11] = clock64();
-  // ---- C. row maximum and minimum --------------------------------------------------------------
+  // ---- C. row maximum and minimum ----------------------------------------------------------------
   // Scores grow with the bin inside a count class, so the highest and lowest non-empty bin of
-  // each class decide (with the side list).  One pass over the table; warps combine with
-  // REDUX and meet in shared memory, one barrier (which also publishes the side list).
+  // each class decide (with the side list).  One pass over the table; warps combine with REDUX
+  // and meet in shared memory, one barrier (which also publishes the side list).
+  constexpr int kPerClass = kV3Bins / kThreads;  // a thread's cells tid + u * kThreads: count class u / kPerClass
+  static_assert(kV3Bins % kThreads == 0 && 3 * kPerClass <= 64, "a thread's u-th cell has the same count class for all threads");
   {
-    uint32_t top[3] = {0u, 0u, 0u}, bot[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
-    constexpr int kPerClass = kV3Bins / kThreads;  // a thread's cells tid + u * kThreads: count class u / kPerClass
-    static_assert(kV3Bins % kThreads == 0, "a thread's u-th cell has the same count class for all threads");
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-#pragma unroll 4
-      for (int u = 0; u < kPerClass; ++u) {
-        const uint32_t cell = (uint32_t)(tid + (k * kPerClass + u) * kThreads);
-        if (c.tab[cell]) { top[k] = cell + 1u; bot[k] = min(bot[k], cell); }
-      }
-    }
     const int lane = tid & 31;
+    for (int k = 0; k < (penalised ? 3 : 1); ++k) {  // (without penalties there is one count class)
+      uint32_t bits = 0;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const uint32_t t = __reduce_max_sync(0xffffffffu, top[k]);
-      const uint32_t l = __reduce_min_sync(0xffffffffu, bot[k]);
+      for (int u = 0; u < kPerClass; ++u) bits |= (c.tab[tid + (k * kPerClass + u) * kThreads] ? 1u : 0u) << u;
+      const uint32_t t = __reduce_max_sync(0xffffffffu, bits ? (uint32_t)(tid + (k * kPerClass + 31 - __clz(bits)) * kThreads) + 1u : 0u);
+      const uint32_t l = __reduce_min_sync(0xffffffffu, bits ? (uint32_t)(tid + (k * kPerClass + __ffs(bits) - 1) * kThreads) : 0xffffffffu);
       if (lane == 0) {
         if (t) atomicMax(reinterpret_cast<unsigned*>(small) + 16 + k, t);
         if (l != 0xffffffffu) atomicMin(reinterpret_cast<unsigned*>(small) + 19 + k, l);
@@ -496,33 +519,17 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
   u64 draw_members = 0, draw_nth = 0;
   bool token_known = false;
 
+  V3Map all_map;        // every token, by score
+  bool filled = false;  // the histogram holds every token under all_map
   {
-  // ---- the row's non-empty classes, each with its key and mass computed once ---------------
-  // Thread t owns classes t, t + kThreads, ... (the populated value range spreads evenly over
-  // the threads) and writes its entries back to back; the order is fixed by the counts alone.
-  {
-    constexpr int kPerCells = kCells / kThreads;
-    int mine = 0;
-#pragma unroll 4
-    for (int u = 0; u < kPerCells; ++u) mine += c.tab[tid + u * kThreads] != 0;
-    const u64 incl = warp_scan_u64((u64)mine);
-    u64 pre, pre_unused, tot, tot_unused;
-    block_warp_prefix2(*c.x, shfl_u64(incl, 31), 0, pre, pre_unused, tot, tot_unused);
-    int at = (int)(pre + incl) - mine;
-    if (clocks && tid == 0) clocks[26] = clock64();
-    for (int u = 0; u < kPerCells; ++u) {
-      const int cell = tid + u * kThreads;
-      const uint32_t n = c.tab[cell];
-      if (!n) continue;
-      const float s = c.cell_score(cell);
-      const u64 q = mass_of(s, m);
-      reinterpret_cast<uint4*>(c.cl)[at] = pack_class(key_of(s), n, (uint32_t)cell, q);
-      ++at;
-    }
-    c.n_cl = (int)tot;
-    __syncthreads();
+  // ---- every token's count and mass, in one histogram over the scores ----------------------------
+  // (in the place of the rare tokens and set-aside chunks, which have served)
+  all_map.by_score(score_of(min_key), m);
+  if (!c.greedy || P.n_logprobs >= 0) {
+    hist_fill<true>(c.hist, AllTokens3{&c}, all_map);
+    filled = true;
   }
-  mark(3);  // (the count table has served: the selection histograms take its place)
+  mark(3);
 
   if (c.greedy) {
     // arg max with penalties: the lowest id among the tokens whose score key is the maximum
@@ -537,12 +544,12 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
     if (token == 0x7fffffff) { token = any_side ? side_arg : 0; status |= 1; }
     if (P.n_logprobs >= 0) {
       u64 cn;
-      totals3(c, 0u, cn, q_kept);
+      totals3(c, 0u, filled, cn, q_kept);
     }
   } else {
     u64 cnt = 0, mass = 0;
     if (P.top_k > 0 && P.top_k < a.vocab) {
-      Selection sk = select_union3<false, true>(c, 0u, (u64)P.top_k, 1.0f);
+      Selection sk = select_key<false, true>(c, AllTokens3{&c}, all_map, filled, (u64)P.top_k);
       if (!sk.ok) status |= 1;
       kept.cut_key = sk.key;
       cnt = sk.above_cnt + sk.bin_cnt;
@@ -553,7 +560,7 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
     }
     mark(4);
     if (P.min_p > 0.0f) {
-      if (!have_totals) { totals3(c, kept.cut_key, cnt, mass); have_totals = true; }
+      if (!have_totals) { totals3(c, kept.cut_key, filled, cnt, mass); have_totals = true; }
       const float z1 = mass_to_float(mass);
       const float thr = __fmul_rn(__fdiv_rn(1.0f, z1), P.min_p);
       uint32_t lowest = 0xffffffffu;
@@ -561,7 +568,7 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
         const uint32_t k = key_of(s);
         if (k >= kept.cut_key && !(__fdiv_rn(expf(s - m), z1) < thr)) lowest = min(lowest, k);
       };
-      for_each_class(c, [&](const ClassEntry& e) { consider(score_of(e.key)); });
+      for_each_class(c, [&](bool valid, uint32_t key, uint32_t, int) { if (valid) consider(score_of(key)); });
       for_each_side3(c, [&](int, float s) { consider(s); });
       lowest = ~block_max_u32(*c.x, ~lowest);
       if (lowest != 0xffffffffu && lowest > kept.cut_key) {
@@ -570,19 +577,20 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
       }
     }
     mark(5);
+    // (what the cuts so far keep lies at the top, so the cut by mass is looked for among all tokens)
+    if (!have_totals) { totals3(c, kept.cut_key, filled, cnt, mass); have_totals = true; }
+    n_minp = cnt;
     if (P.top_p < 1.0f) {
-      {
-        // first level over the scores' own range (from the lowest class that can be kept to the
-        // row maximum) instead of the key's top bits: one level separates a near-flat row
-        const float lo = score_of(max(kept.cut_key, cells_min_key == 0xffffffffu ? min_key : cells_min_key));
-        const float range = m - lo;
-        c.lin = range > 0.f && range < 3.0e38f;
-        c.lin_lo = lo;
-        c.lin_scale = c.lin ? __fdiv_rn(2047.5f, range) : 0.f;
+      Selection sp{};
+      if (mass > 0) {
+        // (double precision, slow: the lanes of one warp try neighbouring candidates at once)
+        if (tid < 32) {
+          const u64 t = top_p_target_warp(mass, P.top_p);
+          if (tid == 0) c.x->bcast[6] = t;
+        }
+        __syncthreads();
+        sp = select_key<true, true>(c, AllTokens3{&c}, all_map, filled, c.x->bcast[6]);
       }
-      Selection sp = select_union3<true, true>(c, kept.cut_key, 0, P.top_p);
-      c.lin = false;
-      n_minp = sp.total_cnt;
       if (sp.ok && sp.bin_cnt > 0) {
         const u64 qv = sp.bin_mass / sp.bin_cnt;  // every token at the cut key has the same mass
         u64 t = sp.bin_cnt;
@@ -598,16 +606,9 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
         cut_ties = (long long)t;
         cut_group_cnt = sp.bin_cnt;
         tie_split = t < sp.bin_cnt;
-        have_totals = true;
       } else {
         status |= 1;
-        cnt = sp.total_cnt;
-        mass = sp.total_mass;
-        have_totals = true;
       }
-    } else {
-      if (!have_totals) { totals3(c, kept.cut_key, cnt, mass); have_totals = true; }
-      n_minp = cnt;
     }
     n_kept = cnt;
     q_kept = mass;
@@ -666,9 +667,48 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
         const Philox4 r = philox4x32_10(0u, 0u, 0u, 0u, (uint32_t)P.seed, (uint32_t)(P.seed >> 32));
         const u64 r64 = ((u64)r.v[0] << 32) | r.v[1];
         const u64 target = __umul64hi(r64, q_kept);
-        // classes above the cut in the order (thread, step): thread t owns entries t, t + kThreads, ...
-        u64 chunk = 0;
-        for_each_class(c, [&](const ClassEntry& e) { if (e.key > kept.cut_key) chunk += e.w; });
+        // Classes above the cut in this order: the non-empty cells t, t + kThreads, ... of every t in
+        // turn make a list, and its entries j, j + kThreads, ... are chunk j.  (Any fixed order
+        // would do; the counts alone decide it.)  A thread adds its cells' masses to their chunks.
+        const int n_cells = (penalised ? 3 : 1) * kPerClass;
+        int mine = 0;
+#pragma unroll 4
+        for (int u = 0; u < n_cells; ++u) mine += c.tab[tid + u * kThreads] ? 1 : 0;
+        uint32_t* chunks = reinterpret_cast<uint32_t*>(c.members);  // [3][kThreads]: mass in limbs
+        static_assert(3 * kThreads * sizeof(uint32_t) <= sizeof(V3Member) * kV3ListCap + sizeof(int) * kV3TieCap, "the chunks fit the members' place");
+#pragma unroll
+        for (int l = 0; l < 3; ++l) chunks[tid + l * kThreads] = 0;
+        int n_cl;
+        const int list_at = block_place(small + 48, mine, n_cl);
+        {
+          int at = list_at;
+          constexpr int kBatch = 3;  // (scoring a cell is a long chain)
+          static_assert(kPerClass % kBatch == 0, "a batch is of one count class");
+#pragma unroll 1
+          for (int u0 = 0; u0 < n_cells; u0 += kBatch) {
+            uint32_t n[kBatch], key[kBatch];
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) n[u] = c.tab[tid + (u0 + u) * kThreads];
+            if (!__any_sync(0xffffffffu, (n[0] | n[1] | n[2]) != 0u)) continue;
+            const int k = u0 / kPerClass;
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) key[u] = c.key_of_bin(tid + (u0 + u) * kThreads - k * kV3Bins, k);
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+              if (!n[u]) continue;
+              if (key[u] > kept.cut_key) {
+                const u64 w = (u64)n[u] * mass_of(score_of(key[u]), m);
+                uint32_t* dst = chunks + (at & (kThreads - 1));
+                atomicAdd(dst, (uint32_t)w & kLimbMask);
+                atomicAdd(dst + kThreads, (uint32_t)(w >> kLimbBits) & kLimbMask);
+                atomicAdd(dst + 2 * kThreads, (uint32_t)(w >> (2 * kLimbBits)));
+              }
+              ++at;
+            }
+          }
+        }
+        __syncthreads();
+        const u64 chunk = (u64)chunks[tid] + ((u64)chunks[tid + kThreads] << kLimbBits) + ((u64)chunks[tid + 2 * kThreads] << (2 * kLimbBits));
         const u64 incl = warp_scan_u64(chunk);
         u64 pre, pre_unused, q_cells, tot_unused;
         block_warp_prefix2(*c.x, shfl_u64(incl, 31), 0, pre, pre_unused, q_cells, tot_unused);
@@ -679,7 +719,8 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
         if (cut_ties < 0) {
           // cut by top-k / min-p / nothing: everything at the cut key is kept; count it
           u64 gc = 0, gm = 0;
-          for_each_class(c, [&](const ClassEntry& e) { if (e.key == kept.cut_key) gc += e.cnt; });
+          for_classes_at(c, 0, 0, [&](uint32_t k) { return k < kept.cut_key ? -1 : (k > kept.cut_key ? 1 : 0); },
+                         [&](uint32_t, uint32_t n, int) { gc += n; });
           for_each_side3(c, [&](int, float s) { if (key_of(s) == kept.cut_key) gc += 1; });
           block_sum2(*c.x, gc, gm);
           group_kept = gc;
@@ -688,21 +729,41 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
         const u64 q_group = group_kept * q_cut;
         mark(13);
         if (target < q_cells) {
+          // the chunk that holds the target, its cells in order (a thread has at most one of them:
+          // its entries of the list are fewer than kThreads and lie side by side), then the cell
+          int* cells = c.list;
+          constexpr int kMostCells = kCells / kThreads;
+          if (tid < kMostCells) cells[tid] = -1;
           if (tid == 0) c.x->bcast[5] = 0;
+          const u64 from = pre + incl - chunk;
+          if (from <= target && target < from + chunk) { c.x->bcast[0] = (u64)tid; c.x->bcast[1] = from; }
           __syncthreads();
-          u64 run = pre + incl - chunk;
-          if (run <= target && target < run + chunk) {
-            bool done = false;
-            for (int i = tid; i < c.n_cl && !done; i += kThreads) {
-              const ClassEntry e = c.class_at(i);
-              if (e.key <= kept.cut_key) continue;
-              if (e.w && target < run + e.w) {
-                c.x->bcast[3] = e.cnt;
-                c.x->bcast[4] = (target - run) / e.q + 1;
-                c.x->bcast[5] = (u64)e.cell + 1;
-                done = true;
+          {
+            int skip = ((int)c.x->bcast[0] - list_at) & (kThreads - 1);
+            if (skip < mine) {
+              const int slot = (list_at + skip) / kThreads;
+              int cell = tid;
+              while (c.tab[cell] == 0u || skip-- > 0) cell += kThreads;
+              cells[slot] = cell;
+            }
+          }
+          __syncthreads();
+          if (tid < 32) {
+            u64 run = c.x->bcast[1];
+            for (int base = 0; base < kMostCells; base += 32) {
+              const int cell = base + tid < kMostCells ? cells[base + tid] : -1;
+              u64 q = 0, w = 0;
+              if (cell >= 0) {
+                const uint32_t key = key_of(c.cell_score(cell));
+                if (key > kept.cut_key) { q = mass_of(score_of(key), m); w = (u64)c.tab[cell] * q; }
               }
-              run += e.w;
+              const u64 in = warp_scan_u64(w);
+              if (w && run + in - w <= target && target < run + in) {
+                c.x->bcast[3] = c.tab[cell];
+                c.x->bcast[4] = (target - (run + in - w)) / q + 1;
+                c.x->bcast[5] = (u64)cell + 1;
+              }
+              run += shfl_u64(in, 31);
             }
           }
           __syncthreads();
@@ -718,8 +779,10 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
           if (token == 0x7fffffff) { token = any_side ? side_arg : 0; status |= 1; }
           token_known = true;
         } else {
-          SideDrawFill3 fill{&c, kept.cut_key};
-          Selection sd = descend_local<true>(c, fill, 0u, target - q_cells - q_group + 1, -1.0f, 0, 1, 0x7FFu);
+          V3Map by_id;
+          by_id.by_key(~(uint32_t)(c.vocab - 1), 0xffffffffu);
+          filled = false;
+          const Selection sd = select_key<true, true>(c, KeptSide3{&c, kept.cut_key}, by_id, filled, target - q_cells - q_group + 1);
           if (sd.ok) token = (int)(~sd.key);
           else { token = any_side ? side_arg : 0; status |= 1; }
           token_known = true;
@@ -769,22 +832,23 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
     int n_want = min(P.n_logprobs, a.vocab);
     if ((u64)n_want > n_kept) n_want = (int)n_kept;
     if (n_want > 0) {
-      Selection sn = select_union3<false, false>(c, kept.cut_key, (u64)n_want, 1.0f);
+      // (the kept tokens are the highest: the N highest of them are the N highest of all)
+      const Selection sn = select_key<false, false>(c, AllTokens3{&c}, all_map, filled, (u64)n_want);
       if (sn.ok) {
         const int need = n_want - (int)sn.above_cnt;  // lowest ids of the group at the N-th key
         // The tokens above the N-th key (fewer than N) and the group at it: side elements come
         // from the side list, the rest from one walk of the row against per-class raw
         // thresholds.  The group's ids go to a list of their own (the member list's memory);
         // a group too large for it is walked the slow way.
-        int* tie_ids = reinterpret_cast<int*>(c.list);
-        constexpr int kTieCap = (int)(kV3ListCap * sizeof(V3Entry) / sizeof(int));
+        int* tie_ids = c.list;
+        constexpr int kTieCap = kV3TieCap;
         int* tie_n = small + 3;
         if (tid == 0) { *c.gbuf_n = 0; *tie_n = 0; }
         __syncthreads();
         auto take = [&](uint32_t k, int id) {
           if (k > sn.key) {
             const int slot = atomicAdd(c.gbuf_n, 1);
-            if (slot < kV3ListCap) c.gbuf[slot] = V3Entry{k, id, 1u, 0u, 0ull};
+            if (slot < kV3ListCap) c.gbuf[slot] = V3Entry{k, id};
           } else if (k == sn.key && need > 0) {
             const int slot = atomicAdd(tie_n, 1);
             if (slot < kTieCap) tie_ids[slot] = id;
@@ -807,7 +871,7 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
               for (int j = 0; j < n_tie; ++j) below += tie_ids[j] < mine ? 1 : 0;
               if (below < need) {
                 const int slot = atomicAdd(c.gbuf_n, 1);
-                if (slot < kV3ListCap) c.gbuf[slot] = V3Entry{sn.key, mine, 1u, 0u, 0ull};
+                if (slot < kV3ListCap) c.gbuf[slot] = V3Entry{sn.key, mine};
               }
             }
           } else {
@@ -874,7 +938,8 @@ __device__ __forceinline__ void count_row(const RowV3Args& args, unsigned char* 
     }
   }
   (void)cut_group_cnt;
-  release_scratch();  // (a barrier first: the record is complete)
+  __syncthreads();  // (the record is complete)
+  if (scratch >= 0 && tid == 0) { __threadfence(); atomicExch(&args.scratch_busy[scratch], 0); }
   if (tid < 32) write_record(a.out + c.row, *out, P.n_logprobs >= 0);
   mark(9);
 }
@@ -910,7 +975,7 @@ __device__ __forceinline__ bool cand_part(const RowV3Args& args, unsigned char* 
   const bool slot_ok = P.slot >= 0 && P.slot < a.pool.slots_total;
   const bool penalised = slot_ok && (c.rp != 1.0f || c.pp != 0.0f || c.fp != 0.0f);
   c.cls = penalised ? a.pool.cls + (size_t)P.slot * a.pool.cls_stride : nullptr;
-  c.s_pair = nullptr; c.n_s = 0; c.s_cap = 0; c.cl = nullptr; c.n_cl = 0; c.m = 0.f;
+  c.s_pair = nullptr; c.n_s = 0; c.s_cap = 0; c.m = 0.f;
   c.tab = nullptr; c.hist = nullptr; c.gbuf = nullptr; c.list = nullptr; c.gbuf_n = nullptr;
   unsigned long long* clocks = args.phase_clocks ? args.phase_clocks + (size_t)c.row * kV3PhaseSlots : nullptr;
   auto mark = [&](int slot) {
@@ -1031,7 +1096,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel_bf16(const __grid_cons
   __syncthreads();
   // (tuning aid: when each item started and ended, in ns of the global timer, slots 48.. of its row)
   unsigned long long* when = nullptr;
-  if (args.phase_clocks && threadIdx.x == 0) {
+  if (args.phase_clocks && threadIdx.x == 0 && part < 4) {
     when = args.phase_clocks + (size_t)row * kV3PhaseSlots + (count ? 48 : 56) + 2 * part;
     when[0] = global_timer_ns();
   }

@@ -11,11 +11,11 @@
 // individual (id, score) entries of a small side list.
 //
 // Selection (top-k by count, min-p by threshold, top-p by probability mass, top-N for the
-// log-probabilities) is a radix descent over 32-bit order-preserving keys of the class
-// scores: each non-empty class contributes (count, count * mass) to a bucket, the buckets
-// are scanned from the top, and once the deciding bucket holds few members they are
-// gathered, sorted and resolved exactly.  Probability mass is an integer multiple of 2^-40,
-// so all sums are exact and order-independent.
+// log-probabilities) needs ONE pass over the count table: a histogram of count and mass over 1,024
+// buckets of equal width in score.  Every cut names a bucket from the top, and the bucket's members
+// are resolved exactly against one another; a bucket with too many members is spread over 1,024
+// again.  Probability mass is an integer multiple of 2^-40, so all sums are exact and
+// order-independent.
 //
 // Token ids are only needed at the very end ("a uniformly chosen member of this class",
 // "the lowest ids of this tie group").  A class of more than kV3ListCap tokens is sampled by
@@ -24,11 +24,9 @@
 // or one the probes keep missing, is found by scanning the row once more for its bit
 // pattern.  Lowest-id tie-breaks walk the row hierarchically.
 //
-// A row's CTA keeps the count table, a short side list and (once the table has served, in its
-// place) the selection histograms in shared memory, about 88 KB, so that two CTAs share an
-// SM and one row's barrier-bound selection phases overlap another row's counting.  The list
-// of the row's non-empty classes (16 bytes each) lives in per-CTA global scratch and is
-// streamed from L2.  What is left of L1 is small, so the streaming loads go past it.
+// A row's CTA keeps the count table, the histogram and a short side list in shared memory, 111 KB, so
+// that two CTAs share an SM and one row's barrier-bound selection phases overlap another row's
+// counting.  What is left of L1 is small, so the streaming loads go past it.
 #pragma once
 
 #include "hs_common.cuh"
@@ -43,9 +41,13 @@ constexpr int kV3Half = 3072;                 // 24 binades x 128 mantissas
 constexpr int kV3Bins = 2 * kV3Half;          // per count class
 constexpr int kCells = 3 * kV3Bins;           // count classes 0, 1, 2
 constexpr uint32_t kV3Base = 113u << 7;       // smallest binned magnitude: 2^-14
-constexpr int kV3ListCap = 256;               // members resolved by sorting
+constexpr int kV3ListCap = 256;               // members of a bucket resolved against one another; top-N ids
 constexpr int kV3RejectMin = 128;             // classes of up to this many tokens are found by scanning the row, larger ones by rejection
-constexpr int kV3ScanCap = 1024;              // ids one class scan can hold (in the gather and list buffers)
+constexpr int kV3ScanCap = 1024;              // ids one class scan can hold
+constexpr int kV3TieCap = 1536;               // token ids ranked in shared memory
+constexpr int kV3Buckets = 1024;              // of a selection's histogram
+constexpr int kV3Staged = 7168;               // (class, count) entries of a hand-over staged in shared memory
+constexpr uint32_t kMostHanded = 0x1fffe;     // highest count of one such entry (17 bits beside a 15-bit class)
 #ifndef HS_RARE_CAP
 #define HS_RARE_CAP 512
 #endif
@@ -63,58 +65,25 @@ constexpr int kSplitCap = 4096;               // candidate entries one CTA of a 
 
 struct V3Entry {
   uint32_t key;  // 32-bit key of the score
-  int32_t id;    // token id of a side element, -1 for a class
-  uint32_t cnt;  // tokens this entry stands for
-  uint32_t cell; // class index (count class * kV3Bins + bin) of a class entry
-  u64 q;         // mass of one token
+  int32_t id;    // token id
 };
-
-struct LocalHist {
-  uint32_t ent[kBins];  // entries (classes + side elements) per bucket
-  uint32_t cnt[kBins];
-  uint32_t l0[kBins], l1[kBins], l2[kBins];  // mass in 14-bit limbs: 32-bit shared atomics only
-  __device__ __forceinline__ u64 mass(int b) const {
-    return (u64)l0[b] + ((u64)l1[b] << kLimbBits) + ((u64)l2[b] << (2 * kLimbBits));
-  }
+// A member of a selection's deciding bucket: a class or a side element.
+struct __align__(16) V3Member {
+  uint32_t key, cnt;
+  u64 w;  // mass of all its tokens
 };
-
-// A non-empty class with its score key and mass, computed once per row.  Stored in 16 bytes
-// in the CTA's global scratch and handed to the visitors of for_each_class unpacked.
-struct __align__(16) ClassPacked {
-  uint32_t key;  // 32-bit key of the class score
-  uint32_t cnt;  // tokens in the class
-  u64 qc;        // bits 0..47: mass of one token (<= 2^40); bits 48..63: count class * kV3Bins + bin
-};
-struct ClassEntry {
-  uint32_t key, cnt, cell;
-  u64 q;  // mass of one token
-  u64 w;  // cnt * q
-};
-__device__ __forceinline__ ClassEntry unpack_class(const uint4& v) {
-  ClassEntry e;
-  e.key = v.x;
-  e.cnt = v.y;
-  e.cell = v.w >> 16;
-  e.q = ((u64)(v.w & 0xffffu) << 32) | v.z;
-  e.w = (u64)e.cnt * e.q;
-  return e;
-}
-__device__ __forceinline__ uint4 pack_class(uint32_t key, uint32_t cnt, uint32_t cell, u64 q) {
-  return make_uint4(key, cnt, (uint32_t)q, (uint32_t)(q >> 32) | (cell << 16));
-}
 
 struct RowV3Args {
   RowKernelArgs base;
-  ClassPacked* clist;  // [n_scratch, kCells] scratch: the class list of the row a CTA is working on
   int2* s_pair;   // [n_scratch, s_cap] side lists too long for shared memory: (token id or -1, fp32 bits of the score)
   int s_cap;
   int n_scratch;       // scratch sets: as many as CTAs of the kernel can be resident at once
   int* scratch_busy;   // [n_scratch] 1 while a CTA holds the set
   unsigned long long* phase_clocks;  // [batch, kV3PhaseSlots] or null
-  int csplit;                        // CTAs per row on the counting path (1, 2 or 4)
-  uint32_t* ctab;                    // [batch, csplit, kCells] count tables handed over by the parts of a row
+  int csplit;                        // CTAs per row on the counting path
+  uint32_t* ctab;                    // [batch, csplit, kCells] classes and counts handed over by the parts of a row
   int2* crare;                       // [batch, csplit, kV3RareCap] their rare lists
-  int* crare_n;                      // [batch, csplit]
+  int2* crare_n;                     // [batch, csplit] (classes, rare tokens)
   int* count_ticket;                 // [batch] arrival counter (returns to 0)
   int split;                         // CTAs per row on the candidate path
   unsigned long long* split_lists;   // [batch, split, kSplitCap] candidate lists of the row's CTAs
@@ -123,10 +92,10 @@ struct RowV3Args {
   int batch;                         // rows in the launch
 };
 
-// Shared memory of a counting row.  The selection histograms and the two member buffers are
-// only needed after the count table has been turned into the class list, and take its place.
+// Shared memory of a counting row.  What only the counting needs (rare tokens, set-aside chunks, the
+// staged hand-over) and what only the selections need (histogram, members, token ids) share a place.
 struct LayoutV3 {
-  size_t x, tab, hist, gbuf, list, side, rare, defer, small, total;
+  size_t x, tab, side, hist, members, list, staged, rare, defer, small, total;
 };
 __host__ __device__ inline LayoutV3 layout_v3() {
   LayoutV3 l{};
@@ -138,26 +107,20 @@ __host__ __device__ inline LayoutV3 layout_v3() {
   };
   l.x = take(sizeof(Exchange));
   l.tab = take(sizeof(uint32_t) * kCells);
-  {
-    size_t in_tab = l.tab;
-    auto sub = [&](size_t bytes) {
-      const size_t at = in_tab;
-      in_tab = (in_tab + bytes + 15) & ~size_t(15);
-      return at;
-    };
-    l.hist = sub(sizeof(LocalHist));
-    l.gbuf = sub(sizeof(V3Entry) * kV3ListCap);
-    l.list = sub(sizeof(V3Entry) * kV3ListCap);
-  }
   l.side = take(sizeof(int2) * kV3SideShared);
-  l.rare = take(sizeof(int2) * kV3RareCap);
-  l.defer = take(sizeof(int) * kV3DeferCap);
-  l.small = take(sizeof(int) * 32);
+  l.staged = take(sizeof(uint32_t) * kV3Staged);
+  l.rare = l.staged;
+  l.defer = l.rare + sizeof(int2) * kV3RareCap;
+  l.hist = l.staged;
+  l.members = l.hist + sizeof(uint32_t) * 4 * kV3Buckets;
+  l.list = l.members + sizeof(V3Member) * kV3ListCap;
+  l.small = take(sizeof(int) * 64);
   l.total = off;
   return l;
 }
-static_assert(sizeof(LocalHist) + 2 * sizeof(V3Entry) * kV3ListCap + 32 <= sizeof(uint32_t) * kCells,
-              "the selection buffers fit in the count table's place");
+static_assert(sizeof(uint32_t) * (4 * kV3Buckets + kV3TieCap) + sizeof(V3Member) * kV3ListCap <= sizeof(uint32_t) * kV3Staged &&
+              sizeof(int2) * kV3RareCap + sizeof(int) * kV3DeferCap <= sizeof(uint32_t) * kV3Staged,
+              "the two uses fit the shared place");
 
 __device__ __forceinline__ int v3_bin_of_raw(uint32_t raw) {
   const uint32_t idx = (raw & 0x7fffu) - kV3Base;
@@ -172,10 +135,14 @@ __device__ __forceinline__ uint32_t v3_raw_of_bin(int b) {
 struct Ctx3 {
   Exchange* x;
   uint32_t* tab;     // [kCells] tokens per class
-  LocalHist* hist;
-  V3Entry* gbuf;     // gather buffer
-  V3Entry* list;     // sorted members
+  uint32_t* hist;    // [4 * kV3Buckets] count, mass in three 14-bit limbs (32-bit shared atomics only)
+  V3Member* members; // [kV3ListCap] members of a selection's deciding bucket
+  V3Entry* gbuf;     // [kV3ListCap] top-N tokens (in the same place)
+  int* list;         // [kV3TieCap] token ids
   int* gbuf_n;
+  uint32_t* span;    // lowest and highest key of a deciding bucket
+  int* range = nullptr;  // [6] scratch of for_classes_at
+  int* ends = nullptr;  // [6] per count class: highest non-empty cell + 1 (0 = none), lowest non-empty cell
   int* step_n = nullptr;  // two counters the early-exit scan alternates between
   int row, vocab;
   unsigned long long* dbg = nullptr;
@@ -209,33 +176,17 @@ struct Ctx3 {
   int slot;
   int2* s_pair;
   int n_s, s_cap;
-  ClassPacked* cl;   // this row's non-empty classes (global scratch of this CTA)
-  // entry i of the row's class list
-  __device__ __forceinline__ ClassEntry class_at(int i) const {
-    return unpack_class(__ldcg(reinterpret_cast<const uint4*>(cl) + i));
-  }
-  int n_cl;
   float T, rp, pp, fp;
   bool greedy;
   float m;
-  // Linear bucketing of the first level of a mass descent (see descend_local): bucket =
-  // (score - lin_lo) * lin_scale, which grows with the key like the key's own top bits do,
-  // but spreads a row whose scores lie close together over all buckets.
-  bool lin = false;
-  float lin_lo = 0.f, lin_scale = 0.f;
-  __device__ __forceinline__ uint32_t lin_bucket(uint32_t key) const {
-    const float t = (hs::score_of(key) - lin_lo) * lin_scale;
-    return (uint32_t)min(max(__float2int_rz(t), 0), kBins - 1);
-  }
-
   __device__ __forceinline__ float score_of_value(float v) const {
-    return greedy ? canonical(v) : canonical(__fdiv_rn(v, T));
+    return greedy || T == 1.0f ? canonical(v) : canonical(__fdiv_rn(v, T));
   }
   // score of a token with raw value bits `raw` that the history holds `count` times
   __device__ __forceinline__ float score_of(uint32_t raw, int count) const {
     float v = canonical(__uint_as_float(raw << 16));
     if (count > 0) {
-      v = v < 0.0f ? __fmul_rn(v, rp) : __fdiv_rn(v, rp);
+      if (rp != 1.0f) v = v < 0.0f ? __fmul_rn(v, rp) : __fdiv_rn(v, rp);
       v = __fsub_rn(v, pp);
       v = __fsub_rn(v, __fmul_rn(fp, (float)count));
     }
@@ -245,6 +196,8 @@ struct Ctx3 {
     const int c = cell / kV3Bins;
     return score_of(v3_raw_of_bin(cell - c * kV3Bins), c);
   }
+  // score key of a bin of count class k
+  __device__ __forceinline__ uint32_t key_of_bin(int bin, int k) const { return key_of(score_of(v3_raw_of_bin(bin), k)); }
   __device__ __forceinline__ int class_of(int id) const {
     return cls ? (int)((cls[id >> 4] >> ((id & 15) * 2)) & 3u) : 0;
   }
@@ -273,299 +226,302 @@ __device__ __forceinline__ void for_each_side3(const Ctx3& c, F&& f) {
       if (e[u].x >= 0) f(e[u].x, __int_as_float(e[u].y));
   }
 }
-// Calls f(entry) for the row's non-empty classes, thread t taking entries t, t + kThreads, ...
-// (four 16-byte loads in flight per thread; the list sits in L2).
+// ---- the row's classes, in order --------------------------------------------------------------
+// Scores grow with the bin inside a count class, so a count class's cells, from its lowest to its
+// highest non-empty one, are in the order of their scores.
+//
+// Calls f(valid, key, tokens, cell) for them, a thread's cells kThreads apart, WHOLE WARPS together
+// (valid = the cell is not empty); a warp whose cells are all empty is passed over.  Scoring a cell is
+// a chain of a few hundred cycles, so three of a thread's cells are worked on at a time.
 template <class F>
 __device__ __forceinline__ void for_each_class(const Ctx3& c, F&& f) {
-  const uint4* src = reinterpret_cast<const uint4*>(c.cl);
-  for (int i0 = threadIdx.x; i0 < c.n_cl; i0 += 4 * kThreads) {
-    uint4 v[4];
+  constexpr int kBatch = 3;
+#pragma unroll 1
+  for (int k = 0; k < 3; ++k) {
+    const int top = c.ends[k], bot = c.ends[3 + k];  // (highest + 1; 0 = the class is empty)
+    if (top == 0) continue;
+#pragma unroll 1
+    for (int base = bot + (int)threadIdx.x; base - (int)(threadIdx.x & 31) < top; base += kBatch * kThreads) {
+      uint32_t n[kBatch], key[kBatch];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = i0 + u * kThreads;
-      if (i < c.n_cl) v[u] = __ldcg(src + i);
+      for (int u = 0; u < kBatch; ++u) n[u] = base + u * kThreads < top ? c.tab[base + u * kThreads] : 0u;
+      if (!__any_sync(0xffffffffu, (n[0] | n[1] | n[2]) != 0u)) continue;
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) key[u] = c.key_of_bin(min(base + u * kThreads, top - 1) - k * kV3Bins, k);
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) f(n[u] != 0u, key[u], n[u], base + u * kThreads);
     }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = i0 + u * kThreads;
-      if (i >= c.n_cl) break;
-      f(unpack_class(v[u]));
+  }
+}
+// Calls f(key, tokens, cell) for the non-empty cells whose keys k have low <= place(k) <= high, for a
+// place that grows with the key.  Warp w looks for one end of count class w % 3's range, 32 cells
+// at a time; then the ranges' cells go to the threads one by one.  Called by the whole CTA.
+template <class Place, class F>
+__device__ __forceinline__ void for_classes_at(const Ctx3& c, int low, int high, Place&& place, F&& f) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __syncthreads();
+  if (warp < 6) {
+    const int k = warp % 3, top = c.ends[k];
+    const int want = warp < 3 ? low : high + 1;  // the first cell whose place is at least this
+    int lo = top ? c.ends[3 + k] : 0, hi = top;
+#pragma unroll 1
+    while (lo < hi) {
+      const int step = (hi - lo + 31) >> 5;
+      const int t = lo + (lane + 1) * step - 1;
+      const bool pass = t >= hi || place(c.key_of_bin(min(t, hi - 1) - k * kV3Bins, k)) >= want;
+      const uint32_t votes = __ballot_sync(0xffffffffu, pass);
+      if (votes == 0) { lo = hi; break; }
+      const int first = __ffs(votes) - 1;
+      hi = min(lo + (first + 1) * step - 1, hi);
+      lo = lo + first * step;
+    }
+    if (lane == 0) c.range[warp] = lo;
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int k = 0; k < 3; ++k) {
+#pragma unroll 1
+    for (int cell = c.range[k] + (int)threadIdx.x; cell < c.range[3 + k]; cell += kThreads) {
+      const uint32_t n = c.tab[cell];
+      if (n) f(c.key_of_bin(cell - k * kV3Bins, k), n, cell);
     }
   }
 }
 
-// ---- radix descent inside one CTA ----------------------------------------------------
-struct LocalAdder {
-  LocalHist* h;
-  __device__ __forceinline__ void operator()(bool valid, uint32_t bin, uint32_t count, u64 mass) const {
-    if (!valid) return;
-    atomicAdd(&h->ent[bin], 1u);
-    atomicAdd(&h->cnt[bin], count);
-    const uint32_t a0 = (uint32_t)mass & kLimbMask;
-    const uint32_t a1 = (uint32_t)(mass >> kLimbBits) & kLimbMask;
-    const uint32_t a2 = (uint32_t)(mass >> (2 * kLimbBits));
-    if (a0) atomicAdd(&h->l0[bin], a0);
-    if (a1) atomicAdd(&h->l1[bin], a1);
-    if (a2) atomicAdd(&h->l2[bin], a2);
+// ---- selection inside one CTA ------------------------------------------------------------
+// Where a key falls among the buckets: by score, over equal widths from `lo` to the row maximum
+// (lin), or by the key itself, over [klo, khi].  Both grow with the key.
+struct V3Map {
+  bool lin;
+  float lo, scale;
+  uint32_t klo, khi;
+  int shift;
+  __device__ __forceinline__ bool in(uint32_t key) const { return key >= klo && key <= khi; }
+  __device__ __forceinline__ int bucket(uint32_t key) const {
+    if (lin) return min(max(__float2int_rz((score_of(key) - lo) * scale), 0), kV3Buckets - 1);
+    return key < klo ? -1 : (key > khi ? kV3Buckets : (int)((key - klo) >> shift));
+  }
+  // buckets over the keys of [from, to]
+  __device__ __forceinline__ void by_key(uint32_t from, uint32_t to) {
+    lin = false;
+    klo = from;
+    khi = to;
+    shift = max(0, 32 - __clz(to - from) - 10);  // ((to - from) >> shift) < 1,024
+  }
+  // buckets over the scores from `lowest` (or 30 below the maximum m, where no mass is left) to m;
+  // by key when the scores do not spread
+  __device__ __forceinline__ void by_score(float lowest, float m) {
+    by_key(0u, 0xffffffffu);
+    lo = fmaxf(lowest, m - 30.0f);
+    const float range = m - lo;
+    lin = range > 0.f && range < 3.0e38f;
+    scale = lin ? __fdiv_rn((float)kV3Buckets - 0.5f, range) : 0.f;
   }
 };
+template <bool WITH_MASS>
+__device__ __forceinline__ void hist_add(uint32_t* hist, int b, uint32_t cnt, u64 mass) {
+  atomicAdd(hist + b, cnt);
+  if (!WITH_MASS) return;
+  const uint32_t a0 = (uint32_t)mass & kLimbMask, a1 = (uint32_t)(mass >> kLimbBits) & kLimbMask, a2 = (uint32_t)(mass >> (2 * kLimbBits));
+  if (a0) atomicAdd(hist + kV3Buckets + b, a0);
+  if (a1) atomicAdd(hist + 2 * kV3Buckets + b, a1);
+  if (a2) atomicAdd(hist + 3 * kV3Buckets + b, a2);
+}
+__device__ __forceinline__ u64 hist_mass(const uint32_t* hist, int b) {
+  return (u64)hist[kV3Buckets + b] + ((u64)hist[2 * kV3Buckets + b] << kLimbBits) + ((u64)hist[3 * kV3Buckets + b] << (2 * kLimbBits));
+}
 
-template <bool BY_MASS, class Fill>
-__device__ Selection descend_local(Ctx3& c, Fill& fill, uint32_t lo_key, u64 target_cnt, float top_p,
-                                   u64 stop_pop = 0, int first_level = 0, uint32_t prefix0 = 0) {
-  LocalHist& h = *c.hist;
-  Selection sel;
-  sel.above_cnt = sel.above_mass = 0;
-  sel.total_cnt = sel.total_mass = 0;
-  sel.bin_cnt = sel.bin_mass = 0;
-  sel.target = target_cnt;
-  sel.ok = true;
-  sel.levels = first_level;
-  uint32_t prefix = prefix0;
+// Every token of the row: side elements one by one, classes with their count.
+struct AllTokens3 {
+  const Ctx3* c;
+  // into the histogram.  The thousands of values next to zero share a bucket, and would queue up at
+  // one address: a warp whose cells all fall into one bucket adds them up first.
+  template <bool WITH_MASS>
+  __device__ __forceinline__ void fill(const V3Map& map) const {
+    const float m = c->m;
+    uint32_t* hist = c->hist;
+    for_each_side3(*c, [&](int, float s) {
+      const uint32_t key = key_of(s);
+      if (map.in(key)) hist_add<WITH_MASS>(hist, map.bucket(key), 1u, WITH_MASS ? mass_of(s, m) : 0ull);
+    });
+    for_each_class(*c, [&](bool valid, uint32_t key, uint32_t n, int) {
+      valid = valid && map.in(key);
+      const int b = map.bucket(key);
+      const u64 w = WITH_MASS ? (u64)n * mass_of(score_of(key), m) : 0ull;
+      const int first = __reduce_min_sync(0xffffffffu, valid ? b : 0x7fffffff);
+      if (__all_sync(0xffffffffu, !valid || b == first)) {
+        const uint32_t cnt = __reduce_add_sync(0xffffffffu, valid ? n : 0u);
+        const u64 sum = WITH_MASS ? warp_sum_u64(valid ? w : 0ull) : 0ull;
+        if (cnt && (threadIdx.x & 31) == 0) hist_add<WITH_MASS>(hist, first, cnt, sum);
+      } else if (valid) {
+        hist_add<WITH_MASS>(hist, b, n, w);
+      }
+    });
+  }
+  // f(key, count, mass) of bucket b
+  template <bool WITH_MASS, class F>
+  __device__ __forceinline__ void members(const V3Map& map, int b, F&& f) const {
+    const float m = c->m;
+    for_each_side3(*c, [&](int, float s) {
+      const uint32_t key = key_of(s);
+      if (map.in(key) && map.bucket(key) == b) f(key, 1u, WITH_MASS ? mass_of(s, m) : 0ull);
+    });
+    for_classes_at(*c, b, b, [&](uint32_t key) { return map.bucket(key); }, [&](uint32_t key, uint32_t n, int) {
+      f(key, n, WITH_MASS ? (u64)n * mass_of(score_of(key), m) : 0ull);
+    });
+  }
+};
+// Kept side elements keyed by ~id: the side part of the draw.
+struct KeptSide3 {
+  const Ctx3* c;
+  uint32_t cut_key;
+  template <bool WITH_MASS>
+  __device__ __forceinline__ void fill(const V3Map& map) const {
+    for_each_side3(*c, [&](int id, float s) {
+      const uint32_t key = ~(uint32_t)id;
+      if (key_of(s) > cut_key && map.in(key)) hist_add<WITH_MASS>(c->hist, map.bucket(key), 1u, mass_of(s, c->m));
+    });
+  }
+  template <bool WITH_MASS, class F>
+  __device__ __forceinline__ void members(const V3Map& map, int b, F&& f) const {
+    for_each_side3(*c, [&](int id, float s) {
+      const uint32_t key = ~(uint32_t)id;
+      if (key_of(s) > cut_key && map.in(key) && map.bucket(key) == b) f(key, 1u, mass_of(s, c->m));
+    });
+  }
+};
+template <bool WITH_MASS, class From>
+__device__ __forceinline__ void hist_fill(uint32_t* hist, const From& from, const V3Map& map) {
+#pragma unroll
+  for (int b = 0; b < 4 * kV3Buckets / kThreads; ++b) hist[threadIdx.x + b * kThreads] = 0;
+  __syncthreads();
+  from.template fill<WITH_MASS>(map);
+  __syncthreads();
+}
+
+// The key, from the top, at which the running count (BY_MASS: mass) of the elements reaches
+// `target`, with what lies above and at it.  filled: the histogram holds all elements under `map`
+// already (false afterwards if it had to be used for something else).
+template <bool BY_MASS, bool WITH_MASS, class From>
+__device__ Selection select_key(Ctx3& c, const From& from, V3Map map, bool& filled, u64 target) {
+  static_assert(WITH_MASS || !BY_MASS, "a cut by mass needs masses");
   const int tid = threadIdx.x;
-  const LocalAdder add{&h};
-  for (int level = first_level; level < 3; ++level) {
-    const int shift = level_shift(level);
-    const int bits = level_bits(level);
-    for (int b = tid; b < kBins; b += kThreads) { h.ent[b] = 0; h.cnt[b] = 0; h.l0[b] = 0; h.l1[b] = 0; h.l2[b] = 0; }
-    if (tid == 0) c.x->bcast[7] = 0;
-    __syncthreads();
-    if (c.dbg && tid == 0 && BY_MASS && level == first_level) c.dbg[16] = clock64();
-    fill(level, shift, bits, prefix, lo_key, add);
-    __syncthreads();
-    if (c.dbg && tid == 0 && BY_MASS && level == first_level) c.dbg[17] = clock64();
-    constexpr int kPer = kBins / kThreads;
-    const int hi = kBins - 1 - kPer * tid;
-    u64 c_sum = 0, m_sum = 0;
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) { c_sum += h.cnt[hi - u]; m_sum += h.mass(hi - u); }
-    const u64 ia = warp_scan_u64(c_sum);
-    const u64 ib = warp_scan_u64(m_sum);
-    if (c.dbg && tid == 0 && BY_MASS && level == first_level) c.dbg[30] = clock64();
-    u64 pa, pb, ta, tb;
-    block_warp_prefix2(*c.x, shfl_u64(ia, 31), shfl_u64(ib, 31), pa, pb, ta, tb);
-    if (c.dbg && tid == 0 && BY_MASS && level == first_level) c.dbg[31] = clock64();
-    u64 ex_cnt = pa + ia - c_sum;
-    u64 ex_mass = pb + ib - m_sum;
-    if (level == first_level) {
-      sel.total_cnt = ta;
-      sel.total_mass = tb;
-      if (BY_MASS && top_p >= 0.0f) {
-        // (double precision, slow: the lanes of one warp try neighbouring candidates at once)
-        if (tid < 32) {
-          const u64 t = top_p_target_warp(tb, top_p);
-          if (tid == 0) c.x->bcast[6] = t;
-        }
-        __syncthreads();
-        sel.target = c.x->bcast[6];
-      }
+  uint32_t* hist = c.hist;
+  Selection sel{};
+  sel.target = target;
+  sel.levels = 3;
+#pragma unroll 1
+  for (int round = 0; round < 8; ++round) {
+    if (!filled || round > 0) {
+      hist_fill<WITH_MASS>(hist, from, map);
+      filled = false;
     }
-    if (c.dbg && tid == 0 && BY_MASS && level == first_level) c.dbg[32] = clock64();
-    const u64 want = sel.target - (BY_MASS ? sel.above_mass : sel.above_cnt);
+    if (tid == 0) { c.x->bcast[7] = 0; *c.gbuf_n = 0; c.span[0] = 0xffffffffu; c.span[1] = 0u; }
+    // thread t owns the two buckets 1,023 - 2 t and 1,022 - 2 t
+    static_assert(kV3Buckets == 2 * kThreads, "two buckets per thread");
+    const int hi = kV3Buckets - 1 - 2 * tid;
+    u64 ac = 0, am = 0;  // above this thread's buckets
     {
-      const u64 ex = BY_MASS ? ex_mass : ex_cnt;
-      const u64 mine = BY_MASS ? m_sum : c_sum;
-      if (ex < want && want <= ex + mine) {
+      const u64 n = (u64)hist[hi] + hist[hi - 1];
+      const u64 q = WITH_MASS ? hist_mass(hist, hi) + hist_mass(hist, hi - 1) : 0ull;
+      const u64 ia = warp_scan_u64(n), ib = WITH_MASS ? warp_scan_u64(q) : 0ull;
+      u64 pa, pb, ta, tb;
+      block_warp_prefix2(*c.x, shfl_u64(ia, 31), WITH_MASS ? shfl_u64(ib, 31) : 0ull, pa, pb, ta, tb);
+      ac = pa + ia - n;
+      am = pb + ib - q;
+    }
+    const u64 want = sel.target - (BY_MASS ? sel.above_mass : sel.above_cnt);
 #pragma unroll
-        for (int u = 0; u < kPer; ++u) {
-          const u64 bc = h.cnt[hi - u], bm = h.mass(hi - u);
-          const u64 e = BY_MASS ? ex_mass : ex_cnt;
-          if (want <= e + (BY_MASS ? bm : bc)) {
-            c.x->bcast[0] = (u64)(hi - u);
-            c.x->bcast[1] = ex_cnt;
-            c.x->bcast[2] = ex_mass;
-            c.x->bcast[3] = bc;
-            c.x->bcast[4] = bm;
-            c.x->bcast[5] = h.ent[hi - u];
-            c.x->bcast[7] = 1;
-            break;
-          }
-          ex_cnt += bc;
-          ex_mass += bm;
-        }
+    for (int u = 0; u < 2; ++u) {
+      const u64 n = hist[hi - u], q = WITH_MASS ? hist_mass(hist, hi - u) : 0ull;
+      const u64 over = BY_MASS ? am : ac;
+      if (over < want && want <= over + (BY_MASS ? q : n)) {
+        c.x->bcast[0] = (u64)(hi - u);
+        c.x->bcast[1] = ac;
+        c.x->bcast[2] = am;
+        c.x->bcast[3] = n;
+        c.x->bcast[4] = q;
+        c.x->bcast[7] = 1;
       }
+      ac += n;
+      am += q;
     }
     __syncthreads();
-    if (c.x->bcast[7] == 0) {
+    if (c.x->bcast[7] == 0) {  // nothing reaches the target
       sel.ok = false;
-      sel.key = lo_key;
-      sel.prefix = prefix;
-      sel.bin_cnt = sel.bin_mass = 0;
+      sel.key = map.klo;
       __syncthreads();
       return sel;
     }
-    const uint32_t bin = (uint32_t)c.x->bcast[0];
+    const int bucket = (int)c.x->bcast[0];
+    sel.ok = true;
     sel.above_cnt += c.x->bcast[1];
     sel.above_mass += c.x->bcast[2];
     sel.bin_cnt = c.x->bcast[3];
     sel.bin_mass = c.x->bcast[4];
-    const u64 entries = c.x->bcast[5];
-    prefix = (prefix << bits) | bin;
-    sel.levels = level + 1;
+    from.template members<WITH_MASS>(map, bucket, [&](uint32_t key, uint32_t cnt, u64 w) {
+      const int slot = atomicAdd(c.gbuf_n, 1);
+      if (slot < kV3ListCap) c.members[slot] = V3Member{key, cnt, w};
+      atomicMin(c.span, key);
+      atomicMax(c.span + 1, key);
+    });
     __syncthreads();
-    if (c.dbg && tid == 0 && BY_MASS && level == first_level) c.dbg[18] = clock64();
-    if (stop_pop && level < 2 && entries <= stop_pop) break;  // few enough members to sort
-    if (c.lin && level == 0) {
-      // the linear buckets did not separate the row: once more, by the key's own bits
-      c.lin = false;
-      sel.above_cnt = sel.above_mass = 0;
-      prefix = prefix0;
-      level = first_level - 1;
+    const int members = *c.gbuf_n;
+    const uint32_t key_lo = c.span[0], key_hi = c.span[1];
+    if (key_lo == key_hi) { sel.key = key_lo; break; }
+    if (members <= kV3ListCap) {
+      // each member against all: what lies above its key, and at it
+      const u64 still = sel.target - (BY_MASS ? sel.above_mass : sel.above_cnt);
+      if (tid < members) {
+        const uint32_t mine = c.members[tid].key;
+        u64 oc = 0, om = 0, gc = 0, gm = 0;
+#pragma unroll 2
+        for (int j = 0; j < members; ++j) {
+          const V3Member o = c.members[j];
+          if (o.key > mine) { oc += o.cnt; om += o.w; }
+          if (o.key == mine) { gc += o.cnt; gm += o.w; }
+        }
+        const u64 over = BY_MASS ? om : oc;
+        if (over < still && still <= over + (BY_MASS ? gm : gc)) {  // (members of one key write the same)
+          c.x->bcast[0] = mine;
+          c.x->bcast[1] = oc; c.x->bcast[2] = om; c.x->bcast[3] = gc; c.x->bcast[4] = gm;
+        }
+      }
+      __syncthreads();
+      sel.key = (uint32_t)c.x->bcast[0];
+      sel.above_cnt += c.x->bcast[1];
+      sel.above_mass += c.x->bcast[2];
+      sel.bin_cnt = c.x->bcast[3];
+      sel.bin_mass = c.x->bcast[4];
+      break;
     }
+    map.by_key(key_lo, key_hi);
+    __syncthreads();
   }
-  sel.prefix = prefix;
-  sel.key = sel.levels == 3 ? prefix : (prefix << (sel.levels == 1 ? 21 : 10));
+  sel.prefix = sel.key;
+  __syncthreads();
   return sel;
 }
 
-// All tokens of the row: side elements individually, classes as (count, count * mass).
-template <bool WITH_MASS>
-struct UnionFill3 {
-  Ctx3* c;
-  template <class Add>
-  __device__ __forceinline__ void operator()(int level, int shift, int bits, uint32_t prefix,
-                                             uint32_t lo_key, const Add& add) const {
-    const uint32_t mask = (1u << bits) - 1u;
-    auto ok = [&](uint32_t k) { return k >= lo_key && (level == 0 || (k >> (shift + bits)) == prefix); };
-    const bool lin = c->lin && level == 0;
-    for_each_side3(*c, [&](int, float s) {
-      const uint32_t k = key_of(s);
-      const bool valid = ok(k);
-      add(valid, lin ? c->lin_bucket(k) : (k >> shift) & mask, 1u, (WITH_MASS && valid) ? mass_of(s, c->m) : 0ull);
-    });
-    for_each_class(*c, [&](const ClassEntry& e) {
-      add(ok(e.key), lin ? c->lin_bucket(e.key) : (e.key >> shift) & mask, e.cnt, WITH_MASS ? e.w : 0ull);
-    });
-  }
-};
-
-// Kept side elements keyed by ~id with their mass: the side part of the draw.
-struct SideDrawFill3 {
-  Ctx3* c;
-  uint32_t cut_key;
-  template <class Add>
-  __device__ __forceinline__ void operator()(int level, int shift, int bits, uint32_t prefix,
-                                             uint32_t, const Add& add) const {
-    const uint32_t mask = (1u << bits) - 1u;
-    for_each_side3(*c, [&](int id, float s) {
-      const uint32_t k = ~(uint32_t)id;
-      const bool valid = key_of(s) > cut_key && (level == 0 || (k >> (shift + bits)) == prefix);
-      add(valid, (k >> shift) & mask, 1u, valid ? mass_of(s, c->m) : 0ull);
-    });
-  }
-};
-
-// Gathers the members (side elements, classes) with key >= lo_key whose top `levels` radix
-// digits equal `prefix` into `list`, sorted by (key descending, classes first, id ascending).
-__device__ int gather_members3(Ctx3& c, uint32_t lo_key, int levels, uint32_t prefix) {
-  const int tid = threadIdx.x;
-  if (tid == 0) *c.gbuf_n = 0;
-  __syncthreads();
-  const int drop = levels == 1 ? 21 : (levels == 2 ? 10 : 0);
-  const bool lin = c.lin && levels == 1;
-  auto matches = [&](uint32_t k) {
-    if (k < lo_key) return false;
-    if (lin) return c.lin_bucket(k) == prefix;
-    return levels == 0 || (levels == 3 ? k == prefix : (k >> drop) == prefix);
-  };
-  for_each_side3(c, [&](int id, float s) {
-    const uint32_t k = key_of(s);
-    if (!matches(k)) return;
-    const int slot = atomicAdd(c.gbuf_n, 1);
-    if (slot < kV3ListCap) c.gbuf[slot] = V3Entry{k, id, 1u, 0u, mass_of(s, c.m)};
-  });
-  for_each_class(c, [&](const ClassEntry& e) {
-    if (!matches(e.key)) return;
-    const int slot = atomicAdd(c.gbuf_n, 1);
-    if (slot < kV3ListCap) c.gbuf[slot] = V3Entry{e.key, -1, e.cnt, e.cell, e.q};
-  });
-  __syncthreads();
-  if (c.dbg && tid == 0) c.dbg[20] = clock64();
-  const int n = min(*c.gbuf_n, kV3ListCap);
-  if (tid < n) {
-    const V3Entry mine = c.gbuf[tid];
-    int pos = 0;
-    for (int j = 0; j < n; ++j) {
-      const uint32_t kj = c.gbuf[j].key;
-      const int idj = c.gbuf[j].id;
-      // classes (id -1) sort before side elements of the same key; two classes of one key
-      // are ordered by their class index
-      const bool before = kj > mine.key ||
-                          (kj == mine.key && (idj < mine.id || (idj == mine.id && c.gbuf[j].cell < mine.cell)));
-      pos += before ? 1 : 0;
+// Count and mass of all tokens with key >= lo_key; hist (or null): a histogram that holds every token,
+// used when lo_key is 0.
+__device__ void totals3(Ctx3& c, uint32_t lo_key, bool filled, u64& cnt, u64& mass) {
+  u64 a = 0, b = 0;
+  if (filled && lo_key == 0u) {
+#pragma unroll
+    for (int u = 0; u < kV3Buckets / kThreads; ++u) {
+      const int i = threadIdx.x + u * kThreads;
+      a += c.hist[i];
+      b += hist_mass(c.hist, i);
     }
-    c.list[pos] = mine;
+  } else {
+    for_each_side3(c, [&](int, float s) {
+      if (key_of(s) >= lo_key) { ++a; b += mass_of(s, c.m); }
+    });
+    for_each_class(c, [&](bool valid, uint32_t key, uint32_t n, int) {
+      if (valid && key >= lo_key) { a += n; b += (u64)n * mass_of(score_of(key), c.m); }
+    });
   }
-  __syncthreads();
-  return n;
-}
-
-template <bool BY_MASS>
-__device__ Selection resolve3(Ctx3& c, Selection sel, uint32_t lo_key) {
-  if (!sel.ok || sel.levels == 3) return sel;
-  if (c.dbg && threadIdx.x == 0 && BY_MASS) { c.dbg[19] = clock64(); c.dbg[23] = (unsigned long long)sel.levels; }
-  const int n = gather_members3(c, lo_key, sel.levels, sel.prefix);
-  const int tid = threadIdx.x;
-  if (c.dbg && tid == 0 && BY_MASS) { c.dbg[21] = clock64(); c.dbg[24] = (unsigned long long)n; }
-  u64 a = 0, b = 0;
-  if (tid < n) { a = c.list[tid].cnt; b = a * c.list[tid].q; }
-  const u64 ia = warp_scan_u64(a), ib = warp_scan_u64(b);
-  u64 pa, pb, tc, tm;
-  block_warp_prefix2(*c.x, shfl_u64(ia, 31), shfl_u64(ib, 31), pa, pb, tc, tm);
-  if (c.dbg && tid == 0 && BY_MASS) c.dbg[34] = clock64();
-  const u64 want = sel.target - (BY_MASS ? sel.above_mass : sel.above_cnt);
-  if (tid == 0) c.x->bcast[7] = 0;
-  __syncthreads();
-  if (tid < n) {
-    const u64 incl = BY_MASS ? pb + ib : pa + ia;
-    const u64 excl = incl - (BY_MASS ? b : a);
-    if (excl < want && want <= incl) { c.x->bcast[0] = c.list[tid].key; c.x->bcast[7] = 1; }
-  }
-  __syncthreads();
-  if (c.x->bcast[7] == 0) {
-    sel.ok = false;
-    __syncthreads();
-    return sel;
-  }
-  const uint32_t key = (uint32_t)c.x->bcast[0];
-  if (c.dbg && tid == 0 && BY_MASS) c.dbg[35] = clock64();
-  // the list is sorted by key: what lies above the key's group and the group itself are read
-  // off the running sums at the group's two ends
-  if (tid < n && c.list[tid].key == key) {
-    if (tid == 0 || c.list[tid - 1].key != key) { c.x->bcast[1] = pa + ia - a; c.x->bcast[2] = pb + ib - b; }
-    if (tid == n - 1 || c.list[tid + 1].key != key) { c.x->bcast[3] = pa + ia; c.x->bcast[4] = pb + ib; }
-  }
-  __syncthreads();
-  const u64 ac = c.x->bcast[1], am = c.x->bcast[2];
-  const u64 bc = c.x->bcast[3] - ac, bm = c.x->bcast[4] - am;
-  sel.key = key;
-  sel.prefix = key;
-  sel.levels = 3;
-  sel.above_cnt += ac;
-  sel.above_mass += am;
-  sel.bin_cnt = bc;
-  sel.bin_mass = bm;
-  __syncthreads();
-  if (c.dbg && tid == 0 && BY_MASS) c.dbg[36] = clock64();
-  return sel;
-}
-
-template <bool BY_MASS, bool WITH_MASS>
-__device__ Selection select_union3(Ctx3& c, uint32_t lo_key, u64 target, float top_p) {
-  UnionFill3<WITH_MASS> fill{&c};
-  Selection sel = descend_local<BY_MASS>(c, fill, lo_key, target, top_p, (u64)kV3ListCap);
-  return resolve3<BY_MASS>(c, sel, lo_key);
-}
-
-// Count and mass of all tokens with key >= lo_key.
-__device__ void totals3(Ctx3& c, uint32_t lo_key, u64& cnt, u64& mass) {
-  u64 a = 0, b = 0;
-  for_each_side3(c, [&](int, float s) {
-    if (key_of(s) >= lo_key) { ++a; b += mass_of(s, c.m); }
-  });
-  for_each_class(c, [&](const ClassEntry& e) {
-    if (e.key >= lo_key) { a += e.cnt; b += e.w; }
-  });
   block_sum2(*c.x, a, b);
   cnt = a;
   mass = b;
@@ -581,8 +537,8 @@ struct Group {
 __device__ Group find_group(Ctx3& c, uint32_t key) {
   if (threadIdx.x < 3) c.x->bcast[threadIdx.x] = 0;
   __syncthreads();
-  for_each_class(c, [&](const ClassEntry& e) {
-    if (e.key == key) c.x->bcast[e.cell / kV3Bins] = (u64)e.cell + 1;
+  for_classes_at(c, 0, 0, [&](uint32_t k) { return k < key ? -1 : (k > key ? 1 : 0); }, [&](uint32_t, uint32_t, int cell) {
+    c.x->bcast[cell / kV3Bins] = (u64)cell + 1;
   });
   __syncthreads();
   Group g;
@@ -639,10 +595,10 @@ __device__ __forceinline__ u64 count_members(const Ctx3& c, const Group& g, int 
 }
 
 // Token id of the n-th (1-based, ascending id) member of the group (classes and side
-// elements whose score key is g.key), or 0x7fffffff.  The row is cut into one segment per
+// elements whose score key is g.key), or 0x7fffffff: for groups of any size.  The row is cut into one segment per
 // warp, members are counted, and the segment that holds the n-th is cut again until one
 // warp can rank its members with ballots.
-__device__ int nth_in_group(Ctx3& c, const Group& g, u64 n) {
+__device__ int nth_in_large_group(Ctx3& c, const Group& g, u64 n) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
   int b = 0, e = c.n8();
   u64 before = 0;
@@ -707,39 +663,47 @@ __device__ int nth_in_group(Ctx3& c, const Group& g, u64 n) {
   return result;
 }
 
-// Token id of the n-th (1-based, ascending id) of the `members` tokens of ONE class (count
-// class and one-value bin `cell`), for classes of at most kV3ScanCap tokens.  The row is walked from the end that is nearer to the n-th
-// member, 16,384 tokens per step, and the walk stops soon after the step that reaches it (it
-// looks every fourth step): members are spread evenly over the row, so on average a third of
-// it is read.  A class is one bf16 bit
-// pattern and a normal number (the bin window holds neither zeros nor NaNs), so two tokens are
-// compared with it by one native bf16x2 equality per 32-bit word; a hit looks its count class
-// up in the 16 class bits that travel with its chunk.  The ids found (in the gather and list
-// buffers, which are contiguous) are ranked among themselves.
-static_assert(kV3ScanCap * sizeof(int) <= 2 * kV3ListCap * sizeof(V3Entry), "scan ids fit the two buffers");
-// (Not inlined, and handed plain values instead of the row's context: inside the kernel's main
-// body its eight 128-bit registers in flight were spilled to local memory, which this kernel's
-// small L1 turns into round trips to L2 inside the loop.)
+// Token id of the n-th (1-based, ascending id) member of up to three classes, one per count class,
+// of at most kV3ScanCap tokens together.  The row is walked from the end that is nearer to the n-th
+// member, 16,384 tokens per step, and the walk stops soon after the step that reaches it (it looks
+// every other step): members are spread evenly over the row, so on average a third of it is read.
+// A class is one bf16 bit pattern and a normal number (the bin window holds neither zeros nor NaNs),
+// so two tokens are compared with it by one native bf16x2 equality per 32-bit word; a hit looks its
+// count class up in the 16 class bits that travel with its chunk.  The ids found are ranked among
+// themselves.  Bound by the latency of the row's loads (out of L2, or HBM when the row has left it):
+// a chunk's successor is requested as soon as the chunk has been compared, and one batch of four
+// 128-bit registers is all that is held (two batches were spilled: 26 thousand cycles for a third of
+// a 248,320-token row).
+static_assert(kV3ScanCap <= kV3TieCap - 4, "scan ids fit the list of ids");
+// (Not inlined, and handed plain values instead of the row's context: the registers of the kernel's
+// main body are all taken.)
 struct ScanArgs {
   const unsigned short* logits;
   const uint32_t* cls;
   int vocab, head, n8;
-  int* ids;       // [kV3ScanCap]
-  int* slot_n;    // ids used
+  int* ids;       // [kV3TieCap]
+  int* slot_n;    // ids in the list so far (the caller's own members first)
   int* step_n;    // [2]
   u64* result;    // id + 1 of the answer, or 0
-  unsigned long long* dbg;
 };
-__device__ __noinline__ void scan_small_class(const ScanArgs c, uint32_t raw, int cc, int n, int members) {
+constexpr uint32_t kNoRaw = 0x7fc0u;  // a NaN: equal to nothing
+template <bool ONE>  // one class (cc0, raw0); else raw0 / raw1 / raw2 of the count classes 0 / 1 / 2
+__device__ __noinline__ void scan_members(const ScanArgs c, uint32_t raw0, uint32_t raw1, uint32_t raw2, int cc0, int n, int members) {
   const int tid = threadIdx.x;
-  const uint32_t vv = raw | (raw << 16);
-  const __nv_bfloat162 vv2 = *reinterpret_cast<const __nv_bfloat162*>(&vv);
+  auto pair_of = [](uint32_t raw) {
+    const uint32_t v = raw | (raw << 16);
+    return *reinterpret_cast<const __nv_bfloat162*>(&v);
+  };
+  const __nv_bfloat162 v0 = pair_of(raw0), v1 = pair_of(raw1), v2 = pair_of(raw2);
+  auto member = [&](uint32_t raw, int cc) {
+    if (ONE) return raw == raw0 && cc == cc0;
+    return cc < 3 && raw == (cc == 0 ? raw0 : (cc == 1 ? raw1 : raw2));
+  };
   int* ids = c.ids;
   const bool forward = 2 * n <= members + 1;
   const int need = forward ? n : members - n + 1;  // counted from the end the walk starts at
-  if (tid == 0) { *c.slot_n = 0; c.step_n[0] = 0; c.step_n[1] = 0; *c.result = 0; }
+  if (tid == 0) { c.step_n[0] = 0; c.step_n[1] = 0; *c.result = 0; }
   __syncthreads();
-  if (c.dbg && tid == 0) c.dbg[40] = clock64();
   const int n8 = c.n8;
   const uint4* src4 = reinterpret_cast<const uint4*>(c.logits + c.head);
   // Members found are counted in two counters that take turns from one look to the next:
@@ -753,54 +717,56 @@ __device__ __noinline__ void scan_small_class(const ScanArgs c, uint32_t raw, in
   // the loose tokens at the end the walk starts from, and later those at its other end
   auto loose = [&](int from, int to, int parity) {
     const int id = from + tid;
-    if (id < to && (uint32_t)c.logits[id] == raw && (c.cls ? (int)((c.cls[id >> 4] >> ((id & 15) * 2)) & 3u) : 0) == cc) note(id, parity);
+    if (id < to && member((uint32_t)c.logits[id], c.cls ? (int)((c.cls[id >> 4] >> ((id & 15) * 2)) & 3u) : 0)) note(id, parity);
   };
   const int tail_at = c.head + 8 * n8;
   if (forward) loose(0, c.head, 0); else loose(tail_at, c.vocab, 0);
   constexpr int kBatch = 4;
   constexpr int kStep = kBatch * kThreads;  // chunks per step
-  constexpr int kCheckShift = 2;            // the walk looks whether it may stop every 2^kCheckShift steps
+  constexpr int kCheckShift = 1;            // the walk looks whether it may stop every 2^kCheckShift steps
   const int n_steps = (n8 + kStep - 1) / kStep;
-  uint4 w[kBatch], wn[kBatch];
-  uint32_t cl[kBatch], cn[kBatch];
+  uint4 w[kBatch];
+  uint32_t cl[kBatch];
   // chunk u of step s for this thread (steps are numbered in walking order)
   auto chunk_of = [&](int s, int u) { return (forward ? s : n_steps - 1 - s) * kStep + u * kThreads + tid; };
-  auto fetch = [&](uint4 (&dw)[kBatch], uint32_t (&dc)[kBatch], int s) {
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) {
-      const int i = chunk_of(s, u);
-      const bool in = s < n_steps && i < n8;
-      dw[u] = in ? __ldcg(src4 + i) : make_uint4(~vv, ~vv, ~vv, ~vv);
-      dc[u] = 0u;
-      if (in && c.cls) {
-        if (c.head == 0) {
-          dc[u] = (uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(c.cls) + i);
-        } else {
-          const int id = c.head + 8 * i;
-          dc[u] = __funnelshift_r(__ldcg(c.cls + (id >> 4)), __ldcg(c.cls + (id >> 4) + 1), (uint32_t)(id & 15) * 2u);
-        }
-      }
+  auto fetch = [&](int u, int s) {
+    const int i = chunk_of(s, u);
+    if (s >= n_steps || i >= n8) { w[u] = make_uint4(~0u, ~0u, ~0u, ~0u); return; }  // (NaNs: no hits)
+    w[u] = __ldcg(src4 + i);
+    if (!c.cls) return;
+    if (c.head == 0) {
+      cl[u] = (uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(c.cls) + i);
+    } else {
+      const int id = c.head + 8 * i;
+      cl[u] = __funnelshift_r(__ldcg(c.cls + (id >> 4)), __ldcg(c.cls + (id >> 4) + 1), (uint32_t)(id & 15) * 2u);
     }
   };
-  fetch(w, cl, 0);
+#pragma unroll
+  for (int u = 0; u < kBatch; ++u) { cl[u] = 0u; fetch(u, 0); }
   bool reached = false;
   int total = 0, seen[2] = {0, 0};
   for (int s = 0; s < n_steps; ++s) {
-    fetch(wn, cn, s + 1);
 #pragma unroll
     for (int u = 0; u < kBatch; ++u) {
-      const uint32_t m0 = __heq2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[u].x), vv2);
-      const uint32_t m1 = __heq2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[u].y), vv2);
-      const uint32_t m2 = __heq2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[u].z), vv2);
-      const uint32_t m3 = __heq2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[u].w), vv2);
+      const uint4 cur = w[u];
+      const uint32_t cur_cl = cl[u];
+      fetch(u, s + 1);
+      auto same = [&](uint32_t word) {
+        const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(&word);
+        uint32_t m = __heq2_mask(x, v0);
+        if (!ONE) m |= __heq2_mask(x, v1) | __heq2_mask(x, v2);
+        return m;
+      };
+      const uint32_t m0 = same(cur.x), m1 = same(cur.y), m2 = same(cur.z), m3 = same(cur.w);
       if (m0 | m1 | m2 | m3) {
-        const int id = c.head + 8 * chunk_of(s, u);
         uint32_t hits = ((m0 & 1u) | ((m0 >> 15) & 2u)) | (((m1 & 1u) | ((m1 >> 15) & 2u)) << 2) |
                         (((m2 & 1u) | ((m2 >> 15) & 2u)) << 4) | (((m3 & 1u) | ((m3 >> 15) & 2u)) << 6);
         while (hits) {
           const int q = __ffs(hits) - 1;
           hits &= hits - 1;
-          if ((int)((cl[u] >> (2 * q)) & 3u) == cc) note(id + q, (s >> kCheckShift) & 1);
+          const uint32_t word = q < 2 ? cur.x : (q < 4 ? cur.y : (q < 6 ? cur.z : cur.w));
+          if (member((word >> (16 * (q & 1))) & 0xffffu, (int)((cur_cl >> (2 * q)) & 3u)))
+            note(c.head + 8 * chunk_of(s, u) + q, (s >> kCheckShift) & 1);
         }
       }
     }
@@ -814,33 +780,65 @@ __device__ __noinline__ void scan_small_class(const ScanArgs c, uint32_t raw, in
       seen[turn] = now;
       if (total >= need) { reached = true; break; }
     }
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) { w[u] = wn[u]; cl[u] = cn[u]; }
   }
   if (!reached) { if (forward) loose(tail_at, c.vocab, 0); else loose(0, c.head, 0); }
-  if (c.dbg && tid == 0) c.dbg[43] = clock64();
   __syncthreads();
-  if (c.dbg && tid == 0) c.dbg[41] = clock64();
   const int found = min(*c.slot_n, kV3ScanCap);
+  if (tid < 4) ids[found + tid] = forward ? 0x7fffffff : -1;
+  __syncthreads();
   // every member on the near side of the last step's far end was noted: the one that `need - 1`
   // others precede (follow, when walking backwards) is the answer
   for (int t = tid; t < found; t += kThreads) {
     const int mine = ids[t];
     int before = 0;
-    for (int j = 0; j < found; ++j) before += (forward ? ids[j] < mine : ids[j] > mine) ? 1 : 0;
+    for (int j = 0; j < found; j += 4) {
+      const int4 o = *reinterpret_cast<const int4*>(ids + j);
+      before += forward ? (o.x < mine) + (o.y < mine) + (o.z < mine) + (o.w < mine)
+                        : (o.x > mine) + (o.y > mine) + (o.z > mine) + (o.w > mine);
+    }
     if (before + 1 == need) *c.result = (u64)mine + 1;
   }
   __syncthreads();
-  if (c.dbg && tid == 0) { c.dbg[42] = clock64(); c.dbg[44] = (unsigned long long)found; }
 }
+__device__ __forceinline__ ScanArgs scan_args(const Ctx3& c) {
+  return ScanArgs{c.logits, c.cls, c.vocab, c.head(), c.n8(), c.list, c.gbuf_n, c.step_n, &c.x->bcast[6]};
+}
+// ... of ONE class (cell), or -1 when it has more members than a scan holds.
 __device__ __forceinline__ int nth_in_small_class(Ctx3& c, int cell, u64 n, u64 members) {
   if (members > (u64)kV3ScanCap || n < 1 || n > members) return -1;
   const int cc = cell / kV3Bins;
-  const ScanArgs sa{c.logits, c.cls, c.vocab, c.head(), c.n8(), reinterpret_cast<int*>(c.gbuf), c.gbuf_n, c.step_n, &c.x->bcast[6], c.dbg};
-  scan_small_class(sa, v3_raw_of_bin(cell - cc * kV3Bins), cc, (int)n, (int)members);
+  if (threadIdx.x == 0) *c.gbuf_n = 0;
+  scan_members<true>(scan_args(c), v3_raw_of_bin(cell - cc * kV3Bins), kNoRaw, kNoRaw, cc, (int)n, (int)members);
   const u64 hit = c.x->bcast[6];
   __syncthreads();
   return hit ? (int)(hit - 1) : 0x7fffffff;
+}
+
+// Token id of the n-th member of a group: by one scan when the group is small enough.
+__device__ int nth_in_group(Ctx3& c, const Group& g, u64 n) {
+  auto count = [&](int cell) { return cell >= 0 ? (u64)c.tab[cell] : 0ull; };
+  auto raw = [&](int cell, int cc) { return cell >= 0 ? v3_raw_of_bin(cell - cc * kV3Bins) : kNoRaw; };
+  const u64 in_classes = count(g.cell0) + count(g.cell1) + count(g.cell2);
+  if (in_classes <= (u64)kV3ScanCap) {
+    // the group's side elements are noted first, whatever the walk will see
+    __syncthreads();
+    if (threadIdx.x == 0) *c.gbuf_n = 0;
+    __syncthreads();
+    for_each_side3(c, [&](int id, float s) {
+      if (key_of(s) != g.key) return;
+      const int slot = atomicAdd(c.gbuf_n, 1);
+      if (slot < kV3ScanCap) c.list[slot] = id;
+    });
+    __syncthreads();
+    const u64 all = in_classes + (u64)*c.gbuf_n;
+    if (all <= (u64)kV3ScanCap && n >= 1 && n <= all) {
+      scan_members<false>(scan_args(c), raw(g.cell0, 0), raw(g.cell1, 1), raw(g.cell2, 2), 0, (int)n, (int)all);
+      const u64 hit = c.x->bcast[6];
+      __syncthreads();
+      if (hit) return (int)(hit - 1);
+    }
+  }
+  return nth_in_large_group(c, g, n);
 }
 
 // Appends to the gather buffer the ids of all group members with id <= id_limit.
@@ -849,7 +847,7 @@ __device__ void emit_group_upto(Ctx3& c, const Group& g, int id_limit) {
   const uint4* src4 = c.chunks();
   auto emit = [&](int id) {
     const int slot = atomicAdd(c.gbuf_n, 1);
-    if (slot < kV3ListCap) c.gbuf[slot] = V3Entry{g.key, id, 1u, 0u, 0ull};
+    if (slot < kV3ListCap) c.gbuf[slot] = V3Entry{g.key, id};
   };
   for (int i = threadIdx.x; i < last; i += kThreads) {
     uint32_t memb = chunk_members(c, g, i, __ldcg(src4 + i), c.cls ? c.chunk_classes(i) : 0u);

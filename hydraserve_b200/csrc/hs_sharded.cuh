@@ -18,7 +18,7 @@ struct ShardArgs {
   hs_shard_rec* recs;   // [batch]
 };
 
-// smem: Exchange | cand[kCandCap] | mass[kCandCap] | count[kBins] | small[16]
+// smem: Exchange | cand[kCandCap] | mass[kCandCap] | count[kBins] | small[32]
 struct LayoutCand {
   size_t x, cand, mass, count, small, total;
 };
@@ -30,7 +30,7 @@ __host__ __device__ inline LayoutCand layout_cand() {
   l.cand = take(sizeof(u64) * kCandCap);
   l.mass = take(sizeof(u64) * kCandCap);
   l.count = take(sizeof(uint32_t) * kBins);
-  l.small = take(sizeof(int) * 16);
+  l.small = take(sizeof(int) * 32);
   l.total = off;
   return l;
 }
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kThreads, 2) shard_partial_kernel(const ShardA
   const bool slot_ok = P.slot >= 0 && P.slot < a.pool.slots_total;
   const bool penalised = slot_ok && (c.rp != 1.0f || c.pp != 0.0f || c.fp != 0.0f);
   c.cls = penalised ? a.pool.cls + (size_t)P.slot * a.pool.cls_stride : nullptr;
-  c.s_pair = nullptr; c.n_s = 0; c.s_cap = 0; c.cl = nullptr; c.n_cl = 0; c.m = 0.f;
+  c.s_pair = nullptr; c.n_s = 0; c.s_cap = 0; c.m = 0.f;
   c.tab = nullptr; c.hist = nullptr; c.gbuf = nullptr; c.list = nullptr; c.gbuf_n = nullptr;
   hs_shard_rec* rec = args.recs + c.row;
   if (tid < 16) small[tid] = 0;
