@@ -1,0 +1,702 @@
+// The counting path after the counting: one CTA turns a row's count table (hs_row_v3.cuh) into its
+// sample, in a few phases.  What the phases hand on lives in shared memory, and each phase is a function
+// of its own: in one body the values that are alive across it filled the 64 registers twice over,
+// and with two CTAs on an SM almost all of L1 is shared memory, so every spilled value was a round
+// trip to L2.
+#pragma once
+
+#include "hs_row_v3.cuh"
+#include "hs_row_topk.cuh"
+
+namespace hs {
+
+struct CountState {
+  Ctx3 c;
+  hs_row_params P;
+  hs_row_out out;        // the row's record, written out in one piece at the end
+  KeptSet kept;
+  V3Map all_map;         // every token, by score
+  u64 q_kept, n_kept, cut_group_cnt;
+  long long cut_ties;
+  u64 side_best;         // highest side element, (key, ~id); 0 = none
+  uint32_t max_key;
+  int status, token, scratch;
+  Group cut_group;
+  bool have_cut_group, tie_split, filled, slot_ok, penalised;
+  // from the launch's arguments
+  int row, flags, token_draw, s_cap_all, n_scratch;
+  int2* s_pair_all;
+  int* scratch_busy;
+  const float* noise;
+  float* scores_out;
+  int32_t* tokens_out;
+  hs_row_out* out_row;
+  unsigned long long* clocks;
+};
+static_assert(sizeof(CountState) <= kStateBytes, "the state fits its place");
+__device__ __forceinline__ CountState& count_state() { return *at_smem<kLayV3.state, CountState>(); }
+__device__ __forceinline__ int* count_small() { return at_smem<kLayV3.small, int>(); }
+__device__ __forceinline__ void phase_mark(const CountState& S, int slot) {
+  if (S.clocks && threadIdx.x == 0) S.clocks[slot] = clock64();
+}
+// Sets a field of the state (the same value in every thread; visible after the next barrier).
+template <class T, class V>
+__device__ __forceinline__ void put_state(T& field, V value) {
+  if (threadIdx.x == 0) field = (T)value;
+}
+__device__ __forceinline__ void raise_status(CountState& S, int bits) {
+  if (threadIdx.x == 0) S.status |= bits;
+}
+
+// Global scratch, for side lists that shared memory does not hold, is kept per RESIDENT CTA: a CTA in
+// need claims one of the n_scratch sets (as many as CTAs can be resident, so one is always free),
+// starting its search at the pair of its SM, and gives it back at the end.
+__device__ bool claim_scratch(CountState& S) {
+  if (threadIdx.x == 0) {
+    unsigned smid;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+    int got = -1;
+    for (int k = 0; k < 2 * S.n_scratch && got < 0; ++k) {
+      const int at = (int)((2u * smid + (unsigned)k) % (unsigned)S.n_scratch);
+      if (atomicCAS(&S.scratch_busy[at], 0, 1) == 0) got = at;
+    }
+    S.scratch = got;
+    if (got >= 0) { S.c.s_pair = S.s_pair_all + (size_t)got * S.s_cap_all; S.c.s_cap = S.s_cap_all; }
+  }
+  __syncthreads();
+  return S.scratch >= 0;
+}
+
+// The side list (tokens held three times or more, values outside the bin window), the row's maximum
+// and minimum, and every token's count and mass in one histogram over the scores.  False: no scratch.
+__device__ __noinline__ bool phase_histogram() {
+  CountState& S = count_state();
+  Ctx3& c = S.c;
+  int* small = count_small();
+  const int tid = threadIdx.x, lane = tid & 31;
+  const bool penalised = S.penalised;
+  // (id, count, value) of a token held three times or more are three dependent reads: thread t
+  // starts the chain for list entry t here and takes one step of it at each stop below
+  int n_heavy = 0, hv_q = -1;
+  const int cap = c.pool.unique_cap;
+  const int32_t* heavy = c.pool.heavy + (size_t)max(c.slot, 0) * cap;
+  const int2* pairs = c.pool.pairs + (size_t)max(c.slot, 0) * cap;
+  if (penalised) {
+    n_heavy = load_now_s32(c.pool.n_heavy + c.slot);
+    if (tid < cap) hv_q = load_now_s32(heavy + tid);
+  }
+  // ---- highest and lowest non-empty cell of each count class: scores grow with the bin inside one
+#pragma unroll 1
+  for (int k = 0; k < (penalised ? 3 : 1); ++k) {  // (without penalties there is one count class)
+    uint32_t bits = 0;
+#pragma unroll
+    for (int u = 0; u < kPerClass; ++u) bits |= (c.tab()[tid + (k * kPerClass + u) * kThreads] ? 1u : 0u) << u;
+    const uint32_t t = __reduce_max_sync(0xffffffffu, bits ? (uint32_t)(tid + (k * kPerClass + 31 - __clz(bits)) * kThreads) + 1u : 0u);
+    const uint32_t l = __reduce_min_sync(0xffffffffu, bits ? (uint32_t)(tid + (k * kPerClass + __ffs(bits) - 1) * kThreads) : 0xffffffffu);
+    if (lane == 0) {
+      if (t) atomicMax(reinterpret_cast<unsigned*>(small) + 16 + k, t);
+      if (l != 0xffffffffu) atomicMin(reinterpret_cast<unsigned*>(small) + 19 + k, l);
+    }
+  }
+  // (more often-repeated tokens than the side list holds: the general kernel's row)
+  if (n_heavy > min(cap, S.s_cap_all)) raise_status(S, 4);
+  n_heavy = min(n_heavy, min(cap, S.s_cap_all));
+  int2 hv_pair = make_int2(-1, 0);
+  if (tid < n_heavy && hv_q >= 0 && hv_q < cap) hv_pair = load_now_int2(pairs + hv_q);  // (id, count)
+  const int n_rare = small[1];
+  if (n_rare > kV3RareCap || n_heavy + kV3RareCap > kV3SideShared) {
+    if (!claim_scratch(S)) return false;
+  }
+  // ---- the side list.  It is walked by every selection, so it lives in shared memory when it fits.
+  {
+    const Ctx3 k = c;  // (what scoring needs, in registers)
+    u64 side_best = 0;
+    uint32_t side_worst = 0xffffffffu;  // this thread's lowest side key
+    auto put = [&](int slot, int id, float s) {
+      if (slot >= k.s_cap) return;  // (reported below, from the counts, by every thread alike)
+      k.s_pair[slot] = make_int2(id, __float_as_int(s));
+      const u64 packed = ((u64)key_of(s) << 32) | (uint32_t)(~(uint32_t)id);
+      side_best = packed > side_best ? packed : side_best;
+      side_worst = min(side_worst, key_of(s));
+    };
+    for (int j = tid; j < n_heavy; j += kThreads) {
+      if (j != tid) {  // (the first entry's reads were started early)
+        const int q = heavy[j];
+        hv_pair = q >= 0 && q < cap ? pairs[q] : make_int2(-1, 0);
+      }
+      if (hv_pair.x < 0 || hv_pair.x >= k.vocab) { if (j < k.s_cap) k.s_pair[j] = make_int2(-1, 0); }
+      else put(j, hv_pair.x, k.score_of(k.logits[hv_pair.x], hv_pair.y));
+    }
+    int n_s = n_heavy + n_rare;
+    if (n_rare <= kV3RareCap) {
+      const int2* rare = c.rare();
+      for (int t = tid; t < n_rare; t += kThreads) {
+        const int2 e = rare[t];
+        put(n_heavy + t, e.x, k.score_of((uint32_t)e.y & 0xffffu, (e.y >> 16) & 3));
+      }
+    } else {
+      // too many to remember: sweep the row again for out-of-window values
+      for (int id = tid; id < k.vocab; id += kThreads) {
+        const uint32_t raw = k.logits[id];
+        const int cc = k.class_of(id);
+        if (cc == 3 || v3_bin_of_raw(raw) >= 0) continue;
+        put(n_heavy + atomicAdd(small + 2, 1), id, k.score_of(raw, cc));
+      }
+      __syncthreads();
+      n_s = n_heavy + small[2];
+    }
+    // more than the list holds: the row is reported for the general kernel (from the counts, not by
+    // the thread whose token found no room)
+    if (n_s > k.s_cap) raise_status(S, 4);
+    put_state(c.n_s, min(n_s, k.s_cap));
+    const u64 sb = warp_max_u64(side_best);
+    const uint32_t sl = __reduce_min_sync(0xffffffffu, side_worst);
+    if (lane == 0) {
+      if (sb) atomicMax(&c.x()->bcast[5], sb);
+      if (sl != 0xffffffffu) atomicMin(reinterpret_cast<unsigned*>(small) + 22, sl);
+    }
+  }
+  __syncthreads();
+  phase_mark(S, 11);
+  // ---- row maximum and minimum: the scores of six cells, one per lane, and the side list's ends
+  {
+    const bool top = lane < 3;
+    const uint32_t mark_at = reinterpret_cast<unsigned*>(small)[(top ? 16 : 19) + lane % 3];
+    const bool valid = lane < 6 && (top ? mark_at != 0u : mark_at != 0xffffffffu);
+    uint32_t key = 0;
+    if (valid) key = key_of(c.cell_score(top ? (int)mark_at - 1 : (int)mark_at));
+    const u64 side_best = c.x()->bcast[5];
+    const uint32_t max_key = max(__reduce_max_sync(0xffffffffu, valid && top ? key : 0u), (uint32_t)(side_best >> 32));
+    const uint32_t min_key = min(__reduce_min_sync(0xffffffffu, valid && !top ? key : 0xffffffffu), reinterpret_cast<unsigned*>(small)[22]);
+    if (tid == 0) {
+      S.side_best = side_best;
+      S.max_key = max_key;
+      c.m = score_of(max_key);
+      V3Map map;
+      map.by_score(score_of(min_key), score_of(max_key));
+      S.all_map = map;
+    }
+  }
+  __syncthreads();
+  phase_mark(S, 2);
+  // ---- the histogram (in the place of the rare tokens and set-aside chunks, which have served)
+  if (!c.greedy || S.P.n_logprobs >= 0) {
+    hist_fill<true>(c.hist(), AllTokens3{&c}, S.all_map);
+    put_state(S.filled, true);
+    __syncthreads();
+  }
+  phase_mark(S, 3);
+  return true;
+}
+
+// Top-k, min-p and top-p.  What a cut keeps lies at the top, so every cut is looked for among all tokens.
+__device__ __noinline__ void phase_cuts() {
+  CountState& S = count_state();
+  Ctx3& c = S.c;
+  const hs_row_params& P = S.P;
+  const int tid = threadIdx.x;
+  const float m = c.m;
+  bool filled = S.filled;
+  uint32_t cut_key = 0;
+  u64 cnt = 0, mass = 0;
+  bool have_totals = false;
+  if (P.top_k > 0 && P.top_k < c.vocab) {
+    const Selection sk = select_key<false, true>(c, AllTokens3{&c}, S.all_map, filled, (u64)P.top_k);
+    if (!sk.ok) raise_status(S, 1);
+    cut_key = sk.key;
+    cnt = sk.above_cnt + sk.bin_cnt;
+    mass = sk.above_mass + sk.bin_mass;
+    have_totals = sk.ok;
+    put_state(S.out.n_after_topk, cnt);
+    put_state(S.cut_group_cnt, sk.bin_cnt);
+  }
+  phase_mark(S, 4);
+  if (P.min_p > 0.0f) {
+    if (!have_totals) { totals3(c, cut_key, filled, cnt, mass); have_totals = true; }
+    const float z1 = mass_to_float(mass);
+    const float thr = __fmul_rn(__fdiv_rn(1.0f, z1), P.min_p);
+    uint32_t lowest = 0xffffffffu;
+    auto consider = [&](uint32_t k) {
+      if (k >= cut_key && !(__fdiv_rn(expf(score_of(k) - m), z1) < thr)) lowest = min(lowest, k);
+    };
+    for_each_class(c, [&](bool valid, uint32_t key, uint32_t, int) { if (valid) consider(key); });
+    for_each_side3(c, [&](int, float s) { consider(key_of(s)); });
+    lowest = ~block_max_u32(*c.x(), ~lowest);
+    if (lowest != 0xffffffffu && lowest > cut_key) {
+      cut_key = lowest;
+      have_totals = false;
+    }
+  }
+  phase_mark(S, 5);
+  if (!have_totals) totals3(c, cut_key, filled, cnt, mass);
+  put_state(S.out.n_after_minp, cnt);
+  if (P.top_p < 1.0f) {
+    Selection sp{};
+    if (mass > 0) {
+      // (double precision, slow: the lanes of one warp try neighbouring candidates at once)
+      if (tid < 32) {
+        const u64 t = top_p_target_warp(mass, P.top_p);
+        if (tid == 0) c.x()->bcast[6] = t;
+      }
+      __syncthreads();
+      phase_mark(S, 20);
+      sp = select_key<true, true>(c, AllTokens3{&c}, S.all_map, filled, c.x()->bcast[6]);
+      phase_mark(S, 21);
+    }
+    if (sp.ok && sp.bin_cnt > 0) {
+      const u64 qv = sp.bin_mass / sp.bin_cnt;  // every token at the cut key has the same mass
+      u64 t = sp.bin_cnt;
+      if (qv > 0) {
+        const u64 want = sp.target - sp.above_mass;
+        t = (want + qv - 1) / qv;
+        if (t < 1) t = 1;
+        if (t > sp.bin_cnt) t = sp.bin_cnt;
+      }
+      cut_key = sp.key;
+      cnt = sp.above_cnt + t;
+      mass = sp.above_mass + t * qv;
+      put_state(S.cut_ties, (long long)t);
+      put_state(S.cut_group_cnt, sp.bin_cnt);
+      put_state(S.tie_split, t < sp.bin_cnt);
+    } else {
+      raise_status(S, 1);
+    }
+  }
+  put_state(S.kept.cut_key, cut_key);
+  put_state(S.n_kept, cnt);
+  put_state(S.q_kept, mass);
+  put_state(S.filled, filled);
+  __syncthreads();
+  phase_mark(S, 6);
+}
+
+__device__ __forceinline__ void need_cut_group(CountState& S) {
+  if (S.have_cut_group) return;
+  const Group g = find_group(S.c, S.kept.cut_key);
+  put_state(S.cut_group, g);
+  put_state(S.have_cut_group, true);
+  __syncthreads();
+}
+// The highest id of the cut's tie group that is kept, when top-p split the group.
+__device__ __noinline__ void need_tie_limit() {
+  CountState& S = count_state();
+  if (!S.tie_split || S.kept.tie_limit != 0x7fffffff) return;
+  need_cut_group(S);
+  const int limit = nth_in_group(S.c, S.cut_group, (u64)S.cut_ties);
+  __syncthreads();
+  put_state(S.kept.tie_limit, limit);
+  __syncthreads();
+}
+
+// What a draw asks for when it does not know the token yet: the nth (by ascending id) member of
+// the cut's tie group, or of one class.
+struct DrawAsk {
+  int kind;  // 0 = the token is known (or there is none), 1 = of the group, 2 = of a class
+  int token;
+  int cell;
+  u64 nth, members;
+};
+
+// The draw by classes: inverse CDF over exact integer masses in the order: classes above the cut, the
+// tie group at the cut (its lowest ids), side elements above the cut (by id).
+__device__ __forceinline__ DrawAsk draw_by_classes(CountState& S, uint64_t seed) {
+  Ctx3& c = S.c;
+  const int tid = threadIdx.x;
+  const uint32_t cut_key = S.kept.cut_key;
+  const float m = c.m;
+  DrawAsk ask{0, -1, -1, 0ull, 0ull};
+  u64 target;
+  {
+    const Philox4 r = philox4x32_10(0u, 0u, 0u, 0u, (uint32_t)seed, (uint32_t)(seed >> 32));
+    target = __umul64hi(((u64)r.v[0] << 32) | r.v[1], S.q_kept);
+  }
+  // Classes above the cut in this order: the non-empty cells t, t + kThreads, ... of every t in
+  // turn make a list, and its entries j, j + kThreads, ... are chunk j.  (Any fixed order
+  // would do; the counts alone decide it.)  A thread adds its cells' masses to their chunks.
+  const uint32_t* tab = c.tab();
+  const int n_cells = (S.penalised ? 3 : 1) * kPerClass;
+  int mine = 0;
+#pragma unroll 4
+  for (int u = 0; u < n_cells; ++u) mine += tab[tid + u * kThreads] ? 1 : 0;
+  uint32_t* chunks = reinterpret_cast<uint32_t*>(c.members());  // [3][kThreads]: mass in limbs
+  static_assert(3 * kThreads * sizeof(uint32_t) <= sizeof(V3Member) * kV3ListCap + sizeof(int) * kV3TieCap, "the chunks fit the members' place");
+#pragma unroll
+  for (int l = 0; l < 3; ++l) chunks[tid + l * kThreads] = 0;
+  int n_cl;
+  const int list_at = block_place(count_small() + 48, mine, n_cl);
+  {
+    const Scorer sc = c;
+    int at = list_at;
+    constexpr int kBatch = 3;  // (scoring a cell is a long chain)
+    static_assert(kPerClass % kBatch == 0, "a batch is of one count class");
+#pragma unroll 1
+    for (int u0 = 0; u0 < n_cells; u0 += kBatch) {
+      uint32_t n[kBatch], key[kBatch];
+      u64 w[kBatch];
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) n[u] = tab[tid + (u0 + u) * kThreads];
+      if (!__any_sync(0xffffffffu, (n[0] | n[1] | n[2]) != 0u)) continue;
+      const int k = u0 / kPerClass;
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) {
+        key[u] = sc.key_of_bin(tid + (u0 + u) * kThreads - k * kV3Bins, k);
+        w[u] = (u64)n[u] * mass_of(score_of(key[u]), m);
+      }
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) {
+        if (!n[u]) continue;
+        if (key[u] > cut_key) {
+          uint32_t* dst = chunks + (at & (kThreads - 1));
+          atomicAdd(dst, (uint32_t)w[u] & kLimbMask);
+          atomicAdd(dst + kThreads, (uint32_t)(w[u] >> kLimbBits) & kLimbMask);
+          atomicAdd(dst + 2 * kThreads, (uint32_t)(w[u] >> (2 * kLimbBits)));
+        }
+        ++at;
+      }
+    }
+  }
+  __syncthreads();
+  const u64 chunk = (u64)chunks[tid] + ((u64)chunks[tid + kThreads] << kLimbBits) + ((u64)chunks[tid + 2 * kThreads] << (2 * kLimbBits));
+  const u64 incl = warp_scan_u64(chunk);
+  u64 pre, pre_unused, q_cells, tot_unused;
+  block_warp_prefix2(*c.x(), shfl_u64(incl, 31), 0, pre, pre_unused, q_cells, tot_unused);
+  phase_mark(S, 12);
+  if (target < q_cells) {
+    // the chunk that holds the target, its cells in order (a thread has at most one of them:
+    // its entries of the list are fewer than kThreads and lie side by side), then the cell
+    int* cells = c.list();
+    constexpr int kMostCells = kCells / kThreads;
+    if (tid < kMostCells) cells[tid] = -1;
+    if (tid == 0) c.x()->bcast[5] = 0;
+    const u64 from = pre + incl - chunk;
+    if (from <= target && target < from + chunk) { c.x()->bcast[0] = (u64)tid; c.x()->bcast[1] = from; }
+    __syncthreads();
+    {
+      int skip = ((int)c.x()->bcast[0] - list_at) & (kThreads - 1);
+      if (skip < mine) {
+        const int slot = (list_at + skip) / kThreads;
+        int cell = tid;
+        while (tab[cell] == 0u || skip-- > 0) cell += kThreads;
+        cells[slot] = cell;
+      }
+    }
+    __syncthreads();
+    if (tid < 32) {
+      u64 run = c.x()->bcast[1];
+      for (int base = 0; base < kMostCells; base += 32) {
+        const int cell = base + tid < kMostCells ? cells[base + tid] : -1;
+        u64 q = 0, w = 0;
+        if (cell >= 0) {
+          const uint32_t key = key_of(c.cell_score(cell));
+          if (key > cut_key) { q = mass_of(score_of(key), m); w = (u64)tab[cell] * q; }
+        }
+        const u64 in = warp_scan_u64(w);
+        if (w && run + in - w <= target && target < run + in) {
+          c.x()->bcast[3] = tab[cell];
+          c.x()->bcast[4] = (target - (run + in - w)) / q + 1;
+          c.x()->bcast[5] = (u64)cell + 1;
+        }
+        run += shfl_u64(in, 31);
+      }
+    }
+    __syncthreads();
+    ask.cell = (int)c.x()->bcast[5] - 1;
+    ask.members = c.x()->bcast[3];
+    ask.nth = c.x()->bcast[4];
+    ask.kind = ask.cell >= 0 ? 2 : 0;
+    __syncthreads();
+    return ask;
+  }
+  // the group at the cut key: cut_ties members when top-p split it, else all of them
+  u64 group_kept = (u64)S.cut_ties;
+  if (S.cut_ties < 0) {
+    // cut by top-k / min-p / nothing: everything at the cut key is kept; count it
+    u64 gc = 0, gm = 0;
+    for_classes_at(c, 0, 0, [&](uint32_t k) { return k < cut_key ? -1 : (k > cut_key ? 1 : 0); },
+                   [&](uint32_t, uint32_t n, int) { gc += n; });
+    for_each_side3(c, [&](int, float s) { if (key_of(s) == cut_key) gc += 1; });
+    block_sum2(*c.x(), gc, gm);
+    group_kept = gc;
+  }
+  const u64 q_cut = mass_of(score_of(cut_key), m);
+  const u64 q_group = group_kept * q_cut;
+  if (target < q_cells + q_group) {
+    ask.kind = 1;
+    ask.nth = q_cut ? (target - q_cells) / q_cut + 1 : 1;
+    return ask;
+  }
+  V3Map by_id;
+  by_id.by_key(~(uint32_t)(c.vocab - 1), 0xffffffffu);
+  bool filled = false;
+  const Selection sd = select_key<true, true>(c, KeptSide3{&c, cut_key}, by_id, filled, target - q_cells - q_group + 1);
+  put_state(S.filled, false);
+  if (sd.ok) ask.token = (int)(~sd.key);
+  return ask;
+}
+
+// Finds what a draw asks for: its own function, for the registers of the scan.
+__device__ __noinline__ int phase_find(const DrawAsk ask) {
+  CountState& S = count_state();
+  Ctx3& c = S.c;
+  if (ask.kind == 1) {
+    need_cut_group(S);
+    return nth_in_group(c, S.cut_group, ask.nth);  // the kept members are the lowest ids
+  }
+  // a uniformly chosen member of ONE class (not of other classes that share its key):
+  // large classes by rejection (about vocab / members scattered probes, which a lone CTA
+  // issues slowly), classes of up to kV3RejectMin tokens by one scan of the row
+  int token = -1;
+  const int cell = ask.cell;
+  if (ask.members > (u64)kV3RejectMin) {
+    const u64 per_round = ((u64)c.vocab + ask.members - 1) / ask.members;  // probes for ~63 % success
+    const int trials = (int)min((u64)kRandomTrials, max(1ull, (per_round + kThreads - 1) / kThreads));
+    // a class the scan can hold gets a few rounds, then the scan; a larger one many
+    token = random_in_class(c, cell, trials, S.P.seed, ask.members <= (u64)kV3ScanCap ? 4 : 32);
+  }
+  if (token >= 0) return token;
+  // (no key: no other member can match)
+  const Group only{0xffffffffu, cell < kV3Bins ? cell : -1, cell >= kV3Bins && cell < 2 * kV3Bins ? cell : -1,
+                   cell >= 2 * kV3Bins ? cell : -1};
+  return nth_in_group(c, only, ask.nth);
+}
+
+__device__ __noinline__ DrawAsk phase_draw() {
+  CountState& S = count_state();
+  Ctx3& c = S.c;
+  const int tid = threadIdx.x;
+  const uint64_t seed = S.P.seed;
+  DrawAsk ask{0, -1, -1, 0ull, 0ull};
+  if (S.q_kept == 0) return ask;  // (nothing has any mass: reported by the caller)
+  if (S.noise) {
+    // reference draws: arg max of fl(fl(e / z) / noise) over the kept set, lowest id on ties
+    need_tie_limit();
+    const KeptSet kept = S.kept;
+    const float zf = mass_to_float(S.q_kept), m = c.m;
+    const float* noise_row = S.noise + (size_t)S.row * c.vocab;
+    u64 best = 0;
+    for (int id = tid; id < c.vocab; id += kThreads) {
+      const float s = c.element_score(id, c.logits[id], c.class_of(id));
+      if (!kept.has(key_of(s), id)) continue;
+      const float p = __fdiv_rn(expf(s - m), zf);
+      const float ratio = __fdiv_rn(p, noise_row[id]);
+      const u64 packed = ((u64)__float_as_uint(ratio) << 32) | (uint32_t)(~(uint32_t)id);
+      best = packed > best ? packed : best;
+    }
+    best = block_max_u64(*c.x(), best);
+    ask.token = (int)(~(uint32_t)(best & 0xffffffffu));
+    return ask;
+  }
+  // Near-flat rows: rejection on tokens, when one round is all but sure to accept.
+  const float q = mass_to_float(S.q_kept);
+  if (S.token_draw && q * (float)(kTokenTrials * kThreads) >= 4.0f * (float)c.vocab) {
+    bool group_hit;
+    // (a sixteenth of the trials accepted on average: one per thread is plenty)
+    const int trials = q * 16.0f >= (float)c.vocab ? 1 : kTokenTrials;
+    const u64 ties = S.cut_ties > 0 ? (u64)S.cut_ties : 0ull;
+    const int t = draw_by_token_rejection(c, S.kept, S.tie_split, ties, S.cut_group_cnt, seed, 4, trials, group_hit);
+    if (t >= 0) {
+      ask.token = t;
+      if (group_hit) {
+        // one of the kept members of the group the cut splits: its lowest ids
+        const Philox4 r = philox4x32_10(0u, 0u, 0u, 4u, (uint32_t)seed, (uint32_t)(seed >> 32));
+        ask.kind = 1;
+        ask.nth = 1 + __umul64hi(((u64)r.v[0] << 32) | r.v[1], ties);
+      }
+      return ask;
+    }
+  }
+  return draw_by_classes(S, seed);
+}
+
+// Arg max with penalties: the lowest id among the tokens whose score key is the maximum.
+__device__ __noinline__ void phase_greedy() {
+  CountState& S = count_state();
+  Ctx3& c = S.c;
+  int* small = count_small();
+  int* low_id = small + 3;
+  const uint32_t max_key = S.max_key;
+  const int side_arg = (int)(~(uint32_t)(S.side_best & 0xffffffffu));
+  if (threadIdx.x == 0) *low_id = (uint32_t)(S.side_best >> 32) == max_key ? side_arg : 0x7fffffff;
+  CandCtx bound_ctx{nullptr, nullptr, nullptr, nullptr, small + 8, nullptr};
+  cand_thresholds(c, bound_ctx, max_key);  // (ends with a barrier)
+  {
+    const Ctx3 k = c;
+    stream_at_or_above(k, bound_ctx.thr, [&](int id, uint32_t raw, int cc) {
+      if (v3_bin_of_raw(raw) >= 0 && key_of(k.score_of(raw, cc)) == max_key) atomicMin(low_id, id);
+    });
+  }
+  __syncthreads();
+  int token = *low_id;
+  if (token == 0x7fffffff) { token = S.side_best ? side_arg : 0; raise_status(S, 1); }
+  put_state(S.token, token);
+  if (S.P.n_logprobs >= 0) {
+    u64 cn, q;
+    totals3(c, 0u, S.filled, cn, q);
+    put_state(S.q_kept, q);
+  }
+  __syncthreads();
+}
+
+// Log-probabilities: of the token, and of the N highest kept ones.
+__device__ __noinline__ void phase_logprobs() {
+  CountState& S = count_state();
+  Ctx3& c = S.c;
+  int* small = count_small();
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    S.out.log_z = (float)(log((double)S.q_kept) - (double)kMassShift * 0.6931471805599453);
+    const int token = S.token;
+    if (token >= 0 && token < c.vocab)
+      S.out.logprob = (c.element_score(token, c.logits[token], c.class_of(token)) - c.m) - S.out.log_z;
+  }
+  int n_want = min(S.P.n_logprobs, c.vocab);
+  if ((u64)n_want > S.n_kept) n_want = (int)S.n_kept;
+  if (n_want > 0) {
+    bool filled = S.filled;
+    // (the kept tokens are the highest: the N highest of them are the N highest of all)
+    const Selection sn = select_key<false, false>(c, AllTokens3{&c}, S.all_map, filled, (u64)n_want);
+    if (sn.ok) {
+      const int need = n_want - (int)sn.above_cnt;  // lowest ids of the group at the N-th key
+      // The tokens above the N-th key (fewer than N) and the group at it: side elements come
+      // from the side list, the rest from one walk of the row against per-class raw
+      // thresholds.  The group's ids go to a list of their own; a group too large for it is
+      // walked the slow way.
+      int* tie_ids = c.list();
+      int* tie_n = small + 3;
+      int* gbuf_n = c.gbuf_n();
+      V3Entry* gbuf = c.gbuf();
+      if (tid == 0) { *gbuf_n = 0; *tie_n = 0; }
+      __syncthreads();
+      const uint32_t nth_key = sn.key;
+      auto take = [&](uint32_t k, int id) {
+        if (k > nth_key) {
+          const int slot = atomicAdd(gbuf_n, 1);
+          if (slot < kV3ListCap) gbuf[slot] = V3Entry{k, id};
+        } else if (k == nth_key && need > 0) {
+          const int slot = atomicAdd(tie_n, 1);
+          if (slot < kV3TieCap) tie_ids[slot] = id;
+        }
+      };
+      for_each_side3(c, [&](int id, float s) { take(key_of(s), id); });
+      CandCtx bound_ctx{nullptr, nullptr, nullptr, nullptr, small + 8, nullptr};
+      cand_thresholds(c, bound_ctx, nth_key);  // (ends with a barrier)
+      phase_mark(S, 16);
+      {
+        const Ctx3 k = c;
+        stream_at_or_above(k, bound_ctx.thr, [&](int id, uint32_t raw, int cc) {
+          if (v3_bin_of_raw(raw) < 0) return;  // outside the bin window: a side element, taken above
+          take(key_of(k.score_of(raw, cc)), id);
+        });
+      }
+      __syncthreads();
+      phase_mark(S, 17);
+      if (need > 0) {
+        const int n_tie = *tie_n;
+        if (n_tie <= kV3TieCap) {
+          // the `need` lowest ids of the group: each id counts the ids below it
+          for (int t = tid; t < n_tie; t += kThreads) {
+            const int mine = tie_ids[t];
+            int below = 0;
+#pragma unroll 4
+            for (int j = 0; j < n_tie; ++j) below += tie_ids[j] < mine ? 1 : 0;
+            if (below < need) {
+              const int slot = atomicAdd(gbuf_n, 1);
+              if (slot < kV3ListCap) gbuf[slot] = V3Entry{nth_key, mine};
+            }
+          }
+        } else {
+          const int have = *gbuf_n;  // (the walk below counts in the same place)
+          const Group g = find_group(c, nth_key);
+          const int last_id = nth_in_group(c, g, (u64)need);
+          if (tid == 0) *gbuf_n = have;
+          __syncthreads();
+          emit_group_upto(c, g, last_id == 0x7fffffff ? -1 : last_id);
+        }
+      }
+      __syncthreads();
+      if (tid < 32) {
+        const int n = min(*gbuf_n, HS_MAX_LOGPROBS);
+        uint32_t kv = 0;
+        int id = 0x7fffffff;
+        if (tid < n) { kv = gbuf[tid].key; id = gbuf[tid].id; }
+        int pos = 0;
+        for (int j = 0; j < n; ++j) {
+          const uint32_t kj = __shfl_sync(0xffffffffu, kv, j);
+          const int idj = __shfl_sync(0xffffffffu, id, j);
+          if (kj > kv || (kj == kv && idj < id)) ++pos;
+        }
+        const float log_z = S.out.log_z;
+        if (tid < n) {
+          S.out.top_ids[pos] = id;
+          S.out.top_logprobs[pos] = (score_of(kv) - c.m) - log_z;
+        }
+        if (tid == 0 && n != n_want) S.status |= 8;
+      }
+    } else {
+      n_want = 0;
+      raise_status(S, 1);
+    }
+  }
+  put_state(S.out.n_top, n_want);
+  __syncthreads();
+  phase_mark(S, 8);
+}
+
+// From the row's count table (and rare tokens) to its record.
+__device__ __forceinline__ void finish_counted_row() {
+  CountState& S = count_state();
+  Ctx3& c = S.c;
+  const int tid = threadIdx.x;
+  if (!phase_histogram()) {  // cannot happen while n_scratch covers the resident CTAs; fail the row, do not wait
+    if (tid == 0) { S.out.token = 0; S.out.status = 128; S.out.n_top = 0; S.out.n_kept = 0; }
+    __syncthreads();
+    if (tid < 32) write_record(S.out_row, S.out, false);
+    return;
+  }
+  if (c.greedy) {
+    phase_greedy();
+  } else {
+    phase_cuts();
+    const DrawAsk ask = phase_draw();
+    phase_mark(S, 14);
+    int token = ask.token;
+    if (ask.kind) token = phase_find(ask);
+    if (token < 0 || token == 0x7fffffff) {
+      token = S.side_best ? (int)(~(uint32_t)(S.side_best & 0xffffffffu)) : 0;
+      raise_status(S, 1);
+    }
+    put_state(S.token, token);
+    __syncthreads();
+  }
+  phase_mark(S, 7);
+  if (S.P.n_logprobs >= 0) phase_logprobs();
+  // ---- optional dump of the final scores (parity tests)
+  if (S.scores_out) {
+    need_tie_limit();
+    float* dst = S.scores_out + (size_t)S.row * c.vocab;
+    const float ninf = __int_as_float(0xff800000);
+    for (int id = tid; id < c.vocab; id += kThreads) {
+      const float s = c.element_score(id, c.logits[id], c.class_of(id));
+      dst[id] = (c.greedy || S.kept.has(key_of(s), id)) ? s : ninf;
+    }
+  }
+  if (tid == 0) {
+    const int token = S.token;
+    S.out.token = token;
+    S.out.n_kept = S.out.n_after_topp = (int32_t)S.n_kept;
+    S.out.cut_bits = __float_as_uint(score_of(S.kept.cut_key));
+    S.out.n_cut_ties = (int32_t)S.cut_ties;
+    S.out.row_max = c.m;
+    if (S.tokens_out) S.tokens_out[S.row] = token;
+    if ((S.flags & HS_SAMPLE_APPEND_TOKEN) && S.slot_ok && token >= 0 && token < c.vocab) {
+      if (!slot_append_one(c.pool, S.P.slot, token)) S.status |= 2;
+    }
+    S.out.status = S.status;
+  }
+  __syncthreads();
+  if (tid < 32) write_record(S.out_row, S.out, S.P.n_logprobs >= 0);
+  if (S.scratch >= 0 && tid == 0) { __threadfence(); atomicExch(&S.scratch_busy[S.scratch], 0); }
+  phase_mark(S, 9);
+}
+
+}  // namespace hs
