@@ -18,6 +18,7 @@
 #include "hs_row_v3.cuh"
 #include "hs_row_topk.cuh"
 #include "hs_sharded.cuh"
+#include "hs_row_finish.cuh"
 #include "hs_row_bf16_kernel.cuh"
 #include "hs_row_resident.cuh"
 

@@ -520,9 +520,9 @@ __device__ __noinline__ void phase_greedy() {
   CandCtx bound_ctx{nullptr, nullptr, nullptr, nullptr, small + 8, nullptr};
   cand_thresholds(c, bound_ctx, max_key);  // (ends with a barrier)
   {
-    const Ctx3 k = c;
-    stream_at_or_above(k, bound_ctx.thr, [&](int id, uint32_t raw, int cc) {
-      if (v3_bin_of_raw(raw) >= 0 && key_of(k.score_of(raw, cc)) == max_key) atomicMin(low_id, id);
+    const Scorer sc = c;
+    stream_at_or_above(c, bound_ctx.thr, [&](int id, uint32_t raw, int cc) {
+      if (v3_bin_of_raw(raw) >= 0 && key_of(sc.score_of(raw, cc)) == max_key) atomicMin(low_id, id);
     });
   }
   __syncthreads();
@@ -535,6 +535,16 @@ __device__ __noinline__ void phase_greedy() {
     put_state(S.q_kept, q);
   }
   __syncthreads();
+}
+
+// Appends the `need` lowest ids of a large tie group to the top-N tokens.
+__device__ __noinline__ void emit_lowest_of_group(Ctx3& c, uint32_t key, int need) {
+  const int have = *c.gbuf_n();  // (the walk below counts in the same place)
+  const Group g = find_group(c, key);
+  const int last_id = nth_in_large_group(c, g, (u64)need);
+  if (threadIdx.x == 0) *c.gbuf_n() = have;
+  __syncthreads();
+  emit_group_upto(c, g, last_id == 0x7fffffff ? -1 : last_id);
 }
 
 // Log-probabilities: of the token, and of the N highest kept ones.
@@ -582,10 +592,10 @@ __device__ __noinline__ void phase_logprobs() {
       cand_thresholds(c, bound_ctx, nth_key);  // (ends with a barrier)
       phase_mark(S, 16);
       {
-        const Ctx3 k = c;
-        stream_at_or_above(k, bound_ctx.thr, [&](int id, uint32_t raw, int cc) {
+        const Scorer sc = c;
+        stream_at_or_above(c, bound_ctx.thr, [&](int id, uint32_t raw, int cc) {
           if (v3_bin_of_raw(raw) < 0) return;  // outside the bin window: a side element, taken above
-          take(key_of(k.score_of(raw, cc)), id);
+          take(key_of(sc.score_of(raw, cc)), id);
         });
       }
       __syncthreads();
@@ -605,12 +615,7 @@ __device__ __noinline__ void phase_logprobs() {
             }
           }
         } else {
-          const int have = *gbuf_n;  // (the walk below counts in the same place)
-          const Group g = find_group(c, nth_key);
-          const int last_id = nth_in_group(c, g, (u64)need);
-          if (tid == 0) *gbuf_n = have;
-          __syncthreads();
-          emit_group_upto(c, g, last_id == 0x7fffffff ? -1 : last_id);
+          emit_lowest_of_group(c, nth_key, need);
         }
       }
       __syncthreads();

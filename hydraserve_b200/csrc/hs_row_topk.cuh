@@ -327,7 +327,7 @@ __device__ int sample_kth_t16(const Ctx3& c, CandCtx& L, int k, const SampleRegs
           const uint32_t bc = L.count[hi - u];
           if ((uint32_t)want <= ex + bc) {
             L.thr[3] = hi - u;
-            c.x->bcast[1] = ex;
+            c.x()->bcast[1] = ex;
             break;
           }
           ex += bc;
@@ -336,7 +336,7 @@ __device__ int sample_kth_t16(const Ctx3& c, CandCtx& L, int k, const SampleRegs
     }
     __syncthreads();
     const int found = L.thr[3];
-    const int above = (int)c.x->bcast[1];
+    const int above = (int)c.x()->bcast[1];
     __syncthreads();
     if (found < 0) return -32768;  // fewer than k groups with a token outside the history
     want -= above;
@@ -484,7 +484,7 @@ __device__ int topk_candidates(Ctx3& c, CandCtx& L, int k) {
       if (*L.lost) return -1;
       n = min(*L.n, kCandCap);
       score_pending(n_scored, n);
-      bound = cand_kth_key(*c.x, L, n, k);
+      bound = cand_kth_key(*c.x(), L, n, k);
       n = cand_compact(L, n, bound);
       n_scored = n;
       cand_thresholds(c, L, bound);

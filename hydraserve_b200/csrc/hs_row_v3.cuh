@@ -94,18 +94,20 @@ struct RowV3Args {
 
 // Shared memory of a counting row.  What only the counting needs (rare tokens, set-aside chunks, the
 // staged hand-over) and what only the selections need (histogram, members, token ids) share a place.
+constexpr size_t kStateBytes = 1024;  // CountState
 struct LayoutV3 {
-  size_t x, tab, side, hist, members, list, staged, rare, defer, small, total;
+  size_t x, state, tab, side, hist, members, list, staged, rare, defer, small, total;
 };
-__host__ __device__ inline LayoutV3 layout_v3() {
+__host__ __device__ constexpr LayoutV3 layout_v3() {
   LayoutV3 l{};
   size_t off = 0;
-  auto take = [&](size_t bytes) {
+  auto take = [&off](size_t bytes) {
     const size_t at = off;
     off = (off + bytes + 15) & ~size_t(15);
     return at;
   };
   l.x = take(sizeof(Exchange));
+  l.state = take(kStateBytes);
   l.tab = take(sizeof(uint32_t) * kCells);
   l.side = take(sizeof(int2) * kV3SideShared);
   l.staged = take(sizeof(uint32_t) * kV3Staged);
@@ -118,6 +120,9 @@ __host__ __device__ inline LayoutV3 layout_v3() {
   l.total = off;
   return l;
 }
+constexpr LayoutV3 kLayV3 = layout_v3();
+constexpr int kPerClass = kV3Bins / kThreads;  // a thread's cells tid + u * kThreads: count class u / kPerClass
+static_assert(kV3Bins % kThreads == 0, "a thread's u-th cell has the same count class for all threads");
 static_assert(sizeof(uint32_t) * (4 * kV3Buckets + kV3TieCap) + sizeof(V3Member) * kV3ListCap <= sizeof(uint32_t) * kV3Staged &&
               sizeof(int2) * kV3RareCap + sizeof(int) * kV3DeferCap <= sizeof(uint32_t) * kV3Staged,
               "the two uses fit the shared place");
@@ -132,20 +137,53 @@ __device__ __forceinline__ uint32_t v3_raw_of_bin(int b) {
                       : 0x8000u | ((uint32_t)(kV3Half - 1 - b) + kV3Base);
 }
 
-struct Ctx3 {
-  Exchange* x;
-  uint32_t* tab;     // [kCells] tokens per class
-  uint32_t* hist;    // [4 * kV3Buckets] count, mass in three 14-bit limbs (32-bit shared atomics only)
-  V3Member* members; // [kV3ListCap] members of a selection's deciding bucket
-  V3Entry* gbuf;     // [kV3ListCap] top-N tokens (in the same place)
-  int* list;         // [kV3TieCap] token ids
-  int* gbuf_n;
-  uint32_t* span;    // lowest and highest key of a deciding bucket
-  int* range = nullptr;  // [6] scratch of for_classes_at
-  int* ends = nullptr;  // [6] per count class: highest non-empty cell + 1 (0 = none), lowest non-empty cell
-  int* step_n = nullptr;  // two counters the early-exit scan alternates between
+// What turns a token's raw value and count into its score.
+struct Scorer {
+  float T, rp, pp, fp;
+  bool greedy;
+  __device__ __forceinline__ float score_of_value(float v) const {
+    return greedy || T == 1.0f ? canonical(v) : canonical(__fdiv_rn(v, T));
+  }
+  // score of a token with raw value bits `raw` that the history holds `count` times
+  __device__ __forceinline__ float score_of(uint32_t raw, int count) const {
+    float v = canonical(__uint_as_float(raw << 16));
+    if (count > 0) {
+      if (rp != 1.0f) v = v < 0.0f ? __fmul_rn(v, rp) : __fdiv_rn(v, rp);
+      v = __fsub_rn(v, pp);
+      v = __fsub_rn(v, __fmul_rn(fp, (float)count));
+    }
+    return score_of_value(v);
+  }
+  __device__ __forceinline__ float cell_score(int cell) const {
+    const int c = cell / kV3Bins;
+    return score_of(v3_raw_of_bin(cell - c * kV3Bins), c);
+  }
+  // score key of a bin of count class k
+  __device__ __forceinline__ uint32_t key_of_bin(int bin, int k) const { return key_of(score_of(v3_raw_of_bin(bin), k)); }
+};
+template <size_t AT, class T>
+__device__ __forceinline__ T* at_smem() {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  return reinterpret_cast<T*>(smem_raw + AT);
+}
+struct Ctx3 : Scorer {
+  // (places in shared memory; the block primitives' scratch comes first in every kernel's layout)
+  __device__ __forceinline__ Exchange* x() const { return at_smem<0, Exchange>(); }
+  __device__ __forceinline__ uint32_t* tab() const { return at_smem<kLayV3.tab, uint32_t>(); }     // [kCells] tokens per class
+  __device__ __forceinline__ uint32_t* hist() const { return at_smem<kLayV3.hist, uint32_t>(); }   // [4 * kV3Buckets] count, mass in three 14-bit limbs
+  __device__ __forceinline__ V3Member* members() const { return at_smem<kLayV3.members, V3Member>(); }  // [kV3ListCap] of a selection's deciding bucket
+  __device__ __forceinline__ V3Entry* gbuf() const { return at_smem<kLayV3.members, V3Entry>(); }  // [kV3ListCap] top-N tokens (in the same place)
+  __device__ __forceinline__ int* list() const { return at_smem<kLayV3.list, int>(); }             // [kV3TieCap] token ids
+  __device__ __forceinline__ int2* rare() const { return at_smem<kLayV3.rare, int2>(); }           // [kV3RareCap] (id, raw bits | count class << 16)
+  __device__ __forceinline__ int2* side() const { return at_smem<kLayV3.side, int2>(); }           // [kV3SideShared]
+  // (of the small counters: 0 gbuf_n, 1 rare_n, 2 side_n, 3 low id / ties, 8..11 thresholds, 14 ticket,
+  // 16..21 ends, 22 lowest side key, 24..25 step_n, 27 defer_n, 30..31 span, 40..45 range, 48..63 warps)
+  __device__ __forceinline__ int* gbuf_n() const { return at_smem<kLayV3.small, int>(); }
+  __device__ __forceinline__ int* step_n() const { return at_smem<kLayV3.small, int>() + 24; }     // [2] of a scan
+  __device__ __forceinline__ uint32_t* span() const { return at_smem<kLayV3.small, uint32_t>() + 30; }  // lowest and highest key of a deciding bucket
+  __device__ __forceinline__ int* range() const { return at_smem<kLayV3.small, int>() + 40; }      // [6] of for_classes_at
+  __device__ __forceinline__ int* ends() const { return at_smem<kLayV3.small, int>() + 16; }       // [6] per count class: highest non-empty cell + 1 (0 = none), lowest
   int row, vocab;
-  unsigned long long* dbg = nullptr;
   int lo, hi;                    // token range this CTA streams in the candidate path ...
   int chunk_lo, chunk_hi;        // ... and the whole chunks in it
   const unsigned short* logits;  // this row
@@ -176,28 +214,7 @@ struct Ctx3 {
   int slot;
   int2* s_pair;
   int n_s, s_cap;
-  float T, rp, pp, fp;
-  bool greedy;
   float m;
-  __device__ __forceinline__ float score_of_value(float v) const {
-    return greedy || T == 1.0f ? canonical(v) : canonical(__fdiv_rn(v, T));
-  }
-  // score of a token with raw value bits `raw` that the history holds `count` times
-  __device__ __forceinline__ float score_of(uint32_t raw, int count) const {
-    float v = canonical(__uint_as_float(raw << 16));
-    if (count > 0) {
-      if (rp != 1.0f) v = v < 0.0f ? __fmul_rn(v, rp) : __fdiv_rn(v, rp);
-      v = __fsub_rn(v, pp);
-      v = __fsub_rn(v, __fmul_rn(fp, (float)count));
-    }
-    return score_of_value(v);
-  }
-  __device__ __forceinline__ float cell_score(int cell) const {
-    const int c = cell / kV3Bins;
-    return score_of(v3_raw_of_bin(cell - c * kV3Bins), c);
-  }
-  // score key of a bin of count class k
-  __device__ __forceinline__ uint32_t key_of_bin(int bin, int k) const { return key_of(score_of(v3_raw_of_bin(bin), k)); }
   __device__ __forceinline__ int class_of(int id) const {
     return cls ? (int)((cls[id >> 4] >> ((id & 15) * 2)) & 3u) : 0;
   }
@@ -236,18 +253,19 @@ __device__ __forceinline__ void for_each_side3(const Ctx3& c, F&& f) {
 template <class F>
 __device__ __forceinline__ void for_each_class(const Ctx3& c, F&& f) {
   constexpr int kBatch = 3;
+  const Scorer sc = c;
 #pragma unroll 1
   for (int k = 0; k < 3; ++k) {
-    const int top = c.ends[k], bot = c.ends[3 + k];  // (highest + 1; 0 = the class is empty)
+    const int top = c.ends()[k], bot = c.ends()[3 + k];  // (highest + 1; 0 = the class is empty)
     if (top == 0) continue;
 #pragma unroll 1
     for (int base = bot + (int)threadIdx.x; base - (int)(threadIdx.x & 31) < top; base += kBatch * kThreads) {
       uint32_t n[kBatch], key[kBatch];
 #pragma unroll
-      for (int u = 0; u < kBatch; ++u) n[u] = base + u * kThreads < top ? c.tab[base + u * kThreads] : 0u;
+      for (int u = 0; u < kBatch; ++u) n[u] = base + u * kThreads < top ? c.tab()[base + u * kThreads] : 0u;
       if (!__any_sync(0xffffffffu, (n[0] | n[1] | n[2]) != 0u)) continue;
 #pragma unroll
-      for (int u = 0; u < kBatch; ++u) key[u] = c.key_of_bin(min(base + u * kThreads, top - 1) - k * kV3Bins, k);
+      for (int u = 0; u < kBatch; ++u) key[u] = sc.key_of_bin(min(base + u * kThreads, top - 1) - k * kV3Bins, k);
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) f(n[u] != 0u, key[u], n[u], base + u * kThreads);
     }
@@ -259,31 +277,32 @@ __device__ __forceinline__ void for_each_class(const Ctx3& c, F&& f) {
 template <class Place, class F>
 __device__ __forceinline__ void for_classes_at(const Ctx3& c, int low, int high, Place&& place, F&& f) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const Scorer sc = c;
   __syncthreads();
   if (warp < 6) {
-    const int k = warp % 3, top = c.ends[k];
+    const int k = warp % 3, top = c.ends()[k];
     const int want = warp < 3 ? low : high + 1;  // the first cell whose place is at least this
-    int lo = top ? c.ends[3 + k] : 0, hi = top;
+    int lo = top ? c.ends()[3 + k] : 0, hi = top;
 #pragma unroll 1
     while (lo < hi) {
       const int step = (hi - lo + 31) >> 5;
       const int t = lo + (lane + 1) * step - 1;
-      const bool pass = t >= hi || place(c.key_of_bin(min(t, hi - 1) - k * kV3Bins, k)) >= want;
+      const bool pass = t >= hi || place(sc.key_of_bin(min(t, hi - 1) - k * kV3Bins, k)) >= want;
       const uint32_t votes = __ballot_sync(0xffffffffu, pass);
       if (votes == 0) { lo = hi; break; }
       const int first = __ffs(votes) - 1;
       hi = min(lo + (first + 1) * step - 1, hi);
       lo = lo + first * step;
     }
-    if (lane == 0) c.range[warp] = lo;
+    if (lane == 0) c.range()[warp] = lo;
   }
   __syncthreads();
 #pragma unroll 1
   for (int k = 0; k < 3; ++k) {
 #pragma unroll 1
-    for (int cell = c.range[k] + (int)threadIdx.x; cell < c.range[3 + k]; cell += kThreads) {
-      const uint32_t n = c.tab[cell];
-      if (n) f(c.key_of_bin(cell - k * kV3Bins, k), n, cell);
+    for (int cell = c.range()[k] + (int)threadIdx.x; cell < c.range()[3 + k]; cell += kThreads) {
+      const uint32_t n = c.tab()[cell];
+      if (n) f(sc.key_of_bin(cell - k * kV3Bins, k), n, cell);
     }
   }
 }
@@ -339,7 +358,7 @@ struct AllTokens3 {
   template <bool WITH_MASS>
   __device__ __forceinline__ void fill(const V3Map& map) const {
     const float m = c->m;
-    uint32_t* hist = c->hist;
+    uint32_t* hist = c->hist();
     for_each_side3(*c, [&](int, float s) {
       const uint32_t key = key_of(s);
       if (map.in(key)) hist_add<WITH_MASS>(hist, map.bucket(key), 1u, WITH_MASS ? mass_of(s, m) : 0ull);
@@ -379,7 +398,7 @@ struct KeptSide3 {
   __device__ __forceinline__ void fill(const V3Map& map) const {
     for_each_side3(*c, [&](int id, float s) {
       const uint32_t key = ~(uint32_t)id;
-      if (key_of(s) > cut_key && map.in(key)) hist_add<WITH_MASS>(c->hist, map.bucket(key), 1u, mass_of(s, c->m));
+      if (key_of(s) > cut_key && map.in(key)) hist_add<WITH_MASS>(c->hist(), map.bucket(key), 1u, mass_of(s, c->m));
     });
   }
   template <bool WITH_MASS, class F>
@@ -406,7 +425,7 @@ template <bool BY_MASS, bool WITH_MASS, class From>
 __device__ Selection select_key(Ctx3& c, const From& from, V3Map map, bool& filled, u64 target) {
   static_assert(WITH_MASS || !BY_MASS, "a cut by mass needs masses");
   const int tid = threadIdx.x;
-  uint32_t* hist = c.hist;
+  uint32_t* hist = c.hist();
   Selection sel{};
   sel.target = target;
   sel.levels = 3;
@@ -416,7 +435,7 @@ __device__ Selection select_key(Ctx3& c, const From& from, V3Map map, bool& fill
       hist_fill<WITH_MASS>(hist, from, map);
       filled = false;
     }
-    if (tid == 0) { c.x->bcast[7] = 0; *c.gbuf_n = 0; c.span[0] = 0xffffffffu; c.span[1] = 0u; }
+    if (tid == 0) { c.x()->bcast[7] = 0; *c.gbuf_n() = 0; c.span()[0] = 0xffffffffu; c.span()[1] = 0u; }
     // thread t owns the two buckets 1,023 - 2 t and 1,022 - 2 t
     static_assert(kV3Buckets == 2 * kThreads, "two buckets per thread");
     const int hi = kV3Buckets - 1 - 2 * tid;
@@ -426,7 +445,7 @@ __device__ Selection select_key(Ctx3& c, const From& from, V3Map map, bool& fill
       const u64 q = WITH_MASS ? hist_mass(hist, hi) + hist_mass(hist, hi - 1) : 0ull;
       const u64 ia = warp_scan_u64(n), ib = WITH_MASS ? warp_scan_u64(q) : 0ull;
       u64 pa, pb, ta, tb;
-      block_warp_prefix2(*c.x, shfl_u64(ia, 31), WITH_MASS ? shfl_u64(ib, 31) : 0ull, pa, pb, ta, tb);
+      block_warp_prefix2(*c.x(), shfl_u64(ia, 31), WITH_MASS ? shfl_u64(ib, 31) : 0ull, pa, pb, ta, tb);
       ac = pa + ia - n;
       am = pb + ib - q;
     }
@@ -436,63 +455,63 @@ __device__ Selection select_key(Ctx3& c, const From& from, V3Map map, bool& fill
       const u64 n = hist[hi - u], q = WITH_MASS ? hist_mass(hist, hi - u) : 0ull;
       const u64 over = BY_MASS ? am : ac;
       if (over < want && want <= over + (BY_MASS ? q : n)) {
-        c.x->bcast[0] = (u64)(hi - u);
-        c.x->bcast[1] = ac;
-        c.x->bcast[2] = am;
-        c.x->bcast[3] = n;
-        c.x->bcast[4] = q;
-        c.x->bcast[7] = 1;
+        c.x()->bcast[0] = (u64)(hi - u);
+        c.x()->bcast[1] = ac;
+        c.x()->bcast[2] = am;
+        c.x()->bcast[3] = n;
+        c.x()->bcast[4] = q;
+        c.x()->bcast[7] = 1;
       }
       ac += n;
       am += q;
     }
     __syncthreads();
-    if (c.x->bcast[7] == 0) {  // nothing reaches the target
+    if (c.x()->bcast[7] == 0) {  // nothing reaches the target
       sel.ok = false;
       sel.key = map.klo;
       __syncthreads();
       return sel;
     }
-    const int bucket = (int)c.x->bcast[0];
+    const int bucket = (int)c.x()->bcast[0];
     sel.ok = true;
-    sel.above_cnt += c.x->bcast[1];
-    sel.above_mass += c.x->bcast[2];
-    sel.bin_cnt = c.x->bcast[3];
-    sel.bin_mass = c.x->bcast[4];
+    sel.above_cnt += c.x()->bcast[1];
+    sel.above_mass += c.x()->bcast[2];
+    sel.bin_cnt = c.x()->bcast[3];
+    sel.bin_mass = c.x()->bcast[4];
     from.template members<WITH_MASS>(map, bucket, [&](uint32_t key, uint32_t cnt, u64 w) {
-      const int slot = atomicAdd(c.gbuf_n, 1);
-      if (slot < kV3ListCap) c.members[slot] = V3Member{key, cnt, w};
-      atomicMin(c.span, key);
-      atomicMax(c.span + 1, key);
+      const int slot = atomicAdd(c.gbuf_n(), 1);
+      if (slot < kV3ListCap) c.members()[slot] = V3Member{key, cnt, w};
+      atomicMin(c.span(), key);
+      atomicMax(c.span() + 1, key);
     });
     __syncthreads();
-    const int members = *c.gbuf_n;
-    const uint32_t key_lo = c.span[0], key_hi = c.span[1];
+    const int members = *c.gbuf_n();
+    const uint32_t key_lo = c.span()[0], key_hi = c.span()[1];
     if (key_lo == key_hi) { sel.key = key_lo; break; }
     if (members <= kV3ListCap) {
       // each member against all: what lies above its key, and at it
       const u64 still = sel.target - (BY_MASS ? sel.above_mass : sel.above_cnt);
       if (tid < members) {
-        const uint32_t mine = c.members[tid].key;
+        const uint32_t mine = c.members()[tid].key;
         u64 oc = 0, om = 0, gc = 0, gm = 0;
 #pragma unroll 2
         for (int j = 0; j < members; ++j) {
-          const V3Member o = c.members[j];
+          const V3Member o = c.members()[j];
           if (o.key > mine) { oc += o.cnt; om += o.w; }
           if (o.key == mine) { gc += o.cnt; gm += o.w; }
         }
         const u64 over = BY_MASS ? om : oc;
         if (over < still && still <= over + (BY_MASS ? gm : gc)) {  // (members of one key write the same)
-          c.x->bcast[0] = mine;
-          c.x->bcast[1] = oc; c.x->bcast[2] = om; c.x->bcast[3] = gc; c.x->bcast[4] = gm;
+          c.x()->bcast[0] = mine;
+          c.x()->bcast[1] = oc; c.x()->bcast[2] = om; c.x()->bcast[3] = gc; c.x()->bcast[4] = gm;
         }
       }
       __syncthreads();
-      sel.key = (uint32_t)c.x->bcast[0];
-      sel.above_cnt += c.x->bcast[1];
-      sel.above_mass += c.x->bcast[2];
-      sel.bin_cnt = c.x->bcast[3];
-      sel.bin_mass = c.x->bcast[4];
+      sel.key = (uint32_t)c.x()->bcast[0];
+      sel.above_cnt += c.x()->bcast[1];
+      sel.above_mass += c.x()->bcast[2];
+      sel.bin_cnt = c.x()->bcast[3];
+      sel.bin_mass = c.x()->bcast[4];
       break;
     }
     map.by_key(key_lo, key_hi);
@@ -511,8 +530,8 @@ __device__ void totals3(Ctx3& c, uint32_t lo_key, bool filled, u64& cnt, u64& ma
 #pragma unroll
     for (int u = 0; u < kV3Buckets / kThreads; ++u) {
       const int i = threadIdx.x + u * kThreads;
-      a += c.hist[i];
-      b += hist_mass(c.hist, i);
+      a += c.hist()[i];
+      b += hist_mass(c.hist(), i);
     }
   } else {
     for_each_side3(c, [&](int, float s) {
@@ -522,7 +541,7 @@ __device__ void totals3(Ctx3& c, uint32_t lo_key, bool filled, u64& cnt, u64& ma
       if (valid && key >= lo_key) { a += n; b += (u64)n * mass_of(score_of(key), c.m); }
     });
   }
-  block_sum2(*c.x, a, b);
+  block_sum2(*c.x(), a, b);
   cnt = a;
   mass = b;
 }
@@ -535,17 +554,17 @@ struct Group {
   __device__ __forceinline__ int cell_of(int cc) const { return cc == 0 ? cell0 : (cc == 1 ? cell1 : cell2); }
 };
 __device__ Group find_group(Ctx3& c, uint32_t key) {
-  if (threadIdx.x < 3) c.x->bcast[threadIdx.x] = 0;
+  if (threadIdx.x < 3) c.x()->bcast[threadIdx.x] = 0;
   __syncthreads();
   for_classes_at(c, 0, 0, [&](uint32_t k) { return k < key ? -1 : (k > key ? 1 : 0); }, [&](uint32_t, uint32_t, int cell) {
-    c.x->bcast[cell / kV3Bins] = (u64)cell + 1;
+    c.x()->bcast[cell / kV3Bins] = (u64)cell + 1;
   });
   __syncthreads();
   Group g;
   g.key = key;
-  g.cell0 = (int)c.x->bcast[0] - 1;
-  g.cell1 = (int)c.x->bcast[1] - 1;
-  g.cell2 = (int)c.x->bcast[2] - 1;
+  g.cell0 = (int)c.x()->bcast[0] - 1;
+  g.cell1 = (int)c.x()->bcast[1] - 1;
+  g.cell2 = (int)c.x()->bcast[2] - 1;
   __syncthreads();
   return g;
 }
@@ -598,7 +617,7 @@ __device__ __forceinline__ u64 count_members(const Ctx3& c, const Group& g, int 
 // elements whose score key is g.key), or 0x7fffffff: for groups of any size.  The row is cut into one segment per
 // warp, members are counted, and the segment that holds the n-th is cut again until one
 // warp can rank its members with ballots.
-__device__ int nth_in_large_group(Ctx3& c, const Group& g, u64 n) {
+__device__ __noinline__ int nth_in_large_group(Ctx3& c, const Group g, u64 n) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
   int b = 0, e = c.n8();
   u64 before = 0;
@@ -617,20 +636,20 @@ __device__ int nth_in_large_group(Ctx3& c, const Group& g, u64 n) {
     const int mb = min(b + warp * seg, e), me = min(mb + seg, e);
     const u64 wtot = warp_sum_u64(count_members(c, g, mb, me));
     u64 pre, pre_unused, tot, tot_unused;
-    block_warp_prefix2(*c.x, wtot, 0, pre, pre_unused, tot, tot_unused);
+    block_warp_prefix2(*c.x(), wtot, 0, pre, pre_unused, tot, tot_unused);
     if (before + tot < n) { before += tot; in_tail = true; break; }
     if (before + pre < n && n <= before + pre + wtot && lane == 0) {
-      c.x->bcast[4] = (u64)mb;
-      c.x->bcast[5] = (u64)me;
-      c.x->bcast[6] = before + pre;
+      c.x()->bcast[4] = (u64)mb;
+      c.x()->bcast[5] = (u64)me;
+      c.x()->bcast[6] = before + pre;
     }
     __syncthreads();
-    b = (int)c.x->bcast[4];
-    e = (int)c.x->bcast[5];
-    before = c.x->bcast[6];
+    b = (int)c.x()->bcast[4];
+    e = (int)c.x()->bcast[5];
+    before = c.x()->bcast[6];
     __syncthreads();
   }
-  if (tid == 0) c.x->bcast[6] = 0;
+  if (tid == 0) c.x()->bcast[6] = 0;
   __syncthreads();
   if (warp == 0) {
     // at most 128 chunks, then the loose tokens behind the last one: rank members with warp scans
@@ -644,7 +663,7 @@ __device__ int nth_in_large_group(Ctx3& c, const Group& g, u64 n) {
       u64 rank = running + incl - __popc(memb);
       for (int k = 0; k < 8; ++k) {
         if (!((memb >> k) & 1u)) continue;
-        if (++rank == n) c.x->bcast[6] = (u64)(c.first_of(i) + k) + 1;
+        if (++rank == n) c.x()->bcast[6] = (u64)(c.first_of(i) + k) + 1;
       }
       running += shfl_u64(incl, 31);
     }
@@ -653,11 +672,11 @@ __device__ int nth_in_large_group(Ctx3& c, const Group& g, u64 n) {
       const bool mbr = id < c.vocab && in_group(c, g, id, c.logits[id], c.class_of(id));
       const uint32_t ballot = __ballot_sync(0xffffffffu, mbr);
       const u64 rank = running + __popc(ballot & ((1u << lane) - 1u)) + 1;
-      if (mbr && rank == n) c.x->bcast[6] = (u64)id + 1;
+      if (mbr && rank == n) c.x()->bcast[6] = (u64)id + 1;
     }
   }
   __syncthreads();
-  const u64 found = c.x->bcast[6];
+  const u64 found = c.x()->bcast[6];
   __syncthreads();
   if (found) result = (int)(found - 1);
   return result;
@@ -801,39 +820,32 @@ __device__ __noinline__ void scan_members(const ScanArgs c, uint32_t raw0, uint3
   __syncthreads();
 }
 __device__ __forceinline__ ScanArgs scan_args(const Ctx3& c) {
-  return ScanArgs{c.logits, c.cls, c.vocab, c.head(), c.n8(), c.list, c.gbuf_n, c.step_n, &c.x->bcast[6]};
+  return ScanArgs{c.logits, c.cls, c.vocab, c.head(), c.n8(), c.list(), c.gbuf_n(), c.step_n(), &c.x()->bcast[6]};
 }
-// ... of ONE class (cell), or -1 when it has more members than a scan holds.
-__device__ __forceinline__ int nth_in_small_class(Ctx3& c, int cell, u64 n, u64 members) {
-  if (members > (u64)kV3ScanCap || n < 1 || n > members) return -1;
-  const int cc = cell / kV3Bins;
-  if (threadIdx.x == 0) *c.gbuf_n = 0;
-  scan_members<true>(scan_args(c), v3_raw_of_bin(cell - cc * kV3Bins), kNoRaw, kNoRaw, cc, (int)n, (int)members);
-  const u64 hit = c.x->bcast[6];
-  __syncthreads();
-  return hit ? (int)(hit - 1) : 0x7fffffff;
-}
-
 // Token id of the n-th member of a group: by one scan when the group is small enough.
 __device__ int nth_in_group(Ctx3& c, const Group& g, u64 n) {
-  auto count = [&](int cell) { return cell >= 0 ? (u64)c.tab[cell] : 0ull; };
+  auto count = [&](int cell) { return cell >= 0 ? (u64)c.tab()[cell] : 0ull; };
   auto raw = [&](int cell, int cc) { return cell >= 0 ? v3_raw_of_bin(cell - cc * kV3Bins) : kNoRaw; };
   const u64 in_classes = count(g.cell0) + count(g.cell1) + count(g.cell2);
   if (in_classes <= (u64)kV3ScanCap) {
     // the group's side elements are noted first, whatever the walk will see
     __syncthreads();
-    if (threadIdx.x == 0) *c.gbuf_n = 0;
+    if (threadIdx.x == 0) *c.gbuf_n() = 0;
     __syncthreads();
     for_each_side3(c, [&](int id, float s) {
       if (key_of(s) != g.key) return;
-      const int slot = atomicAdd(c.gbuf_n, 1);
-      if (slot < kV3ScanCap) c.list[slot] = id;
+      const int slot = atomicAdd(c.gbuf_n(), 1);
+      if (slot < kV3ScanCap) c.list()[slot] = id;
     });
     __syncthreads();
-    const u64 all = in_classes + (u64)*c.gbuf_n;
+    const u64 all = in_classes + (u64)*c.gbuf_n();
     if (all <= (u64)kV3ScanCap && n >= 1 && n <= all) {
-      scan_members<false>(scan_args(c), raw(g.cell0, 0), raw(g.cell1, 1), raw(g.cell2, 2), 0, (int)n, (int)all);
-      const u64 hit = c.x->bcast[6];
+      const int cc = g.cell0 >= 0 ? 0 : (g.cell1 >= 0 ? 1 : 2);
+      if ((g.cell0 >= 0) + (g.cell1 >= 0) + (g.cell2 >= 0) == 1)
+        scan_members<true>(scan_args(c), raw(g.cell_of(cc), cc), kNoRaw, kNoRaw, cc, (int)n, (int)all);
+      else
+        scan_members<false>(scan_args(c), raw(g.cell0, 0), raw(g.cell1, 1), raw(g.cell2, 2), 0, (int)n, (int)all);
+      const u64 hit = c.x()->bcast[6];
       __syncthreads();
       if (hit) return (int)(hit - 1);
     }
@@ -846,8 +858,8 @@ __device__ void emit_group_upto(Ctx3& c, const Group& g, int id_limit) {
   const int last = min(c.n8(), max(0, id_limit - c.head()) / 8 + 1);
   const uint4* src4 = c.chunks();
   auto emit = [&](int id) {
-    const int slot = atomicAdd(c.gbuf_n, 1);
-    if (slot < kV3ListCap) c.gbuf[slot] = V3Entry{g.key, id};
+    const int slot = atomicAdd(c.gbuf_n(), 1);
+    if (slot < kV3ListCap) c.gbuf()[slot] = V3Entry{g.key, id};
   };
   for (int i = threadIdx.x; i < last; i += kThreads) {
     uint32_t memb = chunk_members(c, g, i, __ldcg(src4 + i), c.cls ? c.chunk_classes(i) : 0u);
@@ -898,11 +910,11 @@ __device__ int random_in_class(Ctx3& c, int cell, int trials, uint64_t seed, int
         mine = id[j];
       }
     }
-    const uint32_t best = block_max_u32(*c.x, key);
+    const uint32_t best = block_max_u32(*c.x(), key);
     if (best) {
-      if (key == best) c.x->bcast[6] = (u64)mine;
+      if (key == best) c.x()->bcast[6] = (u64)mine;
       __syncthreads();
-      const int token = (int)c.x->bcast[6];
+      const int token = (int)c.x()->bcast[6];
       __syncthreads();
       return token;
     }
@@ -961,7 +973,7 @@ __device__ int draw_by_token_rejection(Ctx3& c, const KeptSet& kept, bool tie_sp
       const u64 packed = ((u64)((kTokenTrials - j) * kThreads - tid) << 33) | ((u64)(group ? 1u : 0u) << 32) | (uint32_t)id[j];
       best = packed > best ? packed : best;
     }
-    best = block_max_u64(*c.x, best);
+    best = block_max_u64(*c.x(), best);
     if (best) {
       group_hit = ((best >> 32) & 1ull) != 0;
       return (int)(uint32_t)best;

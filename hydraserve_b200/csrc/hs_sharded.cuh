@@ -18,15 +18,16 @@ struct ShardArgs {
   hs_shard_rec* recs;   // [batch]
 };
 
-// smem: Exchange | cand[kCandCap] | mass[kCandCap] | count[kBins] | small[32]
+// smem: Exchange | state | cand[kCandCap] | mass[kCandCap] | count[kBins] | small[32]
 struct LayoutCand {
-  size_t x, cand, mass, count, small, total;
+  size_t x, state, cand, mass, count, small, total;
 };
 __host__ __device__ inline LayoutCand layout_cand() {
   LayoutCand l{};
   size_t off = 0;
   auto take = [&](size_t bytes) { const size_t at = off; off = (off + bytes + 15) & ~size_t(15); return at; };
   l.x = take(sizeof(Exchange));
+  l.state = take(kStateBytes);  // (the counting path's state: a row may turn out to be one of its)
   l.cand = take(sizeof(u64) * kCandCap);
   l.mass = take(sizeof(u64) * kCandCap);
   l.count = take(sizeof(uint32_t) * kBins);
@@ -40,7 +41,6 @@ __global__ void __launch_bounds__(kThreads, 2) shard_partial_kernel(const ShardA
   const RowKernelArgs& a = args.base;
   const LayoutCand lay = layout_cand();
   Ctx3 c;
-  c.x = reinterpret_cast<Exchange*>(smem_raw + lay.x);
   int* small = reinterpret_cast<int*>(smem_raw + lay.small);
   CandCtx L{reinterpret_cast<u64*>(smem_raw + lay.cand), small + 4, small + 5,
             reinterpret_cast<uint32_t*>(smem_raw + lay.count), small + 8, nullptr};
@@ -61,7 +61,6 @@ __global__ void __launch_bounds__(kThreads, 2) shard_partial_kernel(const ShardA
   const bool penalised = slot_ok && (c.rp != 1.0f || c.pp != 0.0f || c.fp != 0.0f);
   c.cls = penalised ? a.pool.cls + (size_t)P.slot * a.pool.cls_stride : nullptr;
   c.s_pair = nullptr; c.n_s = 0; c.s_cap = 0; c.m = 0.f;
-  c.tab = nullptr; c.hist = nullptr; c.gbuf = nullptr; c.list = nullptr; c.gbuf_n = nullptr;
   hs_shard_rec* rec = args.recs + c.row;
   if (tid < 16) small[tid] = 0;
   __syncthreads();
@@ -72,7 +71,7 @@ __global__ void __launch_bounds__(kThreads, 2) shard_partial_kernel(const ShardA
   // and the merge reports the row as failed
   if (n < 0) { status |= 16; n = 0; }
   if (n > k) {
-    const uint32_t cut = cand_kth_key(*c.x, L, n, k);
+    const uint32_t cut = cand_kth_key(*c.x(), L, n, k);
     n = cand_compact(L, n, cut);
   } else if (n > 0) {
     n = cand_compact(L, n, 0u);  // drops entries the scoring pass voided
@@ -122,7 +121,7 @@ __global__ void __launch_bounds__(kThreads, 2) shard_partial_kernel(const ShardA
       if (count) z += (u64)count * mass_of(c.cell_score(cell), m);
     }
   }
-  block_sum2(*c.x, z, unused);
+  block_sum2(*c.x(), z, unused);
   if (tid == 0) {
     rec->row_max = m;
     rec->pad = 0.f;
