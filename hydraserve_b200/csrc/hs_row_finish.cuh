@@ -10,6 +10,15 @@
 
 namespace hs {
 
+// What a draw asks for when it does not know the token yet: the nth (by ascending id) member of
+// the cut's tie group, or of one class.
+struct DrawAsk {
+  int kind;  // 0 = the token is known (or there is none), 1 = of the group, 2 = of a class
+  int token;
+  int cell;
+  u64 nth, members;
+};
+
 struct CountState {
   Ctx3 c;
   hs_row_params P;
@@ -21,6 +30,8 @@ struct CountState {
   u64 side_best;         // highest side element, (key, ~id); 0 = none
   uint32_t max_key;
   int status, token, scratch;
+  Selection sel;         // what select_key found
+  DrawAsk ask;           // what the draw left to be found
   Group cut_group;
   bool have_cut_group, tie_split, filled, slot_ok, penalised;
   // from the launch's arguments
@@ -65,6 +76,212 @@ __device__ bool claim_scratch(CountState& S) {
   }
   __syncthreads();
   return S.scratch >= 0;
+}
+
+// ---- selection -------------------------------------------------------------------------------------
+// A CTA goes through the chain of selections once per row, so what it costs is first of all the
+// fetching of its instructions: one copy of each function, loops that are not unrolled.
+__device__ __forceinline__ void hist_add(uint32_t* hist, int b, uint32_t cnt, u64 mass) {
+  atomicAdd(hist + b, cnt);
+  const uint32_t a0 = (uint32_t)mass & kLimbMask, a1 = (uint32_t)(mass >> kLimbBits) & kLimbMask, a2 = (uint32_t)(mass >> (2 * kLimbBits));
+  if (a0) atomicAdd(hist + kV3Buckets + b, a0);
+  if (a1) atomicAdd(hist + 2 * kV3Buckets + b, a1);
+  if (a2) atomicAdd(hist + 3 * kV3Buckets + b, a2);
+}
+__device__ __forceinline__ u64 hist_mass(const uint32_t* hist, int b) {
+  return (u64)hist[kV3Buckets + b] + ((u64)hist[2 * kV3Buckets + b] << kLimbBits) + ((u64)hist[3 * kV3Buckets + b] << (2 * kLimbBits));
+}
+// The histogram of count and mass: of every token (side elements one by one, classes with their
+// count), or (side_ids) of the kept side elements keyed by ~id.  The thousands of values next to
+// zero share a bucket, and would queue up at one address: a warp whose cells all fall into one bucket
+// adds them up first.
+__device__ __noinline__ void fill_hist(const V3Map map, bool side_ids) {
+  CountState& S = count_state();
+  Ctx3& c = S.c;
+  uint32_t* hist = c.hist();
+  const float m = c.m;
+#pragma unroll
+  for (int b = 0; b < 4 * kV3Buckets / kThreads; ++b) hist[threadIdx.x + b * kThreads] = 0;
+  __syncthreads();
+  const uint32_t cut_key = S.kept.cut_key;
+  for_each_side3(c, [&](int id, float s) {
+    const uint32_t key = side_ids ? ~(uint32_t)id : key_of(s);
+    if (side_ids && key_of(s) <= cut_key) return;
+    if (map.in(key)) hist_add(hist, map.bucket(key), 1u, mass_of(s, m));
+  });
+  if (!side_ids) {
+    for_each_class(c, [&](bool valid, uint32_t key, uint32_t n, int) {
+      valid = valid && map.in(key);
+      const int b = map.bucket(key);
+      const u64 w = (u64)n * mass_of(score_of(key), m);
+      const int first = __reduce_min_sync(0xffffffffu, valid ? b : 0x7fffffff);
+      if (__all_sync(0xffffffffu, !valid || b == first)) {
+        const uint32_t cnt = __reduce_add_sync(0xffffffffu, valid ? n : 0u);
+        const u64 sum = warp_sum_u64(valid ? w : 0ull);
+        if (cnt && (threadIdx.x & 31) == 0) hist_add(hist, first, cnt, sum);
+      } else if (valid) {
+        hist_add(hist, b, n, w);
+      }
+    });
+  }
+  __syncthreads();
+}
+
+// The key, from the top, at which the running count (by_mass: mass) of the elements reaches
+// `target`, with what lies above and at it, in S.sel.  S.filled: the histogram holds all tokens
+// under S.all_map (kept up to date).
+__device__ __noinline__ void select_key(bool by_mass, bool side_ids, u64 target) {
+  CountState& S = count_state();
+  Ctx3& c = S.c;
+  const int tid = threadIdx.x;
+  uint32_t* hist = c.hist();
+  V3Map map = S.all_map;
+  if (side_ids) map.by_key(~(uint32_t)(c.vocab - 1), 0xffffffffu);
+  u64 above = 0;  // of what is counted, above the buckets looked at so far
+  if (tid == 0) {
+    S.sel.above_cnt = S.sel.above_mass = 0;
+    S.sel.target = target;
+    S.sel.ok = true;
+  }
+#pragma unroll 1
+  for (int round = 0; round < 8; ++round) {
+    if (round > 0 || side_ids || !S.filled) {
+      __syncthreads();
+      fill_hist(map, side_ids);
+      put_state(S.filled, round == 0 && !side_ids);
+    }
+    if (tid == 0) { c.x()->bcast[7] = 0; *c.gbuf_n() = 0; c.span()[0] = 0xffffffffu; c.span()[1] = 0u; }
+    // thread t owns the two buckets 1,023 - 2 t and 1,022 - 2 t
+    static_assert(kV3Buckets == 2 * kThreads, "two buckets per thread");
+    const int hi = kV3Buckets - 1 - 2 * tid;
+    u64 ac, am;  // above this thread's buckets
+    {
+      const u64 n = (u64)hist[hi] + hist[hi - 1];
+      const u64 q = hist_mass(hist, hi) + hist_mass(hist, hi - 1);
+      const u64 ia = warp_scan_u64(n), ib = warp_scan_u64(q);
+      u64 pa, pb, ta, tb;
+      block_warp_prefix2(*c.x(), shfl_u64(ia, 31), shfl_u64(ib, 31), pa, pb, ta, tb);
+      ac = pa + ia - n;
+      am = pb + ib - q;
+    }
+    const u64 want = target - above;
+#pragma unroll 1
+    for (int b = hi; b >= hi - 1; --b) {
+      const u64 n = hist[b], q = hist_mass(hist, b);
+      const u64 over = by_mass ? am : ac;
+      if (over < want && want <= over + (by_mass ? q : n)) {
+        c.x()->bcast[0] = (u64)b;
+        c.x()->bcast[1] = ac;
+        c.x()->bcast[2] = am;
+        c.x()->bcast[3] = n;
+        c.x()->bcast[4] = q;
+        c.x()->bcast[7] = 1;
+      }
+      ac += n;
+      am += q;
+    }
+    __syncthreads();
+    if (c.x()->bcast[7] == 0) {  // nothing reaches the target
+      put_state(S.sel.ok, false);
+      put_state(S.sel.key, map.klo);
+      put_state(S.sel.bin_cnt, 0);
+      break;
+    }
+    const int bucket = (int)c.x()->bcast[0];
+    above += by_mass ? c.x()->bcast[2] : c.x()->bcast[1];
+    if (tid == 0) {
+      S.sel.above_cnt += c.x()->bcast[1];
+      S.sel.above_mass += c.x()->bcast[2];
+      S.sel.bin_cnt = c.x()->bcast[3];
+      S.sel.bin_mass = c.x()->bcast[4];
+    }
+    // its members
+    {
+      const float m = c.m;
+      const Scorer sc = c;
+      const uint32_t cut_key = S.kept.cut_key;
+      auto note = [&](uint32_t key, uint32_t cnt, u64 w) {
+        const int slot = atomicAdd(c.gbuf_n(), 1);
+        if (slot < kV3ListCap) c.members()[slot] = V3Member{key, cnt, w};
+        atomicMin(c.span(), key);
+        atomicMax(c.span() + 1, key);
+      };
+      for_each_side3(c, [&](int id, float s) {
+        const uint32_t key = side_ids ? ~(uint32_t)id : key_of(s);
+        if (side_ids && key_of(s) <= cut_key) return;
+        if (map.in(key) && map.bucket(key) == bucket) note(key, 1u, mass_of(s, m));
+      });
+      if (!side_ids) {
+        locate_cells(c, map, bucket);
+        for_located_cells(c, [&](uint32_t n, int cell) {
+          const float s = sc.cell_score(cell);
+          note(key_of(s), n, (u64)n * mass_of(s, m));
+        });
+      }
+    }
+    __syncthreads();
+    const int members = *c.gbuf_n();
+    const uint32_t key_lo = c.span()[0], key_hi = c.span()[1];
+    if (key_lo == key_hi) { put_state(S.sel.key, key_lo); break; }
+    if (members <= kV3ListCap) {
+      // each member against all: what lies above its key, and at it
+      const u64 still = target - above;
+      if (tid < members) {
+        const uint32_t mine = c.members()[tid].key;
+        u64 oc = 0, om = 0, gc = 0, gm = 0;
+#pragma unroll 2
+        for (int j = 0; j < members; ++j) {
+          const V3Member o = c.members()[j];
+          if (o.key > mine) { oc += o.cnt; om += o.w; }
+          if (o.key == mine) { gc += o.cnt; gm += o.w; }
+        }
+        const u64 over = by_mass ? om : oc;
+        if (over < still && still <= over + (by_mass ? gm : gc)) {  // (members of one key write the same)
+          c.x()->bcast[0] = mine;
+          c.x()->bcast[1] = oc; c.x()->bcast[2] = om; c.x()->bcast[3] = gc; c.x()->bcast[4] = gm;
+        }
+      }
+      __syncthreads();
+      if (tid == 0) {
+        S.sel.key = (uint32_t)c.x()->bcast[0];
+        S.sel.above_cnt += c.x()->bcast[1];
+        S.sel.above_mass += c.x()->bcast[2];
+        S.sel.bin_cnt = c.x()->bcast[3];
+        S.sel.bin_mass = c.x()->bcast[4];
+      }
+      break;
+    }
+    map.by_key(key_lo, key_hi);
+    __syncthreads();
+  }
+  __syncthreads();
+}
+
+// Count and mass of all tokens with key >= lo_key, in S.sel.total_cnt / total_mass.
+__device__ __noinline__ void totals3(uint32_t lo_key) {
+  CountState& S = count_state();
+  Ctx3& c = S.c;
+  u64 a = 0, b = 0;
+  if (S.filled && lo_key == 0u) {
+#pragma unroll
+    for (int u = 0; u < kV3Buckets / kThreads; ++u) {
+      const int i = threadIdx.x + u * kThreads;
+      a += c.hist()[i];
+      b += hist_mass(c.hist(), i);
+    }
+  } else {
+    const float m = c.m;
+    for_each_side3(c, [&](int, float s) {
+      if (key_of(s) >= lo_key) { ++a; b += mass_of(s, m); }
+    });
+    for_each_class(c, [&](bool valid, uint32_t key, uint32_t n, int) {
+      if (valid && key >= lo_key) { a += n; b += (u64)n * mass_of(score_of(key), m); }
+    });
+  }
+  block_sum2(*c.x(), a, b);
+  put_state(S.sel.total_cnt, a);
+  put_state(S.sel.total_mass, b);
+  __syncthreads();
 }
 
 // The side list (tokens held three times or more, values outside the bin window), the row's maximum
@@ -181,7 +398,7 @@ __device__ __noinline__ bool phase_histogram() {
   phase_mark(S, 2);
   // ---- the histogram (in the place of the rare tokens and set-aside chunks, which have served)
   if (!c.greedy || S.P.n_logprobs >= 0) {
-    hist_fill<true>(c.hist(), AllTokens3{&c}, S.all_map);
+    fill_hist(S.all_map, false);
     put_state(S.filled, true);
     __syncthreads();
   }
@@ -195,25 +412,23 @@ __device__ __noinline__ void phase_cuts() {
   Ctx3& c = S.c;
   const hs_row_params& P = S.P;
   const int tid = threadIdx.x;
-  const float m = c.m;
-  bool filled = S.filled;
   uint32_t cut_key = 0;
   u64 cnt = 0, mass = 0;
   bool have_totals = false;
   if (P.top_k > 0 && P.top_k < c.vocab) {
-    const Selection sk = select_key<false, true>(c, AllTokens3{&c}, S.all_map, filled, (u64)P.top_k);
-    if (!sk.ok) raise_status(S, 1);
-    cut_key = sk.key;
-    cnt = sk.above_cnt + sk.bin_cnt;
-    mass = sk.above_mass + sk.bin_mass;
-    have_totals = sk.ok;
+    select_key(false, false, (u64)P.top_k);
+    if (!S.sel.ok) raise_status(S, 1);
+    cut_key = S.sel.key;
+    cnt = S.sel.above_cnt + S.sel.bin_cnt;
+    mass = S.sel.above_mass + S.sel.bin_mass;
+    have_totals = S.sel.ok;
     put_state(S.out.n_after_topk, cnt);
-    put_state(S.cut_group_cnt, sk.bin_cnt);
+    put_state(S.cut_group_cnt, S.sel.bin_cnt);
   }
   phase_mark(S, 4);
   if (P.min_p > 0.0f) {
-    if (!have_totals) { totals3(c, cut_key, filled, cnt, mass); have_totals = true; }
-    const float z1 = mass_to_float(mass);
+    if (!have_totals) { totals3(cut_key); cnt = S.sel.total_cnt; mass = S.sel.total_mass; have_totals = true; }
+    const float z1 = mass_to_float(mass), m = c.m;
     const float thr = __fmul_rn(__fdiv_rn(1.0f, z1), P.min_p);
     uint32_t lowest = 0xffffffffu;
     auto consider = [&](uint32_t k) {
@@ -228,10 +443,9 @@ __device__ __noinline__ void phase_cuts() {
     }
   }
   phase_mark(S, 5);
-  if (!have_totals) totals3(c, cut_key, filled, cnt, mass);
+  if (!have_totals) { totals3(cut_key); cnt = S.sel.total_cnt; mass = S.sel.total_mass; }
   put_state(S.out.n_after_minp, cnt);
   if (P.top_p < 1.0f) {
-    Selection sp{};
     if (mass > 0) {
       // (double precision, slow: the lanes of one warp try neighbouring candidates at once)
       if (tid < 32) {
@@ -240,32 +454,32 @@ __device__ __noinline__ void phase_cuts() {
       }
       __syncthreads();
       phase_mark(S, 20);
-      sp = select_key<true, true>(c, AllTokens3{&c}, S.all_map, filled, c.x()->bcast[6]);
+      select_key(true, false, c.x()->bcast[6]);
       phase_mark(S, 21);
     }
-    if (sp.ok && sp.bin_cnt > 0) {
-      const u64 qv = sp.bin_mass / sp.bin_cnt;  // every token at the cut key has the same mass
-      u64 t = sp.bin_cnt;
+    if (mass > 0 && S.sel.ok && S.sel.bin_cnt > 0) {
+      const u64 qv = S.sel.bin_mass / S.sel.bin_cnt;  // every token at the cut key has the same mass
+      u64 t = S.sel.bin_cnt;
       if (qv > 0) {
-        const u64 want = sp.target - sp.above_mass;
+        const u64 want = S.sel.target - S.sel.above_mass;
         t = (want + qv - 1) / qv;
         if (t < 1) t = 1;
-        if (t > sp.bin_cnt) t = sp.bin_cnt;
+        if (t > S.sel.bin_cnt) t = S.sel.bin_cnt;
       }
-      cut_key = sp.key;
-      cnt = sp.above_cnt + t;
-      mass = sp.above_mass + t * qv;
+      cut_key = S.sel.key;
+      cnt = S.sel.above_cnt + t;
+      mass = S.sel.above_mass + t * qv;
       put_state(S.cut_ties, (long long)t);
-      put_state(S.cut_group_cnt, sp.bin_cnt);
-      put_state(S.tie_split, t < sp.bin_cnt);
+      put_state(S.cut_group_cnt, S.sel.bin_cnt);
+      put_state(S.tie_split, t < S.sel.bin_cnt);
     } else {
       raise_status(S, 1);
     }
   }
+  __syncthreads();
   put_state(S.kept.cut_key, cut_key);
   put_state(S.n_kept, cnt);
   put_state(S.q_kept, mass);
-  put_state(S.filled, filled);
   __syncthreads();
   phase_mark(S, 6);
 }
@@ -288,23 +502,14 @@ __device__ __noinline__ void need_tie_limit() {
   __syncthreads();
 }
 
-// What a draw asks for when it does not know the token yet: the nth (by ascending id) member of
-// the cut's tie group, or of one class.
-struct DrawAsk {
-  int kind;  // 0 = the token is known (or there is none), 1 = of the group, 2 = of a class
-  int token;
-  int cell;
-  u64 nth, members;
-};
-
 // The draw by classes: inverse CDF over exact integer masses in the order: classes above the cut, the
 // tie group at the cut (its lowest ids), side elements above the cut (by id).
-__device__ __forceinline__ DrawAsk draw_by_classes(CountState& S, uint64_t seed) {
+__device__ __noinline__ void draw_by_classes(uint64_t seed) {
+  CountState& S = count_state();
   Ctx3& c = S.c;
   const int tid = threadIdx.x;
   const uint32_t cut_key = S.kept.cut_key;
   const float m = c.m;
-  DrawAsk ask{0, -1, -1, 0ull, 0ull};
   u64 target;
   {
     const Philox4 r = philox4x32_10(0u, 0u, 0u, 0u, (uint32_t)seed, (uint32_t)(seed >> 32));
@@ -400,20 +605,19 @@ __device__ __forceinline__ DrawAsk draw_by_classes(CountState& S, uint64_t seed)
       }
     }
     __syncthreads();
-    ask.cell = (int)c.x()->bcast[5] - 1;
-    ask.members = c.x()->bcast[3];
-    ask.nth = c.x()->bcast[4];
-    ask.kind = ask.cell >= 0 ? 2 : 0;
-    __syncthreads();
-    return ask;
+    const int cell = (int)c.x()->bcast[5] - 1;
+    put_state(S.ask, DrawAsk{cell >= 0 ? 2 : 0, -1, cell, c.x()->bcast[4], c.x()->bcast[3]});
+    return;
   }
   // the group at the cut key: cut_ties members when top-p split it, else all of them
   u64 group_kept = (u64)S.cut_ties;
   if (S.cut_ties < 0) {
     // cut by top-k / min-p / nothing: everything at the cut key is kept; count it
     u64 gc = 0, gm = 0;
-    for_classes_at(c, 0, 0, [&](uint32_t k) { return k < cut_key ? -1 : (k > cut_key ? 1 : 0); },
-                   [&](uint32_t, uint32_t n, int) { gc += n; });
+    V3Map at_key;
+    at_key.by_key(cut_key, cut_key);
+    locate_cells(c, at_key, 0);
+    for_located_cells(c, [&](uint32_t n, int) { gc += n; });
     for_each_side3(c, [&](int, float s) { if (key_of(s) == cut_key) gc += 1; });
     block_sum2(*c.x(), gc, gm);
     group_kept = gc;
@@ -421,23 +625,18 @@ __device__ __forceinline__ DrawAsk draw_by_classes(CountState& S, uint64_t seed)
   const u64 q_cut = mass_of(score_of(cut_key), m);
   const u64 q_group = group_kept * q_cut;
   if (target < q_cells + q_group) {
-    ask.kind = 1;
-    ask.nth = q_cut ? (target - q_cells) / q_cut + 1 : 1;
-    return ask;
+    put_state(S.ask, DrawAsk{1, -1, -1, q_cut ? (target - q_cells) / q_cut + 1 : 1ull, 0ull});
+    return;
   }
-  V3Map by_id;
-  by_id.by_key(~(uint32_t)(c.vocab - 1), 0xffffffffu);
-  bool filled = false;
-  const Selection sd = select_key<true, true>(c, KeptSide3{&c, cut_key}, by_id, filled, target - q_cells - q_group + 1);
-  put_state(S.filled, false);
-  if (sd.ok) ask.token = (int)(~sd.key);
-  return ask;
+  select_key(true, true, target - q_cells - q_group + 1);
+  put_state(S.ask, DrawAsk{0, S.sel.ok ? (int)(~S.sel.key) : -1, -1, 0ull, 0ull});
 }
 
 // Finds what a draw asks for: its own function, for the registers of the scan.
-__device__ __noinline__ int phase_find(const DrawAsk ask) {
+__device__ __noinline__ int phase_find() {
   CountState& S = count_state();
   Ctx3& c = S.c;
+  const DrawAsk ask = S.ask;
   if (ask.kind == 1) {
     need_cut_group(S);
     return nth_in_group(c, S.cut_group, ask.nth);  // the kept members are the lowest ids
@@ -460,31 +659,39 @@ __device__ __noinline__ int phase_find(const DrawAsk ask) {
   return nth_in_group(c, only, ask.nth);
 }
 
-__device__ __noinline__ DrawAsk phase_draw() {
+// The token under the reference's own draws: arg max of fl(fl(e / z) / noise) over the kept set, lowest
+// id on ties.
+__device__ __noinline__ int draw_from_noise() {
   CountState& S = count_state();
   Ctx3& c = S.c;
-  const int tid = threadIdx.x;
+  need_tie_limit();
+  const KeptSet kept = S.kept;
+  const float zf = mass_to_float(S.q_kept), m = c.m;
+  const float* noise_row = S.noise + (size_t)S.row * c.vocab;
+  u64 best = 0;
+#pragma unroll 1
+  for (int id = threadIdx.x; id < c.vocab; id += kThreads) {
+    const float s = c.element_score(id, c.logits[id], c.class_of(id));
+    if (!kept.has(key_of(s), id)) continue;
+    const float p = __fdiv_rn(expf(s - m), zf);
+    const float ratio = __fdiv_rn(p, noise_row[id]);
+    const u64 packed = ((u64)__float_as_uint(ratio) << 32) | (uint32_t)(~(uint32_t)id);
+    best = packed > best ? packed : best;
+  }
+  best = block_max_u64(*c.x(), best);
+  return (int)(~(uint32_t)(best & 0xffffffffu));
+}
+
+// The draw: the token, or what is left to be found of it, in S.ask.
+__device__ __noinline__ void phase_draw() {
+  CountState& S = count_state();
+  Ctx3& c = S.c;
   const uint64_t seed = S.P.seed;
-  DrawAsk ask{0, -1, -1, 0ull, 0ull};
-  if (S.q_kept == 0) return ask;  // (nothing has any mass: reported by the caller)
-  if (S.noise) {
-    // reference draws: arg max of fl(fl(e / z) / noise) over the kept set, lowest id on ties
-    need_tie_limit();
-    const KeptSet kept = S.kept;
-    const float zf = mass_to_float(S.q_kept), m = c.m;
-    const float* noise_row = S.noise + (size_t)S.row * c.vocab;
-    u64 best = 0;
-    for (int id = tid; id < c.vocab; id += kThreads) {
-      const float s = c.element_score(id, c.logits[id], c.class_of(id));
-      if (!kept.has(key_of(s), id)) continue;
-      const float p = __fdiv_rn(expf(s - m), zf);
-      const float ratio = __fdiv_rn(p, noise_row[id]);
-      const u64 packed = ((u64)__float_as_uint(ratio) << 32) | (uint32_t)(~(uint32_t)id);
-      best = packed > best ? packed : best;
-    }
-    best = block_max_u64(*c.x(), best);
-    ask.token = (int)(~(uint32_t)(best & 0xffffffffu));
-    return ask;
+  if (S.q_kept == 0 || S.noise) {
+    // (nothing has any mass: no token, reported by the caller)
+    const int token = S.q_kept == 0 ? -1 : draw_from_noise();
+    put_state(S.ask, DrawAsk{0, token, -1, 0ull, 0ull});
+    return;
   }
   // Near-flat rows: rejection on tokens, when one round is all but sure to accept.
   const float q = mass_to_float(S.q_kept);
@@ -495,44 +702,62 @@ __device__ __noinline__ DrawAsk phase_draw() {
     const u64 ties = S.cut_ties > 0 ? (u64)S.cut_ties : 0ull;
     const int t = draw_by_token_rejection(c, S.kept, S.tie_split, ties, S.cut_group_cnt, seed, 4, trials, group_hit);
     if (t >= 0) {
-      ask.token = t;
+      u64 nth = 0;
       if (group_hit) {
         // one of the kept members of the group the cut splits: its lowest ids
         const Philox4 r = philox4x32_10(0u, 0u, 0u, 4u, (uint32_t)seed, (uint32_t)(seed >> 32));
-        ask.kind = 1;
-        ask.nth = 1 + __umul64hi(((u64)r.v[0] << 32) | r.v[1], ties);
+        nth = 1 + __umul64hi(((u64)r.v[0] << 32) | r.v[1], ties);
       }
-      return ask;
+      put_state(S.ask, DrawAsk{group_hit ? 1 : 0, t, -1, nth, 0ull});
+      return;
     }
   }
-  return draw_by_classes(S, seed);
+  draw_by_classes(seed);
+}
+
+// The tokens of the row at or above `key`: those above it into the gather buffer, with their keys,
+// those at it into the list of ids (at most kV3TieCap are kept) with the lowest of them in *low_id.
+// Side elements come from the side list, the rest from one walk of the row against per-class raw
+// thresholds.
+__device__ __noinline__ void collect_at_or_above(uint32_t key, int* low_id) {
+  CountState& S = count_state();
+  Ctx3& c = S.c;
+  int* small = count_small();
+  int* tie_n = small + 26;
+  if (threadIdx.x == 0) { *c.gbuf_n() = 0; *tie_n = 0; *low_id = 0x7fffffff; }
+  __syncthreads();
+  auto take = [&](uint32_t k, int id) {
+    if (k > key) {
+      const int slot = atomicAdd(c.gbuf_n(), 1);
+      if (slot < kV3ListCap) c.gbuf()[slot] = V3Entry{k, id};
+    } else if (k == key) {
+      const int slot = atomicAdd(tie_n, 1);
+      if (slot < kV3TieCap) c.list()[slot] = id;
+      atomicMin(low_id, id);
+    }
+  };
+  for_each_side3(c, [&](int id, float s) { take(key_of(s), id); });
+  CandCtx bound_ctx{nullptr, nullptr, nullptr, nullptr, small + 8, nullptr};
+  cand_thresholds(c, bound_ctx, key);  // (ends with a barrier)
+  const Scorer sc = c;
+  stream_at_or_above(c, bound_ctx.thr, [&](int id, uint32_t raw, int cc) {
+    if (v3_bin_of_raw(raw) < 0) return;  // outside the bin window: a side element, taken above
+    take(key_of(sc.score_of(raw, cc)), id);
+  });
+  __syncthreads();
 }
 
 // Arg max with penalties: the lowest id among the tokens whose score key is the maximum.
 __device__ __noinline__ void phase_greedy() {
   CountState& S = count_state();
-  Ctx3& c = S.c;
-  int* small = count_small();
-  int* low_id = small + 3;
-  const uint32_t max_key = S.max_key;
-  const int side_arg = (int)(~(uint32_t)(S.side_best & 0xffffffffu));
-  if (threadIdx.x == 0) *low_id = (uint32_t)(S.side_best >> 32) == max_key ? side_arg : 0x7fffffff;
-  CandCtx bound_ctx{nullptr, nullptr, nullptr, nullptr, small + 8, nullptr};
-  cand_thresholds(c, bound_ctx, max_key);  // (ends with a barrier)
-  {
-    const Scorer sc = c;
-    stream_at_or_above(c, bound_ctx.thr, [&](int id, uint32_t raw, int cc) {
-      if (v3_bin_of_raw(raw) >= 0 && key_of(sc.score_of(raw, cc)) == max_key) atomicMin(low_id, id);
-    });
-  }
-  __syncthreads();
+  int* low_id = count_small() + 3;
+  collect_at_or_above(S.max_key, low_id);
   int token = *low_id;
-  if (token == 0x7fffffff) { token = S.side_best ? side_arg : 0; raise_status(S, 1); }
+  if (token == 0x7fffffff) { token = S.side_best ? (int)(~(uint32_t)(S.side_best & 0xffffffffu)) : 0; raise_status(S, 1); }
   put_state(S.token, token);
   if (S.P.n_logprobs >= 0) {
-    u64 cn, q;
-    totals3(c, 0u, S.filled, cn, q);
-    put_state(S.q_kept, q);
+    totals3(0u);
+    put_state(S.q_kept, S.sel.total_mass);
   }
   __syncthreads();
 }
@@ -562,46 +787,19 @@ __device__ __noinline__ void phase_logprobs() {
   int n_want = min(S.P.n_logprobs, c.vocab);
   if ((u64)n_want > S.n_kept) n_want = (int)S.n_kept;
   if (n_want > 0) {
-    bool filled = S.filled;
     // (the kept tokens are the highest: the N highest of them are the N highest of all)
-    const Selection sn = select_key<false, false>(c, AllTokens3{&c}, S.all_map, filled, (u64)n_want);
-    if (sn.ok) {
-      const int need = n_want - (int)sn.above_cnt;  // lowest ids of the group at the N-th key
-      // The tokens above the N-th key (fewer than N) and the group at it: side elements come
-      // from the side list, the rest from one walk of the row against per-class raw
-      // thresholds.  The group's ids go to a list of their own; a group too large for it is
-      // walked the slow way.
+    select_key(false, false, (u64)n_want);
+    if (S.sel.ok) {
+      const int need = n_want - (int)S.sel.above_cnt;  // lowest ids of the group at the N-th key
+      const uint32_t nth_key = S.sel.key;
+      phase_mark(S, 16);
+      collect_at_or_above(nth_key, small + 3);
+      phase_mark(S, 17);
       int* tie_ids = c.list();
-      int* tie_n = small + 3;
       int* gbuf_n = c.gbuf_n();
       V3Entry* gbuf = c.gbuf();
-      if (tid == 0) { *gbuf_n = 0; *tie_n = 0; }
-      __syncthreads();
-      const uint32_t nth_key = sn.key;
-      auto take = [&](uint32_t k, int id) {
-        if (k > nth_key) {
-          const int slot = atomicAdd(gbuf_n, 1);
-          if (slot < kV3ListCap) gbuf[slot] = V3Entry{k, id};
-        } else if (k == nth_key && need > 0) {
-          const int slot = atomicAdd(tie_n, 1);
-          if (slot < kV3TieCap) tie_ids[slot] = id;
-        }
-      };
-      for_each_side3(c, [&](int id, float s) { take(key_of(s), id); });
-      CandCtx bound_ctx{nullptr, nullptr, nullptr, nullptr, small + 8, nullptr};
-      cand_thresholds(c, bound_ctx, nth_key);  // (ends with a barrier)
-      phase_mark(S, 16);
-      {
-        const Scorer sc = c;
-        stream_at_or_above(c, bound_ctx.thr, [&](int id, uint32_t raw, int cc) {
-          if (v3_bin_of_raw(raw) < 0) return;  // outside the bin window: a side element, taken above
-          take(key_of(sc.score_of(raw, cc)), id);
-        });
-      }
-      __syncthreads();
-      phase_mark(S, 17);
       if (need > 0) {
-        const int n_tie = *tie_n;
+        const int n_tie = small[26];
         if (n_tie <= kV3TieCap) {
           // the `need` lowest ids of the group: each id counts the ids below it
           for (int t = tid; t < n_tie; t += kThreads) {
@@ -662,10 +860,11 @@ __device__ __forceinline__ void finish_counted_row() {
     phase_greedy();
   } else {
     phase_cuts();
-    const DrawAsk ask = phase_draw();
+    phase_draw();
+    __syncthreads();
     phase_mark(S, 14);
-    int token = ask.token;
-    if (ask.kind) token = phase_find(ask);
+    int token = S.ask.token;
+    if (S.ask.kind) token = phase_find();
     if (token < 0 || token == 0x7fffffff) {
       token = S.side_best ? (int)(~(uint32_t)(S.side_best & 0xffffffffu)) : 0;
       raise_status(S, 1);

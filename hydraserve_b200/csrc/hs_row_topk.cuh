@@ -174,7 +174,7 @@ __device__ int cand_compact(CandCtx& L, int n, uint32_t bound) {
 // Per count class, the lowest raw value (as signed 16-bit image) whose score reaches `bound`
 // (32768 if none does).  Scores grow with the value inside a class, so warp cc searches the
 // 65,536 values of class cc 32 at a time: four rounds of one evaluation per lane and a ballot.
-__device__ void cand_thresholds(const Ctx3& c, CandCtx& L, uint32_t bound) {
+__device__ __noinline__ void class_thresholds(const Scorer sc, int* thr, uint32_t bound) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < 3) {
     const int cc = warp;
@@ -184,7 +184,7 @@ __device__ void cand_thresholds(const Ctx3& c, CandCtx& L, uint32_t bound) {
     while (lo < hi) {
       const int step = (hi - lo + 31) >> 5;
       const int t = lo + (lane + 1) * step - 1;  // last value of this lane's block
-      const bool pass = t >= hi || key_of(c.score_of(raw_of_t16(t), cc)) >= bound;
+      const bool pass = t >= hi || key_of(sc.score_of(raw_of_t16(t), cc)) >= bound;
       const uint32_t votes = __ballot_sync(0xffffffffu, pass);
       if (votes == 0) { lo = hi; break; }
       const int f = __ffs(votes) - 1;  // the answer lies in block f
@@ -194,11 +194,12 @@ __device__ void cand_thresholds(const Ctx3& c, CandCtx& L, uint32_t bound) {
     if (lane == 0) {
       // -0.0 scores like +0.0 but sits one step below it in the integer order
       if (lo == 0) lo = -1;
-      L.thr[cc] = lo;
+      thr[cc] = lo;
     }
   }
   __syncthreads();
 }
+__device__ __forceinline__ void cand_thresholds(const Ctx3& c, CandCtx& L, uint32_t bound) { class_thresholds(c, L.thr, bound); }
 
 // Calls hit(id, raw, count class) for every token of the row whose score key can reach the
 // bound the thresholds stand for: raw value (as signed 16-bit image) >= thr[class] for the
@@ -223,31 +224,31 @@ __device__ void stream_at_or_above(const Ctx3& c, const int* thr, Hit&& hit) {
   const int n8 = c.n8();
   const uint4* src4 = c.chunks();
   constexpr int kInFlight = 8;
+#pragma unroll 1
   for (int base = 0; base < n8; base += kInFlight * kThreads) {
     uint4 w[kInFlight];
 #pragma unroll
     for (int u = 0; u < kInFlight; ++u) {
       const int i = base + tid + u * kThreads;
-      if (i < n8) w[u] = __ldcg(src4 + i);
+      w[u] = i < n8 ? __ldcg(src4 + i) : make_uint4(~0u, ~0u, ~0u, ~0u);  // (NaNs: no hits)
     }
+    u64 hits = 0;  // bit 8 u + q: token q of chunk u (the rare hit is handled in one place, its value read again)
 #pragma unroll
     for (int u = 0; u < kInFlight; ++u) {
-      const int i = base + tid + u * kThreads;
-      if (i >= n8) break;
       const uint32_t m0 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[u].x), thr2);
       const uint32_t m1 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[u].y), thr2);
       const uint32_t m2 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[u].z), thr2);
       const uint32_t m3 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[u].w), thr2);
       if (!(m0 | m1 | m2 | m3)) continue;  // the common case
-      uint32_t hits = ((m0 & 1u) | ((m0 >> 15) & 2u)) | (((m1 & 1u) | ((m1 >> 15) & 2u)) << 2) |
-                      (((m2 & 1u) | ((m2 >> 15) & 2u)) << 4) | (((m3 & 1u) | ((m3 >> 15) & 2u)) << 6);
+      const uint32_t h = ((m0 & 1u) | ((m0 >> 15) & 2u)) | (((m1 & 1u) | ((m1 >> 15) & 2u)) << 2) |
+                         (((m2 & 1u) | ((m2 >> 15) & 2u)) << 4) | (((m3 & 1u) | ((m3 >> 15) & 2u)) << 6);
+      hits |= (u64)h << (8 * u);
+    }
 #pragma unroll 1
-      while (hits) {
-        const int q = __ffs(hits) - 1;
-        hits &= hits - 1;
-        const uint32_t word = q < 2 ? w[u].x : (q < 4 ? w[u].y : (q < 6 ? w[u].z : w[u].w));
-        look(c.first_of(i) + q, (word >> (16 * (q & 1))) & 0xffffu);
-      }
+    for (; hits; hits &= hits - 1) {
+      const int q = __ffsll((long long)hits) - 1;
+      const int id = c.first_of(base + tid + (q >> 3) * kThreads) + (q & 7);
+      look(id, c.logits[id]);
     }
   }
   if (tid < c.n_loose()) {

@@ -231,18 +231,15 @@ struct Ctx3 : Scorer {
 
 template <class F>
 __device__ __forceinline__ void for_each_side3(const Ctx3& c, F&& f) {
-  for (int j0 = threadIdx.x; j0 < c.n_s; j0 += 4 * kThreads) {
-    int2 e[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = j0 + u * kThreads;
-      e[u] = j < c.n_s ? c.s_pair[j] : make_int2(-1, 0);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (e[u].x >= 0) f(e[u].x, __int_as_float(e[u].y));
+  const int2* pairs = c.s_pair;
+  const int n = c.n_s;
+#pragma unroll 1
+  for (int j = threadIdx.x; j < n; j += kThreads) {
+    const int2 e = pairs[j];
+    if (e.x >= 0) f(e.x, __int_as_float(e.y));
   }
 }
+
 // ---- the row's classes, in order --------------------------------------------------------------
 // Scores grow with the bin inside a count class, so a count class's cells, from its lowest to its
 // highest non-empty one, are in the order of their scores.
@@ -271,43 +268,6 @@ __device__ __forceinline__ void for_each_class(const Ctx3& c, F&& f) {
     }
   }
 }
-// Calls f(key, tokens, cell) for the non-empty cells whose keys k have low <= place(k) <= high, for a
-// place that grows with the key.  Warp w looks for one end of count class w % 3's range, 32 cells
-// at a time; then the ranges' cells go to the threads one by one.  Called by the whole CTA.
-template <class Place, class F>
-__device__ __forceinline__ void for_classes_at(const Ctx3& c, int low, int high, Place&& place, F&& f) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const Scorer sc = c;
-  __syncthreads();
-  if (warp < 6) {
-    const int k = warp % 3, top = c.ends()[k];
-    const int want = warp < 3 ? low : high + 1;  // the first cell whose place is at least this
-    int lo = top ? c.ends()[3 + k] : 0, hi = top;
-#pragma unroll 1
-    while (lo < hi) {
-      const int step = (hi - lo + 31) >> 5;
-      const int t = lo + (lane + 1) * step - 1;
-      const bool pass = t >= hi || place(sc.key_of_bin(min(t, hi - 1) - k * kV3Bins, k)) >= want;
-      const uint32_t votes = __ballot_sync(0xffffffffu, pass);
-      if (votes == 0) { lo = hi; break; }
-      const int first = __ffs(votes) - 1;
-      hi = min(lo + (first + 1) * step - 1, hi);
-      lo = lo + first * step;
-    }
-    if (lane == 0) c.range()[warp] = lo;
-  }
-  __syncthreads();
-#pragma unroll 1
-  for (int k = 0; k < 3; ++k) {
-#pragma unroll 1
-    for (int cell = c.range()[k] + (int)threadIdx.x; cell < c.range()[3 + k]; cell += kThreads) {
-      const uint32_t n = c.tab()[cell];
-      if (n) f(sc.key_of_bin(cell - k * kV3Bins, k), n, cell);
-    }
-  }
-}
-
-// ---- selection inside one CTA ------------------------------------------------------------
 // Where a key falls among the buckets: by score, over equal widths from `lo` to the row maximum
 // (lin), or by the key itself, over [klo, khi].  Both grow with the key.
 struct V3Map {
@@ -337,213 +297,43 @@ struct V3Map {
     scale = lin ? __fdiv_rn((float)kV3Buckets - 0.5f, range) : 0.f;
   }
 };
-template <bool WITH_MASS>
-__device__ __forceinline__ void hist_add(uint32_t* hist, int b, uint32_t cnt, u64 mass) {
-  atomicAdd(hist + b, cnt);
-  if (!WITH_MASS) return;
-  const uint32_t a0 = (uint32_t)mass & kLimbMask, a1 = (uint32_t)(mass >> kLimbBits) & kLimbMask, a2 = (uint32_t)(mass >> (2 * kLimbBits));
-  if (a0) atomicAdd(hist + kV3Buckets + b, a0);
-  if (a1) atomicAdd(hist + 2 * kV3Buckets + b, a1);
-  if (a2) atomicAdd(hist + 3 * kV3Buckets + b, a2);
-}
-__device__ __forceinline__ u64 hist_mass(const uint32_t* hist, int b) {
-  return (u64)hist[kV3Buckets + b] + ((u64)hist[2 * kV3Buckets + b] << kLimbBits) + ((u64)hist[3 * kV3Buckets + b] << (2 * kLimbBits));
-}
-
-// Every token of the row: side elements one by one, classes with their count.
-struct AllTokens3 {
-  const Ctx3* c;
-  // into the histogram.  The thousands of values next to zero share a bucket, and would queue up at
-  // one address: a warp whose cells all fall into one bucket adds them up first.
-  template <bool WITH_MASS>
-  __device__ __forceinline__ void fill(const V3Map& map) const {
-    const float m = c->m;
-    uint32_t* hist = c->hist();
-    for_each_side3(*c, [&](int, float s) {
-      const uint32_t key = key_of(s);
-      if (map.in(key)) hist_add<WITH_MASS>(hist, map.bucket(key), 1u, WITH_MASS ? mass_of(s, m) : 0ull);
-    });
-    for_each_class(*c, [&](bool valid, uint32_t key, uint32_t n, int) {
-      valid = valid && map.in(key);
-      const int b = map.bucket(key);
-      const u64 w = WITH_MASS ? (u64)n * mass_of(score_of(key), m) : 0ull;
-      const int first = __reduce_min_sync(0xffffffffu, valid ? b : 0x7fffffff);
-      if (__all_sync(0xffffffffu, !valid || b == first)) {
-        const uint32_t cnt = __reduce_add_sync(0xffffffffu, valid ? n : 0u);
-        const u64 sum = WITH_MASS ? warp_sum_u64(valid ? w : 0ull) : 0ull;
-        if (cnt && (threadIdx.x & 31) == 0) hist_add<WITH_MASS>(hist, first, cnt, sum);
-      } else if (valid) {
-        hist_add<WITH_MASS>(hist, b, n, w);
-      }
-    });
-  }
-  // f(key, count, mass) of bucket b
-  template <bool WITH_MASS, class F>
-  __device__ __forceinline__ void members(const V3Map& map, int b, F&& f) const {
-    const float m = c->m;
-    for_each_side3(*c, [&](int, float s) {
-      const uint32_t key = key_of(s);
-      if (map.in(key) && map.bucket(key) == b) f(key, 1u, WITH_MASS ? mass_of(s, m) : 0ull);
-    });
-    for_classes_at(*c, b, b, [&](uint32_t key) { return map.bucket(key); }, [&](uint32_t key, uint32_t n, int) {
-      f(key, n, WITH_MASS ? (u64)n * mass_of(score_of(key), m) : 0ull);
-    });
-  }
-};
-// Kept side elements keyed by ~id: the side part of the draw.
-struct KeptSide3 {
-  const Ctx3* c;
-  uint32_t cut_key;
-  template <bool WITH_MASS>
-  __device__ __forceinline__ void fill(const V3Map& map) const {
-    for_each_side3(*c, [&](int id, float s) {
-      const uint32_t key = ~(uint32_t)id;
-      if (key_of(s) > cut_key && map.in(key)) hist_add<WITH_MASS>(c->hist(), map.bucket(key), 1u, mass_of(s, c->m));
-    });
-  }
-  template <bool WITH_MASS, class F>
-  __device__ __forceinline__ void members(const V3Map& map, int b, F&& f) const {
-    for_each_side3(*c, [&](int id, float s) {
-      const uint32_t key = ~(uint32_t)id;
-      if (key_of(s) > cut_key && map.in(key) && map.bucket(key) == b) f(key, 1u, mass_of(s, c->m));
-    });
-  }
-};
-template <bool WITH_MASS, class From>
-__device__ __forceinline__ void hist_fill(uint32_t* hist, const From& from, const V3Map& map) {
-#pragma unroll
-  for (int b = 0; b < 4 * kV3Buckets / kThreads; ++b) hist[threadIdx.x + b * kThreads] = 0;
+// Where the cells of bucket b lie: c.range()[k] to c.range()[3 + k] of count class k (a bucket grows with
+// the key, and keys grow with the cell).  Warp w looks for one end of class w % 3's range, 32 cells
+// at a time.  Called by the whole CTA; barriers on both sides.
+__device__ __noinline__ void locate_cells(const Ctx3& c, const V3Map map, int b) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __syncthreads();
-  from.template fill<WITH_MASS>(map);
-  __syncthreads();
-}
-
-// The key, from the top, at which the running count (BY_MASS: mass) of the elements reaches
-// `target`, with what lies above and at it.  filled: the histogram holds all elements under `map`
-// already (false afterwards if it had to be used for something else).
-template <bool BY_MASS, bool WITH_MASS, class From>
-__device__ Selection select_key(Ctx3& c, const From& from, V3Map map, bool& filled, u64 target) {
-  static_assert(WITH_MASS || !BY_MASS, "a cut by mass needs masses");
-  const int tid = threadIdx.x;
-  uint32_t* hist = c.hist();
-  Selection sel{};
-  sel.target = target;
-  sel.levels = 3;
+  if (warp < 6) {
+    const Scorer sc = c;
+    const int k = warp % 3, top = c.ends()[k];
+    const int want = warp < 3 ? b : b + 1;  // the first cell whose bucket is at least this
+    int lo = top ? c.ends()[3 + k] : 0, hi = top;
 #pragma unroll 1
-  for (int round = 0; round < 8; ++round) {
-    if (!filled || round > 0) {
-      hist_fill<WITH_MASS>(hist, from, map);
-      filled = false;
+    while (lo < hi) {
+      const int step = (hi - lo + 31) >> 5;
+      const int t = lo + (lane + 1) * step - 1;
+      const bool pass = t >= hi || map.bucket(sc.key_of_bin(min(t, hi - 1) - k * kV3Bins, k)) >= want;
+      const uint32_t votes = __ballot_sync(0xffffffffu, pass);
+      if (votes == 0) { lo = hi; break; }
+      const int first = __ffs(votes) - 1;
+      hi = min(lo + (first + 1) * step - 1, hi);
+      lo = lo + first * step;
     }
-    if (tid == 0) { c.x()->bcast[7] = 0; *c.gbuf_n() = 0; c.span()[0] = 0xffffffffu; c.span()[1] = 0u; }
-    // thread t owns the two buckets 1,023 - 2 t and 1,022 - 2 t
-    static_assert(kV3Buckets == 2 * kThreads, "two buckets per thread");
-    const int hi = kV3Buckets - 1 - 2 * tid;
-    u64 ac = 0, am = 0;  // above this thread's buckets
-    {
-      const u64 n = (u64)hist[hi] + hist[hi - 1];
-      const u64 q = WITH_MASS ? hist_mass(hist, hi) + hist_mass(hist, hi - 1) : 0ull;
-      const u64 ia = warp_scan_u64(n), ib = WITH_MASS ? warp_scan_u64(q) : 0ull;
-      u64 pa, pb, ta, tb;
-      block_warp_prefix2(*c.x(), shfl_u64(ia, 31), WITH_MASS ? shfl_u64(ib, 31) : 0ull, pa, pb, ta, tb);
-      ac = pa + ia - n;
-      am = pb + ib - q;
-    }
-    const u64 want = sel.target - (BY_MASS ? sel.above_mass : sel.above_cnt);
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const u64 n = hist[hi - u], q = WITH_MASS ? hist_mass(hist, hi - u) : 0ull;
-      const u64 over = BY_MASS ? am : ac;
-      if (over < want && want <= over + (BY_MASS ? q : n)) {
-        c.x()->bcast[0] = (u64)(hi - u);
-        c.x()->bcast[1] = ac;
-        c.x()->bcast[2] = am;
-        c.x()->bcast[3] = n;
-        c.x()->bcast[4] = q;
-        c.x()->bcast[7] = 1;
-      }
-      ac += n;
-      am += q;
-    }
-    __syncthreads();
-    if (c.x()->bcast[7] == 0) {  // nothing reaches the target
-      sel.ok = false;
-      sel.key = map.klo;
-      __syncthreads();
-      return sel;
-    }
-    const int bucket = (int)c.x()->bcast[0];
-    sel.ok = true;
-    sel.above_cnt += c.x()->bcast[1];
-    sel.above_mass += c.x()->bcast[2];
-    sel.bin_cnt = c.x()->bcast[3];
-    sel.bin_mass = c.x()->bcast[4];
-    from.template members<WITH_MASS>(map, bucket, [&](uint32_t key, uint32_t cnt, u64 w) {
-      const int slot = atomicAdd(c.gbuf_n(), 1);
-      if (slot < kV3ListCap) c.members()[slot] = V3Member{key, cnt, w};
-      atomicMin(c.span(), key);
-      atomicMax(c.span() + 1, key);
-    });
-    __syncthreads();
-    const int members = *c.gbuf_n();
-    const uint32_t key_lo = c.span()[0], key_hi = c.span()[1];
-    if (key_lo == key_hi) { sel.key = key_lo; break; }
-    if (members <= kV3ListCap) {
-      // each member against all: what lies above its key, and at it
-      const u64 still = sel.target - (BY_MASS ? sel.above_mass : sel.above_cnt);
-      if (tid < members) {
-        const uint32_t mine = c.members()[tid].key;
-        u64 oc = 0, om = 0, gc = 0, gm = 0;
-#pragma unroll 2
-        for (int j = 0; j < members; ++j) {
-          const V3Member o = c.members()[j];
-          if (o.key > mine) { oc += o.cnt; om += o.w; }
-          if (o.key == mine) { gc += o.cnt; gm += o.w; }
-        }
-        const u64 over = BY_MASS ? om : oc;
-        if (over < still && still <= over + (BY_MASS ? gm : gc)) {  // (members of one key write the same)
-          c.x()->bcast[0] = mine;
-          c.x()->bcast[1] = oc; c.x()->bcast[2] = om; c.x()->bcast[3] = gc; c.x()->bcast[4] = gm;
-        }
-      }
-      __syncthreads();
-      sel.key = (uint32_t)c.x()->bcast[0];
-      sel.above_cnt += c.x()->bcast[1];
-      sel.above_mass += c.x()->bcast[2];
-      sel.bin_cnt = c.x()->bcast[3];
-      sel.bin_mass = c.x()->bcast[4];
-      break;
-    }
-    map.by_key(key_lo, key_hi);
-    __syncthreads();
+    if (lane == 0) c.range()[warp] = lo;
   }
-  sel.prefix = sel.key;
   __syncthreads();
-  return sel;
 }
-
-// Count and mass of all tokens with key >= lo_key; hist (or null): a histogram that holds every token,
-// used when lo_key is 0.
-__device__ void totals3(Ctx3& c, uint32_t lo_key, bool filled, u64& cnt, u64& mass) {
-  u64 a = 0, b = 0;
-  if (filled && lo_key == 0u) {
-#pragma unroll
-    for (int u = 0; u < kV3Buckets / kThreads; ++u) {
-      const int i = threadIdx.x + u * kThreads;
-      a += c.hist()[i];
-      b += hist_mass(c.hist(), i);
+// Calls f(tokens, cell) for the non-empty cells that were located, one per thread and step.
+template <class F>
+__device__ __forceinline__ void for_located_cells(const Ctx3& c, F&& f) {
+#pragma unroll 1
+  for (int k = 0; k < 3; ++k) {
+#pragma unroll 1
+    for (int cell = c.range()[k] + (int)threadIdx.x; cell < c.range()[3 + k]; cell += kThreads) {
+      const uint32_t n = c.tab()[cell];
+      if (n) f(n, cell);
     }
-  } else {
-    for_each_side3(c, [&](int, float s) {
-      if (key_of(s) >= lo_key) { ++a; b += mass_of(s, c.m); }
-    });
-    for_each_class(c, [&](bool valid, uint32_t key, uint32_t n, int) {
-      if (valid && key >= lo_key) { a += n; b += (u64)n * mass_of(score_of(key), c.m); }
-    });
   }
-  block_sum2(*c.x(), a, b);
-  cnt = a;
-  mass = b;
 }
 
 // ---- the tie group of a key: the classes (at most one per count class, scores grow with
@@ -553,12 +343,12 @@ struct Group {
   int cell0, cell1, cell2;  // class index per count class, or -1
   __device__ __forceinline__ int cell_of(int cc) const { return cc == 0 ? cell0 : (cc == 1 ? cell1 : cell2); }
 };
-__device__ Group find_group(Ctx3& c, uint32_t key) {
+__device__ __forceinline__ Group find_group(Ctx3& c, uint32_t key) {
   if (threadIdx.x < 3) c.x()->bcast[threadIdx.x] = 0;
-  __syncthreads();
-  for_classes_at(c, 0, 0, [&](uint32_t k) { return k < key ? -1 : (k > key ? 1 : 0); }, [&](uint32_t, uint32_t, int cell) {
-    c.x()->bcast[cell / kV3Bins] = (u64)cell + 1;
-  });
+  V3Map at_key;
+  at_key.by_key(key, key);
+  locate_cells(c, at_key, 0);
+  for_located_cells(c, [&](uint32_t, int cell) { c.x()->bcast[cell / kV3Bins] = (u64)cell + 1; });
   __syncthreads();
   Group g;
   g.key = key;
@@ -583,7 +373,7 @@ __device__ __forceinline__ uint32_t chunk_members(const Ctx3& c, const Group& g,
                                                   uint32_t cls16) {
   const uint32_t words[4] = {w.x, w.y, w.z, w.w};
   uint32_t memb = 0;
-#pragma unroll
+#pragma unroll 1
   for (int k = 0; k < 4; ++k) {
     memb |= (in_group(c, g, c.first_of(i) + 2 * k, words[k] & 0xffffu, (cls16 >> (4 * k)) & 3) ? 1u : 0u) << (2 * k);
     memb |= (in_group(c, g, c.first_of(i) + 2 * k + 1, words[k] >> 16, (cls16 >> (4 * k + 2)) & 3) ? 1u : 0u) << (2 * k + 1);
