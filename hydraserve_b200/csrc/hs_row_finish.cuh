@@ -110,10 +110,16 @@ __device__ __noinline__ void fill_hist(const V3Map map, bool side_ids) {
     if (map.in(key)) hist_add(hist, map.bucket(key), 1u, mass_of(s, m));
   });
   if (!side_ids) {
-    for_each_class(c, [&](bool valid, uint32_t key, uint32_t n, int) {
-      valid = valid && map.in(key);
-      const int b = map.bucket(key);
-      const u64 w = (u64)n * mass_of(score_of(key), m);
+    for_each_class(c, [&](bool valid, float s, uint32_t n, int) {
+      int b;
+      if (map.lin) {
+        b = map.bucket_of(s);
+      } else {
+        const uint32_t key = key_of(s);
+        valid = valid && map.in(key);
+        b = map.bucket(key);
+      }
+      const u64 w = (u64)n * mass_of(s, m);
       const int first = __reduce_min_sync(0xffffffffu, valid ? b : 0x7fffffff);
       if (__all_sync(0xffffffffu, !valid || b == first)) {
         const uint32_t cnt = __reduce_add_sync(0xffffffffu, valid ? n : 0u);
@@ -195,6 +201,7 @@ __device__ __noinline__ void select_key(bool by_mass, bool side_ids, u64 target)
       S.sel.bin_cnt = c.x()->bcast[3];
       S.sel.bin_mass = c.x()->bcast[4];
     }
+    phase_mark(S, 22);
     // its members
     {
       const float m = c.m;
@@ -220,6 +227,7 @@ __device__ __noinline__ void select_key(bool by_mass, bool side_ids, u64 target)
       }
     }
     __syncthreads();
+    phase_mark(S, 23);
     const int members = *c.gbuf_n();
     const uint32_t key_lo = c.span()[0], key_hi = c.span()[1];
     if (key_lo == key_hi) { put_state(S.sel.key, key_lo); break; }
@@ -274,8 +282,8 @@ __device__ __noinline__ void totals3(uint32_t lo_key) {
     for_each_side3(c, [&](int, float s) {
       if (key_of(s) >= lo_key) { ++a; b += mass_of(s, m); }
     });
-    for_each_class(c, [&](bool valid, uint32_t key, uint32_t n, int) {
-      if (valid && key >= lo_key) { a += n; b += (u64)n * mass_of(score_of(key), m); }
+    for_each_class(c, [&](bool valid, float s, uint32_t n, int) {
+      if (valid && key_of(s) >= lo_key) { a += n; b += (u64)n * mass_of(s, m); }
     });
   }
   block_sum2(*c.x(), a, b);
@@ -431,11 +439,12 @@ __device__ __noinline__ void phase_cuts() {
     const float z1 = mass_to_float(mass), m = c.m;
     const float thr = __fmul_rn(__fdiv_rn(1.0f, z1), P.min_p);
     uint32_t lowest = 0xffffffffu;
-    auto consider = [&](uint32_t k) {
-      if (k >= cut_key && !(__fdiv_rn(expf(score_of(k) - m), z1) < thr)) lowest = min(lowest, k);
+    auto consider = [&](float s) {
+      const uint32_t k = key_of(s);
+      if (k >= cut_key && k < lowest && !(__fdiv_rn(expf(s - m), z1) < thr)) lowest = k;
     };
-    for_each_class(c, [&](bool valid, uint32_t key, uint32_t, int) { if (valid) consider(key); });
-    for_each_side3(c, [&](int, float s) { consider(key_of(s)); });
+    for_each_class(c, [&](bool valid, float s, uint32_t, int) { if (valid) consider(s); });
+    for_each_side3(c, [&](int, float s) { consider(s); });
     lowest = ~block_max_u32(*c.x(), ~lowest);
     if (lowest != 0xffffffffu && lowest > cut_key) {
       cut_key = lowest;
@@ -519,10 +528,13 @@ __device__ __noinline__ void draw_by_classes(uint64_t seed) {
   // turn make a list, and its entries j, j + kThreads, ... are chunk j.  (Any fixed order
   // would do; the counts alone decide it.)  A thread adds its cells' masses to their chunks.
   const uint32_t* tab = c.tab();
-  const int n_cells = (S.penalised ? 3 : 1) * kPerClass;
   int mine = 0;
-#pragma unroll 4
-  for (int u = 0; u < n_cells; ++u) mine += tab[tid + u * kThreads] ? 1 : 0;
+#pragma unroll 1
+  for (int k = 0; k < 3; ++k) {
+    if (c.ends()[k] == 0) continue;
+#pragma unroll
+    for (int u = 0; u < kPerClass; ++u) mine += tab[tid + (k * kPerClass + u) * kThreads] ? 1 : 0;
+  }
   uint32_t* chunks = reinterpret_cast<uint32_t*>(c.members());  // [3][kThreads]: mass in limbs
   static_assert(3 * kThreads * sizeof(uint32_t) <= sizeof(V3Member) * kV3ListCap + sizeof(int) * kV3TieCap, "the chunks fit the members' place");
 #pragma unroll
@@ -530,35 +542,18 @@ __device__ __noinline__ void draw_by_classes(uint64_t seed) {
   int n_cl;
   const int list_at = block_place(count_small() + 48, mine, n_cl);
   {
-    const Scorer sc = c;
-    int at = list_at;
-    constexpr int kBatch = 3;  // (scoring a cell is a long chain)
-    static_assert(kPerClass % kBatch == 0, "a batch is of one count class");
-#pragma unroll 1
-    for (int u0 = 0; u0 < n_cells; u0 += kBatch) {
-      uint32_t n[kBatch], key[kBatch];
-      u64 w[kBatch];
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) n[u] = tab[tid + (u0 + u) * kThreads];
-      if (!__any_sync(0xffffffffu, (n[0] | n[1] | n[2]) != 0u)) continue;
-      const int k = u0 / kPerClass;
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) {
-        key[u] = sc.key_of_bin(tid + (u0 + u) * kThreads - k * kV3Bins, k);
-        w[u] = (u64)n[u] * mass_of(score_of(key[u]), m);
+    int at = list_at;  // (a thread's cells come in the order of the list)
+    for_each_class(c, [&](bool valid, float s, uint32_t n, int) {
+      if (!valid) return;
+      if (key_of(s) > cut_key) {
+        const u64 w = (u64)n * mass_of(s, m);
+        uint32_t* dst = chunks + (at & (kThreads - 1));
+        atomicAdd(dst, (uint32_t)w & kLimbMask);
+        atomicAdd(dst + kThreads, (uint32_t)(w >> kLimbBits) & kLimbMask);
+        atomicAdd(dst + 2 * kThreads, (uint32_t)(w >> (2 * kLimbBits)));
       }
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) {
-        if (!n[u]) continue;
-        if (key[u] > cut_key) {
-          uint32_t* dst = chunks + (at & (kThreads - 1));
-          atomicAdd(dst, (uint32_t)w[u] & kLimbMask);
-          atomicAdd(dst + kThreads, (uint32_t)(w[u] >> kLimbBits) & kLimbMask);
-          atomicAdd(dst + 2 * kThreads, (uint32_t)(w[u] >> (2 * kLimbBits)));
-        }
-        ++at;
-      }
-    }
+      ++at;
+    });
   }
   __syncthreads();
   const u64 chunk = (u64)chunks[tid] + ((u64)chunks[tid + kThreads] << kLimbBits) + ((u64)chunks[tid + 2 * kThreads] << (2 * kLimbBits));

@@ -240,34 +240,33 @@ __device__ __forceinline__ void for_each_side3(const Ctx3& c, F&& f) {
   }
 }
 
-// ---- the row's classes, in order --------------------------------------------------------------
+// ---- the row's classes --------------------------------------------------------------------------
 // Scores grow with the bin inside a count class, so a count class's cells, from its lowest to its
-// highest non-empty one, are in the order of their scores.
-//
-// Calls f(valid, key, tokens, cell) for them, a thread's cells kThreads apart, WHOLE WARPS together
-// (valid = the cell is not empty); a warp whose cells are all empty is passed over.  Scoring a cell is
-// a chain of a few hundred cycles, so three of a thread's cells are worked on at a time.
+// highest non-empty one, are in the order of their scores.  Thread t owns cells t, t + kThreads, ... of
+// each.  Calls f(valid, score, tokens, cell) for the non-empty ones, WHOLE WARPS together; empty cells
+// cost a look, not a call (a pass is bound by the instructions it issues, and two cells in three
+// may be empty), and neighbouring lanes have neighbouring cells, so they mostly go in step.
 template <class F>
 __device__ __forceinline__ void for_each_class(const Ctx3& c, F&& f) {
-  constexpr int kBatch = 3;
   const Scorer sc = c;
+  const uint32_t* tab = c.tab() + threadIdx.x;
 #pragma unroll 1
   for (int k = 0; k < 3; ++k) {
-    const int top = c.ends()[k], bot = c.ends()[3 + k];  // (highest + 1; 0 = the class is empty)
-    if (top == 0) continue;
+    if (c.ends()[k] == 0) continue;  // (nothing in this count class)
+    uint32_t bits = 0;
+#pragma unroll
+    for (int u = 0; u < kPerClass; ++u) bits |= (tab[(k * kPerClass + u) * kThreads] ? 1u : 0u) << u;
 #pragma unroll 1
-    for (int base = bot + (int)threadIdx.x; base - (int)(threadIdx.x & 31) < top; base += kBatch * kThreads) {
-      uint32_t n[kBatch], key[kBatch];
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) n[u] = base + u * kThreads < top ? c.tab()[base + u * kThreads] : 0u;
-      if (!__any_sync(0xffffffffu, (n[0] | n[1] | n[2]) != 0u)) continue;
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) key[u] = sc.key_of_bin(min(base + u * kThreads, top - 1) - k * kV3Bins, k);
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) f(n[u] != 0u, key[u], n[u], base + u * kThreads);
+    while (__any_sync(0xffffffffu, bits != 0u)) {
+      const bool valid = bits != 0u;
+      const int at = (k * kPerClass + (valid ? __ffs(bits) - 1 : 0)) * kThreads;
+      bits &= bits - 1u;
+      const int cell = at + (int)threadIdx.x;
+      f(valid, sc.score_of(v3_raw_of_bin(cell - k * kV3Bins), k), tab[at], cell);
     }
   }
 }
+
 // Where a key falls among the buckets: by score, over equal widths from `lo` to the row maximum
 // (lin), or by the key itself, over [klo, khi].  Both grow with the key.
 struct V3Map {
@@ -276,8 +275,11 @@ struct V3Map {
   uint32_t klo, khi;
   int shift;
   __device__ __forceinline__ bool in(uint32_t key) const { return key >= klo && key <= khi; }
+  __device__ __forceinline__ int bucket_of(float score) const {  // (lin)
+    return min(max(__float2int_rz((score - lo) * scale), 0), kV3Buckets - 1);
+  }
   __device__ __forceinline__ int bucket(uint32_t key) const {
-    if (lin) return min(max(__float2int_rz((score_of(key) - lo) * scale), 0), kV3Buckets - 1);
+    if (lin) return bucket_of(score_of(key));
     return key < klo ? -1 : (key > khi ? kV3Buckets : (int)((key - klo) >> shift));
   }
   // buckets over the keys of [from, to]
