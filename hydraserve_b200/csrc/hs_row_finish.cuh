@@ -67,6 +67,7 @@ __device__ bool claim_scratch(CountState& S) {
     unsigned smid;
     asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
     int got = -1;
+#pragma unroll 1
     for (int k = 0; k < 2 * S.n_scratch && got < 0; ++k) {
       const int at = (int)((2u * smid + (unsigned)k) % (unsigned)S.n_scratch);
       if (atomicCAS(&S.scratch_busy[at], 0, 1) == 0) got = at;
@@ -344,6 +345,7 @@ __device__ __noinline__ bool phase_histogram() {
       side_best = packed > side_best ? packed : side_best;
       side_worst = min(side_worst, key_of(s));
     };
+#pragma unroll 1
     for (int j = tid; j < n_heavy; j += kThreads) {
       if (j != tid) {  // (the first entry's reads were started early)
         const int q = heavy[j];
@@ -355,12 +357,14 @@ __device__ __noinline__ bool phase_histogram() {
     int n_s = n_heavy + n_rare;
     if (n_rare <= kV3RareCap) {
       const int2* rare = c.rare();
+#pragma unroll 1
       for (int t = tid; t < n_rare; t += kThreads) {
         const int2 e = rare[t];
         put(n_heavy + t, e.x, k.score_of((uint32_t)e.y & 0xffffu, (e.y >> 16) & 3));
       }
     } else {
       // too many to remember: sweep the row again for out-of-window values
+#pragma unroll 1
       for (int id = tid; id < k.vocab; id += kThreads) {
         const uint32_t raw = k.logits[id];
         const int cc = k.class_of(id);
@@ -576,6 +580,7 @@ __device__ __noinline__ void draw_by_classes(uint64_t seed) {
       if (skip < mine) {
         const int slot = (list_at + skip) / kThreads;
         int cell = tid;
+#pragma unroll 1
         while (tab[cell] == 0u || skip-- > 0) cell += kThreads;
         cells[slot] = cell;
       }
@@ -583,6 +588,7 @@ __device__ __noinline__ void draw_by_classes(uint64_t seed) {
     __syncthreads();
     if (tid < 32) {
       u64 run = c.x()->bcast[1];
+#pragma unroll 1
       for (int base = 0; base < kMostCells; base += 32) {
         const int cell = base + tid < kMostCells ? cells[base + tid] : -1;
         u64 q = 0, w = 0;
@@ -797,6 +803,7 @@ __device__ __noinline__ void phase_logprobs() {
         const int n_tie = small[26];
         if (n_tie <= kV3TieCap) {
           // the `need` lowest ids of the group: each id counts the ids below it
+#pragma unroll 1
           for (int t = tid; t < n_tie; t += kThreads) {
             const int mine = tie_ids[t];
             int below = 0;
@@ -818,6 +825,7 @@ __device__ __noinline__ void phase_logprobs() {
         int id = 0x7fffffff;
         if (tid < n) { kv = gbuf[tid].key; id = gbuf[tid].id; }
         int pos = 0;
+#pragma unroll 1
         for (int j = 0; j < n; ++j) {
           const uint32_t kj = __shfl_sync(0xffffffffu, kv, j);
           const int idj = __shfl_sync(0xffffffffu, id, j);
@@ -874,6 +882,7 @@ __device__ __forceinline__ void finish_counted_row() {
     need_tie_limit();
     float* dst = S.scores_out + (size_t)S.row * c.vocab;
     const float ninf = __int_as_float(0xff800000);
+#pragma unroll 1
     for (int id = tid; id < c.vocab; id += kThreads) {
       const float s = c.element_score(id, c.logits[id], c.class_of(id));
       dst[id] = (c.greedy || S.kept.has(key_of(s), id)) ? s : ninf;
