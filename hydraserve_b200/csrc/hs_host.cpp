@@ -17,6 +17,7 @@
 #include <structmember.h>
 
 #include <cstddef>
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -61,7 +62,7 @@ struct Ref {  // an owned reference
 struct Row {  // what one SamplingParams object comes to
   hs_row_params p;
   int logprobs;     // as asked for, -1 = none
-  bool penalised, greedy, seeded;
+  bool penalised, greedy, seeded, zero_t;
   uint64_t seed;
 };
 
@@ -99,7 +100,8 @@ bool pack_row(PyObject* o, Row& r) {
   r.greedy = t == 0.0 && r.logprobs < 0 && !r.penalised;               // reference sampling.py:86-91
   r.p.flags = r.greedy ? HS_ROW_PLAIN_GREEDY : 0u;
   r.p.slot = -1;
-  r.seeded = seed.p != Py_None || t == 0.0;
+  r.zero_t = t == 0.0;
+  r.seeded = seed.p != Py_None || r.zero_t;
   if (seed.p != Py_None) {
     Ref i(PyNumber_Index(seed.p));
     if (!i) return false;
@@ -137,7 +139,8 @@ struct Batch {
   std::vector<uint64_t> seeds;
   std::vector<int8_t> logprobs;
   std::vector<uint8_t> penalised;
-  bool all_greedy = true, any_unseeded = false, any_penalised = false, any_logprobs = false;
+  bool all_greedy = true, any_unseeded = false, any_penalised = false, any_logprobs = false, any_zero_t = false;
+  int top_k_lo = 0x7fffffff, top_k_hi = 0;  // over all rows
   uint64_t used = 0;
   Batch() = default;
   Batch(const Batch&) = delete;
@@ -192,6 +195,9 @@ BatchRef batch_of(PyObject** items, Py_ssize_t n) {
     b->any_unseeded = b->any_unseeded || !r->seeded;
     b->any_penalised = b->any_penalised || r->penalised;
     b->any_logprobs = b->any_logprobs || r->logprobs >= 0;
+    b->any_zero_t = b->any_zero_t || r->zero_t;
+    b->top_k_lo = std::min(b->top_k_lo, r->p.top_k);
+    b->top_k_hi = std::max(b->top_k_hi, r->p.top_k);
   }
   if (ok) b->view = batch_view(*b);
   for (PyObject* o : b->key) Py_DECREF(o);  // (view holds them now)
@@ -897,6 +903,16 @@ PyObject* mod_batch(PyObject*, PyObject* params) {
   const BatchRef b = batch_of(reinterpret_cast<PyTupleObject*>(t.p)->ob_item, PyTuple_GET_SIZE(t.p));
   return b ? Py_NewRef(b->view) : nullptr;
 }
+// traits(params) -> (lowest top_k, highest top_k, any row with temperature 0, any unseeded row, any
+// row with penalties)
+PyObject* mod_traits(PyObject*, PyObject* params) {
+  Ref t(PySequence_Tuple(params));
+  if (!t) return nullptr;
+  const BatchRef b = batch_of(reinterpret_cast<PyTupleObject*>(t.p)->ob_item, PyTuple_GET_SIZE(t.p));
+  if (!b) return nullptr;
+  return Py_BuildValue("(iiOOO)", b->top_k_lo, b->top_k_hi, b->any_zero_t ? Py_True : Py_False,
+                       b->any_unseeded ? Py_True : Py_False, b->any_penalised ? Py_True : Py_False);
+}
 // survey(histories, params) -> -1 when every row is plain greedy, else the longest history of a
 // row with penalties
 PyObject* mod_survey(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
@@ -1031,6 +1047,7 @@ PyMethodDef module_methods[] = {
     {"batched_greedy", mod_batched_greedy, METH_NOARGS, "Whether the batched arg-max path is on."},
     {"bind", mod_bind, METH_VARARGS, "Hand over the Python objects this module works with."},
     {"batch", mod_batch, METH_O, "What depends on a batch's parameters alone."},
+    {"traits", mod_traits, METH_O, "What a vocabulary-sharded call asks about a batch's parameters."},
     {"survey", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(mod_survey)), METH_FASTCALL, "-1 for an all plain-greedy batch, else the longest penalised history."},
     {"pack", mod_pack, METH_VARARGS, "hs_row_params of a batch."},
     {"plan", mod_plan, METH_VARARGS, "Histogram slots of a batch."},

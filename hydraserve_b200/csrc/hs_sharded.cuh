@@ -150,25 +150,28 @@ __global__ void __launch_bounds__(kThreads, 2) shard_merge_kernel(const MergeArg
   u64* mass = reinterpret_cast<u64*>(smem_raw + lay.mass);
   const int tid = threadIdx.x, row = blockIdx.x;
   const hs_row_params P = a.params[row];
-  hs_row_out* out = a.out + row;
+  __shared__ hs_row_out rec;  // (the records may go straight to pinned host memory)
   if (tid < 16) small[tid] = 0;
+  if (tid < 12) reinterpret_cast<uint32_t*>(&rec)[tid] = 0;
   __syncthreads();
   int status = 0;
   // union of the ranks' candidates
   for (int i = tid; i < a.ranks * HS_SHARD_CAND; i += kThreads) {
-    const hs_shard_rec* rec = a.recs + (size_t)(i / HS_SHARD_CAND) * a.batch + row;
+    const hs_shard_rec* part = a.recs + (size_t)(i / HS_SHARD_CAND) * a.batch + row;
     const int j = i % HS_SHARD_CAND;
-    if (j < rec->n && rec->ids[j] >= 0) {
+    if (j < part->n && part->ids[j] >= 0) {
       const int slot = atomicAdd(L.n, 1);
-      if (slot < kCandCap) L.cand[slot] = cand_pack(key_of(rec->scores[j]), rec->ids[j]);
+      if (slot < kCandCap) L.cand[slot] = cand_pack(key_of(part->scores[j]), part->ids[j]);
     }
-    if (j == 0 && rec->status) atomicOr(small + 6, rec->status);
+    if (j == 0 && part->status) atomicOr(small + 6, part->status);
   }
   __syncthreads();
   int n = min(*L.n, kCandCap);
   status = small[6];
   if (n == 0) {
-    if (tid == 0) { out->token = 0; out->status = status | 1; out->n_top = 0; out->n_kept = 0; }
+    if (tid == 0) rec.status = status | 1;
+    __syncthreads();
+    if (tid < 32) write_record(a.out + row, rec, false);
     return;
   }
   const int k = P.top_k > 0 ? P.top_k : n;
@@ -178,16 +181,18 @@ __global__ void __launch_bounds__(kThreads, 2) shard_merge_kernel(const MergeArg
   }
   cand_sort(L, n);
   const float* noise_row = a.noise ? a.noise + (size_t)row * a.vocab_total : nullptr;
-  FinishOut r = finish_sorted(*x, L.cand, mass, n, P, noise_row, out);
+  FinishOut r = finish_sorted(*x, L.cand, mass, n, P, noise_row, &rec);
   r.status |= status;
+  if (tid == 0) write_finish(r, &rec);
+  __syncthreads();
+  if (tid < 32) write_record(a.out + row, rec, P.n_logprobs >= 0);
   if (tid == 0) {
-    write_finish(r, out);
     if (a.full_lse) {
       // log sum exp over the whole vocabulary from the slices' (max, denominator) pairs
       double acc = 0.0;
       for (int rk = 0; rk < a.ranks; ++rk) {
-        const hs_shard_rec* rec = a.recs + (size_t)rk * a.batch + row;
-        if (rec->n > 0) acc += (double)rec->z_mass * 9.094947017729282e-13 * exp((double)rec->row_max - (double)r.m);
+        const hs_shard_rec* part = a.recs + (size_t)rk * a.batch + row;
+        if (part->n > 0) acc += (double)part->z_mass * 9.094947017729282e-13 * exp((double)part->row_max - (double)r.m);
       }
       a.full_lse[row] = (float)((double)r.m + log(acc));
     }

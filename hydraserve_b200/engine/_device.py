@@ -62,6 +62,13 @@ _host.bind(TokenSample, _as_int64, draw_unseeded_keys)
 # lives).
 batch_static = _host.batch
 
+# (lowest top_k, highest top_k, any row with temperature 0, any unseeded row, any row with
+# penalties) of a batch's SamplingParams, kept with it.
+batch_traits = _host.traits
+
+# -1 for an all plain-greedy batch, else the length of the longest history of a row with penalties.
+longest_history = _host.survey
+
 # Whether HYDRASERVE_BATCHED_GREEDY (reference sampling.py:69) is anything but "0" right now.
 batched_greedy = _host.batched_greedy
 
@@ -548,7 +555,7 @@ def sample_batch(logits, histories, params, steps, request_ids, packed: bool = F
     batch, vocab = logits.shape
     if batch == 0:
         return PackedSamples(np.zeros(0, _lib.ROW_OUT), [], vocab) if packed else ()
-    longest = _host.survey(histories, params)
+    longest = longest_history(histories, params)
     with lease_sampler(device, vocab, batch, longest) as sampler:
         if longest < 0 and fast_greedy:
             return sampler.step_greedy(logits, packed)

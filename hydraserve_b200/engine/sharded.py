@@ -32,6 +32,9 @@ def local_history(history, lo: int, hi: int) -> np.ndarray:
 
 
 def check_params(params) -> None:
+    k_lo, k_hi, any_greedy, _, _ = _device.batch_traits(params)
+    if 0 < k_lo and k_hi <= MAX_TOP_K and not any_greedy:
+        return
     for p in params:
         if not 0 < p.top_k <= MAX_TOP_K:
             raise ValueError(f"vocabulary-sharded sampling needs 0 < top_k <= {MAX_TOP_K} on every row")
@@ -46,7 +49,7 @@ def agree_on_unseeded_keys(params, group=None):
     import torch
     import torch.distributed as dist
 
-    if not any(p.seed is None and p.temperature != 0.0 for p in params):
+    if not _device.batch_traits(params)[3]:
         return None
     keys = _device.draw_unseeded_keys(params)
     if dist.is_available() and dist.is_initialized() and dist.get_world_size(group) > 1:
@@ -68,19 +71,21 @@ def partial_records(sampler, local_logits, histories, params, steps, vocab_offse
     batch, width = logits.shape
     lo, hi = vocab_offset, vocab_offset + width
     with sampler.lock:
-        slots = [-1] * batch
-        resets, appends = [], []
-        for i, p in enumerate(params):
-            if not _has_penalties(p):
-                continue
-            tokens = local_history(histories[i], lo, hi)
-            if tokens.size == 0:
-                continue
-            slots[i] = sampler.scratch_base + i
-            resets.append(slots[i])
-            appends.append((slots[i], tokens))
-        sampler.reset_slots(resets)
-        sampler.append_tokens([s for s, _ in appends], [t for _, t in appends], width)
+        slots = None
+        if _device.batch_traits(params)[4]:
+            slots = [-1] * batch
+            resets, appends = [], []
+            for i, p in enumerate(params):
+                if not _has_penalties(p):
+                    continue
+                tokens = local_history(histories[i], lo, hi)
+                if tokens.size == 0:
+                    continue
+                slots[i] = sampler.scratch_base + i
+                resets.append(slots[i])
+                appends.append((slots[i], tokens))
+            sampler.reset_slots(resets)
+            sampler.append_tokens([s for s, _ in appends], [t for _, t in appends], width)
         rec = _device.pack_params(params, steps, slots, unseeded_keys)
         d_params = sampler._to_device(rec.view(np.uint8).reshape(batch, -1))
         recs = torch.empty((batch, _lib.SHARD_REC.itemsize), dtype=torch.uint8, device=sampler.device)
@@ -93,16 +98,14 @@ def partial_records(sampler, local_logits, histories, params, steps, vocab_offse
 def merge_records(sampler, all_recs, ranks: int, d_params, batch: int, vocab_total: int, *, noise=None):
     """all_recs: [ranks, batch, 536] uint8 CUDA tensor.  Returns (records, full log-sum-exp)."""
     torch = sampler.torch
-    d_out = torch.empty((batch, _lib.ROW_OUT.itemsize), dtype=torch.uint8, device=sampler.device)
+    host = sampler._pinned_records(batch)  # (the kernel writes the records straight into it)
     lse = torch.empty(batch, dtype=torch.float32, device=sampler.device)
     d_noise = noise.to(sampler.device, dtype=torch.float32).contiguous() if noise is not None else None
     st = sampler.lib.hs_sharded_merge(sampler.handle, all_recs.data_ptr(), ranks, batch, vocab_total,
-                                      d_params.data_ptr(), d_out.data_ptr(),
+                                      d_params.data_ptr(), host.data_ptr(),
                                       d_noise.data_ptr() if d_noise is not None else None, lse.data_ptr(),
                                       sampler._stream())
     _lib.check(sampler.lib, sampler.handle, st, "hs_sharded_merge")
-    host = sampler._pinned_records(batch)
-    host.copy_(d_out, non_blocking=True)
     torch.cuda.current_stream(sampler.device).synchronize()
     return host.numpy().view(_lib.ROW_OUT).reshape(batch).copy(), lse
 
@@ -134,7 +137,7 @@ def sample_logits_sharded(local_logits, histories, params, *, steps, vocab_offse
         raise ValueError("sampling metadata must match the logits batch")
     batch, width = int(local_logits.shape[0]), int(local_logits.shape[1])
     keys = agree_on_unseeded_keys(params, group)
-    hist_need = max((len(h) for h, p in zip(histories, params) if _has_penalties(p)), default=0)
+    hist_need = max(_device.longest_history(histories, params), 0)
     with _device.lease_sampler(local_logits.device, width, batch, hist_need) as sampler:
         recs, d_params = partial_records(sampler, local_logits, histories, params, steps, vocab_offset, keys)
         ranks = dist.get_world_size(group) if dist.is_initialized() else 1
