@@ -20,6 +20,7 @@
 #include "hs_sharded.cuh"
 #include "hs_row_finish.cuh"
 #include "hs_row_bf16_kernel.cuh"
+#include "hs_row_f32_stream.cuh"
 #include "hs_row_resident.cuh"
 
 namespace {
@@ -295,7 +296,19 @@ int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride
   }
   if (!make_plan(h, vocab, batch, plan)) return fail(h, HS_ERR_CAPACITY, "vocabulary too wide for the row kernel");
   // (bf16 rows that get here, and whatever is asked for by flag, are finished in token order)
-  a.general_order = dtype == HS_DTYPE_BF16 || h->force_general || (flags & HS_SAMPLE_GENERAL_KERNEL) ? 1 : 0;
+  const bool in_order = dtype == HS_DTYPE_BF16 || h->force_general || (flags & HS_SAMPLE_GENERAL_KERNEL);
+  a.small_k = in_order ? hs::kSmallKOrder : hs::kSmallKList;
+  // fp32 rows with a small top_k: as clusters while these are at most two waves of two CTAs per SM, one
+  // CTA each in the streaming kernel beyond that (a row takes longer there, but 296 of them run side by
+  // side; figures at that kernel).  Such a batch is too large for inline parameters.
+  if (!in_order && params && n_count != batch && (long long)batch * plan.cluster > 4ll * h->sm_count) {
+    a.small_k = hs::kSmallKLeave;
+    HS_CUDA(h, launch(hs::row_kernel_f32_stream, dim3((unsigned)batch), hs::kThreads, hs::layout_cand().total, stream,
+                      LaunchAttrs(0, false), a));
+    h->launches += 1;
+    if (n_count == 0) return HS_OK;
+    behind = false;  // (the launch before the resident kernel is not a histogram kernel any more)
+  }
   if (plan.global_stage) {
     const size_t need = (size_t)batch * plan.slice * plan.cluster;
     if (need > h->gstage_elems) return fail(h, HS_ERR_CAPACITY, "global stage too small for this batch x vocab");
@@ -487,6 +500,7 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
   if (cudaFuncSetAttribute(hs::row_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, h->smem_optin) != cudaSuccess) return bail(HS_ERR_CUDA);
   if (cudaFuncSetAttribute(hs::row_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, h->smem_optin) != cudaSuccess) return bail(HS_ERR_CUDA);
   if (cudaFuncSetAttribute(hs::row_kernel_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs::bf16_kernel_smem()) != cudaSuccess) return bail(HS_ERR_CUDA);
+  if (cudaFuncSetAttribute(hs::row_kernel_f32_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs::layout_cand().total) != cudaSuccess) return bail(HS_ERR_CUDA);
   if (cudaFuncSetAttribute(hs::shard_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs::layout_cand().total) != cudaSuccess) return bail(HS_ERR_CUDA);
   if (cudaFuncSetAttribute(hs::shard_merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs::layout_cand().total) != cudaSuccess) return bail(HS_ERR_CUDA);
   {
@@ -880,8 +894,14 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
                    rows_inline ? nullptr : reinterpret_cast<const hs_row_params*>(h->d_block), rows_inline ? inl : kNoInlineRows,
                    n_count_of(params, batch, vocab), h->h_out, nullptr, nullptr, nullptr, 0u, behind, stream);
   if (rc != HS_OK) return rc;
-  HS_CUDA(h, cudaStreamSynchronize(stream));
-  h->have_last = false;  // everything enqueued so far has been waited for
+  HS_CUDA(h, serial.done());
+  return HS_OK;
+}
+
+int hs_step_wait(hs_sampler* h, void* stream) {
+  if (!h) return HS_ERR_INVALID;
+  DeviceGuard guard(h->device);
+  HS_CUDA(h, cudaStreamSynchronize((cudaStream_t)stream));
   return HS_OK;
 }
 
@@ -901,8 +921,7 @@ int hs_step_greedy(hs_sampler* h, const void* logits, int dtype, int64_t row_str
   *tokens = h->h_tokens;
   rc = launch_greedy(h, logits, dtype, row_stride, batch, vocab, h->h_tokens, stream);
   if (rc != HS_OK) return rc;
-  HS_CUDA(h, cudaStreamSynchronize(stream));
-  h->have_last = false;
+  HS_CUDA(h, serial.done());
   return HS_OK;
 }
 

@@ -581,72 +581,84 @@ bool gather(const Append& a, int vocab, int32_t* out) {
 inline PyObject** slot_at(PyObject* o, Py_ssize_t offset) {
   return reinterpret_cast<PyObject**>(reinterpret_cast<char*>(o) + offset);
 }
-// TokenSample(token, logprob, top) without the frozen dataclass's __init__ (steals the references).
-// The object holds numbers and tuples of numbers only, so it cannot be part of a cycle: the
-// collector need not look at the thousand of them a step makes.
-PyObject* make_sample(PyObject* token, PyObject* logprob, PyObject* top) {
+// TokenSample objects without the frozen dataclass's __init__.
+// A step's results are made in two parts: the objects while the GPU is at work, then, from the
+// records, the numbers in them (1,024 samples: 30 of 42 us pass before the records are there).
+// They hold numbers and tuples of numbers only, so they cannot be part of a cycle: the collector need
+// not look at the thousands of them a step makes.
+PyObject* blank_pairs(int n) {  // ((id, value), ...), to be filled in
+  if (n == 0) return Py_NewRef(g.empty);
+  Ref top(PyTuple_New(n));
+  for (int i = 0; top && i < n; ++i) {
+    PyObject* t = PyTuple_New(2);
+    if (!t) return nullptr;
+    PyObject_GC_UnTrack(t);
+    PyTuple_SET_ITEM(top.p, i, t);
+  }
+  if (top) PyObject_GC_UnTrack(top.p);
+  return top.take();
+}
+PyObject* blank_samples(Py_ssize_t n, const int8_t* logprobs, int vocab) {
   auto* type = reinterpret_cast<PyTypeObject*>(g.token_sample);
-  PyObject* o = token && logprob && top ? type->tp_alloc(type, 0) : nullptr;
-  if (!o) {
-    Py_XDECREF(token); Py_XDECREF(logprob); Py_XDECREF(top);
-    return nullptr;
-  }
-  *slot_at(o, g.off_token) = token;
-  *slot_at(o, g.off_logprob) = logprob;
-  *slot_at(o, g.off_top) = top;
-  if (PyObject_GC_IsTracked(o)) PyObject_GC_UnTrack(o);
-  return o;
-}
-PyObject* pair(long id, PyObject* value) {  // steals value
-  PyObject* t = PyTuple_New(2);
-  PyObject* i = PyLong_FromLong(id);
-  if (!t || !i || !value) { Py_XDECREF(t); Py_XDECREF(i); Py_XDECREF(value); return nullptr; }
-  PyTuple_SET_ITEM(t, 0, i);
-  PyTuple_SET_ITEM(t, 1, value);
-  PyObject_GC_UnTrack(t);
-  return t;
-}
-PyObject* sample_of(const hs_row_out& r, int logprobs, int vocab) {
-  if (logprobs < 0) return make_sample(PyLong_FromLong(r.token), Py_NewRef(Py_None), Py_NewRef(g.empty));
-  const int want = logprobs < vocab ? logprobs : vocab;
-  int n = r.n_top < 0 ? 0 : (r.n_top > HS_MAX_LOGPROBS ? HS_MAX_LOGPROBS : r.n_top);
-  const int total = n > want ? n : want;
-  PyObject* top = PyTuple_New(total);
-  if (!top) return nullptr;
-  int at = 0;
-  for (; at < n; ++at) {
-    PyObject* t = pair(r.top_ids[at], PyFloat_FromDouble((double)r.top_logprobs[at]));
-    if (!t) { Py_DECREF(top); return nullptr; }
-    PyTuple_SET_ITEM(top, at, t);
-  }
-  // fewer candidates than requested: the reference lists filtered ids at -inf
-  for (int id = 0; at < total; ++id) {
-    bool taken = false;
-    for (int j = 0; j < n; ++j) taken = taken || r.top_ids[j] == id;
-    if (taken) continue;
-    PyObject* t = pair(id, Py_NewRef(g.neg_inf));
-    if (!t) { Py_DECREF(top); return nullptr; }
-    PyTuple_SET_ITEM(top, at++, t);
-  }
-  if (total) PyObject_GC_UnTrack(top);
-  return make_sample(PyLong_FromLong(r.token), PyFloat_FromDouble((double)r.logprob), top);
-}
-PyObject* samples_of(const hs_row_out* rec, const Batch& b, int vocab) {
-  const Py_ssize_t n = (Py_ssize_t)b.key.size();
   Ref out(PyTuple_New(n));
   if (!out) return nullptr;
   for (Py_ssize_t i = 0; i < n; ++i) {
-    PyObject* s = sample_of(rec[i], b.logprobs[(size_t)i], vocab);
-    if (!s) return nullptr;
-    PyTuple_SET_ITEM(out.p, i, s);
+    PyObject* o = type->tp_alloc(type, 0);
+    if (!o) return nullptr;
+    if (PyObject_GC_IsTracked(o)) PyObject_GC_UnTrack(o);
+    PyTuple_SET_ITEM(out.p, i, o);
+    const int asked = logprobs ? logprobs[i] : -1;
+    if (asked < 0) *slot_at(o, g.off_logprob) = Py_NewRef(Py_None);
+    PyObject* top = blank_pairs(asked < 0 ? 0 : std::min(asked, vocab));
+    if (!top) return nullptr;
+    *slot_at(o, g.off_top) = top;
   }
+  if (n) PyObject_GC_UnTrack(out.p);
   return out.take();
+}
+inline bool set_token(PyObject* sample, int32_t token) {
+  return (*slot_at(sample, g.off_token) = PyLong_FromLong(token)) != nullptr;
+}
+bool fill_sample(PyObject* o, const hs_row_out& r, int asked, int vocab) {
+  if (!set_token(o, r.token)) return false;
+  if (asked < 0) return true;
+  if (!(*slot_at(o, g.off_logprob) = PyFloat_FromDouble((double)r.logprob))) return false;
+  PyObject* top = *slot_at(o, g.off_top);
+  const int want = std::min(asked, vocab);
+  const int n = std::max(0, std::min((int)r.n_top, want));
+  auto set = [&](int at, int id, PyObject* value) {
+    PyObject* t = PyTuple_GET_ITEM(top, at);
+    PyObject* i = PyLong_FromLong(id);
+    PyTuple_SET_ITEM(t, 0, i);
+    PyTuple_SET_ITEM(t, 1, value);
+    return i && value;
+  };
+  int at = 0;
+  for (; at < n; ++at)
+    if (!set(at, r.top_ids[at], PyFloat_FromDouble((double)r.top_logprobs[at]))) return false;
+  // fewer candidates than requested: the reference lists filtered ids at -inf
+  for (int id = 0; at < want; ++id) {
+    bool taken = false;
+    for (int j = 0; j < n; ++j) taken = taken || r.top_ids[j] == id;
+    if (!taken && !set(at++, id, Py_NewRef(g.neg_inf))) return false;
+  }
+  return true;
+}
+PyObject* filled_samples(Ref& out, const hs_row_out* rec, const Batch& b, int vocab) {
+  for (Py_ssize_t i = 0; i < (Py_ssize_t)b.key.size(); ++i)
+    if (!fill_sample(PyTuple_GET_ITEM(out.p, i), rec[i], b.logprobs[(size_t)i], vocab)) return nullptr;
+  return out.take();
+}
+PyObject* samples_of(const hs_row_out* rec, const Batch& b, int vocab) {
+  Ref out(blank_samples((Py_ssize_t)b.key.size(), b.logprobs.data(), vocab));
+  return out ? filled_samples(out, rec, b, vocab) : nullptr;
 }
 
 // ---- the stepper ---------------------------------------------------------------------------------------
 typedef int (*BlockFn)(hs_sampler*, size_t, void**);
 typedef int (*StepFn)(hs_sampler*, const void*, int, int64_t, int, int, const hs_step_desc*, const hs_row_out**, void*);
 typedef int (*GreedyFn)(hs_sampler*, const void*, int, int64_t, int, int, const int32_t**, void*);
+typedef int (*WaitFn)(hs_sampler*, void*);
 typedef const char* (*TextFn)(hs_sampler*);
 
 struct Stepper {
@@ -658,15 +670,16 @@ struct Stepper {
   BlockFn block;
   StepFn step;
   GreedyFn greedy;
+  WaitFn wait;
   TextFn text;
 };
 PyTypeObject StepperType = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
 PyObject* stepper_new(PyTypeObject* type, PyObject* args, PyObject*) {
-  unsigned long long h, block, step, greedy, text;
+  unsigned long long h, block, step, greedy, wait, text;
   PyObject *book, *error;
   int base;
-  if (!PyArg_ParseTuple(args, "KO!iOKKKK", &h, &SlotBookType, &book, &base, &error, &block, &step, &greedy, &text)) return nullptr;
+  if (!PyArg_ParseTuple(args, "KO!iOKKKKK", &h, &SlotBookType, &book, &base, &error, &block, &step, &greedy, &wait, &text)) return nullptr;
   auto* s = reinterpret_cast<Stepper*>(type->tp_alloc(type, 0));
   if (!s) return nullptr;
   s->h = reinterpret_cast<hs_sampler*>(h);
@@ -676,6 +689,7 @@ PyObject* stepper_new(PyTypeObject* type, PyObject* args, PyObject*) {
   s->block = reinterpret_cast<BlockFn>(block);
   s->step = reinterpret_cast<StepFn>(step);
   s->greedy = reinterpret_cast<GreedyFn>(greedy);
+  s->wait = reinterpret_cast<WaitFn>(wait);
   s->text = reinterpret_cast<TextFn>(text);
   return reinterpret_cast<PyObject*>(s);
 }
@@ -808,10 +822,18 @@ PyObject* stepper_step(PyObject* self, PyObject* const* args, Py_ssize_t n_args)
   Py_BEGIN_ALLOW_THREADS
   st = s->step(s->h, logits, dtype, stride, (int)n, vocab, &d, &rec, stream);
   Py_END_ALLOW_THREADS
+  Ref out(st == HS_OK && !packed ? blank_samples(n, logprobs.data(), vocab) : nullptr);
+  if (st == HS_OK) {
+    Py_BEGIN_ALLOW_THREADS
+    st = s->wait(s->h, stream);
+    Py_END_ALLOW_THREADS
+  }
   if (st != HS_OK) {
+    PyErr_Clear();
     forget(book, plan);
     return failed(s, "hs_step", st);
   }
+  if (!out && !packed) return nullptr;
   int status = 0;
   for (Py_ssize_t i = 0; i < n; ++i) status |= rec[i].status;
   if (status & (2 | 4 | 64 | 128)) {
@@ -833,7 +855,7 @@ PyObject* stepper_step(PyObject* self, PyObject* const* args, Py_ssize_t n_args)
       }
     return Py_BuildValue("(OO)", r.p, l.p);
   }
-  return samples_of(rec, *b, vocab);
+  return filled_samples(out, rec, *b, vocab);
 }
 
 // greedy(logits address, dtype, row stride, batch, vocabulary, stream, packed) -> tuple of
@@ -857,15 +879,20 @@ PyObject* stepper_greedy(PyObject* self, PyObject* const* args, Py_ssize_t n_arg
   Py_BEGIN_ALLOW_THREADS
   st = s->greedy(s->h, logits, dtype, stride, n, vocab, &tokens, stream);
   Py_END_ALLOW_THREADS
-  if (st != HS_OK) return failed(s, "hs_step_greedy", st);
-  if (packed) return PyByteArray_FromStringAndSize(reinterpret_cast<const char*>(tokens), n * (Py_ssize_t)4);
-  Ref out(PyTuple_New(n));
-  if (!out) return nullptr;
-  for (int i = 0; i < n; ++i) {
-    PyObject* t = make_sample(PyLong_FromLong(tokens[i]), Py_NewRef(Py_None), Py_NewRef(g.empty));
-    if (!t) return nullptr;
-    PyTuple_SET_ITEM(out.p, i, t);
+  Ref out(st == HS_OK && !packed ? blank_samples(n, nullptr, vocab) : nullptr);
+  if (st == HS_OK) {
+    Py_BEGIN_ALLOW_THREADS
+    st = s->wait(s->h, stream);
+    Py_END_ALLOW_THREADS
   }
+  if (st != HS_OK) {
+    PyErr_Clear();
+    return failed(s, "hs_step_greedy", st);
+  }
+  if (packed) return PyByteArray_FromStringAndSize(reinterpret_cast<const char*>(tokens), n * (Py_ssize_t)4);
+  if (!out) return nullptr;
+  for (int i = 0; i < n; ++i)
+    if (!set_token(PyTuple_GET_ITEM(out.p, i), tokens[i])) return nullptr;
   return out.take();
 }
 

@@ -9,6 +9,12 @@
 
 namespace hs {
 
+enum SmallK {
+  kSmallKList = 0,   // lists their candidates
+  kSmallKOrder = 1,  // finishes them in token order like any other (rows another kernel gave up)
+  kSmallKLeave = 2,  // leaves them to the streaming kernel
+};
+
 struct RowKernelArgs {
   const void* logits;
   int dtype;
@@ -23,7 +29,7 @@ struct RowKernelArgs {
   Pool pool;            // token-count histograms
   uint32_t flags;
   int32_t* tokens_out;  // [batch] or null: the sampled ids once more, as the next step's input ids
-  int general_order;    // the resident kernel finishes rows with a small top_k in token order too (rows another kernel gave up)
+  int small_k;          // what the resident kernel does with rows of a small top_k: SmallK
   int token_draw;       // bf16 counting rows draw near-flat rows by rejection on tokens (tuning / test switch)
 };
 

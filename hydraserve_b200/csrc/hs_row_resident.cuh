@@ -524,7 +524,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
 
   const int tid = threadIdx.x;
   const bool greedy = P.temperature == 0.0f;
-  const bool candidate = is_candidate_row(P, a.vocab) && !a.general_order;
+  const bool candidate = is_candidate_row(P, a.vocab) && a.small_k != kSmallKOrder;
+  if (candidate && a.small_k == kSmallKLeave) return;  // (all CTAs of the cluster alike)
   const bool slot_ok = P.slot >= 0 && P.slot < a.pool.slots_total;
   const bool penalised = slot_ok && (P.repetition_penalty != 1.0f || P.presence_penalty != 0.0f ||
                                      P.frequency_penalty != 0.0f);

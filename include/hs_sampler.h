@@ -186,8 +186,9 @@ int hs_sample_host(hs_sampler* h, const void* logits, int dtype, int64_t row_str
 /* One step of a serving loop, host to host: everything but the logits starts and ends in host
  * memory (the reference's sample_logits as its callers see it, sampling.py:54-83), without the
  * copies hs_sample_host makes.  The caller fills ONE pinned block that the sampler owns and hands
- * the step's description over; hs_step counts the new tokens into the histograms, samples, waits
- * for `stream` and points *out at the records, in pinned memory of the sampler.
+ * the step's description over; hs_step counts the new tokens into the histograms, samples, and points
+ * *out at the records, in pinned memory of the sampler: they are there once hs_step_wait (or the
+ * caller's own wait for `stream`) has returned.
  *   hs_step_block   the block, at least `bytes` long (grown as needed, kept, freed by hs_destroy)
  *   hs_step_desc    where in the block things are: hs_row_params[batch] at its start (slots filled
  *                   in); int32 reset_slots[n_resets] at resets_at; and for the tokens to count
@@ -196,7 +197,7 @@ int hs_sample_host(hs_sampler* h, const void* logits, int dtype, int64_t row_str
  *                   aligned; bytes = end of the last one; repeats = 1 when a slot is listed twice)
  * A record's top_ids / top_logprobs are written on rows with n_logprobs >= 0 only.
  * The block and the records belong to one step at a time: the caller serialises
- * hs_step_block .. hs_step .. reading the records against other steps of the same sampler. */
+ * hs_step_block .. hs_step .. hs_step_wait .. reading the records against other steps of the same sampler. */
 typedef struct hs_step_desc {
   size_t bytes, resets_at, slots_at, offsets_at, tokens_at;
   int32_t n_resets, n_appends, max_tokens, repeats;
@@ -204,7 +205,8 @@ typedef struct hs_step_desc {
 int hs_step_block(hs_sampler* h, size_t bytes, void** block);
 int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
             const hs_step_desc* desc, const hs_row_out** out, void* stream);
-/* The same for a batch of plain-greedy rows: hs_greedy, waited for, the ids in pinned memory. */
+int hs_step_wait(hs_sampler* h, void* stream);
+/* The same for a batch of plain-greedy rows: hs_greedy with the ids in pinned memory. */
 int hs_step_greedy(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
                    const int32_t** tokens, void* stream);
 
