@@ -9,6 +9,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/hs_sampler.h"
@@ -123,6 +124,7 @@ struct hs_sampler {
   cudaEvent_t ev_done = nullptr;
   cudaStream_t last_stream = nullptr;
   bool have_last = false;
+  void* d_held = nullptr;  // the one allocation the arrays above live in (DeviceBlock)
   size_t device_bytes = 0;
   unsigned long long launches = 0;
 };
@@ -165,12 +167,27 @@ struct Serial {
   }
 };
 
-template <class T>
-bool dmalloc(hs_sampler* h, T** p, size_t bytes) {
-  if (cudaMalloc(reinterpret_cast<void**>(p), bytes ? bytes : 1) != cudaSuccess) return false;
-  h->device_bytes += bytes;
-  return true;
-}
+// What a sampler holds on the device from the start: ONE allocation (each takes the driver a
+// round of mapping and a lock), what starts at zero in front, so that one memset clears it.
+struct DeviceBlock {
+  std::vector<std::pair<void**, size_t>> zeroed, others;
+  template <class T>
+  void add(T** p, size_t bytes, bool zero) {
+    (zero ? zeroed : others).emplace_back(reinterpret_cast<void**>(p), (bytes + 255) & ~size_t(255));
+  }
+  bool allocate(hs_sampler* h) {
+    size_t clear = 0, total = 0;
+    for (auto& e : zeroed) clear += e.second;
+    total = clear;
+    for (auto& e : others) total += e.second;
+    if (cudaMalloc(&h->d_held, total) != cudaSuccess) return false;
+    h->device_bytes += total;
+    unsigned char* at = static_cast<unsigned char*>(h->d_held);
+    for (auto* list : {&zeroed, &others})
+      for (auto& e : *list) { *e.first = at; at += e.second; }
+    return cudaMemset(h->d_held, 0, clear) == cudaSuccess;
+  }
+};
 
 // The resident kernel's geometry.  As many CTAs per row as leave each at least 4,096 tokens (below
 // that a row's time is its barriers), eight at most (the portable cluster size): the row's passes
@@ -355,14 +372,8 @@ int launch_append(hs_sampler* h, const int32_t* tokens, const int32_t* offsets, 
 }
 
 void release(hs_sampler* h) {
-  cudaFree(h->pool.pairs); cudaFree(h->pool.cls); cudaFree(h->pool.heavy); cudaFree(h->pool.n_heavy); cudaFree(h->pool.n); cudaFree(h->pool.pos);
-  cudaFree(h->side_pair); cudaFree(h->scratch_busy);
-  cudaFree(h->ctab); cudaFree(h->crare); cudaFree(h->crare_n); cudaFree(h->count_ticket);
-  cudaFree(h->split_lists); cudaFree(h->split_n); cudaFree(h->split_ticket);
+  cudaFree(h->d_held); cudaFree(h->d_block); cudaFree(h->d_logits); cudaFree(h->d_hist);
   if (h->ev_done) cudaEventDestroy(h->ev_done);
-  cudaFree(h->phase_clocks);
-  cudaFree(h->pool.error); cudaFree(h->greedy_best); cudaFree(h->greedy_ticket); cudaFree(h->d_block); cudaFree(h->gstage); cudaFree(h->d_logits);
-  cudaFree(h->d_params); cudaFree(h->d_out); cudaFree(h->d_hist); cudaFree(h->d_offsets); cudaFree(h->d_slots);
   if (h->h_params) cudaFreeHost(h->h_params);
   if (h->h_small) cudaFreeHost(h->h_small);
   if (h->h_block) cudaFreeHost(h->h_block);
@@ -516,60 +527,47 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
   h->pool.unique_cap = h->unique_cap;
   h->pool.pos_stride = vocab_max;
   h->pool.cls_stride = (vocab_max + 15) / 16 + 4;  // words; padded so 128-bit reads of the tail stay inside
-  bool ok = true;
-  ok = ok && dmalloc(h, &h->pool.pairs, st * h->unique_cap * sizeof(int2));
-  ok = ok && dmalloc(h, &h->pool.n, st * sizeof(int32_t));
-  ok = ok && dmalloc(h, &h->pool.n_heavy, st * sizeof(int32_t));
-  ok = ok && dmalloc(h, &h->pool.heavy, st * h->unique_cap * sizeof(int32_t));
-  ok = ok && dmalloc(h, &h->pool.cls, st * (size_t)h->pool.cls_stride * sizeof(uint32_t));
-  ok = ok && dmalloc(h, &h->pool.pos, st * (size_t)vocab_max * sizeof(int32_t));
-  ok = ok && dmalloc(h, &h->pool.error, sizeof(int32_t));
-  ok = ok && dmalloc(h, &h->greedy_best, (size_t)batch_max * sizeof(u64));
-  ok = ok && dmalloc(h, &h->greedy_ticket, (size_t)batch_max * sizeof(int));
-  ok = ok && dmalloc(h, &h->d_params, (size_t)batch_max * sizeof(hs_row_params));
-  ok = ok && dmalloc(h, &h->d_out, (size_t)batch_max * sizeof(hs_row_out));
-  ok = ok && dmalloc(h, &h->d_offsets, ((size_t)batch_max + 1) * sizeof(int32_t));
-  ok = ok && dmalloc(h, &h->d_slots, (size_t)batch_max * sizeof(int32_t));
+  DeviceBlock held;
+  held.add(&h->pool.pairs, st * h->unique_cap * sizeof(int2), false);
+  held.add(&h->pool.n, st * sizeof(int32_t), true);
+  held.add(&h->pool.n_heavy, st * sizeof(int32_t), true);
+  held.add(&h->pool.heavy, st * h->unique_cap * sizeof(int32_t), false);
+  held.add(&h->pool.cls, st * (size_t)h->pool.cls_stride * sizeof(uint32_t), true);
+  held.add(&h->pool.pos, st * (size_t)vocab_max * sizeof(int32_t), true);
+  held.add(&h->pool.error, sizeof(int32_t), true);
+  held.add(&h->greedy_best, (size_t)batch_max * sizeof(u64), true);
+  held.add(&h->greedy_ticket, (size_t)batch_max * sizeof(int), true);
+  held.add(&h->d_params, (size_t)batch_max * sizeof(hs_row_params), false);
+  held.add(&h->d_out, (size_t)batch_max * sizeof(hs_row_out), false);
+  held.add(&h->d_offsets, ((size_t)batch_max + 1) * sizeof(int32_t), false);
+  held.add(&h->d_slots, (size_t)batch_max * sizeof(int32_t), false);
   // scratch of the bf16 kernel, per resident CTA (not per row of the batch)
   h->side_cap = std::min((vocab_max + 7) & ~7, kSideCapMax);
-  ok = ok && dmalloc(h, &h->side_pair, (size_t)h->resident_bf16 * h->side_cap * sizeof(int2));
-  ok = ok && dmalloc(h, &h->scratch_busy, (size_t)h->resident_bf16 * sizeof(int));
+  held.add(&h->side_pair, (size_t)h->resident_bf16 * h->side_cap * sizeof(int2), false);
+  held.add(&h->scratch_busy, (size_t)h->resident_bf16 * sizeof(int), true);
   // hand-over scratch of rows split over several CTAs: two parts per resident CTA
   h->ctab_tables = 2 * h->resident_bf16;
   h->split_tables = std::max(2 * h->resident_bf16, 2 * batch_max);
-  ok = ok && dmalloc(h, &h->ctab, (size_t)h->ctab_tables * hs::kCells * sizeof(uint32_t));
-  ok = ok && dmalloc(h, &h->crare, (size_t)h->ctab_tables * hs::kV3RareCap * sizeof(int2));
-  ok = ok && dmalloc(h, &h->crare_n, (size_t)h->ctab_tables * sizeof(int2));
-  ok = ok && dmalloc(h, &h->count_ticket, (size_t)batch_max * sizeof(int));
-  ok = ok && cudaEventCreateWithFlags(&h->ev_done, cudaEventDisableTiming) == cudaSuccess;
-  ok = ok && dmalloc(h, &h->split_lists, (size_t)h->split_tables * hs::kSplitCap * sizeof(unsigned long long));
-  ok = ok && dmalloc(h, &h->split_n, (size_t)h->split_tables * sizeof(int));
-  ok = ok && dmalloc(h, &h->split_ticket, (size_t)batch_max * sizeof(int));
-  ok = ok && cudaMallocHost(&h->h_params, (size_t)batch_max * sizeof(hs_row_params)) == cudaSuccess;
-  ok = ok && cudaMallocHost(&h->h_small, (2 * (size_t)batch_max + 1) * sizeof(int32_t)) == cudaSuccess;
-  if (flags & HS_CREATE_PHASE_CLOCKS) {
-    const size_t bytes = (size_t)batch_max * hs::kV3PhaseSlots * sizeof(unsigned long long);
-    ok = ok && dmalloc(h, &h->phase_clocks, bytes);
-    ok = ok && cudaMemset(h->phase_clocks, 0, bytes) == cudaSuccess;
-  }
-  if (!ok) return bail(HS_ERR_CUDA);
-  ok = ok && cudaMemset(h->split_ticket, 0, (size_t)batch_max * sizeof(int)) == cudaSuccess;
-  ok = ok && cudaMemset(h->greedy_best, 0, (size_t)batch_max * sizeof(u64)) == cudaSuccess;
-  ok = ok && cudaMemset(h->greedy_ticket, 0, (size_t)batch_max * sizeof(int)) == cudaSuccess;
-  ok = ok && cudaMemset(h->scratch_busy, 0, (size_t)h->resident_bf16 * sizeof(int)) == cudaSuccess;
-  ok = ok && cudaMemset(h->count_ticket, 0, (size_t)batch_max * sizeof(int)) == cudaSuccess;
-  ok = ok && cudaMemset(h->pool.n, 0, st * sizeof(int32_t)) == cudaSuccess;
-  ok = ok && cudaMemset(h->pool.n_heavy, 0, st * sizeof(int32_t)) == cudaSuccess;
-  ok = ok && cudaMemset(h->pool.cls, 0, st * (size_t)h->pool.cls_stride * sizeof(uint32_t)) == cudaSuccess;
-  ok = ok && cudaMemset(h->pool.pos, 0, st * (size_t)vocab_max * sizeof(int32_t)) == cudaSuccess;
-  ok = ok && cudaMemset(h->pool.error, 0, sizeof(int32_t)) == cudaSuccess;
-  if (!ok) return bail(HS_ERR_CUDA);
+  held.add(&h->ctab, (size_t)h->ctab_tables * hs::kCells * sizeof(uint32_t), false);
+  held.add(&h->crare, (size_t)h->ctab_tables * hs::kV3RareCap * sizeof(int2), false);
+  held.add(&h->crare_n, (size_t)h->ctab_tables * sizeof(int2), false);
+  held.add(&h->count_ticket, (size_t)batch_max * sizeof(int), true);
+  held.add(&h->split_lists, (size_t)h->split_tables * hs::kSplitCap * sizeof(unsigned long long), false);
+  held.add(&h->split_n, (size_t)h->split_tables * sizeof(int), false);
+  held.add(&h->split_ticket, (size_t)batch_max * sizeof(int), true);
+  if (flags & HS_CREATE_PHASE_CLOCKS)
+    held.add(&h->phase_clocks, (size_t)batch_max * hs::kV3PhaseSlots * sizeof(unsigned long long), true);
   Plan plan;
   if (!make_plan(h, vocab_max, batch_max, plan)) return bail(HS_ERR_CAPACITY);
   if (plan.global_stage) {
     h->gstage_elems = (size_t)batch_max * plan.slice * plan.cluster;
-    if (!dmalloc(h, &h->gstage, h->gstage_elems * sizeof(float))) return bail(HS_ERR_CUDA);
+    held.add(&h->gstage, h->gstage_elems * sizeof(float), false);
   }
+  bool ok = held.allocate(h);
+  ok = ok && cudaEventCreateWithFlags(&h->ev_done, cudaEventDisableTiming) == cudaSuccess;
+  ok = ok && cudaMallocHost(&h->h_params, (size_t)batch_max * sizeof(hs_row_params)) == cudaSuccess;
+  ok = ok && cudaMallocHost(&h->h_small, (2 * (size_t)batch_max + 1) * sizeof(int32_t)) == cudaSuccess;
+  if (!ok) return bail(HS_ERR_CUDA);
   if (cudaDeviceSynchronize() != cudaSuccess) return bail(HS_ERR_CUDA);
   *out = h;
   return HS_OK;
