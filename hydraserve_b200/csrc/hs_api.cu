@@ -109,11 +109,13 @@ struct hs_sampler {
   int32_t* d_slots = nullptr;
   hs_row_params* h_params = nullptr;  // pinned
   int32_t* h_small = nullptr;         // pinned: offsets[batch_max+1] then slots[batch_max]
-  // hs_step: the pinned block its caller fills, its copy on the device, and pinned results
+  // hs_step: the pinned block its caller fills, its copy on the device, and pinned results.  The first
+  // blocks are part of h_held and d_held; larger ones, when a step needs them, are own allocations.
   unsigned char* h_block = nullptr;
   size_t h_block_bytes = 0;
   unsigned char* d_block = nullptr;
   size_t d_block_bytes = 0;
+  void *h_block_own = nullptr, *d_block_own = nullptr;
   hs_row_out* h_out = nullptr;    // [batch_max]
   int32_t* h_tokens = nullptr;    // [batch_max]
   std::mutex mu;         // the staging buffers of hs_sample_host
@@ -124,6 +126,7 @@ struct hs_sampler {
   cudaEvent_t ev_done = nullptr;
   cudaStream_t last_stream = nullptr;
   bool have_last = false;
+  void* h_held = nullptr;  // the one pinned allocation, likewise
   void* d_held = nullptr;  // the one allocation the arrays above live in (DeviceBlock)
   size_t device_bytes = 0;
   unsigned long long launches = 0;
@@ -372,13 +375,10 @@ int launch_append(hs_sampler* h, const int32_t* tokens, const int32_t* offsets, 
 }
 
 void release(hs_sampler* h) {
-  cudaFree(h->d_held); cudaFree(h->d_block); cudaFree(h->d_logits); cudaFree(h->d_hist);
+  cudaFree(h->d_held); cudaFree(h->d_block_own); cudaFree(h->d_logits); cudaFree(h->d_hist);
   if (h->ev_done) cudaEventDestroy(h->ev_done);
-  if (h->h_params) cudaFreeHost(h->h_params);
-  if (h->h_small) cudaFreeHost(h->h_small);
-  if (h->h_block) cudaFreeHost(h->h_block);
-  if (h->h_out) cudaFreeHost(h->h_out);
-  if (h->h_tokens) cudaFreeHost(h->h_tokens);
+  if (h->h_held) cudaFreeHost(h->h_held);
+  if (h->h_block_own) cudaFreeHost(h->h_block_own);
 }
 
 }  // namespace
@@ -563,10 +563,28 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
     h->gstage_elems = (size_t)batch_max * plan.slice * plan.cluster;
     held.add(&h->gstage, h->gstage_elems * sizeof(float), false);
   }
+  // a step of every row with a new token or two, or a quarter of a million history tokens: growing a
+  // block costs a step 0.2 ms and more
+  const size_t first_block = (size_t)batch_max * (sizeof(hs_row_params) + 32) + (1 << 20);
+  held.add(&h->d_block, first_block, false);
   bool ok = held.allocate(h);
   ok = ok && cudaEventCreateWithFlags(&h->ev_done, cudaEventDisableTiming) == cudaSuccess;
-  ok = ok && cudaMallocHost(&h->h_params, (size_t)batch_max * sizeof(hs_row_params)) == cudaSuccess;
-  ok = ok && cudaMallocHost(&h->h_small, (2 * (size_t)batch_max + 1) * sizeof(int32_t)) == cudaSuccess;
+  if (ok) {
+    const size_t sizes[5] = {(size_t)batch_max * sizeof(hs_row_params), (2 * (size_t)batch_max + 1) * sizeof(int32_t),
+                             (size_t)batch_max * sizeof(hs_row_out), (size_t)batch_max * sizeof(int32_t), first_block};
+    size_t at[6] = {0};
+    for (int i = 0; i < 5; ++i) at[i + 1] = (at[i] + sizes[i] + 255) & ~size_t(255);
+    ok = cudaMallocHost(&h->h_held, at[5]) == cudaSuccess;
+    if (ok) {
+      unsigned char* base = static_cast<unsigned char*>(h->h_held);
+      h->h_params = reinterpret_cast<hs_row_params*>(base);
+      h->h_small = reinterpret_cast<int32_t*>(base + at[1]);
+      h->h_out = reinterpret_cast<hs_row_out*>(base + at[2]);
+      h->h_tokens = reinterpret_cast<int32_t*>(base + at[3]);
+      h->h_block = base + at[4];
+      h->h_block_bytes = h->d_block_bytes = first_block;
+    }
+  }
   if (!ok) return bail(HS_ERR_CUDA);
   if (cudaDeviceSynchronize() != cudaSuccess) return bail(HS_ERR_CUDA);
   *out = h;
@@ -761,30 +779,18 @@ int hs_step_block(hs_sampler* h, size_t bytes, void** block) {
   *block = nullptr;
   if (bytes > h->h_block_bytes) {
     DeviceGuard guard(h->device);
-    const size_t want = std::max<size_t>(bytes + bytes / 2, 64 << 10);
-    if (h->h_block) cudaFreeHost(h->h_block);
+    const size_t want = std::max<size_t>(2 * bytes, 64 << 10);
+    if (h->h_block_own) cudaFreeHost(h->h_block_own);
+    h->h_block_own = nullptr;
     h->h_block = nullptr;
     h->h_block_bytes = 0;
-    HS_CUDA(h, cudaMallocHost(&h->h_block, want));
+    HS_CUDA(h, cudaMallocHost(&h->h_block_own, want));
+    h->h_block = static_cast<unsigned char*>(h->h_block_own);
     h->h_block_bytes = want;
   }
   *block = h->h_block;
   return HS_OK;
 }
-
-}  // extern "C"
-
-namespace {
-// The pinned results of hs_step (records) and hs_step_greedy (ids), made at the first step: a
-// sampler that only ever runs device-chained steps does without.
-template <class T>
-int pinned_results(hs_sampler* h, T** p) {
-  if (!*p) HS_CUDA(h, cudaMallocHost(p, (size_t)h->batch_max * sizeof(T)));
-  return HS_OK;
-}
-}  // namespace
-
-extern "C" {
 
 int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
             const hs_step_desc* d, const hs_row_out** out, void* stream_) {
@@ -805,7 +811,6 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
   Serial serial(h, stream);
   HS_CUDA(h, serial.status);
 
-  if ((rc = pinned_results(h, &h->h_out)) != HS_OK) return rc;
   *out = h->h_out;
 
   // What a small step brings along goes into the launches themselves: 64 rows' parameters (3 KB)
@@ -834,11 +839,13 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
     const size_t bytes = counting && !appends_inline ? d->bytes : (size_t)batch * sizeof(hs_row_params);
     if (bytes > h->d_block_bytes) {
       HS_CUDA(h, cudaStreamSynchronize(stream));
-      cudaFree(h->d_block);
+      cudaFree(h->d_block_own);
+      h->d_block_own = nullptr;
       h->d_block = nullptr;
       h->d_block_bytes = 0;
-      const size_t want = std::max<size_t>(bytes + bytes / 2, 64 << 10);
-      HS_CUDA(h, cudaMalloc(&h->d_block, want));
+      const size_t want = std::max<size_t>(2 * bytes, 64 << 10);
+      HS_CUDA(h, cudaMalloc(&h->d_block_own, want));
+      h->d_block = static_cast<unsigned char*>(h->d_block_own);
       h->d_block_bytes = want;
     }
     HS_CUDA(h, cudaMemcpyAsync(h->d_block, h->h_block, bytes, cudaMemcpyHostToDevice, stream));
@@ -915,7 +922,6 @@ int hs_step_greedy(hs_sampler* h, const void* logits, int dtype, int64_t row_str
   DeviceGuard guard(h->device);
   Serial serial(h, stream);
   HS_CUDA(h, serial.status);
-  if ((rc = pinned_results(h, &h->h_tokens)) != HS_OK) return rc;
   *tokens = h->h_tokens;
   rc = launch_greedy(h, logits, dtype, row_stride, batch, vocab, h->h_tokens, stream);
   if (rc != HS_OK) return rc;

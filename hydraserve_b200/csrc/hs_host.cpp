@@ -31,7 +31,10 @@ namespace {
 
 constexpr uint64_t kSeedStride = 0x1E3779B97F4A7C15ull;  // reference sampling.py:148
 constexpr uint64_t kMask63 = 0x7fffffffffffffffull;
+// What is kept between calls is bounded, and goes a little at a time: dropping a batch can mean freeing
+// its parameter objects, 60 ns each, in whichever call comes next.
 constexpr size_t kBatchesMax = 64;
+constexpr size_t kBatchRowsMax = 4096;  // over all kept batches
 constexpr size_t kRowsMax = 8192;
 
 // Python objects this module works with, handed over once by bind().
@@ -115,19 +118,27 @@ struct RowEntry { PyObject* owner; Row row; };
 // By object; the reference keeps the address its own.  (Both caches live as long as the process:
 // nothing of theirs may be released once the interpreter is gone.)
 auto& g_rows = *new std::unordered_map<PyObject*, RowEntry>();
+auto& g_rows_order = *new std::vector<PyObject*>();
+size_t g_rows_next = 0;
 
 const Row* row_of(PyObject* o) {
   auto it = g_rows.find(o);
   if (it != g_rows.end()) return &it->second.row;
   Row r;
   if (!pack_row(o, r)) return nullptr;
-  if (g_rows.size() >= kRowsMax) {
-    std::unordered_map<PyObject*, RowEntry> old;
-    old.swap(g_rows);
-    for (auto& e : old) Py_DECREF(e.second.owner);
-  }
   Py_INCREF(o);
-  return &(g_rows[o] = RowEntry{o, r}).row;
+  PyObject* gone = nullptr;  // the one that has been here longest
+  if (g_rows_order.size() < kRowsMax) {
+    g_rows_order.push_back(o);
+  } else {
+    gone = g_rows_order[g_rows_next];
+    g_rows_order[g_rows_next] = o;
+    g_rows_next = (g_rows_next + 1) % kRowsMax;
+    g_rows.erase(gone);
+  }
+  const Row* kept = &(g_rows[o] = RowEntry{o, r}).row;
+  Py_XDECREF(gone);  // (last: this may run any code)
+  return kept;
 }
 
 // A batch's parameters.  `view` is what Python sees: (the params, packed static part, any
@@ -151,6 +162,7 @@ struct Batch {
 typedef std::shared_ptr<Batch> BatchRef;
 auto& g_batches = *new std::unordered_multimap<uint64_t, BatchRef>();
 uint64_t g_batch_clock = 0;
+size_t g_batch_rows = 0;  // of the kept batches
 
 PyObject* batch_view(const Batch& b) {
   const Py_ssize_t n = (Py_ssize_t)b.key.size();
@@ -202,14 +214,17 @@ BatchRef batch_of(PyObject** items, Py_ssize_t n) {
   if (ok) b->view = batch_view(*b);
   for (PyObject* o : b->key) Py_DECREF(o);  // (view holds them now)
   if (!ok || !b->view) return nullptr;
-  if (g_batches.size() >= kBatchesMax) {  // the least recently used one goes
+  std::vector<BatchRef> gone;  // the least recently used ones (let go of at the end: this may run any code)
+  while (!g_batches.empty() && (g_batches.size() >= kBatchesMax || g_batch_rows + (size_t)n > kBatchRowsMax)) {
     auto oldest = g_batches.begin();
     for (auto it = g_batches.begin(); it != g_batches.end(); ++it)
       if (it->second->used < oldest->second->used) oldest = it;
-    const BatchRef gone = oldest->second;
+    g_batch_rows -= oldest->second->key.size();
+    gone.push_back(oldest->second);
     g_batches.erase(oldest);
   }
   b->used = ++g_batch_clock;
+  g_batch_rows += (size_t)n;
   g_batches.emplace(h, b);
   return b;
 }
