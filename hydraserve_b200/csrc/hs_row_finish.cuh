@@ -2,7 +2,10 @@
 // sample, in a few phases.  What the phases hand on lives in shared memory, and each phase is a function
 // of its own: in one body the values that are alive across it filled the 64 registers twice over,
 // and with two CTAs on an SM almost all of L1 is shared memory, so every spilled value was a round
-// trip to L2.
+// trip to L2.  What bounds it now is the fetching of instructions a CTA goes through once, and the
+// barriers between the passes.  With its count table kept in shared memory and one histogram for all
+// cuts, 64 rows of 151,936 with 20 log-probabilities take 75 us (90), one row of 248,320 69 us (97),
+// 1,024 mixed rows of 151,936 199 us (231).
 #pragma once
 
 #include "hs_row_v3.cuh"
