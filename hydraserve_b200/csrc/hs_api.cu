@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <atomic>
 #include <mutex>
 #include <new>
 #include <string>
@@ -30,6 +31,7 @@ using hs::u64;
 
 constexpr int kMaxParts = 16;  // CTAs per counting row
 constexpr int kMaxSplit = 8;   // CTAs per candidate row: the parts' lists, top_k entries and ties each, meet in one list
+constexpr int32_t kNoToken = -1;  // where a greedy step's id will stand
 constexpr int kSideCapMax = 16384;  // side-list entries a CTA can keep in global scratch
 
 struct DeviceGuard {
@@ -118,6 +120,7 @@ struct hs_sampler {
   void *h_block_own = nullptr, *d_block_own = nullptr;
   hs_row_out* h_out = nullptr;    // [batch_max]
   int32_t* h_tokens = nullptr;    // [batch_max]
+  std::atomic<int> awaited{0};    // greedy ids on their way into h_tokens
   std::mutex mu;         // the staging buffers of hs_sample_host
   // Every launching call takes launch_mu, and work of one call is ordered after the previous
   // call's on the GPU (an event when the stream changed), because all calls share the
@@ -905,6 +908,16 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
 
 int hs_step_wait(hs_sampler* h, void* stream) {
   if (!h) return HS_ERR_INVALID;
+  // A greedy step's ids are single words in pinned memory, each its row's last store: they are there
+  // two microseconds before the stream reports its end.  (For as long as a large step takes; then,
+  // or if something went wrong, the stream has the word.)
+  const int n = h->awaited.exchange(0);
+  int seen = 0;
+  for (int turn = 0; turn < 200000 && seen < n; ++turn) {
+    while (seen < n && reinterpret_cast<volatile int32_t*>(h->h_tokens)[seen] != kNoToken) ++seen;
+    if (seen < n) __builtin_ia32_pause();
+  }
+  if (n > 0 && seen == n) return HS_OK;
   DeviceGuard guard(h->device);
   HS_CUDA(h, cudaStreamSynchronize((cudaStream_t)stream));
   return HS_OK;
@@ -923,9 +936,11 @@ int hs_step_greedy(hs_sampler* h, const void* logits, int dtype, int64_t row_str
   Serial serial(h, stream);
   HS_CUDA(h, serial.status);
   *tokens = h->h_tokens;
+  std::fill_n(h->h_tokens, batch, kNoToken);
   rc = launch_greedy(h, logits, dtype, row_stride, batch, vocab, h->h_tokens, stream);
   if (rc != HS_OK) return rc;
   HS_CUDA(h, serial.done());
+  h->awaited = batch;
   return HS_OK;
 }
 

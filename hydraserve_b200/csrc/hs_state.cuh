@@ -448,7 +448,9 @@ __global__ void __launch_bounds__(kGreedyThreads) greedy_kernel(
     top = atomicExch(&best[row], 0ull);
     ticket[row] = 0;
   }
-  tokens_out[row] = (int32_t)(~(uint32_t)(top & 0xffffffffu));
+  // (one store, the CTA's last: a host that waits for it in pinned memory sees it at once)
+  *reinterpret_cast<volatile int32_t*>(tokens_out + row) = (int32_t)(~(uint32_t)(top & 0xffffffffu));
+  __threadfence_system();
 }
 
 // The same in two launches, with nothing that has to hold a value between calls.
