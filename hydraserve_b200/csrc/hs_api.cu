@@ -120,7 +120,7 @@ struct hs_sampler {
   void *h_block_own = nullptr, *d_block_own = nullptr;
   hs_row_out* h_out = nullptr;    // [batch_max]
   int32_t* h_tokens = nullptr;    // [batch_max]
-  std::atomic<int> awaited{0};    // greedy ids on their way into h_tokens
+  std::atomic<int> awaited_ids{0}, awaited_records{0};  // on their way into h_tokens and h_out
   std::mutex mu;         // the staging buffers of hs_sample_host
   // Every launching call takes launch_mu, and work of one call is ordered after the previous
   // call's on the GPU (an event when the stream changed), because all calls share the
@@ -280,7 +280,7 @@ int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride
   hs::RowKernelArgs a{};
   a.logits = logits; a.dtype = dtype; a.row_stride = row_stride; a.vocab = vocab; a.slice = 0;
   a.params = params; a.out = out; a.noise = noise; a.scores_out = scores_out; a.gstage = nullptr;
-  a.pool = h->pool; a.flags = flags & HS_SAMPLE_APPEND_TOKEN; a.tokens_out = tokens_out;
+  a.pool = h->pool; a.flags = flags & (HS_SAMPLE_APPEND_TOKEN | hs::kHostWaits); a.tokens_out = tokens_out;
   a.token_draw = h->token_draw;
   if (dtype == HS_DTYPE_BF16 && !h->force_general && !(flags & HS_SAMPLE_GENERAL_KERNEL)) {
     // One launch: the parts of the counting rows, then the parts of the candidate rows, two CTAs
@@ -815,6 +815,7 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
   HS_CUDA(h, serial.status);
 
   *out = h->h_out;
+  for (int r = 0; r < batch; ++r) h->h_out[r].status = hs::kNoStatus;
 
   // What a small step brings along goes into the launches themselves: 64 rows' parameters (3 KB)
   // and 256 (slot, token) pairs (2 KB) are cheaper there than one copy ahead of the kernel
@@ -900,23 +901,30 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
   // (the records go straight to pinned memory, one burst per row: see write_record)
   rc = launch_rows(h, logits, dtype, row_stride, batch, vocab,
                    rows_inline ? nullptr : reinterpret_cast<const hs_row_params*>(h->d_block), rows_inline ? inl : kNoInlineRows,
-                   n_count_of(params, batch, vocab), h->h_out, nullptr, nullptr, nullptr, 0u, behind, stream);
+                   n_count_of(params, batch, vocab), h->h_out, nullptr, nullptr, nullptr, hs::kHostWaits, behind, stream);
   if (rc != HS_OK) return rc;
   HS_CUDA(h, serial.done());
+  h->awaited_records = batch;
   return HS_OK;
 }
 
 int hs_step_wait(hs_sampler* h, void* stream) {
   if (!h) return HS_ERR_INVALID;
-  // A greedy step's ids are single words in pinned memory, each its row's last store: they are there
-  // two microseconds before the stream reports its end.  (For as long as a large step takes; then,
-  // or if something went wrong, the stream has the word.)
-  const int n = h->awaited.exchange(0);
+  // A row's last store is one word in pinned memory (its id in a greedy step, else its record's
+  // status): they are there two microseconds before the stream reports its end.  (For as long as a
+  // large step takes; then, or if something went wrong, the stream has the word.)
+  const int ids = h->awaited_ids.exchange(0), records = h->awaited_records.exchange(0);
+  auto there = [&](int row) {
+    return ids ? *reinterpret_cast<volatile int32_t*>(h->h_tokens + row) != kNoToken
+               : *reinterpret_cast<volatile int32_t*>(&h->h_out[row].status) != hs::kNoStatus;
+  };
+  const int n = ids + records;
   int seen = 0;
   for (int turn = 0; turn < 200000 && seen < n; ++turn) {
-    while (seen < n && reinterpret_cast<volatile int32_t*>(h->h_tokens)[seen] != kNoToken) ++seen;
+    while (seen < n && there(seen)) ++seen;
     if (seen < n) __builtin_ia32_pause();
   }
+  std::atomic_thread_fence(std::memory_order_acquire);
   if (n > 0 && seen == n) return HS_OK;
   DeviceGuard guard(h->device);
   HS_CUDA(h, cudaStreamSynchronize((cudaStream_t)stream));
@@ -940,7 +948,7 @@ int hs_step_greedy(hs_sampler* h, const void* logits, int dtype, int64_t row_str
   rc = launch_greedy(h, logits, dtype, row_stride, batch, vocab, h->h_tokens, stream);
   if (rc != HS_OK) return rc;
   HS_CUDA(h, serial.done());
-  h->awaited = batch;
+  h->awaited_ids = batch;
   return HS_OK;
 }
 

@@ -127,7 +127,7 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
       out->row_max = score_of((uint32_t)(best >> 32)); out->log_z = 0.f;
     }
     __syncthreads();
-    if (tid < 32) write_record(a.out + c.row, *out, false);
+    if (tid < 32) write_record(a.out + c.row, *out, false, a.flags);
     return false;
   }
 
@@ -464,7 +464,7 @@ __device__ __forceinline__ bool cand_part(const RowV3Args& args, unsigned char* 
     }
   }
   __syncthreads();
-  if (tid < 32) write_record(a.out + c.row, *out, P.n_logprobs >= 0);
+  if (tid < 32) write_record(a.out + c.row, *out, P.n_logprobs >= 0, a.flags);
   mark(8);
   return false;
 }

@@ -859,7 +859,7 @@ __device__ __forceinline__ void finish_counted_row() {
   if (!phase_histogram()) {  // cannot happen while n_scratch covers the resident CTAs; fail the row, do not wait
     if (tid == 0) { S.out.token = 0; S.out.status = 128; S.out.n_top = 0; S.out.n_kept = 0; }
     __syncthreads();
-    if (tid < 32) write_record(S.out_row, S.out, false);
+    if (tid < 32) write_record(S.out_row, S.out, false, (uint32_t)S.flags);
     return;
   }
   if (c.greedy) {
@@ -905,7 +905,7 @@ __device__ __forceinline__ void finish_counted_row() {
     S.out.status = S.status;
   }
   __syncthreads();
-  if (tid < 32) write_record(S.out_row, S.out, S.P.n_logprobs >= 0);
+  if (tid < 32) write_record(S.out_row, S.out, S.P.n_logprobs >= 0, (uint32_t)S.flags);
   if (S.scratch >= 0 && tid == 0) { __threadfence(); atomicExch(&S.scratch_busy[S.scratch], 0); }
   phase_mark(S, 9);
 }

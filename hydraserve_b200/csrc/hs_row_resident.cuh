@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
         }
       }
       __syncthreads();
-      if (tid < 32) write_record(out, record, P.n_logprobs >= 0);
+      if (tid < 32) write_record(out, record, P.n_logprobs >= 0, a.flags);
       return;
     }
     // more ties at the k-th value than a list holds: in token order, like any other row
@@ -956,7 +956,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
       }
     }
     __syncthreads();
-    if (tid < 32) write_record(out, record, P.n_logprobs >= 0);
+    if (tid < 32) write_record(out, record, P.n_logprobs >= 0, a.flags);
   }
   // No CTA may leave while a peer can still read its shared memory.
   c.sync_all();

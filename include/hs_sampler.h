@@ -188,7 +188,9 @@ int hs_sample_host(hs_sampler* h, const void* logits, int dtype, int64_t row_str
  * copies hs_sample_host makes.  The caller fills ONE pinned block that the sampler owns and hands
  * the step's description over; hs_step counts the new tokens into the histograms, samples, and points
  * *out at the records, in pinned memory of the sampler: they are there once hs_step_wait (or the
- * caller's own wait for `stream`) has returned.
+ * caller's own wait for `stream`) has returned.  hs_step_wait looks for the rows' last words, which the
+ * kernel writes behind all else, and asks the stream only if they do not come; the stream's end may
+ * be a few microseconds off when it returns.
  *   hs_step_block   the block, at least `bytes` long (grown as needed, kept, freed by hs_destroy)
  *   hs_step_desc    where in the block things are: hs_row_params[batch] at its start (slots filled
  *                   in); int32 reset_slots[n_resets] at resets_at; and for the tokens to count
