@@ -547,10 +547,11 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
 
   // ---- A. the one read of the row from HBM, scored ------------------------------------
   uint32_t top_key = 0, low_key = 0xffffffffu;  // over this thread's elements
-  int top_at = 0;                               // (the first with the highest key)
+  int top_at = 0;                               // (the lowest with the highest key)
   auto note = [&](float s, int i) {
     const uint32_t k = key_of(s);
-    if (k > top_key) { top_key = k; top_at = i; }
+    // (the often-repeated tokens below come in any order)
+    if (k > top_key || (k == top_key && i < top_at)) { top_key = k; top_at = i; }
     low_key = min(low_key, k);
   };
   {

@@ -40,3 +40,21 @@ def test_every_way_to_a_cut_matches_the_checker(sampler, general_sampler, kind, 
     w = Workload(kind, _rows(kind, rng, len(params), vocab), "f32", hist, params, [5] * len(params))
     compare_case(sampler, w).assert_ok(max_sensitive_fraction=0.6)
     compare_case(general_sampler, w).assert_ok(max_sensitive_fraction=0.6)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("heavy", [1, 2_000])
+def test_the_lowest_id_wins_a_tie_with_tokens_held_three_times(built_library, dtype, heavy):
+    """Penalised arg max: `heavy` tokens held three times and one other all score exactly 5; the
+    lowest id among them is a heavy one (with 2,000, a thread meets several of them, in any order)."""
+    from hydraserve_b200.engine import SamplingParams, sample_logits
+
+    vocab = 32_768
+    ids = 5 + np.arange(heavy)
+    logits = torch.full((2, vocab), -1.0)
+    logits[:, ids] = 8.0
+    logits[:, 2_048] = 5.0
+    history = np.repeat(ids[::-1], 3).tolist()
+    params = [SamplingParams(frequency_penalty=1.0), SamplingParams(frequency_penalty=1.0, logprobs=3)]
+    got = sample_logits(logits.to(dtype).cuda(), [history] * 2, params, steps=[0, 0])
+    assert [s.token_id for s in got] == [5, 5]
