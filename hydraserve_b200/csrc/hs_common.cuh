@@ -32,9 +32,10 @@ __device__ __forceinline__ float score_of(uint32_t k) {
   uint32_t u = (k & 0x80000000u) ? (k ^ 0x80000000u) : ~k;
   return __uint_as_float(u);
 }
-// -0.0 and +0.0 compare equal in the reference; give them one key.
+// -0.0 and +0.0 compare equal in the reference; give them one key.  (By the bits: adding zero
+// would also turn a NaN of negative sign, below all values in every kernel, into one above them.)
 __device__ __forceinline__ float canonical(float f) {
-  return __fadd_rn(f, 0.0f);  // (-0 + 0 = +0, everything else stays: one addition)
+  return __float_as_uint(f) == 0x80000000u ? 0.0f : f;
 }
 
 // Hint: bring `bytes` (a multiple of 16) starting at the 16-byte aligned global address p

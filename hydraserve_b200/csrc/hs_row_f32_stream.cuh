@@ -25,7 +25,7 @@ namespace hs {
 
 // score of a token with logit x that the history holds `count` times
 __device__ __forceinline__ float score_of_float(const Scorer& c, float x, int count) {
-  float v = canonical(x);
+  float v = x;  // (a zero's sign goes at the end)
   if (count > 0) {
     v = v < 0.0f ? __fmul_rn(v, c.rp) : __fdiv_rn(v, c.rp);
     v = __fsub_rn(v, c.pp);

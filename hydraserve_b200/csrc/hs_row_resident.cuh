@@ -558,9 +558,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
     const uint32_t* cls = penalised ? a.pool.cls + (size_t)P.slot * a.pool.cls_stride : nullptr;
     const long long gofs = (long long)c.row * a.row_stride + c.base;
     auto put = [&](float x, uint32_t cc, int i) {
-      float v = canonical(x);
-      if (cc == 3u) { c.stage[i] = v; return; }  // (held three times or more: scored below, with its count)
-      v = score(v, (int)cc);
+      if (cc == 3u) { c.stage[i] = x; return; }  // (held three times or more: scored below, with its count)
+      float v = score(x, (int)cc);
       if (candidate && v != v) v = __int_as_float(0xff800000);  // (a NaN is never a candidate)
       c.stage[i] = v;
       note(v, i);
@@ -569,7 +568,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
     // branch per token, one 128-bit store
     auto put4 = [&](const float4& w, uint32_t cl, int i) {
       if ((cl & 0xffu) == 0u) {
-        const float4 v = make_float4(score(canonical(w.x), 0), score(canonical(w.y), 0), score(canonical(w.z), 0), score(canonical(w.w), 0));
+        const float4 v = make_float4(score(w.x, 0), score(w.y, 0), score(w.z, 0), score(w.w, 0));
         const uint32_t k0 = key_of(v.x), k1 = key_of(v.y), k2 = key_of(v.z), k3 = key_of(v.w);
         const uint32_t hi = max(max(k0, k1), max(k2, k3)), lo = min(min(k0, k1), min(k2, k3));
         if (hi <= 0xff800000u && lo >= 0x007fffffu) {  // (keys of +inf and -inf)

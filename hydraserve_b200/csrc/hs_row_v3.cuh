@@ -146,7 +146,7 @@ struct Scorer {
   }
   // score of a token with raw value bits `raw` that the history holds `count` times
   __device__ __forceinline__ float score_of(uint32_t raw, int count) const {
-    float v = canonical(__uint_as_float(raw << 16));
+    float v = __uint_as_float(raw << 16);  // (a zero's sign goes at the end)
     if (count > 0) {
       if (rp != 1.0f) v = v < 0.0f ? __fmul_rn(v, rp) : __fdiv_rn(v, rp);
       v = __fsub_rn(v, pp);

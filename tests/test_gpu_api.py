@@ -141,3 +141,29 @@ def test_host_buffer_entry_point_matches_device_entry_point():
                                   out.ctypes.data, None, None, 0, None) == -2
     finally:
         lib.hs_destroy(handle)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_plain_greedy_row_gives_the_same_token_alone_and_in_a_mixed_batch(dtype):
+    """Signed zeros, infinities and NaNs of either sign: one order of values, whichever kernel has
+    the row (a NaN of positive sign above all else, one of negative sign below)."""
+    special = torch.tensor([0.0, -0.0, float("inf"), float("-inf"), 0.0, 0.0, 1.0, -1.0]).to(dtype)
+    bits = special.view(torch.int32 if dtype == torch.float32 else torch.int16)  # (a conversion may change a NaN's sign)
+    bits[4], bits[5] = (0x7fc00000, -0x400000) if dtype == torch.float32 else (0x7fc0, -0x40)
+    rng = np.random.default_rng(5)
+    rows = [torch.full((1_001,), v, dtype=dtype) for v in (0.0, -3.0, float("-inf"))]
+    for at in range(8):
+        r = torch.full((1_001,), -3.0, dtype=dtype)
+        r[500] = 2.0
+        r[700] = special[at]
+        rows.append(r)
+    for _ in range(8):
+        rows.append(special[torch.from_numpy(rng.integers(0, 8, 1_001))])
+    logits = torch.stack(rows).cuda()
+    n = len(rows)
+    plain = SamplingParams()
+    alone = [s.token_id for s in sample_logits(logits, [[]] * n, [plain] * n, steps=[0] * n)]
+    mixed = sample_logits(torch.cat([logits, logits[:1]]), [[]] * (n + 1), [plain] * n + [SamplingParams(temperature=1.0, seed=1)],
+                          steps=[0] * (n + 1))
+    assert [s.token_id for s in mixed[:n]] == alone
+    assert alone[3 + 5] == 500 and alone[3 + 4] == 700 and alone[3 + 2] == 700
