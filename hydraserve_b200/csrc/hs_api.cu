@@ -318,13 +318,15 @@ int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride
     return HS_OK;
   }
   if (!make_plan(h, vocab, batch, plan)) return fail(h, HS_ERR_CAPACITY, "vocabulary too wide for the row kernel");
-  // (bf16 rows that get here, and whatever is asked for by flag, are finished in token order)
-  const bool in_order = dtype == HS_DTYPE_BF16 || h->force_general || (flags & HS_SAMPLE_GENERAL_KERNEL);
-  a.small_k = in_order ? hs::kSmallKOrder : hs::kSmallKList;
+  // A row with a small top_k is drawn from its sorted list wherever it is sampled, so a row that another
+  // kernel gave up (HS_SAMPLE_GENERAL_KERNEL) is listed here too: which token a seed names must not
+  // depend on the kernel, which depends on the batch around the row.
+  a.small_k = h->force_general ? hs::kSmallKOrder : hs::kSmallKList;
   // fp32 rows with a small top_k: as clusters while these are at most two waves of two CTAs per SM, one
   // CTA each in the streaming kernel beyond that (a row takes longer there, but 296 of them run side by
   // side; figures at that kernel).  Such a batch is too large for inline parameters.
-  if (!in_order && params && n_count != batch && (long long)batch * plan.cluster > 4ll * h->sm_count) {
+  const bool may_stream = dtype == HS_DTYPE_F32 && !h->force_general && !(flags & HS_SAMPLE_GENERAL_KERNEL);
+  if (may_stream && params && n_count != batch && (long long)batch * plan.cluster > 4ll * h->sm_count) {
     a.small_k = hs::kSmallKLeave;
     HS_CUDA(h, launch(hs::row_kernel_f32_stream, dim3((unsigned)batch), hs::kThreads, hs::layout_cand().total, stream,
                       LaunchAttrs(0, false), a));

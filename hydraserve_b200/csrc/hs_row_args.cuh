@@ -11,7 +11,7 @@ namespace hs {
 
 enum SmallK {
   kSmallKList = 0,   // lists their candidates
-  kSmallKOrder = 1,  // finishes them in token order like any other (rows another kernel gave up)
+  kSmallKOrder = 1,  // finishes them in token order like any other (samplers made for that alone)
   kSmallKLeave = 2,  // leaves them to the streaming kernel
 };
 

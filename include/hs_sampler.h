@@ -45,7 +45,7 @@ typedef enum { HS_DTYPE_F32 = 0, HS_DTYPE_BF16 = 1 } hs_dtype;
 
 /* Bits of the `flags` argument of hs_sample / hs_sample_ex. */
 #define HS_SAMPLE_APPEND_TOKEN 1u   /* after sampling, count the sampled token in the row's slot */
-#define HS_SAMPLE_GENERAL_KERNEL 2u /* bf16 rows too take the general kernel (rows reported with status bit 4) */
+#define HS_SAMPLE_GENERAL_KERNEL 2u /* every row takes the general kernel (rows reported with status bit 4) */
 
 /* Bits of the `flags` argument of hs_create_ex (tests and tuning; a serving process passes 0). */
 #define HS_CREATE_FORCE_GENERAL 1u /* every row, bf16 included, takes the general (fp32-resident) kernel */
@@ -80,7 +80,8 @@ typedef struct hs_row_out {
   int32_t n_top;         /* number of valid entries in top_ids / top_logprobs */
   int32_t status;        /* 0 ok.  bit 0 (1): selection fell back (non-finite input); 2: the sampled token
                             could not be counted (histogram full); 4: more individually scored tokens than
-                            the bf16 kernel keeps (values outside 2^-14 <= |x| < 2^10, history counts >= 3):
+                            the bf16 kernel keeps (values outside 2^-14 <= |x| < 2^10, history counts >= 3),
+                            or more candidates than the fp32 streaming kernel's list holds:
                             sample the row again with HS_SAMPLE_GENERAL_KERNEL; 8: fewer top log-probabilities
                             found than expected; 16 / 32: a vocabulary shard's record was cut short;
                             64: params.slot is not a slot of this sampler (the row got no penalties);

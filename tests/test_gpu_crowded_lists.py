@@ -1,0 +1,76 @@
+"""Rows with a small top_k whose candidates do not fit a list on the way (scores that rise with the
+id, penalties that raise scores): which token a seed names is a matter of the row alone, whatever
+the batch around it and however many CTAs share the row."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+from hydraserve_b200.engine import SamplingParams, sample_logits, sample_logits_packed  # noqa: E402
+
+
+@pytest.fixture(autouse=True)
+def _lib(built_library):
+    return built_library
+
+
+def _row(kind, vocab, dtype):
+    """(logits of the row, its history, its parameters beside the seed)"""
+    x = torch.randn(vocab, generator=torch.Generator().manual_seed(vocab)) * 3
+    if kind == "rising":
+        return x.sort().values.to(dtype), [], {}
+    if kind == "rising at the end":  # (only the last CTA of a split row has a crowded list)
+        x[-vocab // 9:] = x[-vocab // 9:].sort().values + 4
+        return x.to(dtype), [], {}
+    if kind == "ties":  # more at the k-th score than a list holds
+        return x.clamp(max=0.5).to(dtype), [], {}
+    # a token of the history would need a score this low to count
+    return x.to(dtype), [1, 2, 3, 3, 3], dict(presence_penalty=-2.0, repetition_penalty=0.5, frequency_penalty=-2.0)
+
+
+@pytest.mark.parametrize("kind", ["rising", "rising at the end", "ties", "raised scores"])
+@pytest.mark.parametrize("vocab", [32_768, 65_541, 151_936])
+@pytest.mark.parametrize("dtype", [torch.float32])
+def test_a_seeded_row_draws_the_same_token_in_every_batch(dtype, vocab, kind):
+    row, history, more = _row(kind, vocab, dtype)
+    params = [SamplingParams(temperature=1.0, top_k=50, seed=100 + i, **more) for i in range(8)]
+    tokens = {}
+    for batch in (1, 8, 80, 256):
+        logits = row.cuda().expand(batch, vocab).contiguous()
+        rows = [sample_logits(logits, [history] * batch, [params[(i + t) % 8] for i in range(batch)], steps=[3] * batch)
+                for t in range(8 if batch < 8 else 1)]
+        for t, samples in enumerate(rows):
+            for i, s in enumerate(samples):
+                tokens.setdefault((i + t) % 8, set()).add(s.token_id)
+    assert all(len(t) == 1 for t in tokens.values()), tokens
+
+
+@pytest.mark.parametrize("kind", ["rising", "ties", "raised scores"])
+@pytest.mark.parametrize("batch", [1, 80])
+@pytest.mark.parametrize("dtype", [torch.float32])
+def test_counts_and_log_probabilities_of_a_crowded_row(dtype, batch, kind):
+    """The filters and the log-probabilities against torch in 64 bits."""
+    vocab, k = 65_541, 50
+    row, history, more = _row(kind, vocab, dtype)
+    score = row.double().clone()
+    for t in set(history):
+        n = history.count(t)
+        v = score[t] * (0.5 if score[t] < 0 else 2.0) + 2.0 + 2.0 * n
+        score[t] = v.float().double()
+    kth = score.topk(k).values[-1]
+    kept = torch.nonzero(score >= kth).flatten()
+    order = sorted(kept.tolist(), key=lambda i: (-float(score[i]), i))
+    logp = torch.log_softmax(score[kept], 0)
+    by_id = dict(zip(kept.tolist(), logp.tolist()))
+    logits = row.cuda().expand(batch, vocab).contiguous()
+    params = [SamplingParams(temperature=1.0, top_k=k, seed=7 + i, logprobs=20, **more) for i in range(batch)]
+    got = sample_logits_packed(logits, [history] * batch, params, steps=[1] * batch)
+    assert (got.records["n_kept"] == len(kept)).all() and (got.records["status"] == 0).all()
+    for s in got:
+        assert s.token_id in by_id
+        # (sums of 2**-40 units behind a 32-bit logarithm: a few ulp of values up to 16)
+        assert abs(s.logprob - by_id[s.token_id]) < 1e-5
+        assert [t for t, _ in s.top_logprobs] == order[:20]
+        np.testing.assert_allclose([v for _, v in s.top_logprobs], [by_id[t] for t in order[:20]], rtol=0, atol=1e-5)
