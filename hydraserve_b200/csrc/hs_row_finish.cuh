@@ -851,8 +851,50 @@ __device__ __noinline__ void phase_logprobs() {
   phase_mark(S, 8);
 }
 
+// Gives a claimed set of global scratch back.
+__device__ __forceinline__ void release_scratch(CountState& S) {
+  if (S.scratch >= 0 && threadIdx.x == 0) { __threadfence(); atomicExch(&S.scratch_busy[S.scratch], 0); }
+}
+
+// A candidate row whose list overflowed while it was streamed.  Whether one does depends on how many
+// CTAs share the row, and so on the batch around it, and the token a seed names must not: with the
+// tokens counted, the k-th highest score is known exactly, and when the k highest and the ties of
+// the last fit a list after all, they are listed (in the count table's place, which has served) and
+// the row is finished like any other of its kind.  False: they do not fit, or the row goes to the
+// general kernel.  Bound by one more walk of the row, in the place of the draw's.
+__device__ __noinline__ bool finish_listed_row(const RowKernelArgs& a) {
+  CountState& S = count_state();
+  Ctx3& c = S.c;
+  if (S.status & 4) return false;
+  select_key(false, false, (u64)S.P.top_k);
+  if (!S.sel.ok || S.sel.above_cnt + S.sel.bin_cnt > (u64)kCandCap) return false;
+  static_assert(2 * kCandCap * sizeof(u64) <= sizeof(uint32_t) * kCells, "list and masses fit the count table's place");
+  u64* list = at_smem<kLayV3.tab, u64>();
+  const uint32_t key = S.sel.key;
+  if (threadIdx.x == 0) *c.gbuf_n() = 0;
+  __syncthreads();
+  auto take = [&](uint32_t k, int id) {
+    if (k < key) return;
+    const int slot = atomicAdd(c.gbuf_n(), 1);
+    if (slot < kCandCap) list[slot] = cand_pack(k, id);
+  };
+  for_each_side3(c, [&](int id, float s) { take(key_of(s), id); });
+  CandCtx L{list, nullptr, nullptr, nullptr, count_small() + 8, nullptr};
+  cand_thresholds(c, L, key);  // (ends with a barrier)
+  const Scorer sc = c;
+  stream_at_or_above(c, L.thr, [&](int id, uint32_t raw, int cc) {
+    if (v3_bin_of_raw(raw) >= 0) take(key_of(sc.score_of(raw, cc)), id);  // (else a side element, taken above)
+  });
+  __syncthreads();
+  const int n = min(*c.gbuf_n(), kCandCap);
+  cand_sort(L, n);
+  finish_candidates(a, S.row, *c.x(), list, list + kCandCap, n, S.P, S.status, &S.out);
+  release_scratch(S);
+  return true;
+}
+
 // From the row's count table (and rare tokens) to its record.
-__device__ __forceinline__ void finish_counted_row() {
+__device__ __forceinline__ void finish_counted_row(const RowKernelArgs& a) {
   CountState& S = count_state();
   Ctx3& c = S.c;
   const int tid = threadIdx.x;
@@ -862,6 +904,7 @@ __device__ __forceinline__ void finish_counted_row() {
     if (tid < 32) write_record(S.out_row, S.out, false, (uint32_t)S.flags);
     return;
   }
+  if (is_candidate_row(S.P, c.vocab) && finish_listed_row(a)) return;
   if (c.greedy) {
     phase_greedy();
   } else {
@@ -906,7 +949,7 @@ __device__ __forceinline__ void finish_counted_row() {
   }
   __syncthreads();
   if (tid < 32) write_record(S.out_row, S.out, S.P.n_logprobs >= 0, (uint32_t)S.flags);
-  if (S.scratch >= 0 && tid == 0) { __threadfence(); atomicExch(&S.scratch_busy[S.scratch], 0); }
+  release_scratch(S);
   phase_mark(S, 9);
 }
 

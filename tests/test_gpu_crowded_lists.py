@@ -32,7 +32,7 @@ def _row(kind, vocab, dtype):
 
 @pytest.mark.parametrize("kind", ["rising", "rising at the end", "ties", "raised scores"])
 @pytest.mark.parametrize("vocab", [32_768, 65_541, 151_936])
-@pytest.mark.parametrize("dtype", [torch.float32])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_a_seeded_row_draws_the_same_token_in_every_batch(dtype, vocab, kind):
     row, history, more = _row(kind, vocab, dtype)
     params = [SamplingParams(temperature=1.0, top_k=50, seed=100 + i, **more) for i in range(8)]
@@ -49,7 +49,7 @@ def test_a_seeded_row_draws_the_same_token_in_every_batch(dtype, vocab, kind):
 
 @pytest.mark.parametrize("kind", ["rising", "ties", "raised scores"])
 @pytest.mark.parametrize("batch", [1, 80])
-@pytest.mark.parametrize("dtype", [torch.float32])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_counts_and_log_probabilities_of_a_crowded_row(dtype, batch, kind):
     """The filters and the log-probabilities against torch in 64 bits."""
     vocab, k = 65_541, 50
