@@ -446,12 +446,12 @@ struct Append {
   int slot;
   PyObject* history;       // borrowed from the call's histories
   long long from, count;   // tokens history[from : from + count]
-  SlotEntry* entry;        // borrowed, or null for a per-call slot
 };
 struct StepPlan {
   std::vector<int> resets;
   std::vector<Append> appends;
-  bool repeats = false;    // a slot is appended to twice
+  std::vector<Ref> entries;  // the book's entries among them
+  bool repeats = false;      // a slot is appended to twice
 };
 
 inline Py_ssize_t length(PyObject* h) {
@@ -507,6 +507,7 @@ bool plan_step(SlotBook* book, int per_call_base, const Batch& b, PyObject** his
       }
       if (e) {
         e->call = call;
+        if (is_new || len != e->counted) plan.entries.emplace_back(Py_NewRef(reinterpret_cast<PyObject*>(e)));
         if (is_new || len < e->counted) {  // (a history that got shorter is counted anew)
           plan.resets.push_back(e->slot);
           e->counted = 0;
@@ -514,7 +515,7 @@ bool plan_step(SlotBook* book, int per_call_base, const Batch& b, PyObject** his
         if (len > e->counted) {
           if (e->appended == call) plan.repeats = true;
           e->appended = call;
-          plan.appends.push_back(Append{e->slot, histories[i], e->counted, len - e->counted, e});
+          plan.appends.push_back(Append{e->slot, histories[i], e->counted, len - e->counted});
           e->counted = len;
         }
         if (len > 0) slots[i] = e->slot;
@@ -524,7 +525,7 @@ bool plan_step(SlotBook* book, int per_call_base, const Batch& b, PyObject** his
     if (len == 0) continue;
     const int slot = per_call_base + (int)i;
     plan.resets.push_back(slot);
-    plan.appends.push_back(Append{slot, histories[i], 0, len, nullptr});
+    plan.appends.push_back(Append{slot, histories[i], 0, len});
     slots[i] = slot;
   }
   return true;
@@ -727,13 +728,15 @@ PyObject* failed(Stepper* s, const char* what, int status) {
 
 inline size_t up16(size_t v) { return (v + 15) & ~size_t(15); }
 
-// What a failed step leaves behind: the histograms it was to bring up to date are not, so their
-// requests start over.
+// What a failed step leaves behind: the histograms it was to empty or bring up to date may not be, so
+// their requests start over.
 void forget(SlotBook* book, const StepPlan& plan) {
   PyObject *type, *value, *trace;
   PyErr_Fetch(&type, &value, &trace);
-  for (const Append& a : plan.appends)
-    if (a.entry && a.entry->slot >= 0 && !drop(book, a.entry)) PyErr_Clear();
+  for (const Ref& r : plan.entries) {
+    auto* e = reinterpret_cast<SlotEntry*>(r.p);
+    if (e->slot >= 0 && !drop(book, e)) PyErr_Clear();
+  }
   PyErr_Restore(type, value, trace);
 }
 
@@ -1029,26 +1032,28 @@ PyObject* mod_plan(PyObject*, PyObject* args) {
   if (!b) return nullptr;
   StepPlan plan;
   std::vector<int> slots((size_t)n, -1);
-  if (!plan_step(reinterpret_cast<SlotBook*>(book), base, *b, reinterpret_cast<PyTupleObject*>(histories.p)->ob_item,
-                 ids ? ids.p : nullptr, slots.data(), plan)) {
+  auto undo = [&]() -> PyObject* {
     forget(reinterpret_cast<SlotBook*>(book), plan);
     return nullptr;
-  }
+  };
+  if (!plan_step(reinterpret_cast<SlotBook*>(book), base, *b, reinterpret_cast<PyTupleObject*>(histories.p)->ob_item,
+                 ids ? ids.p : nullptr, slots.data(), plan))
+    return undo();
   Ref out_slots(PyList_New(0)), resets(PyList_New(0)), appends(PyList_New(0));
-  if (!out_slots || !resets || !appends) return nullptr;
+  if (!out_slots || !resets || !appends) return undo();
   auto push = [](PyObject* list, PyObject* o) {
     const bool ok = o && PyList_Append(list, o) == 0;
     Py_XDECREF(o);
     return ok;
   };
   for (int v : slots)
-    if (!push(out_slots.p, PyLong_FromLong(v))) return nullptr;
+    if (!push(out_slots.p, PyLong_FromLong(v))) return undo();
   for (int v : plan.resets)
-    if (!push(resets.p, PyLong_FromLong(v))) return nullptr;
+    if (!push(resets.p, PyLong_FromLong(v))) return undo();
   for (const Append& a : plan.appends) {
     PyObject* tail = tail_of(a);
-    if (!tail) return nullptr;
-    if (!push(appends.p, Py_BuildValue("(iN)", a.slot, tail))) return nullptr;
+    if (!tail) return undo();
+    if (!push(appends.p, Py_BuildValue("(iN)", a.slot, tail))) return undo();
   }
   return PyTuple_Pack(3, out_slots.p, resets.p, appends.p);
 }

@@ -344,8 +344,13 @@ class DeviceSampler:
         """Slot per row plus the histogram resets / appends that bring the device up to date
         (issued here, on the current stream).  Call with the sampler lock held."""
         slots, resets, appends = _host.plan(self.book, self.scratch_base, histories, params, request_ids)
-        self.reset_slots(resets)
-        self.append_tokens([s for s, _ in appends], [t for _, t in appends], vocab)
+        try:
+            self.reset_slots(resets)
+            self.append_tokens([s for s, _ in appends], [t for _, t in appends], vocab)
+        except BaseException:
+            for request in request_ids or ():  # (the device may hold anything for them: they start over)
+                self.book.release(request)
+            raise
         return slots
 
     def step(self, logits, histories, params, steps, request_ids=None, packed: bool = False):
