@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel_f32_stream(const __gri
     const int i = tid + u * kThreads;
     if (i < n4) w[u] = __ldcs(src4 + i);
   }
-  int iteration = 0, next_look = 1, last_look = -1, last_seen = 0;
+  int iteration = 0, next_look = 1, last_look = -1, last_seen = 0, turn = 0;
 #pragma unroll 1
   for (int base = 0; base < n4; base += kBatch * kThreads, ++iteration) {
     const float t_min = lowest_threshold();
@@ -189,10 +189,12 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel_f32_stream(const __gri
     // a look at the list's length now and then, the sooner the faster it grows (each is a barrier,
     // which makes the batch wait for its slowest load)
     if (iteration != next_look) continue;
-    if (tid == 0) L.lost[2] = *L.n;
+    // (two words in turn: one is written again only after the next look's barrier, when every thread has read it)
+    turn ^= 1;
+    if (tid == 0) L.lost[1 + turn] = *L.n;
     const bool refresh = __syncthreads_or(*L.n >= kCandSoft);
     {
-      const int seen = L.lost[2];
+      const int seen = L.lost[1 + turn];
       const int per_batch = max(0, seen - last_seen) / (iteration - last_look);
       last_seen = seen;
       last_look = iteration;

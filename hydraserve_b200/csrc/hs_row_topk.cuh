@@ -55,7 +55,7 @@ __device__ __forceinline__ uint32_t raw_of_t16(int t) {
 struct CandCtx {
   u64* cand;        // [kCandCap]
   int* n;           // entries in the list
-  int* lost;        // set when an append did not fit; lost[2] is scratch of the stream's looks at the list
+  int* lost;        // set when an append did not fit; lost[1] and lost[2] are scratch of the stream's looks at the list
   uint32_t* count;  // [kBins] radix counters
   int* thr;         // [4] per-class signed 16-bit thresholds
   unsigned long long* dbg;  // optional phase clocks of this row (tuning aid), or null
@@ -434,7 +434,7 @@ __device__ int topk_candidates(Ctx3& c, CandCtx& L, int k) {
     }
   };
   fetch(w, first8);
-  int iteration = 0, next_look = 1, last_look = -1, last_seen = n;
+  int iteration = 0, next_look = 1, last_look = -1, last_seen = n, turn = 0;
   for (int base = first8; base < n8; base += kBatch * kThreads, ++iteration) {
     // threshold as a bf16 value (NaN = nothing passes, -inf = everything passes)
     int t_min = L.thr[0];
@@ -470,11 +470,14 @@ __device__ int topk_candidates(Ctx3& c, CandCtx& L, int k) {
     // its slowest load): after the second batch, then the sooner the faster the list grows, so
     // that it cannot run from the soft limit past its capacity between two looks.
     if (iteration != next_look) continue;
-    if (tid == 0) L.lost[2] = *L.n;  // (a spare slot two behind the flag)
+    // (the looks take two words in turn: a word is written again only after the next look's barrier,
+    // when every thread has read it)
+    turn ^= 1;
+    if (tid == 0) L.lost[1 + turn] = *L.n;
     // raise the bound when the list is getting long (block-uniform decision)
     const bool refresh = __syncthreads_or(*L.n >= kCandSoft);
     {
-      const int seen = L.lost[2];  // (what thread 0 saw: the same value for all)
+      const int seen = L.lost[1 + turn];  // (what thread 0 saw: the same value for all)
       const int per_batch = max(0, seen - last_seen) / (iteration - last_look);
       last_seen = seen;
       last_look = iteration;

@@ -74,3 +74,28 @@ def test_counts_and_log_probabilities_of_a_crowded_row(dtype, batch, kind):
         assert abs(s.logprob - by_id[s.token_id]) < 1e-5
         assert [t for t, _ in s.top_logprobs] == order[:20]
         np.testing.assert_allclose([v for _, v in s.top_logprobs], [by_id[t] for t in order[:20]], rtol=0, atol=1e-5)
+
+
+@pytest.mark.parametrize("slope", [1.0, 4.0, 16.0])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_lists_that_are_looked_at_after_every_batch_of_loads(dtype, slope):
+    """Rows that drift upwards list hundreds of tokens per batch of loads, so the stream looks at
+    its list after every batch, one barrier behind the other; the candidates against torch."""
+    from hydraserve_b200.engine.sharded import sample_logits_sharded
+
+    vocab, batch, k = 248_320, 80, 56
+    x = torch.randn((batch, vocab), generator=torch.Generator().manual_seed(int(slope))) + torch.linspace(0, slope, vocab)
+    logits = x.to(dtype).cuda()
+    kth = logits.topk(k, dim=1).values[:, -1:]
+    kept = (logits >= kth).sum(1).tolist()
+    params = [SamplingParams(temperature=1.0, top_k=k, seed=i) for i in range(batch)]
+    first = sample_logits_packed(logits, [[]] * batch, params, steps=[0] * batch)
+    assert first.records["n_kept"].tolist() == kept and not first.records["status"].any()
+    tokens = torch.from_numpy(first.token_ids.astype(np.int64)).cuda()[:, None]
+    assert (logits.gather(1, tokens) >= kth).all()
+    for _ in range(20):
+        again = sample_logits_packed(logits, [[]] * batch, params, steps=[0] * batch)
+        assert again.token_ids.tolist() == first.token_ids.tolist()
+    if dtype == torch.bfloat16 and max(kept) <= 64:  # (the candidates of a slice that one record holds)
+        sharded = sample_logits_sharded(logits, [[]] * batch, params, steps=[0] * batch, vocab_offset=0, vocab_total=vocab)
+        assert [s.token_id for s in sharded] == first.token_ids.tolist()
