@@ -379,6 +379,10 @@ int launch_append(hs_sampler* h, const int32_t* tokens, const int32_t* offsets, 
   return HS_OK;
 }
 
+// hs_step_wait is for the step before it: what an earlier step left, whose caller waited for the stream
+// instead, counts no more.
+void nothing_awaited(hs_sampler* h) { h->awaited_ids = h->awaited_records = 0; }
+
 void release(hs_sampler* h) {
   cudaFree(h->d_held); cudaFree(h->d_block_own); cudaFree(h->d_logits); cudaFree(h->d_hist);
   if (h->ev_done) cudaEventDestroy(h->ev_done);
@@ -803,6 +807,7 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
   if (rc != HS_OK) return rc;
   if (!d || !out) return fail(h, HS_ERR_INVALID, "desc / out is null");
   *out = nullptr;
+  nothing_awaited(h);
   if (batch == 0) return HS_OK;
   if (row_stride < vocab) return fail(h, HS_ERR_INVALID, "row_stride smaller than vocab");
   if (d->n_resets < 0 || d->n_appends < 0 || d->n_appends > 65535 || d->n_resets > 65535)
@@ -939,6 +944,7 @@ int hs_step_greedy(hs_sampler* h, const void* logits, int dtype, int64_t row_str
   if (rc != HS_OK) return rc;
   if (!tokens) return fail(h, HS_ERR_INVALID, "tokens is null");
   *tokens = nullptr;
+  nothing_awaited(h);
   if (batch == 0) return HS_OK;
   if (row_stride < vocab) return fail(h, HS_ERR_INVALID, "row_stride smaller than vocab");
   cudaStream_t stream = (cudaStream_t)stream_;

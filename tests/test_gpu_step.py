@@ -1,6 +1,8 @@
 """The host-to-host step (hs_step: histories counted by one launch, parameters and single tokens in the
 launches themselves) against the step made of its parts (slots_append and hs_sample), at history
 lengths around what a thread, a CTA and a cluster take at once."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -39,3 +41,52 @@ def test_step_equals_its_parts(built_library, batch, length):
         parts.close()
         for i in ids:
             release_request(i)
+
+
+class _Desc(C.Structure):
+    _fields_ = [(n, C.c_size_t) for n in ("bytes", "resets_at", "slots_at", "offsets_at", "tokens_at")] + \
+               [(n, C.c_int32) for n in ("n_resets", "n_appends", "max_tokens", "repeats")]
+
+
+def test_a_wait_is_for_the_step_before_it(built_library):
+    """hs_step and hs_step_greedy may be followed by the caller's own wait instead of hs_step_wait:
+    a later step's hs_step_wait then waits for that step's results, all of them and no others."""
+    from hydraserve_b200 import _lib
+    from hydraserve_b200.engine import _device
+
+    batch, unwritten = 8, 0x7fffffff
+    logits = torch.randn(batch, VOCAB, generator=torch.Generator().manual_seed(1)).cuda().bfloat16()
+    best = logits.argmax(1).tolist()
+    s = _device.DeviceSampler("cuda:0", vocab_max=VOCAB, batch_max=batch, resident_slots=1)
+    rec = _device.pack_params([SamplingParams(temperature=1.0, top_k=1, seed=i) for i in range(batch)], [0] * batch)
+    stream = s._stream()
+
+    def sample():
+        block, out = C.c_void_p(), C.c_void_p()
+        assert s.lib.hs_step_block(s.handle, rec.nbytes, C.byref(block)) == 0
+        C.memmove(block.value, rec.ctypes.data, rec.nbytes)
+        d = _Desc(rec.nbytes, rec.nbytes, rec.nbytes, rec.nbytes, rec.nbytes, 0, 0, 0, 0)
+        assert s.lib.hs_step(s.handle, logits.data_ptr(), 1, VOCAB, batch, VOCAB, C.byref(d), C.byref(out), stream) == 0
+        return lambda: np.frombuffer((C.c_char * (batch * 208)).from_address(out.value), dtype=_lib.ROW_OUT)
+
+    def greedy():
+        out = C.c_void_p()
+        assert s.lib.hs_step_greedy(s.handle, logits.data_ptr(), 1, VOCAB, batch, VOCAB, C.byref(out), stream) == 0
+        return lambda: np.frombuffer((C.c_int32 * batch).from_address(out.value), dtype=np.int32)
+
+    try:
+        for first in (greedy, sample, greedy, sample):
+            first()
+            torch.cuda.synchronize()  # (the caller's own wait)
+            torch.cuda._sleep(2_000_000)  # a millisecond: the results cannot be there by themselves
+            second = sample if first is greedy else greedy
+            read = second()
+            assert s.lib.hs_step_wait(s.handle, stream) == 0
+            got = read().copy()
+            if second is sample:
+                assert (got["status"] != unwritten).all() and got["token"].tolist() == best
+            else:
+                assert got.tolist() == best
+            torch.cuda.synchronize()
+    finally:
+        s.close()
