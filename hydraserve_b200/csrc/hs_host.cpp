@@ -679,7 +679,7 @@ typedef const char* (*TextFn)(hs_sampler*);
 
 struct Stepper {
   PyObject_HEAD
-  hs_sampler* h;
+  hs_sampler* h;    // null once closed
   PyObject* book;
   PyObject* error;  // the exception type
   int per_call_base;
@@ -726,6 +726,12 @@ PyObject* failed(Stepper* s, const char* what, int status) {
   return nullptr;
 }
 
+// close(): the sampler is about to be destroyed; later steps fail.
+PyObject* stepper_close(PyObject* self, PyObject*) {
+  reinterpret_cast<Stepper*>(self)->h = nullptr;
+  Py_RETURN_NONE;
+}
+
 inline size_t up16(size_t v) { return (v + 15) & ~size_t(15); }
 
 // What a failed step leaves behind: the histograms it was to empty or bring up to date may not be, so
@@ -750,6 +756,7 @@ PyObject* stepper_step(PyObject* self, PyObject* const* args, Py_ssize_t n_args)
     PyErr_SetString(PyExc_TypeError, "step takes ten arguments");
     return nullptr;
   }
+  if (!s->h) return failed(s, "hs_step", HS_ERR_INVALID);
   const void* logits = reinterpret_cast<const void*>((uintptr_t)PyLong_AsUnsignedLongLong(args[0]));
   const int dtype = (int)PyLong_AsLong(args[1]);
   const int64_t stride = PyLong_AsLongLong(args[2]);
@@ -884,6 +891,7 @@ PyObject* stepper_greedy(PyObject* self, PyObject* const* args, Py_ssize_t n_arg
     PyErr_SetString(PyExc_TypeError, "greedy takes seven arguments");
     return nullptr;
   }
+  if (!s->h) return failed(s, "hs_step_greedy", HS_ERR_INVALID);
   const void* logits = reinterpret_cast<const void*>((uintptr_t)PyLong_AsUnsignedLongLong(args[0]));
   const int dtype = (int)PyLong_AsLong(args[1]);
   const int64_t stride = PyLong_AsLongLong(args[2]);
@@ -917,6 +925,7 @@ PyObject* stepper_greedy(PyObject* self, PyObject* const* args, Py_ssize_t n_arg
 PyMethodDef stepper_methods[] = {
     {"step", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(stepper_step)), METH_FASTCALL, "One sampling step."},
     {"greedy", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(stepper_greedy)), METH_FASTCALL, "One plain-greedy step."},
+    {"close", stepper_close, METH_NOARGS, "The sampler is gone: steps fail from here on."},
     {nullptr, nullptr, 0, nullptr}};
 
 // ---- module functions --------------------------------------------------------------------------------

@@ -147,6 +147,8 @@ class DeviceSampler:
     def close(self) -> None:
         with self.lock:
             if getattr(self, "handle", None):
+                if getattr(self, "host", None):
+                    self.host.close()
                 self.lib.hs_destroy(self.handle)
                 self.handle = None
 

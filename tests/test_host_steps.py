@@ -1,6 +1,7 @@
 """The native host side of a step against a stand-in for the CUDA library that notes what each step
 asks of it; no GPU needed."""
 import ctypes as C
+import threading
 from types import SimpleNamespace
 
 import numpy as np
@@ -133,3 +134,21 @@ def test_a_plan_that_does_not_reach_the_device_is_forgotten(tokens):
     fake.append_tokens = lambda slots, arrays, vocab: calls.append((slots, [list(a) for a in arrays]))
     slots = _device.DeviceSampler.plan_slots(fake, [[4], [5]], params, VOCAB, ["a", "b"])
     assert calls == [slots, (slots, [[4], [5]])]
+
+
+def test_a_step_on_a_closed_sampler_fails_without_a_call():
+    s = Sampler()
+    s.step({"a": [1]})
+    destroyed = []
+    sampler = object.__new__(_device.DeviceSampler)
+    sampler.handle, sampler.host, sampler.lock = C.c_void_p(1), s.host, threading.RLock()
+    sampler.lib = SimpleNamespace(hs_destroy=destroyed.append)
+    sampler.close()
+    sampler.close()
+    assert len(destroyed) == 1
+    calls = s.library.calls
+    with pytest.raises(_lib.SamplerError):
+        s.step({"a": [1, 2]})
+    with pytest.raises(_lib.SamplerError):
+        s.host.greedy(0, 1, VOCAB, 2, VOCAB, 0, False)
+    assert s.library.calls == calls
