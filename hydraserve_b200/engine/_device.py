@@ -431,7 +431,7 @@ class _Lease:
 def lease_sampler(device, vocab: int, batch: int, hist_need: int = 0) -> _Lease:
     """The process-wide sampler of a GPU, replaced by a larger one when a call outgrows it.
     The old one is closed only after the last call inside it has returned."""
-    if isinstance(device, str):
+    if isinstance(device, str) or getattr(device, "index", None) is None:
         device = _cuda_device(device)
     if hist_need > vocab:
         hist_need = vocab

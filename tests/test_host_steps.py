@@ -7,8 +7,10 @@ from types import SimpleNamespace
 import numpy as np
 import pytest
 
-from hydraserve_b200 import _lib
-from hydraserve_b200.engine import SamplingParams, _device
+torch = pytest.importorskip("torch")
+
+from hydraserve_b200 import _lib  # noqa: E402
+from hydraserve_b200.engine import SamplingParams, _device  # noqa: E402
 
 VOCAB = 1_000
 
@@ -152,3 +154,25 @@ def test_a_step_on_a_closed_sampler_fails_without_a_call():
     with pytest.raises(_lib.SamplerError):
         s.host.greedy(0, 1, VOCAB, 2, VOCAB, 0, False)
     assert s.library.calls == calls
+
+
+@pytest.mark.parametrize("named", ["cuda", "cuda:0", 0, torch.device("cuda"), torch.device("cuda:0")])
+def test_a_gpu_has_one_sampler_however_it_is_named(monkeypatch, named):
+    made, released = [], []
+
+    class Fake:
+        hist_cap, users, retired = VOCAB, 0, False
+
+        def __init__(self, device, vocab_max, batch_max, **_):
+            self.device, self.vocab_max, self.batch_max = device, vocab_max, batch_max
+            self.release_request = released.append
+            made.append(device)
+
+    monkeypatch.setattr(_device, "DeviceSampler", Fake)
+    monkeypatch.setattr(_device, "_samplers", {})
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    first = _device.sampler_for(named, VOCAB, 4)
+    for other in ("cuda", "cuda:0", 0, torch.device("cuda"), torch.device("cuda:0")):
+        assert _device.sampler_for(other, VOCAB, 4) is first
+        _device.release_request("a", other)
+    assert made == [torch.device("cuda:0")] and released == ["a"] * 5
