@@ -967,12 +967,21 @@ PyObject* mod_traits(PyObject*, PyObject* params) {
   return Py_BuildValue("(iiOOO)", b->top_k_lo, b->top_k_hi, b->any_zero_t ? Py_True : Py_False,
                        b->any_unseeded ? Py_True : Py_False, b->any_penalised ? Py_True : Py_False);
 }
-// survey(histories, params) -> -1 when every row is plain greedy, else the longest history of a
-// row with penalties
+// survey(histories, params[, steps]) -> -1 when every row is plain greedy, else the longest history
+// of a row with penalties.  Raises for a step that is no number (a plain greedy row has no use for its own).
 PyObject* mod_survey(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
-  if (n_args != 2) {
-    PyErr_SetString(PyExc_TypeError, "survey takes two arguments");
+  if (n_args != 2 && n_args != 3) {
+    PyErr_SetString(PyExc_TypeError, "survey takes two or three arguments");
     return nullptr;
+  }
+  if (n_args == 3) {
+    Ref steps(PySequence_Tuple(args[2]));
+    if (!steps) return nullptr;
+    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(steps.p); ++i) {
+      if (PyLong_CheckExact(PyTuple_GET_ITEM(steps.p, i))) continue;
+      Ref number(PyNumber_Long(PyTuple_GET_ITEM(steps.p, i)));
+      if (!number) return nullptr;
+    }
   }
   Ref params(PySequence_Tuple(args[1])), histories(PySequence_Tuple(args[0]));
   if (!params || !histories) return nullptr;

@@ -66,7 +66,8 @@ batch_static = _host.batch
 # penalties) of a batch's SamplingParams, kept with it.
 batch_traits = _host.traits
 
-# -1 for an all plain-greedy batch, else the length of the longest history of a row with penalties.
+# -1 for an all plain-greedy batch, else the length of the longest history of a row with penalties;
+# given the steps too, raises for one that int() would not take.
 longest_history = _host.survey
 
 # Whether HYDRASERVE_BATCHED_GREEDY (reference sampling.py:69) is anything but "0" right now.
@@ -559,11 +560,11 @@ def _check_status(records) -> None:
 def sample_batch(logits, histories, params, steps, request_ids, packed: bool = False, fast_greedy: bool = True):
     """One sampling step on the process-wide sampler of the logits' GPU.  ``fast_greedy``: a batch
     of plain-greedy rows takes the arg-max kernel."""
+    longest = longest_history(histories, params, steps)
     device = _target_device(logits)
     batch, vocab = logits.shape
     if batch == 0:
         return PackedSamples(np.zeros(0, _lib.ROW_OUT), [], vocab) if packed else ()
-    longest = longest_history(histories, params)
     with lease_sampler(device, vocab, batch, longest) as sampler:
         if longest < 0 and fast_greedy:
             return sampler.step_greedy(logits, packed)

@@ -149,6 +149,7 @@ def sample_logits(
     if not gpu.batched_greedy():
         # Per-row routing, as the reference does when its batched fast path is disabled
         # (sampling.py:69, :78-83): every row goes through the module-level _sample_row.
+        steps = tuple(map(int, steps))
         return tuple(
             _sample_row(logits[i], histories[i], params[i], steps[i])
             for i in range(len(params))

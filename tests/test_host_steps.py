@@ -176,3 +176,18 @@ def test_a_gpu_has_one_sampler_however_it_is_named(monkeypatch, named):
         assert _device.sampler_for(other, VOCAB, 4) is first
         _device.release_request("a", other)
     assert made == [torch.device("cuda:0")] and released == ["a"] * 5
+
+
+@pytest.mark.parametrize("batched", ["1", "0"])
+@pytest.mark.parametrize("params", [SamplingParams(), SamplingParams(temperature=1.0, seed=1)])
+def test_a_step_that_is_no_number_is_refused_before_anything_else(monkeypatch, params, batched):
+    """(the reference's int(step) for every row, plain greedy ones too)"""
+    from hydraserve_b200.engine import sample_logits, sample_logits_packed
+
+    monkeypatch.setenv("HYDRASERVE_BATCHED_GREEDY", batched)
+    monkeypatch.setattr(_device, "_target_device", lambda logits: pytest.fail("the call went on"))
+    for call in (sample_logits, sample_logits_packed):
+        for step, error in ((None, TypeError), ("three", ValueError), ([1], TypeError)):
+            with pytest.raises(error):
+                call(torch.zeros(2, 5), [[], []], [params] * 2, steps=[0, step])
+    assert _device.longest_history([[], []], [params] * 2, [2.5, True]) == (-1 if params == SamplingParams() else 0)
