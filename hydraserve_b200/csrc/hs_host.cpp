@@ -861,23 +861,27 @@ PyObject* stepper_step(PyObject* self, PyObject* const* args, Py_ssize_t n_args)
   if (!out && !packed) return nullptr;
   int status = 0;
   for (Py_ssize_t i = 0; i < n; ++i) status |= rec[i].status;
+  // (rows without log-probabilities leave that part of the pinned record as it was)
+  auto records = [&]() -> PyObject* {
+    PyObject* copy = PyByteArray_FromStringAndSize(reinterpret_cast<const char*>(rec), n * (Py_ssize_t)sizeof(hs_row_out));
+    auto* own = copy ? reinterpret_cast<hs_row_out*>(PyByteArray_AS_STRING(copy)) : nullptr;
+    for (Py_ssize_t i = 0; own && i < n; ++i)
+      if (own[i].n_top <= 0) {
+        std::memset(own[i].top_ids, 0, sizeof own[i].top_ids);
+        std::memset(own[i].top_logprobs, 0, sizeof own[i].top_logprobs);
+      }
+    return copy;
+  };
   if (status & (2 | 4 | 64 | 128)) {
-    Ref r(PyByteArray_FromStringAndSize(reinterpret_cast<const char*>(rec), n * (Py_ssize_t)sizeof(hs_row_out)));
+    Ref r(records());
     Ref p(PyByteArray_FromStringAndSize(reinterpret_cast<const char*>(rows), n * (Py_ssize_t)sizeof(hs_row_params)));
     if (!r || !p) return nullptr;
     return Py_BuildValue("[OO]", r.p, p.p);
   }
   if (packed) {
-    Ref r(PyByteArray_FromStringAndSize(reinterpret_cast<const char*>(rec), n * (Py_ssize_t)sizeof(hs_row_out)));
+    Ref r(records());
     Ref l(PyBytes_FromStringAndSize(reinterpret_cast<const char*>(logprobs.data()), n));
     if (!r || !l) return nullptr;
-    // (rows without log-probabilities leave that part of the pinned record as it was)
-    auto* own = reinterpret_cast<hs_row_out*>(PyByteArray_AS_STRING(r.p));
-    for (Py_ssize_t i = 0; i < n; ++i)
-      if (own[i].n_top <= 0) {
-        std::memset(own[i].top_ids, 0, sizeof own[i].top_ids);
-        std::memset(own[i].top_logprobs, 0, sizeof own[i].top_logprobs);
-      }
     return Py_BuildValue("(OO)", r.p, l.p);
   }
   return filled_samples(out, rec, *b, vocab);

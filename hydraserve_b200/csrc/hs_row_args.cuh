@@ -43,16 +43,17 @@ __device__ __forceinline__ hs_row_params row_params(const RowKernelArgs& a, cons
   return a.params ? a.params[row] : inl.p[row];
 }
 
-// A row's record is put together in shared memory and leaves in one piece (one warp): `out` may be
-// pinned host memory, where every store is a transfer of its own.  When the host waits for the record
-// itself (hs_step), its status goes last, behind everything else.
+// A row's record is put together in shared memory (zero where nothing is to be said) and leaves in one
+// piece (one warp): `out` may be pinned host memory, where every store is a transfer of its own.  When
+// the host waits for the record itself (hs_step), its status goes last, behind everything else, and a
+// row without log-probabilities leaves their place as it was.
 constexpr uint32_t kHostWaits = 1u << 31;  // in RowKernelArgs.flags
 constexpr int32_t kNoStatus = 0x7fffffff;  // what stands in the status until then
 __device__ __forceinline__ void write_record(hs_row_out* out, const hs_row_out& rec, bool with_top, uint32_t flags) {
   static_assert(sizeof(hs_row_out) == 52 * 4 && offsetof(hs_row_out, top_ids) == 12 * 4, "words of a record");
   constexpr int kStatus = offsetof(hs_row_out, status) / 4;
-  const int n = with_top ? 52 : 12;
   const bool last = flags & kHostWaits;
+  const int n = with_top || !last ? 52 : 12;
   for (int i = threadIdx.x; i < n; i += 32)
     if (!last || i != kStatus) reinterpret_cast<uint32_t*>(out)[i] = reinterpret_cast<const uint32_t*>(&rec)[i];
   if (!last) return;

@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel_f32_stream(const __gri
   const bool penalised = slot_ok && (c.rp != 1.0f || c.pp != 0.0f || c.fp != 0.0f);
   c.cls = penalised ? a.pool.cls + (size_t)P.slot * a.pool.cls_stride : nullptr;
   if (tid < 16) small[tid] = 0;
-  if (tid < 12) reinterpret_cast<uint32_t*>(&rec)[tid] = 0;
+  if (tid < (int)sizeof(hs_row_out) / 4) reinterpret_cast<uint32_t*>(&rec)[tid] = 0;
   __syncthreads();
   const int k = P.top_k;  // (0 < k <= kTopKMax and k < vocab)
 

@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kThreads, 2) shard_merge_kernel(const MergeArg
   const hs_row_params P = a.params[row];
   __shared__ hs_row_out rec;  // (the records may go straight to pinned host memory)
   if (tid < 16) small[tid] = 0;
-  if (tid < 12) reinterpret_cast<uint32_t*>(&rec)[tid] = 0;
+  if (tid < (int)sizeof(hs_row_out) / 4) reinterpret_cast<uint32_t*>(&rec)[tid] = 0;
   __syncthreads();
   int status = 0;
   // union of the ranks' candidates

@@ -99,3 +99,20 @@ def test_lists_that_are_looked_at_after_every_batch_of_loads(dtype, slope):
     if dtype == torch.bfloat16 and max(kept) <= 64:  # (the candidates of a slice that one record holds)
         sharded = sample_logits_sharded(logits, [[]] * batch, params, steps=[0] * batch, vocab_offset=0, vocab_total=vocab)
         assert [s.token_id for s in sharded] == first.token_ids.tolist()
+
+
+def test_what_a_record_does_not_use_is_zero():
+    """Rows that went through a kernel a second time, and rows with fewer candidates than
+    log-probabilities: a packed result carries nothing of other rows or earlier steps."""
+    vocab, batch = 151_936, 80
+    row, _, _ = _row("rising", vocab, torch.float32)
+    logits = row.cuda().expand(batch, vocab).contiguous()
+    full = [SamplingParams(temperature=1.0, top_k=50, seed=i, logprobs=20) for i in range(batch)]
+    none = [SamplingParams(temperature=1.0, top_k=50, seed=i) for i in range(batch)]
+    few = [SamplingParams(temperature=1.0, top_k=3, seed=i, logprobs=20) for i in range(batch)]
+    normal = torch.randn(batch, vocab, generator=torch.Generator().manual_seed(3)).cuda()
+    for x in (logits, normal):
+        for params, used in ((full, 20), (none, 0), (few, 3)):
+            records = sample_logits_packed(x, [[]] * batch, params, steps=[0] * batch).records
+            assert (records["n_top"] == used).all()
+            assert not records["top_ids"][:, used:].any() and not records["top_logprobs"][:, used:].any()
