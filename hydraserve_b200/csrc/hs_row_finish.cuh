@@ -942,7 +942,8 @@ __device__ __forceinline__ void finish_counted_row(const RowKernelArgs& a) {
     S.out.n_cut_ties = (int32_t)S.cut_ties;
     S.out.row_max = c.m;
     if (S.tokens_out) S.tokens_out[S.row] = token;
-    if ((S.flags & HS_SAMPLE_APPEND_TOKEN) && S.slot_ok && token >= 0 && token < c.vocab) {
+    // (a row for the general kernel is counted by that one)
+    if ((S.flags & HS_SAMPLE_APPEND_TOKEN) && S.slot_ok && !(S.status & 4) && token >= 0 && token < c.vocab) {
       if (!slot_append_one(c.pool, S.P.slot, token)) S.status |= 2;
     }
     S.out.status = S.status;

@@ -90,3 +90,22 @@ def test_a_wait_is_for_the_step_before_it(built_library):
             torch.cuda.synchronize()
     finally:
         s.close()
+
+
+def test_a_row_that_goes_again_is_counted_once(built_library):
+    """HS_SAMPLE_APPEND_TOKEN and a row the bf16 kernel hands to the general one (more values outside
+    its window than the side list holds): one token goes into the histogram, the one sampled."""
+    from hydraserve_b200.engine import _device
+
+    rows = 8
+    logits = 5_000 + 64 * torch.randint(0, 4, (rows, VOCAB), generator=torch.Generator().manual_seed(2))
+    logits = logits.cuda().bfloat16()
+    s = _device.DeviceSampler("cuda:0", vocab_max=VOCAB, batch_max=rows, resident_slots=rows)
+    try:
+        params = [SamplingParams(temperature=2.0, seed=i, presence_penalty=0.5) for i in range(rows)]
+        s.reset_slots(list(range(rows)))
+        records, _ = s.run(logits, _device.pack_params(params, [0] * rows, list(range(rows))), append_token=True)
+        assert not records["status"].any()
+        assert [s.unique_count(i) for i in range(rows)] == [1] * rows
+    finally:
+        s.close()
