@@ -2,7 +2,8 @@
 
 ``hydraserve_b200/lib/libhs_sampler.so``, the C-ABI CUDA library, is what
 ``hydraserve_b200._lib`` loads (nvcc cross-compiles for sm_100a without a GPU);
-``hydraserve_b200/_host.so`` is the Python extension with the host side of a step (plain C++).
+``hydraserve_b200/_host.<interpreter>.so`` is the Python extension with the host side of a step
+(plain C++; Python 3.10 or newer, x86-64 or aarch64).
 """
 from __future__ import annotations
 
@@ -15,11 +16,12 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 ROOT = PKG.parent
 SOURCES = [PKG / "csrc" / "hs_api.cu"]
-HEADERS = sorted((PKG / "csrc").glob("*.cuh")) + [ROOT / "include" / "hs_sampler.h"]
+HEADERS = sorted((PKG / "csrc").glob("*.cuh")) + sorted((PKG / "csrc").glob("*.h")) + [ROOT / "include" / "hs_sampler.h"]
 OUTPUT = PKG / "lib" / "libhs_sampler.so"
 HOST_SOURCES = [PKG / "csrc" / "hs_host.cpp"]
 HOST_HEADERS = [ROOT / "include" / "hs_sampler.h"]
-HOST_OUTPUT = PKG / "_host.so"
+# (named for the interpreter: another one builds its own)
+HOST_OUTPUT = PKG / f"_host{sysconfig.get_config_var('EXT_SUFFIX')}"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

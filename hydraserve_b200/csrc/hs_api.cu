@@ -15,6 +15,7 @@
 
 #include "../../include/hs_sampler.h"
 #include "hs_common.cuh"
+#include "hs_pause.h"
 #include "hs_state.cuh"
 #include "hs_row_args.cuh"
 #include "hs_row_v3.cuh"
@@ -929,7 +930,7 @@ int hs_step_wait(hs_sampler* h, void* stream) {
   int seen = 0;
   for (int turn = 0; turn < 200000 && seen < n; ++turn) {
     while (seen < n && there(seen)) ++seen;
-    if (seen < n) __builtin_ia32_pause();
+    if (seen < n) hs_pause();
   }
   std::atomic_thread_fence(std::memory_order_acquire);
   if (n > 0 && seen == n) return HS_OK;

@@ -27,6 +27,12 @@
 
 #include "../../include/hs_sampler.h"
 
+// Whether the interpreter lets small ints be read without a call (Python 3.12 on).  33 histories of up
+// to 4,096 tokens: 67,000 reads.
+#ifndef HS_COMPACT_INTS
+#define HS_COMPACT_INTS (PY_VERSION_HEX >= 0x030C0000)
+#endif
+
 namespace {
 
 constexpr uint64_t kSeedStride = 0x1E3779B97F4A7C15ull;  // reference sampling.py:148
@@ -563,18 +569,20 @@ bool gather(const Append& a, int vocab, int32_t* out) {
       if (i + 16 < a.count) __builtin_prefetch(items[i + 16]);
       PyObject* o = items[i];
       if (!PyLong_CheckExact(o)) break;
+#if HS_COMPACT_INTS
       const PyLongObject* l = reinterpret_cast<const PyLongObject*>(o);
       if (PyUnstable_Long_IsCompact(l)) {
         out[i] = device_token((long long)PyUnstable_Long_CompactValue(l), vocab);
-      } else {
-        int over = 0;
-        const long long t = PyLong_AsLongLongAndOverflow(o, &over);
-        if (over) {
-          PyErr_SetString(PyExc_OverflowError, "token id too large to convert to 64 bits");
-          return false;
-        }
-        out[i] = device_token(t, vocab);
+        continue;
       }
+#endif
+      int over = 0;
+      const long long t = PyLong_AsLongLongAndOverflow(o, &over);
+      if (over) {
+        PyErr_SetString(PyExc_OverflowError, "token id too large to convert to 64 bits");
+        return false;
+      }
+      out[i] = device_token(t, vocab);
     }
     if (i == a.count) return true;
   }

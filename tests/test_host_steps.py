@@ -1,6 +1,9 @@
 """The native host side of a step against a stand-in for the CUDA library that notes what each step
 asks of it; no GPU needed."""
 import ctypes as C
+import importlib.util
+import subprocess
+import sysconfig
 import threading
 from types import SimpleNamespace
 
@@ -9,8 +12,8 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from hydraserve_b200 import _lib  # noqa: E402
-from hydraserve_b200.engine import SamplingParams, _device  # noqa: E402
+from hydraserve_b200 import _lib, build  # noqa: E402
+from hydraserve_b200.engine import SamplingParams, TokenSample, _device  # noqa: E402
 
 VOCAB = 1_000
 
@@ -36,8 +39,8 @@ class Library:
                         C.CFUNCTYPE(i, p, p)(self._wait),
                         C.CFUNCTYPE(p, p)(lambda h: C.addressof(self.text))]
 
-    def stepper(self, book, base=100):
-        return _device._host.Stepper(1, book, base, _lib.SamplerError, *(C.cast(f, C.c_void_p).value for f in self.entries))
+    def stepper(self, host, book, base=100):
+        return host.Stepper(1, book, base, _lib.SamplerError, *(C.cast(f, C.c_void_p).value for f in self.entries))
 
     def _block(self, h, n, out):
         self.calls += 1
@@ -66,10 +69,10 @@ class Library:
 
 
 class Sampler:
-    def __init__(self, n_slots=4):
+    def __init__(self, n_slots=4, host=_device._host):
         self.library = Library()
-        self.book = _device.SlotBook(n_slots)
-        self.host = self.library.stepper(self.book)
+        self.book = host.SlotBook(n_slots)
+        self.host = self.library.stepper(host, self.book)
         self.params = SamplingParams(temperature=1.0, seed=1, presence_penalty=0.5)
 
     def step(self, requests, steps=None):
@@ -191,3 +194,33 @@ def test_a_step_that_is_no_number_is_refused_before_anything_else(monkeypatch, p
             with pytest.raises(error):
                 call(torch.zeros(2, 5), [[], []], [params] * 2, steps=[0, step])
     assert _device.longest_history([[], []], [params] * 2, [2.5, True]) == (-1 if params == SamplingParams() else 0)
+
+
+def test_the_extension_is_built_for_this_interpreter():
+    assert _device._host.__file__ == str(build.HOST_OUTPUT)
+    assert build.HOST_OUTPUT.name == "_host" + sysconfig.get_config_var("EXT_SUFFIX")
+
+
+def test_histories_read_the_same_without_the_interpreters_compact_ints(tmp_path):
+    """The form older interpreters get, built beside the other."""
+    path = tmp_path / build.HOST_OUTPUT.name
+    subprocess.run(["g++", *build.CXX_FLAGS, "-DHS_COMPACT_INTS=0", "-I", sysconfig.get_paths()["include"],
+                    "-o", str(path), *map(str, build.HOST_SOURCES)], check=True)
+    spec = importlib.util.spec_from_file_location("_host", path)
+    other = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(other)
+    other.bind(TokenSample, _device._as_int64, _device.draw_unseeded_keys)
+    history = [0, 5, VOCAB - 1, VOCAB, -1, -2**31, 2**31, 2**40, 2**62, -2**63, 7]
+    want = [0, 5, VOCAB - 1, -1, -1, -1, -1, -1, -1, -1, 7]
+    for host in (_device._host, other):
+        s = Sampler(host=host)
+        assert s.step({"a": history, "b": tuple(history)})[1] == {s.slot("a"): want, s.slot("b"): want}
+        with pytest.raises(OverflowError):
+            s.step({"a": [*history, 2**63]})
+
+
+@pytest.mark.parametrize("defines,word", [([], "ia32_pause"), (["-U__x86_64__", "-D__aarch64__"], "yield"), (["-U__x86_64__"], None)])
+def test_the_wait_hint_is_the_hosts_own(defines, word):
+    header = build.PKG / "csrc" / "hs_pause.h"
+    text = subprocess.run(["g++", "-E", "-P", "-x", "c++", *defines, str(header)], check=True, capture_output=True, text=True).stdout
+    assert [w for w in ("ia32_pause", "yield") if w in text] == ([word] if word else [])
