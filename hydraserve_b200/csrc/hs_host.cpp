@@ -412,35 +412,8 @@ PyObject* book_release(PyObject* self, PyObject* request) {
   if (!drop(b, e)) return nullptr;
   Py_RETURN_TRUE;
 }
-// lookup(request, in_batch) -> (entry, is new), or (None, False) when every slot is held by a
-// request of the batch
-PyObject* book_lookup(PyObject* self, PyObject* args) {
-  auto* b = reinterpret_cast<SlotBook*>(self);
-  PyObject *request, *in_batch;
-  if (!PyArg_ParseTuple(args, "OO", &request, &in_batch)) return nullptr;
-  SlotEntry* e = find(b, request);
-  if (!e && PyErr_Occurred()) return nullptr;
-  if (e) {
-    touch(b, e);
-    return Py_BuildValue("OO", reinterpret_cast<PyObject*>(e), Py_False);
-  }
-  if (b->free_->empty()) {
-    SlotEntry* v = b->oldest;
-    for (; v; v = v->next) {
-      const int in = PySequence_Contains(in_batch, v->request);
-      if (in < 0) return nullptr;
-      if (!in) break;
-    }
-    if (!v) return Py_BuildValue("OO", Py_None, Py_False);
-    if (!drop(b, v)) return nullptr;
-  }
-  e = add(b, request);
-  if (!e) return nullptr;
-  return Py_BuildValue("OO", reinterpret_cast<PyObject*>(e), Py_True);
-}
 PyMethodDef book_methods[] = {
     {"release", book_release, METH_O, "Forget a request; True if it held a slot."},
-    {"lookup", book_lookup, METH_VARARGS, "(entry, is new) of a request; (None, False) when the batch holds every slot."},
     {nullptr, nullptr, 0, nullptr}};
 PyMemberDef book_members[] = {
     {"n_slots", T_INT, offsetof(SlotBook, n_slots), READONLY, "resident slots"},

@@ -74,8 +74,8 @@ longest_history = _host.survey
 batched_greedy = _host.batched_greedy
 
 # Which request holds which resident histogram slot, and how much of its history the device has
-# already counted: release(request) and lookup(request, requests of the batch) -> (entry, is
-# new); least recently used requests are evicted first, never one that belongs to the batch.
+# already counted.  A step's plan takes slots for its requests: least recently used requests are
+# evicted first, never one that belongs to the batch.
 SlotBook = _host.SlotBook
 
 

@@ -125,33 +125,44 @@ def test_missing_gpu_fails_loudly():
 
 
 def test_slot_book_evicts_least_recently_used_and_never_a_row_of_the_batch():
-    """More live requests than resident slots: the least recently used request outside the
-    current batch loses its slot; when every slot belongs to the batch, the caller is told to
-    use a per-call slot (no two rows of a call may share one)."""
-    from hydraserve_b200.engine._device import SlotBook
+    """More live requests than resident slots, through the plan a step is made from: the least
+    recently used request outside the current batch loses its slot; when every slot belongs to
+    the batch, the row gets a per-call slot (no two rows of a call may share one)."""
+    from hydraserve_b200.engine import _device
 
-    book = SlotBook(3)
-    batch = {"a", "b", "c"}
-    slots = {}
-    for rid in ("a", "b", "c"):
-        entry, new = book.lookup(rid, batch)
-        assert new and entry[1] == 0
-        entry[1] = 10
-        slots[rid] = entry[0]
-    assert sorted(slots.values()) == [0, 1, 2]
-    # a fourth request in the same batch finds every slot held by the batch: no eviction
-    entry, new = book.lookup("d", batch | {"d"})
-    assert entry is None and not new
-    assert {rid: book.entries[rid][0] for rid in "abc"} == slots
-    # touching "a" makes "b" the least recently used; a later batch without "b" evicts it
-    assert book.lookup("a", {"a"})[0][0] == slots["a"]
-    entry, new = book.lookup("d", {"a", "d"})
-    assert new and entry[0] == slots["b"] and entry[1] == 0 and "b" not in book.entries
-    # the evicted request comes back as new (its histogram is rebuilt), evicting "c"
-    entry, new = book.lookup("b", {"b"})
-    assert new and entry[0] == slots["c"] and "c" not in book.entries
-    assert book.release("a") and not book.release("a")
-    assert book.lookup("e", {"e"})[0][0] == slots["a"]
+    book, base = _device.SlotBook(3), 100
+    pen, plain = SamplingParams(temperature=1.0, seed=1, presence_penalty=0.5), SamplingParams(temperature=1.0, seed=1)
+
+    def plan(requests, params=None):
+        """slots, resets, appends of a step of {request: history}"""
+        slots, resets, appends = _device._host.plan(book, base, list(requests.values()), params or [pen] * len(requests), list(requests))
+        return slots, resets, [(s, list(t)) for s, t in appends]
+
+    slots, resets, appends = plan({"a": [1], "b": [2], "c": [3]})
+    assert sorted(slots) == [0, 1, 2] and resets == slots and appends == [(s, [i + 1]) for i, s in enumerate(slots)]
+    at = dict(zip("abc", slots))
+    # a fourth request in the same batch finds every slot held by the batch, whichever row it is:
+    # no eviction, a slot of its own for this call, counted from its whole history
+    for order in ("dabc", "abcd", "abdc"):
+        histories = {"a": [1], "b": [2], "c": [3], "d": [4, 4]}
+        slots, resets, appends = plan({r: histories[r] for r in order})
+        i = order.index("d")
+        assert slots == [base + i if r == "d" else at[r] for r in order]
+        assert resets == [base + i] and appends == [(base + i, [4, 4])] and set(book.entries) == set("abc")
+    # a row without penalties needs no slot, but its request keeps the one it has
+    slots, resets, appends = plan({"d": [4], "a": [1], "b": [2], "c": [3]}, [pen, plain, plain, plain])
+    assert slots == [base, -1, -1, -1] and set(book.entries) == set("abc")
+    # "a" was used last: "b", the least recently used one outside the batch, makes room
+    plan({"b": [2]}); plan({"c": [3]}); plan({"a": [1]})
+    slots, resets, appends = plan({"d": [4, 4], "a": [1, 9]})
+    assert slots == [at["b"], at["a"]] and resets == [at["b"]] and appends == [(at["b"], [4, 4]), (at["a"], [9])]
+    assert set(book.entries) == set("acd")
+    # the evicted request comes back as new, in the place of "c", and two at once take two places
+    assert plan({"b": [2, 5]}) == ([at["c"]], [at["c"]], [(at["c"], [2, 5])])
+    slots, resets, _ = plan({"e": [6], "f": [7]})
+    assert sorted(slots) == sorted([at["b"], at["a"]]) and resets == slots and set(book.entries) == set("bef")
+    assert book.release("b") and not book.release("b")
+    assert plan({"g": [8]})[0] == [at["c"]]
     # slots held never repeat
     held = [e[0] for e in book.entries.values()]
     assert len(held) == len(set(held)) == 3
@@ -271,7 +282,6 @@ def test_a_row_without_history_goes_without_a_slot_with_and_without_request_ids(
                            reset_slots=lambda slots: calls.append(("reset", list(slots))),
                            append_tokens=lambda slots, tokens, vocab: calls.append(
                                ("append", list(slots), [list(t) for t in tokens])))
-    fake._slot_for_request = lambda *a: _device.DeviceSampler._slot_for_request(fake, *a)
     plan = lambda *a, **k: _device.DeviceSampler.plan_slots(fake, *a, **k)  # noqa: E731
     params = [SamplingParams(temperature=1.0, top_k=40, seed=1, presence_penalty=-1.5),
               SamplingParams(temperature=1.0, top_k=40, seed=2, presence_penalty=0.5),
