@@ -38,12 +38,6 @@ __device__ __forceinline__ float canonical(float f) {
   return __float_as_uint(f) == 0x80000000u ? 0.0f : f;
 }
 
-// Hint: bring `bytes` (a multiple of 16) starting at the 16-byte aligned global address p
-// into L2.  No completion to wait for, nothing is written.
-__device__ __forceinline__ void prefetch_l2_bulk(const void* p, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
 // Loads the compiler must issue where they are written (it may otherwise sink a load to its
 // first use, which defeats starting a chain of dependent reads early).
 __device__ __forceinline__ int load_now_s32(const int* p) {
@@ -101,11 +95,6 @@ __device__ __forceinline__ Philox4 philox4x32_10(uint32_t c0, uint32_t c1, uint3
 }
 
 // ---- warp / block primitives ---------------------------------------------------------
-__device__ __forceinline__ u64 shfl_xor_u64(u64 v, int lane_mask) {
-  const uint32_t lo = __shfl_xor_sync(0xffffffffu, (uint32_t)v, lane_mask);
-  const uint32_t hi = __shfl_xor_sync(0xffffffffu, (uint32_t)(v >> 32), lane_mask);
-  return ((u64)hi << 32) | lo;
-}
 __device__ __forceinline__ u64 shfl_u64(u64 v, int src) {
   return __shfl_sync(0xffffffffu, v, src);
 }
@@ -126,9 +115,6 @@ __device__ __forceinline__ u64 warp_max_u64(u64 v) {
 }
 __device__ __forceinline__ uint32_t warp_max_u32(uint32_t v) {
   return __reduce_max_sync(0xffffffffu, v);
-}
-__device__ __forceinline__ uint32_t warp_min_u32(uint32_t v) {
-  return __reduce_min_sync(0xffffffffu, v);
 }
 // Inclusive scan over the lanes of a warp.
 __device__ __forceinline__ u64 warp_scan_u64(u64 v) {

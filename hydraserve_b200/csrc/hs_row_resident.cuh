@@ -427,7 +427,6 @@ __device__ Selection res_resolve(RowCtx& c, int n, float m, u64 want, In&& in) {
   u64 pre, pu, tot, tu;
   block_warp_prefix2(*c.x, shfl_u64(incl, 31), 0, pre, pu, tot, tu);
   Selection sel{};
-  sel.levels = 3;
   sel.target = want;
   sel.ok = want >= 1 && want <= tot;
   if (!sel.ok) return sel;

@@ -17,11 +17,9 @@ struct Hist {
 };
 
 struct Selection {
-  uint32_t key;               // selected key; when `levels` < 3 only its top bits (prefix) are known
-  uint32_t prefix;            // resolved high bits, right aligned
-  int levels;                 // radix levels resolved: 3 = the full 32-bit key
-  u64 above_cnt, above_mass;  // over elements with key above the selected key / bucket
-  u64 bin_cnt, bin_mass;      // over elements inside the selected key / bucket
+  uint32_t key;               // selected key
+  u64 above_cnt, above_mass;  // over elements with key above the selected key
+  u64 bin_cnt, bin_mass;      // over elements with the selected key
   u64 total_cnt, total_mass;  // over all elements with key >= lo
   u64 target;                 // the count / mass that was searched for
   bool ok;
@@ -103,12 +101,8 @@ __device__ __forceinline__ u64 top_p_target_warp(u64 total, float top_p) {
 // must call add(valid, bucket, count, mass), with all lanes of each warp together, where
 // valid marks an element with key >= lo_key whose bits above `shift + bits` equal `prefix`
 // (level 0: all), and bucket = (key >> shift) & mask.
-// Stops early, with sel.levels < 3, once the selected bucket holds at most stop_pop
-// elements (stop_pop = 0: always resolve all 32 bits).
 template <bool BY_MASS, bool WITH_MASS, class Fill>
-__device__ Selection descend_core(ClusterCtx& c, Fill& fill, uint32_t lo_key, u64 target_cnt,
-                                  float top_p, u64 stop_pop = 0, int first_level = 0,
-                                  uint32_t prefix0 = 0) {
+__device__ Selection descend_core(ClusterCtx& c, Fill& fill, uint32_t lo_key, u64 target_cnt, float top_p) {
   static_assert(WITH_MASS || !BY_MASS, "a mass descent needs masses");
   Hist& h = *c.hist;
   u64* full_mass = reinterpret_cast<u64*>(h.l0);
@@ -119,13 +113,12 @@ __device__ Selection descend_core(ClusterCtx& c, Fill& fill, uint32_t lo_key, u6
   sel.bin_cnt = sel.bin_mass = 0;
   sel.target = target_cnt;
   sel.ok = true;
-  sel.levels = first_level;
-  uint32_t prefix = prefix0;
+  uint32_t prefix = 0;
   const int per = kBins / (int)c.nranks;
   const int tid = threadIdx.x;
   const HistAdder<WITH_MASS> add{&h};
 
-  for (int level = first_level; level < 3; ++level) {
+  for (int level = 0; level < 3; ++level) {
     const int shift = level_shift(level);
     const int bits = level_bits(level);
     for (int b = tid; b < kBins; b += kThreads) {
@@ -175,10 +168,10 @@ __device__ Selection descend_core(ClusterCtx& c, Fill& fill, uint32_t lo_key, u6
     block_warp_prefix2(*c.x, shfl_u64(ia, 31), shfl_u64(ib, 31), pa, pb, ta, tb);
     u64 ex_cnt = pa + ia - c_sum;   // exclusive prefix over buckets above `hi`
     u64 ex_mass = pb + ib - m_sum;
-    if (level == first_level) {
+    if (level == 0) {
       sel.total_cnt = ta;
       sel.total_mass = tb;
-      if (BY_MASS && top_p >= 0.0f) sel.target = top_p_target(tb, top_p);  // top_p < 0: explicit mass target
+      if (BY_MASS) sel.target = top_p_target(tb, top_p);
     }
     const u64 want = sel.target - (BY_MASS ? sel.above_mass : sel.above_cnt);
     {
@@ -207,7 +200,6 @@ __device__ Selection descend_core(ClusterCtx& c, Fill& fill, uint32_t lo_key, u6
     if (c.x->bcast[7] == 0) {  // nothing reaches the target (non-finite input)
       sel.ok = false;
       sel.key = lo_key;
-      sel.prefix = prefix;
       sel.bin_cnt = sel.bin_mass = 0;
       __syncthreads();
       return sel;
@@ -218,12 +210,9 @@ __device__ Selection descend_core(ClusterCtx& c, Fill& fill, uint32_t lo_key, u6
     sel.bin_cnt = c.x->bcast[3];
     sel.bin_mass = c.x->bcast[4];
     prefix = (prefix << bits) | bin;
-    sel.levels = level + 1;
     __syncthreads();  // bcast and the aliased arrays are reused by the next level
-    if (stop_pop && level < 2 && sel.bin_cnt <= stop_pop) break;
   }
-  sel.prefix = prefix;
-  sel.key = sel.levels == 3 ? prefix : (prefix << (sel.levels == 1 ? 21 : 10));
+  sel.key = prefix;
   return sel;
 }
 
