@@ -37,6 +37,9 @@ __device__ __forceinline__ float score_of(uint32_t k) {
 __device__ __forceinline__ float canonical(float f) {
   return __float_as_uint(f) == 0x80000000u ? 0.0f : f;
 }
+// The same for what is not a NaN, in one addition (the loops that score token after token, or class
+// after class, take this one: the other costs them 1 to 1.5 % of a launch).
+__device__ __forceinline__ float canonical_number(float f) { return __fadd_rn(f, 0.0f); }
 
 // Loads the compiler must issue where they are written (it may otherwise sink a load to its
 // first use, which defeats starting a chain of dependent reads early).

@@ -543,14 +543,14 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
     if (divide) v = __fdiv_rn(v, T);
     return canonical(v);
   };
+  auto score_new = [&](float v) { return canonical_number(divide ? __fdiv_rn(v, T) : v); };  // (held never, no NaN)
 
   // ---- A. the one read of the row from HBM, scored ------------------------------------
   uint32_t top_key = 0, low_key = 0xffffffffu;  // over this thread's elements
   int top_at = 0;                               // (the lowest with the highest key)
   auto note = [&](float s, int i) {
     const uint32_t k = key_of(s);
-    // (the often-repeated tokens below come in any order)
-    if (k > top_key || (k == top_key && i < top_at)) { top_key = k; top_at = i; }
+    if (k > top_key) { top_key = k; top_at = i; }  // (a thread's elements come in ascending order)
     low_key = min(low_key, k);
   };
   {
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
     // branch per token, one 128-bit store
     auto put4 = [&](const float4& w, uint32_t cl, int i) {
       if ((cl & 0xffu) == 0u) {
-        const float4 v = make_float4(score(w.x, 0), score(w.y, 0), score(w.z, 0), score(w.w, 0));
+        const float4 v = make_float4(score_new(w.x), score_new(w.y), score_new(w.z), score_new(w.w));
         const uint32_t k0 = key_of(v.x), k1 = key_of(v.y), k2 = key_of(v.z), k3 = key_of(v.w);
         const uint32_t hi = max(max(k0, k1), max(k2, k3)), lo = min(min(k0, k1), min(k2, k3));
         if (hi <= 0xff800000u && lo >= 0x007fffffu) {  // (keys of +inf and -inf)
@@ -636,6 +636,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
         float v = score(c.stage[i], e.y);
         if (candidate && v != v) v = __int_as_float(0xff800000);
         c.stage[i] = v;
+        // (these come in any order: an equal score at a lower id takes the place)
+        if (key_of(v) == top_key) top_at = min(top_at, i);
         note(v, i);
       }
     }

@@ -141,10 +141,13 @@ __device__ __forceinline__ uint32_t v3_raw_of_bin(int b) {
 struct Scorer {
   float T, rp, pp, fp;
   bool greedy;
+  template <bool NUMBER = false>
   __device__ __forceinline__ float score_of_value(float v) const {
-    return greedy || T == 1.0f ? canonical(v) : canonical(__fdiv_rn(v, T));
+    if (!greedy && T != 1.0f) v = __fdiv_rn(v, T);
+    return NUMBER ? canonical_number(v) : canonical(v);
   }
-  // score of a token with raw value bits `raw` that the history holds `count` times
+  // score of a token with raw value bits `raw` (NUMBER: not a NaN's) that the history holds `count` times
+  template <bool NUMBER = false>
   __device__ __forceinline__ float score_of(uint32_t raw, int count) const {
     float v = __uint_as_float(raw << 16);  // (a zero's sign goes at the end)
     if (count > 0) {
@@ -152,14 +155,14 @@ struct Scorer {
       v = __fsub_rn(v, pp);
       v = __fsub_rn(v, __fmul_rn(fp, (float)count));
     }
-    return score_of_value(v);
+    return score_of_value<NUMBER>(v);
   }
+  // score of a bin of count class k, and of a cell
+  __device__ __forceinline__ float bin_score(int bin, int k) const { return score_of<true>(v3_raw_of_bin(bin), k); }
   __device__ __forceinline__ float cell_score(int cell) const {
     const int c = cell / kV3Bins;
-    return score_of(v3_raw_of_bin(cell - c * kV3Bins), c);
+    return bin_score(cell - c * kV3Bins, c);
   }
-  // score key of a bin of count class k
-  __device__ __forceinline__ uint32_t key_of_bin(int bin, int k) const { return key_of(score_of(v3_raw_of_bin(bin), k)); }
 };
 template <size_t AT, class T>
 __device__ __forceinline__ T* at_smem() {
@@ -262,7 +265,7 @@ __device__ __forceinline__ void for_each_class(const Ctx3& c, F&& f) {
       const int at = (k * kPerClass + (valid ? __ffs(bits) - 1 : 0)) * kThreads;
       bits &= bits - 1u;
       const int cell = at + (int)threadIdx.x;
-      f(valid, sc.score_of(v3_raw_of_bin(cell - k * kV3Bins), k), tab[at], cell);
+      f(valid, sc.bin_score(cell - k * kV3Bins, k), tab[at], cell);
     }
   }
 }
@@ -314,7 +317,7 @@ __device__ __noinline__ void locate_cells(const Ctx3& c, const V3Map map, int b)
     while (lo < hi) {
       const int step = (hi - lo + 31) >> 5;
       const int t = lo + (lane + 1) * step - 1;
-      const bool pass = t >= hi || map.bucket(sc.key_of_bin(min(t, hi - 1) - k * kV3Bins, k)) >= want;
+      const bool pass = t >= hi || map.bucket(key_of(sc.bin_score(min(t, hi - 1) - k * kV3Bins, k))) >= want;
       const uint32_t votes = __ballot_sync(0xffffffffu, pass);
       if (votes == 0) { lo = hi; break; }
       const int first = __ffs(votes) - 1;
