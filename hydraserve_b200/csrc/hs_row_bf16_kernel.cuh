@@ -447,7 +447,24 @@ __device__ __forceinline__ bool cand_part(const RowV3Args& args, unsigned char* 
     n = (int)keep;
   }
   mark(2);
-  finish_candidates(a, c.row, *c.x(), L.cand, reinterpret_cast<u64*>(smem_raw + lay.mass), n, P, 0, out, clocks);
+  const float* noise_row = a.noise ? a.noise + (size_t)c.row * a.vocab : nullptr;
+  FinishOut r = finish_sorted(*c.x(), L.cand, reinterpret_cast<u64*>(smem_raw + lay.mass), n, P, noise_row, out, clocks);
+  if (P.slot >= a.pool.slots_total) r.status |= 64;  // a slot this sampler does not have: no penalties
+  if (a.scores_out) {
+    float* dst = a.scores_out + (size_t)c.row * a.vocab;
+    for (int id = tid; id < c.vocab; id += kThreads) dst[id] = __int_as_float(0xff800000);
+    __syncthreads();
+    for (int i = tid; i < (int)r.n_kept; i += kThreads) dst[cand_id(L.cand[i])] = score_of(cand_key(L.cand[i]));
+  }
+  if (tid == 0) {
+    write_finish(r, out);
+    if (a.tokens_out) a.tokens_out[c.row] = r.token;
+    if ((a.flags & HS_SAMPLE_APPEND_TOKEN) && slot_ok && r.token >= 0 && r.token < a.vocab) {
+      if (!slot_append_one(a.pool, P.slot, r.token)) out->status = r.status | 2;
+    }
+  }
+  __syncthreads();
+  if (tid < 32) write_record(a.out + c.row, *out, P.n_logprobs >= 0, a.flags);
   mark(8);
   return false;
 }
@@ -496,7 +513,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel_bf16(const __grid_cons
   } else if (args.csplit == 1) {
     part = -1;
   }
-  if (count_tokens(args, row, part)) finish_counted_row(args.base);
+  if (count_tokens(args, row, part)) finish_counted_row();
   if (when) when[1] = global_timer_ns();
 }
 

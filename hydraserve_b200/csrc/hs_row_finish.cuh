@@ -862,7 +862,7 @@ __device__ __forceinline__ void release_scratch(CountState& S) {
 // the last fit a list after all, they are listed (in the count table's place, which has served) and
 // the row is finished like any other of its kind.  False: they do not fit, or the row goes to the
 // general kernel.  Bound by one more walk of the row, in the place of the draw's.
-__device__ __noinline__ bool finish_listed_row(const RowKernelArgs& a) {
+__device__ __noinline__ bool finish_listed_row() {
   CountState& S = count_state();
   Ctx3& c = S.c;
   if (S.status & 4) return false;
@@ -888,13 +888,30 @@ __device__ __noinline__ bool finish_listed_row(const RowKernelArgs& a) {
   __syncthreads();
   const int n = min(*c.gbuf_n(), kCandCap);
   cand_sort(L, n);
-  finish_candidates(a, S.row, *c.x(), list, list + kCandCap, n, S.P, S.status, &S.out);
+  const float* noise_row = S.noise ? S.noise + (size_t)S.row * c.vocab : nullptr;
+  const FinishOut r = finish_sorted(*c.x(), list, list + kCandCap, n, S.P, noise_row, &S.out);
+  if (S.scores_out) {
+    float* dst = S.scores_out + (size_t)S.row * c.vocab;
+    for (int id = threadIdx.x; id < c.vocab; id += kThreads) dst[id] = __int_as_float(0xff800000);
+    __syncthreads();
+    for (int i = threadIdx.x; i < (int)r.n_kept; i += kThreads) dst[cand_id(list[i])] = score_of(cand_key(list[i]));
+  }
+  if (threadIdx.x == 0) {
+    write_finish(r, &S.out);
+    S.out.status |= S.status;
+    if (S.tokens_out) S.tokens_out[S.row] = r.token;
+    if ((S.flags & HS_SAMPLE_APPEND_TOKEN) && S.slot_ok && r.token >= 0 && r.token < c.vocab) {
+      if (!slot_append_one(c.pool, S.P.slot, r.token)) S.out.status |= 2;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) write_record(S.out_row, S.out, S.P.n_logprobs >= 0, (uint32_t)S.flags);
   release_scratch(S);
   return true;
 }
 
 // From the row's count table (and rare tokens) to its record.
-__device__ __forceinline__ void finish_counted_row(const RowKernelArgs& a) {
+__device__ __forceinline__ void finish_counted_row() {
   CountState& S = count_state();
   Ctx3& c = S.c;
   const int tid = threadIdx.x;
@@ -904,7 +921,7 @@ __device__ __forceinline__ void finish_counted_row(const RowKernelArgs& a) {
     if (tid < 32) write_record(S.out_row, S.out, false, (uint32_t)S.flags);
     return;
   }
-  if (is_candidate_row(S.P, c.vocab) && finish_listed_row(a)) return;
+  if (is_candidate_row(S.P, c.vocab) && finish_listed_row()) return;
   if (c.greedy) {
     phase_greedy();
   } else {

@@ -709,30 +709,4 @@ __device__ __forceinline__ void write_finish(const FinishOut& r, hs_row_out* out
   out->log_z = r.log_z;
 }
 
-// From a candidate row's list, cut by top-k and sorted, to its record (called by the whole CTA).
-__device__ __forceinline__ void finish_candidates(const RowKernelArgs& a, int row, Exchange& x, const u64* cand, u64* mass, int n,
-                                                  const hs_row_params& P, int status, hs_row_out* record,
-                                                  unsigned long long* dbg = nullptr) {
-  const int tid = threadIdx.x;
-  const float* noise_row = a.noise ? a.noise + (size_t)row * a.vocab : nullptr;
-  FinishOut r = finish_sorted(x, cand, mass, n, P, noise_row, record, dbg);
-  r.status |= status;
-  if (P.slot >= a.pool.slots_total) r.status |= 64;  // a slot this sampler does not have: no penalties
-  if (a.scores_out) {
-    float* dst = a.scores_out + (size_t)row * a.vocab;
-    for (int id = tid; id < a.vocab; id += kThreads) dst[id] = __int_as_float(0xff800000);
-    __syncthreads();
-    for (int i = tid; i < (int)r.n_kept; i += kThreads) dst[cand_id(cand[i])] = score_of(cand_key(cand[i]));
-  }
-  if (tid == 0) {
-    write_finish(r, record);
-    if (a.tokens_out) a.tokens_out[row] = r.token;
-    if ((a.flags & HS_SAMPLE_APPEND_TOKEN) && P.slot >= 0 && P.slot < a.pool.slots_total && r.token >= 0 && r.token < a.vocab) {
-      if (!slot_append_one(a.pool, P.slot, r.token)) record->status = r.status | 2;
-    }
-  }
-  __syncthreads();
-  if (tid < 32) write_record(a.out + row, *record, P.n_logprobs >= 0, a.flags);
-}
-
 }  // namespace hs
