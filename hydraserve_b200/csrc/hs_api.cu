@@ -325,7 +325,8 @@ int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride
   a.small_k = h->force_general ? hs::kSmallKOrder : hs::kSmallKList;
   // fp32 rows with a small top_k: as clusters while these are at most two waves of two CTAs per SM, one
   // CTA each in the streaming kernel beyond that (a row takes longer there, but 296 of them run side by
-  // side; figures at that kernel).  Such a batch is too large for inline parameters.
+  // side: 64 rows are two waves less a little and 55 us here, 61 there; 75 would be a third, 70 against
+  // 62).  Such a batch is too large for inline parameters.
   const bool may_stream = dtype == HS_DTYPE_F32 && !h->force_general && !(flags & HS_SAMPLE_GENERAL_KERNEL);
   if (may_stream && params && n_count != batch && (long long)batch * plan.cluster > 4ll * h->sm_count) {
     a.small_k = hs::kSmallKLeave;

@@ -12,10 +12,11 @@
 // cut back whenever it gets long, and finished exactly like a bf16 candidate row's.  A list
 // that overflows (more ties than it holds) reports status 4, for the general kernel.
 //
-// What bounds it: the chain of bound, stream and finish of one row, the same 70 us for any batch that
+// What bounds it: the chain of bound, stream and finish of one row, the same 61 us for any batch that
 // is one wave of two CTAs per SM, where the resident kernel's time grows with the waves of its
-// clusters.  151,936 tokens, top_k 50, penalties (us; streaming / resident): 64 rows 69 / 55, 128 rows
-// 70 / 103, 256 rows 80 / 247.
+// clusters.  151,936 tokens, top_k 50, penalties, one plain greedy row for the resident kernel (us a
+// step; streaming / resident): 32 rows 59 / 30, 64 rows 61 / 55, 74 rows 61 / 69, 128 rows 62 / 103, 256
+// rows 76 / 246.
 #pragma once
 
 #include "hs_row_bf16_kernel.cuh"
@@ -145,7 +146,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel_f32_stream(const __gri
     else *L.lost = 1;
   };
   auto score_pending = [&](int from, int to) {
-#pragma unroll 1
+    // (left to the compiler to unroll: the hits' count classes are scattered reads, and one at a time
+    // they make 128 rows take 82 us instead of 62)
     for (int i = from + tid; i < to; i += kThreads) {
       const u64 e = L.cand[i];
       const int id = (int)(uint32_t)e;
