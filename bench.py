@@ -443,7 +443,8 @@ def run_ours(args, world, rank, local_rank):
         "traffic": NCU_DRAM_BYTES_PER_STEP.get(cfg) if default_shape else None,
         "kernel": ("hs::row_kernel_bf16 (one launch per step: counting rows and candidate-row parts, two CTAs per SM)"
                    if w.dtype == "bf16" else
-                   "hs::row_kernel (a cluster of CTAs per row, the row resident in shared memory)"),
+                   "hs::row_kernel (a cluster of CTAs per row, the row resident in shared memory)" if launches == args.steps else
+                   "hs::row_kernel_f32_stream (rows with 0 < top_k <= 256, one CTA each) + hs::row_kernel (the other rows)"),
         "peak_source": peak_src,
         "algorithmic_bytes_per_launch": algo_bytes, "logits_bytes_per_launch": logits_bytes,
         "logits_only_gbs": logits_bytes / (ms_per_step * 1e-3) / 1e9,

@@ -11,7 +11,7 @@ namespace cg = cooperative_groups;
 
 namespace hs {
 
-constexpr int kThreads = 512;           // threads per CTA of the row kernels (128 registers each: no spills)
+constexpr int kThreads = 512;           // threads per CTA of the row kernels (64 registers each, two CTAs per SM)
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxCluster = 8;          // portable cluster limit
 constexpr int kBinBits = 11;            // radix digit of the first two select levels

@@ -3,7 +3,7 @@
 // mixed batch) or one part of a row for the candidate path (small top_k, hs_row_topk.cuh);
 // the hardware hands the items out in grid order as SMs free up, the long ones first.  No CTA
 // waits for another: the last part of a candidate row to arrive finishes that row, and a row
-// whose candidate list overflowed is counted by the CTA that found out.
+// whose candidate list overflowed is counted by the CTA that found out (and then listed after all).
 #pragma once
 #include <type_traits>
 

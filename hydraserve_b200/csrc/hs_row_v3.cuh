@@ -18,13 +18,13 @@
 // order-independent.
 //
 // Token ids are only needed at the very end ("a uniformly chosen member of this class",
-// "the lowest ids of this tie group").  A class of more than kV3ListCap tokens is sampled by
+// "the lowest ids of this tie group").  A class of more than kV3RejectMin tokens is sampled by
 // rejection: Philox-drawn positions are probed until one belongs to the class (exactly
 // uniform over its members); a lone CTA issues scattered reads slowly, so a smaller class,
 // or one the probes keep missing, is found by scanning the row once more for its bit
 // pattern.  Lowest-id tie-breaks walk the row hierarchically.
 //
-// A row's CTA keeps the count table, the histogram and a short side list in shared memory, 111 KB, so
+// A row's CTA keeps the count table, the histogram and a short side list in shared memory, 112.3 KB, so
 // that two CTAs share an SM and one row's barrier-bound selection phases overlap another row's
 // counting.  What is left of L1 is small, so the streaming loads go past it.
 #pragma once

@@ -169,8 +169,8 @@ __device__ __forceinline__ bool slot_append_one(const Pool& p, int s, int token)
 // one another.  A slot that is emptied first (kResetFirst, the usual case) takes two barriers: its
 // old ids are cleared; every token is counted where its position will stand, and the token that
 // found a zero there stands for its id from then on; those write id and count, position and class.
-// Four tokens per thread are under way together.  One slot with an 8,192-token prompt: 14 us to
-// empty it (one CTA) and 10 us for the three passes above, now 9 us in all.
+// Four tokens per thread are under way together.  One slot with an 8,192-token prompt, cold (ncu): 22 us
+// to empty it (one CTA) and 16 us for the three passes above, 12.4 us here in all.
 // A slot that keeps what it has goes through the three passes with barriers in between.
 // Overwrites `tokens` (this sampler's own copy of them).
 constexpr int kBuildThreads = 512;
@@ -309,7 +309,9 @@ __global__ void __launch_bounds__(kBuildThreads) slots_build_kernel(const Pool p
 // the three passes above are one.  Up to kInlineAppends pairs travel in the launch's own
 // parameters; without inline pairs they come from device memory as hs_slots_append takes them.
 // Bound by three dependent scattered accesses: 2.4 us for one request, 3.9 us for 256 (three launches
-// and a copy before).
+// and a copy before).  Where the line lies, calls of 64 and 256 rows that gained a token each: 40.3 and
+// 61.9 us with the pairs in the launch, 42.8 and 62.7 with a copy; room for 1,024 pairs costs every launch
+// that has fewer (128 rows 49.6 us against 48.3).
 constexpr int kInlineAppends = 256;
 struct InlineAppends {
   int n;
