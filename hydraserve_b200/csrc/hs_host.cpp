@@ -546,16 +546,17 @@ bool gather(const Append& a, int vocab, int32_t* out) {
       const PyLongObject* l = reinterpret_cast<const PyLongObject*>(o);
       if (PyUnstable_Long_IsCompact(l)) {
         out[i] = device_token((long long)PyUnstable_Long_CompactValue(l), vocab);
-        continue;
-      }
+      } else
 #endif
-      int over = 0;
-      const long long t = PyLong_AsLongLongAndOverflow(o, &over);
-      if (over) {
-        PyErr_SetString(PyExc_OverflowError, "token id too large to convert to 64 bits");
-        return false;
+      {
+        int over = 0;
+        const long long t = PyLong_AsLongLongAndOverflow(o, &over);
+        if (over) {
+          PyErr_SetString(PyExc_OverflowError, "token id too large to convert to 64 bits");
+          return false;
+        }
+        out[i] = device_token(t, vocab);
       }
-      out[i] = device_token(t, vocab);
     }
     if (i == a.count) return true;
   }
