@@ -88,6 +88,9 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
     S.scores_out = a.scores_out;
     S.tokens_out = a.tokens_out;
     S.out_row = a.out + row_index;
+    S.parts = part < 0 ? 1 : args.csplit;
+    S.lists = args.ctab + (size_t)row_index * args.csplit * kCells;
+    S.lens = args.crare_n + (size_t)row_index * args.csplit;
     S.clocks = args.phase_clocks ? args.phase_clocks + (size_t)row_index * kV3PhaseSlots : nullptr;
     if (S.clocks) S.clocks[0] = clock64();
   }
@@ -136,7 +139,7 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
   const int n8_row = c.n8();
   const int parts = part < 0 ? 1 : args.csplit;
   const int my_part = part < 0 ? 0 : part;
-  const int per_part = (n8_row + parts - 1) / parts;
+  const int per_part = chunks_per_part(n8_row, parts);
   const int chunk_lo = min(my_part * per_part, n8_row), chunk_hi = min(chunk_lo + per_part, n8_row);
   const bool last_part = my_part == parts - 1;
   // small[16..18] / [19..21]: highest (+ 1) / lowest non-empty cell per count class; [22]: lowest side key
@@ -282,31 +285,51 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
     // Hand this part's counts over, as a list of (class, count), with its rare tokens; then a ticket.
     // The part that draws the last ticket adds the other parts' lists to its own table and goes on;
     // the others are done.  Nobody waits for anybody.  (Lists instead of whole tables: about 16 KB a
-    // part instead of 72, so that a lone row can be counted by sixteen CTAs.)
+    // part instead of 72.)  Bound by the banks when a list is added up, and by the round trips to L2: in the
+    // order of the cells, four entries a load and the next piece under way, the first token after a prompt
+    // of 8,192 takes 97.2 us a call, 107.6 before (248,320 tokens, sixteen parts; the look-up in
+    // nth_in_parts has its share in that).
     const size_t mine = (size_t)c.row * parts + my_part;
     const int nr = *rare_n;
     for (int t = tid; t < min(nr, kV3RareCap); t += kThreads) args.crare[mine * kV3RareCap + t] = rare[t];
     {
-      // a count that 17 bits do not hold takes several entries
-      u64 left = 0;
+      // Warp w lists the w-th run of cells, 32 neighbours at a time, so that a list is in the order of
+      // the cells: whoever adds it up finds neighbouring entries in different banks, and can look a
+      // class up in it (part_of_member).  A count that 17 bits do not hold takes several entries.
+      const int lane = tid & 31, warp = tid >> 5;
+      const int rows = (c.cls ? kCells : kV3Bins) / (32 * kWarps);  // (without penalties there is one count class)
+      static_assert(kV3Bins % (32 * kWarps) == 0, "every warp has whole groups of 32 cells");
+      const int first = warp * rows * 32 + lane;
+      const uint32_t* run = c.tab() + first;
       int n = 0;
 #pragma unroll 4
-      for (int u = 0; u < kCells / kThreads; ++u) {
-        const uint32_t v = c.tab()[tid + u * kThreads];
-        if (v) { left |= 1ull << u; n += 1 + (int)((v - 1u) / kMostHanded); }
+      for (int u = 0; u < rows; ++u) {
+        const uint32_t v = run[32 * u];
+        n += v ? 1 : 0;
+        if (v > kMostHanded) n += (int)((v - 1u) / kMostHanded);
       }
-      int total;
-      int at = block_place(small + 48, n, total);  // (a barrier inside: the rare tokens have left)
+      n = __reduce_add_sync(0xffffffffu, n);
+      if (lane == 0) small[48 + warp] = n;
+      __syncthreads();  // (the rare tokens have left, too)
+      const int of_warp = lane < kWarps ? small[48 + lane] : 0;
+      const int total = __reduce_add_sync(0xffffffffu, of_warp);
+      int at = __reduce_add_sync(0xffffffffu, lane < warp ? of_warp : 0);
       uint32_t* gtab = args.ctab + mine * kCells;
       uint32_t* dst = total <= kV3Staged ? staged : gtab;
-      for (; left; left &= left - 1) {
-        const int cell = tid + (__ffsll((long long)left) - 1) * kThreads;
-        uint32_t v = c.tab()[cell];
-        for (; v > kMostHanded; v -= kMostHanded) dst[at++] = (uint32_t)cell | (kMostHanded << 15);
-        dst[at++] = (uint32_t)cell | (v << 15);
+#pragma unroll 1
+      for (int u = 0; u < rows; ++u) {
+        uint32_t v = run[32 * u];
+        const uint32_t cell = (uint32_t)(first + 32 * u);
+        for (uint32_t who = __ballot_sync(0xffffffffu, v != 0u); who; who = __ballot_sync(0xffffffffu, v != 0u)) {
+          const uint32_t part_v = min(v, kMostHanded);
+          if (v) dst[at + __popc(who & ((1u << lane) - 1u))] = cell | (part_v << 15);
+          at += __popc(who);
+          v -= part_v;
+          if (__all_sync(0xffffffffu, v == 0u)) break;  // (but for the largest counts)
+        }
       }
       __syncthreads();
-      if (total <= kV3Staged)
+      if (dst == staged)
         for (int i = tid; i < (total + 3) / 4; i += kThreads)
           reinterpret_cast<uint4*>(gtab)[i] = reinterpret_cast<const uint4*>(staged)[i];
       if (tid == 0) args.crare_n[mine] = make_int2(total, nr);
@@ -318,29 +341,57 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
     if (small[14] != parts - 1) return false;
     __threadfence();
     if (tid == 0) args.count_ticket[c.row] = 0;
-    // all parts' lengths, then every warp takes its share of each list, the next list's entries
-    // on their way while this one's are added
+    // The other parts' lists, piece by piece of up to 4,096 entries, the next piece's on their way while this
+    // one's are added.
     const int2* lens = args.crare_n + (size_t)c.row * parts;
     const uint32_t* lists = args.ctab + (size_t)c.row * parts * kCells;
-    int n_rare_all = 0;
-    for (int g = 0; g < parts; ++g) {
-      const int2 len = __ldcg(lens + g);
-      if (g != my_part) {
-        const uint32_t* src = lists + (size_t)g * kCells;
-        constexpr int kFlight = 8;
-        for (int i0 = tid; i0 < len.x; i0 += kFlight * kThreads) {
-          uint32_t v[kFlight];
+    int2* part_len = reinterpret_cast<int2*>(defer);  // (the staged list has left)
+    if (tid < parts) part_len[tid] = __ldcg(lens + tid);
+    __syncthreads();
+    constexpr int kFlight = 2;  // four entries each
+    struct Piece { int g, at; } next{my_part == 0 ? 1 : 0, 0};
+    auto fetch = [&](uint4 (&v)[kFlight]) {
+      if (next.g >= parts) return;
+      const int n = part_len[next.g].x, n4 = (n + 3) >> 2;
+      const uint4* src = reinterpret_cast<const uint4*>(lists + (size_t)next.g * kCells);
 #pragma unroll
-          for (int u = 0; u < kFlight; ++u) v[u] = i0 + u * kThreads < len.x ? __ldcg(src + i0 + u * kThreads) : 0u;
-#pragma unroll
-          for (int u = 0; u < kFlight; ++u)
-            if (v[u]) atomicAdd(&c.tab()[v[u] & 0x7fffu], v[u] >> 15);
+      for (int u = 0; u < kFlight; ++u) {
+        const int i = next.at + tid + u * kThreads;
+        v[u] = i < n4 ? __ldcg(src + i) : make_uint4(0u, 0u, 0u, 0u);
+        if (i == n4 - 1) {  // (nothing is behind a list's last entry)
+          if (4 * i + 1 >= n) v[u].y = 0u;
+          if (4 * i + 2 >= n) v[u].z = 0u;
+          if (4 * i + 3 >= n) v[u].w = 0u;
         }
       }
+      next.at += kFlight * kThreads;
+      if (next.at >= n4) {
+        next.at = 0;
+        next.g += next.g + 1 == my_part ? 2 : 1;
+      }
+    };
+    uint4 v[kFlight], vn[kFlight];
+    fetch(v);
+    for (bool more = true; more;) {
+      more = next.g < parts;
+      fetch(vn);
+#pragma unroll
+      for (int u = 0; u < kFlight; ++u) {
+        const uint32_t e[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (e[k]) atomicAdd(&c.tab()[e[k] & 0x7fffu], e[k] >> 15);
+        v[u] = vn[u];
+      }
+    }
+    int n_rare_all = 0;
+#pragma unroll 1
+    for (int g = 0; g < parts; ++g) {
       // (a total beyond the capacity is swept up below)
-      for (int t = tid; t < min(len.y, kV3RareCap); t += kThreads)
+      const int n = part_len[g].y;
+      for (int t = tid; t < min(n, kV3RareCap); t += kThreads)
         if (n_rare_all + t < kV3RareCap) rare[n_rare_all + t] = __ldcg(args.crare + ((size_t)c.row * parts + g) * kV3RareCap + t);
-      n_rare_all += len.y;
+      n_rare_all += n;
     }
     if (tid == 0) *rare_n = n_rare_all;
     __syncthreads();

@@ -1,0 +1,79 @@
+"""The bf16 row kernel's rarer ways through a row against its usual ones: rows cut into parts, rows
+of a batch of the stream and a little more or less, values spread over the whole range of a bf16,
+masked rows; greedy rows at any address; and a step's records as the host puts them together."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+from hydraserve_b200 import _lib  # noqa: E402
+from hydraserve_b200.engine import SamplingParams, _device, sample_logits  # noqa: E402
+
+COUNTS = ("status", "n_kept", "n_after_topk", "n_after_minp", "cut_bits", "n_cut_ties", "row_max")
+
+
+@pytest.fixture(autouse=True)
+def _lib_built(built_library):
+    return built_library
+
+
+def _sampler(vocab, batch):
+    return _device.DeviceSampler("cuda:0", vocab_max=vocab, batch_max=batch, resident_slots=batch)
+
+
+def _rows(kind, batch, vocab, seed=0):
+    gen = torch.Generator().manual_seed(seed + vocab)
+    x = torch.randn(batch, vocab, generator=gen) * 3
+    if kind == "masked":           # all but a few hundred tokens are out
+        x[:, torch.randperm(vocab, generator=gen)[: max(0, vocab - 300)]] = -float("inf")
+    elif kind == "lowest":         # ... or at the type's lowest value
+        x[:, torch.randperm(vocab, generator=gen)[: max(0, vocab - 300)]] = torch.finfo(torch.bfloat16).min
+    elif kind == "wide":           # magnitudes from 1e-20 to 1e20
+        x = torch.sign(x) * 10.0 ** (torch.rand(batch, vocab, generator=gen) * 40 - 20)
+    elif kind == "few values":
+        x = x.round()
+    return x.to(torch.bfloat16).cuda()
+
+
+@pytest.mark.parametrize("vocab", [8_192, 50_257, 65_543, 151_936])
+@pytest.mark.parametrize("kind", ["usual", "few values", "masked"])
+def test_a_counted_row_is_the_same_in_any_number_of_parts(kind, vocab):
+    """The token too: it is the n-th member of a class whichever part holds it, and the same whether the
+    class is looked up in the parts' lists or looked for in the whole row (rows off the 16-byte grid have
+    members ahead of the first part)."""
+    batch = 16
+    room = torch.zeros((batch, vocab + 8 - vocab % 8), dtype=torch.bfloat16, device="cuda")
+    logits = room[:, :vocab]  # (every row starts on a boundary; below, none does)
+    logits.copy_(_rows(kind, batch, vocab))
+    odd = torch.zeros((batch, room.shape[1] + 8), dtype=torch.bfloat16, device="cuda")[:, 3:3 + vocab]
+    odd.copy_(logits)
+    params = [SamplingParams(temperature=(0.4, 1.0, 1.4)[i % 3], top_p=(0.95, 0.7, 1.0)[i // 6], min_p=(0.0, 0.01)[i % 2], seed=11 * i + 1,
+                             **(dict(repetition_penalty=1.1, frequency_penalty=0.2) if i % 4 else {})) for i in range(batch)]
+    histories = [[(31 * j * j + i) % vocab for j in range(200 * i)] for i in range(batch)]
+    s = _sampler(vocab, batch)
+    try:
+        with s.lock:
+            slots = s.plan_slots(histories, params, vocab)
+            for step in range(4):
+                rec = _device.pack_params(params, [step] * batch, slots)
+                s.set_count_split(1)
+                want, _ = s.run(logits, rec)
+                general, _ = s.run(logits, rec, general=True)
+                for name in COUNTS:
+                    np.testing.assert_array_equal(want[name], general[name], err_msg=f"{name}, against the general kernel")
+                for split in (2, 4, 0):
+                    s.set_count_split(split)
+                    for rows in (logits, odd):
+                        got, _ = s.run(rows, rec)
+                        for name in (*COUNTS, "token"):
+                            np.testing.assert_array_equal(got[name], want[name], err_msg=f"{name}, {split} parts")
+        # (a step knows which rows count, and cuts them as it sees fit)
+        s.set_count_split(0)
+        got = s.step(odd, histories, params, [3] * batch)
+        assert [x.token_id for x in got] == want["token"].tolist()
+    finally:
+        s.close()
