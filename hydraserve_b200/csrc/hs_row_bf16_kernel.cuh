@@ -146,7 +146,8 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
   if (tid < 64) small[tid] = (tid >= 19 && tid <= 22) ? -1 : 0;
   if (tid == 0) c.x()->bcast[5] = 0;  // highest side element, (key, ~id)
   __syncthreads();
-  for (int i = tid; i < kCells; i += kThreads) c.tab()[i] = 0;
+  for (int i = tid; i < kCells / 4; i += kThreads) reinterpret_cast<uint4*>(c.tab())[i] = make_uint4(0u, 0u, 0u, 0u);
+  cudaGridDependencySynchronize();  // (the histograms are up to date from here on)
   __syncthreads();
   // ---- A. the one read of the row from HBM: count tokens per (count class, value) --------
   {
@@ -545,7 +546,6 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel_bf16(const __grid_cons
   if (threadIdx.x == 0) P = row_params(args.base, inl, row);
   __syncthreads();
   if (is_candidate_row(P, args.base.vocab) == count) return;  // the other path's row
-  cudaGridDependencySynchronize();  // (the histograms are up to date from here on)
   if (threadIdx.x < sizeof(hs_row_out) / 4) reinterpret_cast<uint32_t*>(&record)[threadIdx.x] = 0u;
   __syncthreads();
   // (tuning aid: when each item started and ended, in ns of the global timer, slots 48.. of its row)

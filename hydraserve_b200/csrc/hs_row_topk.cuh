@@ -271,13 +271,20 @@ struct SampleRegs {
   uint4 w[kSampleGroups];
   uint32_t cl[kSampleGroups];
 };
-// Starts the loads of the sample (nothing waits for them here).
-__device__ __forceinline__ void sample_fetch(const Ctx3& c, SampleRegs& r) {
+// Starts the loads of the sample's values, and of its count classes (nothing waits for them here).
+__device__ __forceinline__ void sample_values(const Ctx3& c, SampleRegs& r) {
   const uint4* src4 = c.chunks();
 #pragma unroll
   for (int u = 0; u < kSampleGroups; ++u) {
     const int i = c.chunk_lo + threadIdx.x + u * kThreads;
-    if (i < c.chunk_hi) { r.w[u] = __ldcg(src4 + i); r.cl[u] = c.cls ? c.chunk_classes(i) : 0u; }
+    if (i < c.chunk_hi) r.w[u] = __ldcg(src4 + i);
+  }
+}
+__device__ __forceinline__ void sample_classes(const Ctx3& c, SampleRegs& r) {
+#pragma unroll
+  for (int u = 0; u < kSampleGroups; ++u) {
+    const int i = c.chunk_lo + threadIdx.x + u * kThreads;
+    if (i < c.chunk_hi) r.cl[u] = c.cls ? c.chunk_classes(i) : 0u;
   }
 }
 __device__ int sample_kth_t16(const Ctx3& c, CandCtx& L, int k, const SampleRegs& r) {
@@ -379,13 +386,17 @@ __device__ int topk_candidates(Ctx3& c, CandCtx& L, int k) {
   // The chain heavy -> pairs -> logits is three dependent reads; it is started for list entry
   // `tid` before the sample is fetched and worked off between the sample's steps, so that
   // the waits overlap.
+  SampleRegs sample;
+  sample_values(c, sample);
+  // (the histograms are up to date from here on: the values do not depend on them, so their loads cross the
+  // end of the kernel that counts the new tokens; one row of 151,936 48.7 -> 47.9 us a call)
+  cudaGridDependencySynchronize();
   int n_heavy = 0, hv_q = -1;
   if (c.cls) {
     n_heavy = load_now_s32(c.pool.n_heavy + c.slot);
     if (tid < c.pool.unique_cap) hv_q = load_now_s32(c.pool.heavy + (size_t)c.slot * c.pool.unique_cap + tid);
   }
-  SampleRegs sample;
-  sample_fetch(c, sample);
+  sample_classes(c, sample);
   n_heavy = min(n_heavy, c.pool.unique_cap);
   const int2* pairs = c.pool.pairs + (size_t)c.slot * c.pool.unique_cap;
   int2 hv_pair = make_int2(-1, 0);
@@ -626,7 +637,7 @@ __device__ FinishOut finish_impl(Exchange& x, const u64* cand, u64* mass, int n,
   r.cut_ties = -1;
   if (P.top_p < 1.0f) {
     const u64 z2 = mass[n1 - 1];
-    const u64 target = top_p_target(z2, P.top_p);
+    const u64 target = top_p_target_warp(z2, P.top_p);
     u64 below = 0;
     for (int i = tid; i < n1; i += kLanes) below += mass[i] < target ? 1 : 0;
     n2 = min(n1, (int)sum(below) + 1);
