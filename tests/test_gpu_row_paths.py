@@ -77,3 +77,18 @@ def test_a_counted_row_is_the_same_in_any_number_of_parts(kind, vocab):
         assert [x.token_id for x in got] == want["token"].tolist()
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("vocab", [1, 9, 31, 5_003, 50_257])
+def test_greedy_rows_off_the_16_byte_grid(dtype, vocab):
+    for offset in range(8):
+        room = torch.full((5, vocab + 16), 3.0e4, dtype=dtype, device="cuda")  # (what lies outside a row must not count)
+        rows = room[:, offset:offset + vocab]
+        rows.copy_(torch.randn(5, vocab, generator=torch.Generator().manual_seed(offset)).to(dtype))
+        rows[1] = 0.5                 # (the lowest id of a tie)
+        rows[2, vocab - 1] = 9.0      # (the last token; the first)
+        rows[3, 0] = 9.0
+        got = sample_logits(rows, [[]] * 5, [SamplingParams()] * 5, steps=[0] * 5)
+        want = [int((r == r.max()).nonzero()[0]) for r in rows.float().cpu()]
+        assert [x.token_id for x in got] == want, offset
