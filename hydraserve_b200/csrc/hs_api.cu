@@ -121,7 +121,11 @@ struct hs_sampler {
   void *h_block_own = nullptr, *d_block_own = nullptr;
   hs_row_out* h_out = nullptr;    // [batch_max]
   int32_t* h_tokens = nullptr;    // [batch_max]
-  std::atomic<int> awaited_ids{0}, awaited_records{0};  // on their way into h_tokens and h_out
+  volatile u64* h_mail = nullptr;  // [batch_max, kRecordWords] a record's words as they arrive, each under its step's tag
+  uint32_t mail_tag = 0;           // of the last hs_step
+  bool mail_only = false;          // its records are nowhere else
+  std::vector<uint8_t> mail_words; // [batch_max] words of each row's record of that step
+  std::atomic<int> awaited_ids{0}, awaited_records{0};  // on their way into h_tokens and h_mail
   std::mutex mu;         // the staging buffers of hs_sample_host
   // Every launching call takes launch_mu, and work of one call is ordered after the previous
   // call's on the GPU (an event when the stream changed), because all calls share the
@@ -276,12 +280,14 @@ const hs::InlineRows kNoInlineRows{};  // (stands in when the parameters are in 
 // this one on the stream is one of this sampler's histogram kernels.
 int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
                 const hs_row_params* params, const hs::InlineRows& inl, int n_count, hs_row_out* out, const float* noise,
-                float* scores_out, int32_t* tokens_out, uint32_t flags, bool behind, cudaStream_t stream) {
+                float* scores_out, int32_t* tokens_out, uint32_t flags, bool behind, cudaStream_t stream, bool mailed = false) {
   Plan plan;
   hs::RowKernelArgs a{};
   a.logits = logits; a.dtype = dtype; a.row_stride = row_stride; a.vocab = vocab; a.slice = 0;
   a.params = params; a.out = out; a.noise = noise; a.scores_out = scores_out; a.gstage = nullptr;
-  a.pool = h->pool; a.flags = flags & (HS_SAMPLE_APPEND_TOKEN | hs::kHostWaits); a.tokens_out = tokens_out;
+  a.pool = h->pool; a.flags = flags & HS_SAMPLE_APPEND_TOKEN; a.tokens_out = tokens_out;
+  a.mail = mailed ? reinterpret_cast<ulonglong2*>(const_cast<u64*>(h->h_mail)) : nullptr;
+  a.mail_tag = h->mail_tag;
   a.token_draw = h->token_draw;
   if (dtype == HS_DTYPE_BF16 && !h->force_general && !(flags & HS_SAMPLE_GENERAL_KERNEL)) {
     // One launch: the parts of the counting rows, then the parts of the candidate rows, two CTAs
@@ -581,18 +587,22 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
   bool ok = held.allocate(h);
   ok = ok && cudaEventCreateWithFlags(&h->ev_done, cudaEventDisableTiming) == cudaSuccess;
   if (ok) {
-    const size_t sizes[5] = {(size_t)batch_max * sizeof(hs_row_params), (2 * (size_t)batch_max + 1) * sizeof(int32_t),
-                             (size_t)batch_max * sizeof(hs_row_out), (size_t)batch_max * sizeof(int32_t), first_block};
-    size_t at[6] = {0};
-    for (int i = 0; i < 5; ++i) at[i + 1] = (at[i] + sizes[i] + 255) & ~size_t(255);
-    ok = cudaMallocHost(&h->h_held, at[5]) == cudaSuccess;
+    const size_t mail_bytes = (size_t)batch_max * hs::kRecordWords * sizeof(u64);
+    const size_t sizes[6] = {(size_t)batch_max * sizeof(hs_row_params), (2 * (size_t)batch_max + 1) * sizeof(int32_t),
+                             (size_t)batch_max * sizeof(hs_row_out), (size_t)batch_max * sizeof(int32_t), mail_bytes, first_block};
+    size_t at[7] = {0};
+    for (int i = 0; i < 6; ++i) at[i + 1] = (at[i] + sizes[i] + 255) & ~size_t(255);
+    ok = cudaMallocHost(&h->h_held, at[6]) == cudaSuccess;
     if (ok) {
       unsigned char* base = static_cast<unsigned char*>(h->h_held);
       h->h_params = reinterpret_cast<hs_row_params*>(base);
       h->h_small = reinterpret_cast<int32_t*>(base + at[1]);
       h->h_out = reinterpret_cast<hs_row_out*>(base + at[2]);
       h->h_tokens = reinterpret_cast<int32_t*>(base + at[3]);
-      h->h_block = base + at[4];
+      h->h_mail = reinterpret_cast<u64*>(base + at[4]);
+      std::memset(base + at[4], 0, mail_bytes);
+      h->mail_words.assign((size_t)batch_max, 0);
+      h->h_block = base + at[5];
       h->h_block_bytes = h->d_block_bytes = first_block;
     }
   }
@@ -810,6 +820,7 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
   if (!d || !out) return fail(h, HS_ERR_INVALID, "desc / out is null");
   *out = nullptr;
   nothing_awaited(h);
+  const bool repeats = (d->repeats & ~HS_STEP_WILL_WAIT) != 0;
   if (batch == 0) return HS_OK;
   if (row_stride < vocab) return fail(h, HS_ERR_INVALID, "row_stride smaller than vocab");
   if (d->n_resets < 0 || d->n_appends < 0 || d->n_appends > 65535 || d->n_resets > 65535)
@@ -824,14 +835,21 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
   HS_CUDA(h, serial.status);
 
   *out = h->h_out;
-  for (int r = 0; r < batch; ++r) h->h_out[r].status = hs::kNoStatus;
+  h->mail_only = (d->repeats & HS_STEP_WILL_WAIT) != 0;
+  if (++h->mail_tag == 0) {
+    // (around once: no word may still stand under a tag that comes again)
+    HS_CUDA(h, cudaStreamSynchronize(stream));
+    std::memset(const_cast<u64*>(h->h_mail), 0, (size_t)h->batch_max * hs::kRecordWords * sizeof(u64));
+    h->mail_tag = 1;
+  }
 
   // What a small step brings along goes into the launches themselves: 64 rows' parameters (3 KB)
   // and 256 (slot, token) pairs (2 KB) are cheaper there than one copy ahead of the kernel
   // (about 3 us of host and GPU time); anything larger is copied in one piece.
   const auto* params = reinterpret_cast<const hs_row_params*>(h->h_block);
+  for (int r = 0; r < batch; ++r) h->mail_words[(size_t)r] = (uint8_t)(params[r].n_logprobs >= 0 ? hs::kRecordWords : hs::kBareWords);
   const bool counting = d->n_resets > 0 || d->n_appends > 0;
-  const bool singles = d->n_resets == 0 && d->n_appends > 0 && d->max_tokens == 1 && !d->repeats;
+  const bool singles = d->n_resets == 0 && d->n_appends > 0 && d->max_tokens == 1 && !repeats;
   // a slot that is emptied and then filled again is one entry of the build (the two lists are in
   // the same order); what is only emptied stays in the list of resets
   int n_alone = 0;
@@ -841,8 +859,8 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
     int j = 0;
     for (int i = 0; i < d->n_resets; ++i) {
       int k = j;
-      while (!d->repeats && k < d->n_appends && slots[k] != resets[i]) ++k;
-      if (!d->repeats && k < d->n_appends) { slots[k] |= hs::kResetFirst; j = k + 1; }
+      while (!repeats && k < d->n_appends && slots[k] != resets[i]) ++k;
+      if (!repeats && k < d->n_appends) { slots[k] |= hs::kResetFirst; j = k + 1; }
       else resets[n_alone++] = resets[i];
     }
   }
@@ -891,7 +909,7 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
       HS_CUDA(h, cudaGetLastError());
       h->launches += 1;
     }
-    if (d->n_appends && d->repeats) {
+    if (d->n_appends && repeats) {
       rc = launch_append(h, d_tokens, d_offsets, d_slots, d->n_appends, vocab, d->max_tokens, stream);
       if (rc != HS_OK) return rc;
     } else if (d->n_appends) {
@@ -907,10 +925,10 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
   }
   hs::InlineRows inl;
   if (rows_inline) std::memcpy(inl.p, params, (size_t)batch * sizeof(hs_row_params));
-  // (the records go straight to pinned memory, one burst per row: see write_record)
+  // (the records go straight to pinned memory: see write_record)
   rc = launch_rows(h, logits, dtype, row_stride, batch, vocab,
                    rows_inline ? nullptr : reinterpret_cast<const hs_row_params*>(h->d_block), rows_inline ? inl : kNoInlineRows,
-                   n_count_of(params, batch, vocab), h->h_out, nullptr, nullptr, nullptr, hs::kHostWaits, behind, stream);
+                   n_count_of(params, batch, vocab), h->mail_only ? nullptr : h->h_out, nullptr, nullptr, nullptr, 0u, behind, stream, true);
   if (rc != HS_OK) return rc;
   HS_CUDA(h, serial.done());
   h->awaited_records = batch;
@@ -919,13 +937,23 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
 
 int hs_step_wait(hs_sampler* h, void* stream) {
   if (!h) return HS_ERR_INVALID;
-  // A row's last store is one word in pinned memory (its id in a greedy step, else its record's
-  // status): they are there two microseconds before the stream reports its end.  (For as long as a
-  // large step takes; then, or if something went wrong, the stream has the word.)
+  // A greedy row's id is one word in pinned memory, any other row's record comes word by word (see
+  // write_record) and is put together here: all are there some microseconds before the stream reports
+  // its end.  (For as long as a large step takes; then, or if something went wrong, the stream has
+  // the word, and the records stand where the kernel wrote them in one piece.)
   const int ids = h->awaited_ids.exchange(0), records = h->awaited_records.exchange(0);
   auto there = [&](int row) {
-    return ids ? *reinterpret_cast<volatile int32_t*>(h->h_tokens + row) != kNoToken
-               : *reinterpret_cast<volatile int32_t*>(&h->h_out[row].status) != hs::kNoStatus;
+    if (ids) return *reinterpret_cast<volatile int32_t*>(h->h_tokens + row) != kNoToken;
+    const volatile u64* mail = h->h_mail + (size_t)row * hs::kRecordWords;
+    const int n = h->mail_words[(size_t)row];
+    uint32_t words[hs::kRecordWords];
+    for (int i = 0; i < n; ++i) {
+      const u64 w = mail[i];
+      if ((uint32_t)(w >> 32) != h->mail_tag) return false;
+      words[i] = (uint32_t)w;
+    }
+    std::memcpy(h->h_out + row, words, (size_t)n * 4);
+    return true;
   };
   const int n = ids + records;
   int seen = 0;
@@ -937,6 +965,9 @@ int hs_step_wait(hs_sampler* h, void* stream) {
   if (n > 0 && seen == n) return HS_OK;
   DeviceGuard guard(h->device);
   HS_CUDA(h, cudaStreamSynchronize((cudaStream_t)stream));
+  if (records && h->mail_only)
+    for (; seen < n; ++seen)
+      if (!there(seen)) return fail(h, HS_ERR_CUDA, "a step's records did not come");
   return HS_OK;
 }
 
@@ -1025,6 +1056,10 @@ int hs_debug_set(hs_sampler* h, int what, int value) {
   if (what == 1) {
     if (value != 0 && value != 1 && value != 2 && value != 4) return fail(h, HS_ERR_INVALID, "counting split must be 0, 1, 2 or 4");
     h->force_csplit = value;
+    return HS_OK;
+  }
+  if (what == 4) {
+    h->mail_tag = (uint32_t)value;
     return HS_OK;
   }
   if (what == 3) {

@@ -87,7 +87,9 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
     S.noise = a.noise;
     S.scores_out = a.scores_out;
     S.tokens_out = a.tokens_out;
-    S.out_row = a.out + row_index;
+    S.out_row = record_of(a, row_index);
+    S.mail_row = mail_of(a, row_index);
+    S.mail_tag = a.mail_tag;
     S.parts = part < 0 ? 1 : args.csplit;
     S.lists = args.ctab + (size_t)row_index * args.csplit * kCells;
     S.lens = args.crare_n + (size_t)row_index * args.csplit;
@@ -130,7 +132,7 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
       out->row_max = score_of((uint32_t)(best >> 32)); out->log_z = 0.f;
     }
     __syncthreads();
-    if (tid < 32) write_record(a.out + c.row, *out, false, a.flags);
+    if (tid < 32) write_record(record_of(a, c.row), *out, false, mail_of(a, c.row), a.mail_tag);
     return false;
   }
 
@@ -516,7 +518,7 @@ __device__ __forceinline__ bool cand_part(const RowV3Args& args, unsigned char* 
     }
   }
   __syncthreads();
-  if (tid < 32) write_record(a.out + c.row, *out, P.n_logprobs >= 0, a.flags);
+  if (tid < 32) write_record(record_of(a, c.row), *out, P.n_logprobs >= 0, mail_of(a, c.row), a.mail_tag);
   mark(8);
   return false;
 }

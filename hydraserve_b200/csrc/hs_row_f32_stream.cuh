@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel_f32_stream(const __gri
   if (*L.lost) {  // more ties than the list holds: the general kernel samples this row
     if (tid == 0) rec.status = 4;
     __syncthreads();
-    if (tid < 32) write_record(a.out + row, rec, false, a.flags);
+    if (tid < 32) write_record(record_of(a, row), rec, P.n_logprobs >= 0, mail_of(a, row), a.mail_tag);
     return;
   }
   int n = min(*L.n, kCandCap);
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel_f32_stream(const __gri
     write_finish(r, &rec);
   }
   __syncthreads();
-  if (tid < 32) write_record(a.out + row, rec, P.n_logprobs >= 0, a.flags);
+  if (tid < 32) write_record(record_of(a, row), rec, P.n_logprobs >= 0, mail_of(a, row), a.mail_tag);
 }
 
 }  // namespace hs

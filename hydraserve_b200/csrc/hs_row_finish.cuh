@@ -45,6 +45,8 @@ struct CountState {
   float* scores_out;
   int32_t* tokens_out;
   hs_row_out* out_row;
+  ulonglong2* mail_row;
+  uint32_t mail_tag;
   int parts;              // CTAs that counted the row; of several, each left a list of its classes
   const uint32_t* lists;  // [parts, kCells]
   const int2* lens;       // [parts]
@@ -970,7 +972,7 @@ __device__ __noinline__ bool finish_listed_row() {
     }
   }
   __syncthreads();
-  if (threadIdx.x < 32) write_record(S.out_row, S.out, S.P.n_logprobs >= 0, (uint32_t)S.flags);
+  if (threadIdx.x < 32) write_record(S.out_row, S.out, S.P.n_logprobs >= 0, S.mail_row, S.mail_tag);
   release_scratch(S);
   return true;
 }
@@ -983,7 +985,7 @@ __device__ __forceinline__ void finish_counted_row() {
   if (!phase_histogram()) {  // cannot happen while n_scratch covers the resident CTAs; fail the row, do not wait
     if (tid == 0) { S.out.token = 0; S.out.status = 128; S.out.n_top = 0; S.out.n_kept = 0; }
     __syncthreads();
-    if (tid < 32) write_record(S.out_row, S.out, false, (uint32_t)S.flags);
+    if (tid < 32) write_record(S.out_row, S.out, S.P.n_logprobs >= 0, S.mail_row, S.mail_tag);
     return;
   }
   if (is_candidate_row(S.P, c.vocab) && finish_listed_row()) return;
@@ -1031,7 +1033,7 @@ __device__ __forceinline__ void finish_counted_row() {
     S.out.status = S.status;
   }
   __syncthreads();
-  if (tid < 32) write_record(S.out_row, S.out, S.P.n_logprobs >= 0, (uint32_t)S.flags);
+  if (tid < 32) write_record(S.out_row, S.out, S.P.n_logprobs >= 0, S.mail_row, S.mail_tag);
   release_scratch(S);
   phase_mark(S, 9);
 }

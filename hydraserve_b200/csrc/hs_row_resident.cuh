@@ -661,7 +661,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
   const int argmax_id = (int)(~(uint32_t)(best & 0xffffffffu));
   const float m = score_of(max_key);
   int status = P.slot >= a.pool.slots_total ? 64 : 0;  // a slot this sampler does not have: no penalties
-  hs_row_out* out = a.out + c.row;
+  hs_row_out* out = record_of(a, c.row);
 
   // ---- C. rows with a small top_k -----------------------------------------------------
   if (candidate) {
@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
         }
       }
       __syncthreads();
-      if (tid < 32) write_record(out, record, P.n_logprobs >= 0, a.flags);
+      if (tid < 32) write_record(out, record, P.n_logprobs >= 0, mail_of(a, c.row), a.mail_tag);
       return;
     }
     // more ties at the k-th value than a list holds: in token order, like any other row
@@ -957,7 +957,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
       }
     }
     __syncthreads();
-    if (tid < 32) write_record(out, record, P.n_logprobs >= 0, a.flags);
+    if (tid < 32) write_record(out, record, P.n_logprobs >= 0, mail_of(a, c.row), a.mail_tag);
   }
   // No CTA may leave while a peer can still read its shared memory.
   c.sync_all();

@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(kThreads, 2) shard_merge_kernel(const MergeArg
   if (n == 0) {
     if (tid == 0) rec.status = status | 1;
     __syncthreads();
-    if (tid < 32) write_record(a.out + row, rec, false, 0u);
+    if (tid < 32) write_record(a.out + row, rec, false);
     return;
   }
   const int k = P.top_k > 0 ? P.top_k : n;
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(kThreads, 2) shard_merge_kernel(const MergeArg
   r.status |= status;
   if (tid == 0) write_finish(r, &rec);
   __syncthreads();
-  if (tid < 32) write_record(a.out + row, rec, P.n_logprobs >= 0, 0u);
+  if (tid < 32) write_record(a.out + row, rec, P.n_logprobs >= 0);
   if (tid == 0) {
     if (a.full_lse) {
       // log sum exp over the whole vocabulary from the slices' (max, denominator) pairs

@@ -197,10 +197,13 @@ int hs_sample_host(hs_sampler* h, const void* logits, int dtype, int64_t row_str
  *                   in); int32 reset_slots[n_resets] at resets_at; and for the tokens to count
  *                   int32 slots[n_appends] at slots_at, int32 offsets[n_appends + 1] at offsets_at,
  *                   int32 tokens[] at tokens_at, as hs_slots_append takes them (sections 16-byte
- *                   aligned; bytes = end of the last one; repeats = 1 when a slot is listed twice)
+ *                   aligned; bytes = end of the last one; repeats = 1 when a slot is listed twice, and
+ *                   HS_STEP_WILL_WAIT beside it when the caller is going to call hs_step_wait: the
+ *                   records are then written where that call looks for them and nowhere else)
  * A record's top_ids / top_logprobs are written on rows with n_logprobs >= 0 only.
  * The block and the records belong to one step at a time: the caller serialises
  * hs_step_block .. hs_step .. hs_step_wait .. reading the records against other steps of the same sampler. */
+#define HS_STEP_WILL_WAIT (1 << 30)
 typedef struct hs_step_desc {
   size_t bytes, resets_at, slots_at, offsets_at, tokens_at;
   int32_t n_resets, n_appends, max_tokens, repeats;
@@ -264,7 +267,7 @@ int hs_query(hs_sampler* h, int what, int vocab, int dtype);
 int hs_debug_phase_clocks(hs_sampler* h, int batch, unsigned long long* out_host);
 /* Tests and tuning.  what = 0: CTAs per candidate row, what = 1: CTAs per counting row; value 1, 2
  * or 4 (0 = chosen per call).  what = 3: near-flat counting rows draw by rejection on tokens
- * (1, the default) or always class by class (0). */
+ * (1, the default) or always class by class (0).  what = 4: the tag of the last step's mail. */
 int hs_debug_set(hs_sampler* h, int what, int value);
 
 #ifdef __cplusplus

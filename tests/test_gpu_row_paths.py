@@ -92,3 +92,22 @@ def test_greedy_rows_off_the_16_byte_grid(dtype, vocab):
         got = sample_logits(rows, [[]] * 5, [SamplingParams()] * 5, steps=[0] * 5)
         want = [int((r == r.max()).nonzero()[0]) for r in rows.float().cpu()]
         assert [x.token_id for x in got] == want, offset
+
+
+def test_mail_of_another_step_is_not_taken_for_this_one():
+    """Rows with and without log-probabilities in turn, so that words of older steps stand in the mail;
+    and the tags' way around: the step behind the last tag starts over with clean mail."""
+    vocab, batch = 4_096, 6
+    logits = _rows("usual", batch, vocab)
+    s = _sampler(vocab, batch)
+    try:
+        for step, first in enumerate((None, 0xfffffffd, None, None, None, None)):
+            if first is not None:
+                _lib.check(s.lib, s.handle, s.lib.hs_debug_set(s.handle, 4, C.c_int(first - 2**32)), "hs_debug_set")
+            params = [SamplingParams(temperature=1.0, top_k=(0, 40)[i % 2], seed=step * 10 + i, logprobs=3 if (i + step) % 2 else None)
+                      for i in range(batch)]
+            got = s.step(logits, [[]] * batch, params, [step] * batch)
+            want, _ = s.sample(logits, [[]] * batch, params, [step] * batch)
+            assert got == _device.records_to_samples(want, params, vocab)
+    finally:
+        s.close()
