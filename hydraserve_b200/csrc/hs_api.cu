@@ -30,7 +30,7 @@ namespace {
 
 using hs::u64;
 
-constexpr int kMaxParts = 16;  // CTAs per counting row
+constexpr int kMaxParts = 16;  // CTAs per counting row the hand-over can deal with
 constexpr int kMaxSplit = 8;   // CTAs per candidate row: the parts' lists, top_k entries and ties each, meet in one list
 constexpr int32_t kNoToken = -1;  // where a greedy step's id will stand
 constexpr int kSideCapMax = 16384;  // side-list entries a CTA can keep in global scratch
@@ -292,24 +292,28 @@ int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride
   if (dtype == HS_DTYPE_BF16 && !h->force_general && !(flags & HS_SAMPLE_GENERAL_KERNEL)) {
     // One launch: the parts of the counting rows, then the parts of the candidate rows, two CTAs
     // resident per SM.  How many rows take which path is known when the parameters come from the
-    // host (n_count >= 0).  Then counting rows, whose last part has a long chain of selections
-    // ahead of it, are cut into as many parts (up to sixteen) as three quarters of a wave hold, into
-    // two as long as that is one wave; candidate rows into what the wave has left, up to eight
-    // (a second, partial wave costs more than idle SMs in the first).  No part is below 8,192 tokens
-    // (16,384, its bound's sample, for a candidate row): shorter ones end with the hand-over.
-    // When the host does not know, every row may be either: four parts or two, as the hand-over
-    // scratch allows, and a wave of candidate parts.
+    // host (n_count >= 0).  Counting goes at the rate of an SM's shared atomics, so two counting CTAs on
+    // one gain nothing: the rows are cut into as many parts as give every SM one, eight at most and
+    // none below 32,768 tokens; and not at all when that makes less than four of them, because the
+    // hand-over then costs what the shorter count saves (us a call, whole rows / 2 / 4 parts: 64 rows of
+    // 151,936 82.3 / 91.2 / 81.7, 100 rows 93.5 / 104.3 / -, one row of 50,257 53.7 / 58.7 / 57.9; one
+    // row of 248,320 in 4 / 8 / 12 / 16 parts 89.2 / 85.5 / 88.7 / 93.5).  Candidate rows get what the wave
+    // has left, up to eight CTAs each (a second, partial wave costs more than idle SMs in the first), none
+    // below 16,384 tokens, its bound's sample.
+    // When the host does not know, every row may be either: four parts as far as the hand-over
+    // scratch goes, else whole rows (256 rows of 248,320, half of them counting: 61.9 us a step, 66.0 in two
+    // parts), and a wave of candidate parts.
     const int resident = h->resident_bf16;
     const bool known = n_count >= 0;
     int csplit, split;
     if (known) {
       const int n_cand = batch - n_count;
-      csplit = std::max(resident * 3 / 4 / std::max(1, n_count), 2 * n_count <= resident ? 2 : 1);
-      csplit = std::max(1, std::min({csplit, kMaxParts, vocab / 8192}));
+      csplit = std::min({h->sm_count / std::max(1, n_count), 8, vocab / 32768});
+      if (csplit < 4) csplit = 1;
       split = (resident - std::min(resident, n_count * csplit)) / std::max(1, n_cand);
       split = std::max(1, std::min({split, kMaxSplit, vocab / hs::kSample}));
     } else {
-      csplit = vocab < 65536 ? 1 : (long long)batch * 4 <= h->ctab_tables ? 4 : 2;
+      csplit = vocab < 65536 || (long long)batch * 4 > h->ctab_tables ? 1 : 4;
       split = std::max(1, std::min({resident / batch, 4, vocab / (2 * hs::kSample)}));
     }
     if (h->force_csplit) csplit = h->force_csplit;
@@ -1054,7 +1058,7 @@ int hs_debug_set(hs_sampler* h, int what, int value) {
     return HS_OK;
   }
   if (what == 1) {
-    if (value != 0 && value != 1 && value != 2 && value != 4) return fail(h, HS_ERR_INVALID, "counting split must be 0, 1, 2 or 4");
+    if (value < 0 || value > kMaxParts) return fail(h, HS_ERR_INVALID, "counting split must be 0 to 16");
     h->force_csplit = value;
     return HS_OK;
   }
