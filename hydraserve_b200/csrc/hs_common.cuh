@@ -166,6 +166,18 @@ __device__ __forceinline__ u64 block_max_u64(Exchange& x, u64 v) {
   __syncthreads();
   return warp_max_u64(lane < kWarps ? x.warp_a[lane] : 0ull);
 }
+// Lowest and highest value over the CTA, for every thread.  Two barriers.
+__device__ __forceinline__ void block_ends_u32(Exchange& x, uint32_t& lo, uint32_t& hi) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = warp_max_u32(hi);
+  __syncthreads();
+  if (lane == 0) { x.warp_a[warp] = lo; x.warp_b[warp] = hi; }
+  __syncthreads();
+  const uint32_t l = lane < kWarps ? (uint32_t)x.warp_a[lane] : 0xffffffffu, h = lane < kWarps ? (uint32_t)x.warp_b[lane] : 0u;
+  lo = __reduce_min_sync(0xffffffffu, l);
+  hi = warp_max_u32(h);
+}
 // Exclusive prefix of (a, b) over the warps of the CTA, given per-warp totals held by
 // every lane of each warp; also returns the CTA totals.  Two barriers.
 __device__ __forceinline__ void block_warp_prefix2(Exchange& x, u64 wa, u64 wb, u64& pre_a,

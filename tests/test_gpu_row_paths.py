@@ -39,6 +39,33 @@ def _rows(kind, batch, vocab, seed=0):
     return x.to(torch.bfloat16).cuda()
 
 
+# 16,384 tokens are the bound's sample and a batch of the stream, two of which are on their way at once
+@pytest.mark.parametrize("vocab", [1, 7, 300, 4_096, 4_104, 16_384, 16_392, 32_768, 32_776, 36_864, 65_541, 151_936])
+@pytest.mark.parametrize("kind", ["usual", "masked", "lowest", "wide", "few values"])
+def test_small_top_k_rows_match_the_general_kernel(kind, vocab):
+    """Both kernels finish such a row from its sorted candidates: the whole record is the same."""
+    batch = 12
+    logits = _rows(kind, batch, vocab)
+    params = [SamplingParams(temperature=(0.7, 1.0, 1.3)[i % 3], top_k=min((1, 20, 50, 256)[i % 4], max(1, vocab - 1)), seed=i + 1, logprobs=5,
+                             top_p=(1.0, 0.9)[i % 2], min_p=(0.0, 0.02)[i // 6],
+                             **(dict(repetition_penalty=(1.2, 0.8)[i // 6], presence_penalty=0.5, frequency_penalty=0.3) if i % 5 else {}))
+              for i in range(batch)]
+    histories = [[(37 * j * j) % vocab for j in range(40 * i)] for i in range(batch)]
+    s = _sampler(vocab, batch)
+    try:
+        with s.lock:
+            slots = s.plan_slots(histories, params, vocab)
+            rec = _device.pack_params(params, [2] * batch, slots)
+            want, _ = s.run(logits, rec, general=True)
+            for split in (0, 1, 2, 4):
+                s.set_split(split)
+                got, _ = s.run(logits, rec)
+                for name in (*COUNTS, "token", "logprob", "n_top", "top_ids", "top_logprobs"):
+                    np.testing.assert_array_equal(got[name], want[name], err_msg=f"{name}, {split} parts")
+    finally:
+        s.close()
+
+
 @pytest.mark.parametrize("vocab", [8_192, 50_257, 65_543, 151_936])
 @pytest.mark.parametrize("kind", ["usual", "few values", "masked"])
 def test_a_counted_row_is_the_same_in_any_number_of_parts(kind, vocab):
