@@ -92,13 +92,10 @@ __device__ bool claim_scratch(CountState& S) {
 // fetching of its instructions: one copy of each function, loops that are not unrolled.
 __device__ __forceinline__ void hist_add(uint32_t* hist, int b, uint32_t cnt, u64 mass) {
   atomicAdd(hist + b, cnt);
-  const uint32_t a0 = (uint32_t)mass & kLimbMask, a1 = (uint32_t)(mass >> kLimbBits) & kLimbMask, a2 = (uint32_t)(mass >> (2 * kLimbBits));
-  if (a0) atomicAdd(hist + kV3Buckets + b, a0);
-  if (a1) atomicAdd(hist + 2 * kV3Buckets + b, a1);
-  if (a2) atomicAdd(hist + 3 * kV3Buckets + b, a2);
+  shared_add_u64(hist + kV3Buckets + b, hist + 2 * kV3Buckets + b, mass);
 }
 __device__ __forceinline__ u64 hist_mass(const uint32_t* hist, int b) {
-  return (u64)hist[kV3Buckets + b] + ((u64)hist[2 * kV3Buckets + b] << kLimbBits) + ((u64)hist[3 * kV3Buckets + b] << (2 * kLimbBits));
+  return (u64)hist[kV3Buckets + b] | ((u64)hist[2 * kV3Buckets + b] << 32);
 }
 // The histogram of count and mass: of every token (side elements one by one, classes with their
 // count), or (side_ids) of the kept side elements keyed by ~id.  The thousands of values next to
@@ -110,7 +107,7 @@ __device__ __noinline__ void fill_hist(const V3Map map, bool side_ids) {
   uint32_t* hist = c.hist();
   const float m = c.m;
 #pragma unroll
-  for (int b = 0; b < 4 * kV3Buckets / kThreads; ++b) hist[threadIdx.x + b * kThreads] = 0;
+  for (int b = 0; b < 3 * kV3Buckets / kThreads; ++b) hist[threadIdx.x + b * kThreads] = 0;
   __syncthreads();
   const uint32_t cut_key = S.kept.cut_key;
   for_each_side3(c, [&](int id, float s) {
@@ -567,10 +564,10 @@ __device__ __noinline__ void draw_by_classes(uint64_t seed) {
 #pragma unroll
     for (int u = 0; u < kPerClass; ++u) mine += tab[tid + (k * kPerClass + u) * kThreads] ? 1 : 0;
   }
-  uint32_t* chunks = reinterpret_cast<uint32_t*>(c.members());  // [3][kThreads]: mass in limbs
-  static_assert(3 * kThreads * sizeof(uint32_t) <= sizeof(V3Member) * kV3ListCap + sizeof(int) * kV3TieCap, "the chunks fit the members' place");
+  uint32_t* chunks = reinterpret_cast<uint32_t*>(c.members());  // [2][kThreads]: mass, low and high words
+  static_assert(2 * kThreads * sizeof(uint32_t) <= sizeof(V3Member) * kV3ListCap + sizeof(int) * kV3TieCap, "the chunks fit the members' place");
 #pragma unroll
-  for (int l = 0; l < 3; ++l) chunks[tid + l * kThreads] = 0;
+  for (int l = 0; l < 2; ++l) chunks[tid + l * kThreads] = 0;
   int n_cl;
   const int list_at = block_place(count_small() + 48, mine, n_cl);
   {
@@ -592,15 +589,13 @@ __device__ __noinline__ void draw_by_classes(uint64_t seed) {
         const int cell = tid + (k * kPerClass + u) * kThreads;
         const u64 w = (u64)tab[cell] * mass_of(sc.bin_score(cell - k * kV3Bins, k), m);
         uint32_t* dst = chunks + ((from + __popc(bits & ((1u << u) - 1u))) & (kThreads - 1));
-        atomicAdd(dst, (uint32_t)w & kLimbMask);
-        atomicAdd(dst + kThreads, (uint32_t)(w >> kLimbBits) & kLimbMask);
-        atomicAdd(dst + 2 * kThreads, (uint32_t)(w >> (2 * kLimbBits)));
+        shared_add_u64(dst, dst + kThreads, w);
       }
       from += __popc(bits);
     }
   }
   __syncthreads();
-  const u64 chunk = (u64)chunks[tid] + ((u64)chunks[tid + kThreads] << kLimbBits) + ((u64)chunks[tid + 2 * kThreads] << (2 * kLimbBits));
+  const u64 chunk = (u64)chunks[tid] | ((u64)chunks[tid + kThreads] << 32);
   const u64 incl = warp_scan_u64(chunk);
   u64 pre, pre_unused, q_cells, tot_unused;
   block_warp_prefix2(*c.x(), shfl_u64(incl, 31), 0, pre, pre_unused, q_cells, tot_unused);

@@ -16,7 +16,7 @@
 // are gathered from all slices, sorted, and the cut is read off exactly.  The draw is an inverse
 // CDF in token order: a thread adds up a contiguous run of the slice, and one warp looks into the
 // run that holds the target.  What bounds it: shared-memory atomics and exponentials of the
-// histogram (about 3.3 atomics and 45 instructions per token), then cluster barriers; with eight
+// histogram (about two atomics and 40 instructions per token), then cluster barriers; with eight
 // CTAs a row, two per SM, 32 rows of 151,936 are one wave.  With top_p over all tokens they take 56 us
 // (113 us by radix descents, several passes a cut); four rows with top_k 50 24 us (72 us).
 // A bucket with more members than a list holds (a row of few values) is resolved by radix
@@ -247,16 +247,13 @@ struct BucketHit {
 __device__ void res_histogram(RowCtx& c, const ResHist& rh, float m, u64 (&seg)[2]) {
   uint32_t* cnt = reinterpret_cast<uint32_t*>(c.hist);
   const int tid = threadIdx.x;
-  for (int b = tid; b < 4 * kResBuckets; b += kThreads) cnt[b] = 0;
+  for (int b = tid; b < 3 * kResBuckets; b += kThreads) cnt[b] = 0;
   __syncthreads();
   auto take = [&](float s) {
     const int b = rh.bucket(s);
     atomicAdd(&cnt[b], 1u);
     const u64 q = mass_of(s, m);  // (0 from 28.4 below the maximum on)
-    const uint32_t a0 = (uint32_t)q & kLimbMask, a1 = (uint32_t)(q >> kLimbBits) & kLimbMask, a2 = (uint32_t)(q >> (2 * kLimbBits));
-    if (a0) atomicAdd(&cnt[kResBuckets + b], a0);
-    if (a1) atomicAdd(&cnt[2 * kResBuckets + b], a1);
-    if (a2) atomicAdd(&cnt[3 * kResBuckets + b], a2);
+    shared_add_u64(&cnt[kResBuckets + b], &cnt[2 * kResBuckets + b], q);
   };
   int i = tid;
   for (; i + 3 * kThreads < c.n_local; i += 4 * kThreads) {
@@ -279,8 +276,7 @@ __device__ void res_histogram(RowCtx& c, const ResHist& rh, float m, u64 (&seg)[
       if (r >= c.nranks) break;
       const uint32_t* h = c.nranks > 1 ? c.cluster.map_shared_rank(cnt, r) : cnt;
       n += h[gb];
-      q += (u64)h[kResBuckets + gb] + ((u64)h[2 * kResBuckets + gb] << kLimbBits) +
-           ((u64)h[3 * kResBuckets + gb] << (2 * kLimbBits));
+      q += (u64)h[kResBuckets + gb] | ((u64)h[2 * kResBuckets + gb] << 32);
     }
     c.red_cnt[b] = n;
     c.red_mass[b] = q;

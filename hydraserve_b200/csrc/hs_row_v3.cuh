@@ -114,7 +114,7 @@ __host__ __device__ constexpr LayoutV3 layout_v3() {
   l.rare = l.staged;
   l.defer = l.rare + sizeof(int2) * kV3RareCap;
   l.hist = l.staged;
-  l.members = l.hist + sizeof(uint32_t) * 4 * kV3Buckets;
+  l.members = l.hist + sizeof(uint32_t) * 3 * kV3Buckets;
   l.list = l.members + sizeof(V3Member) * kV3ListCap;
   l.small = take(sizeof(int) * 64);
   l.total = off;
@@ -123,7 +123,7 @@ __host__ __device__ constexpr LayoutV3 layout_v3() {
 constexpr LayoutV3 kLayV3 = layout_v3();
 constexpr int kPerClass = kV3Bins / kThreads;  // a thread's cells tid + u * kThreads: count class u / kPerClass
 static_assert(kV3Bins % kThreads == 0, "a thread's u-th cell has the same count class for all threads");
-static_assert(sizeof(uint32_t) * (4 * kV3Buckets + kV3TieCap) + sizeof(V3Member) * kV3ListCap <= sizeof(uint32_t) * kV3Staged &&
+static_assert(sizeof(uint32_t) * (3 * kV3Buckets + kV3TieCap) + sizeof(V3Member) * kV3ListCap <= sizeof(uint32_t) * kV3Staged &&
               sizeof(int2) * kV3RareCap + sizeof(int) * kV3DeferCap <= sizeof(uint32_t) * kV3Staged,
               "the two uses fit the shared place");
 
@@ -176,7 +176,7 @@ struct Ctx3 : Scorer {
   // (places in shared memory; the block primitives' scratch comes first in every kernel's layout)
   __device__ __forceinline__ Exchange* x() const { return at_smem<0, Exchange>(); }
   __device__ __forceinline__ uint32_t* tab() const { return at_smem<kLayV3.tab, uint32_t>(); }     // [kCells] tokens per class
-  __device__ __forceinline__ uint32_t* hist() const { return at_smem<kLayV3.hist, uint32_t>(); }   // [4 * kV3Buckets] count, mass in three 14-bit limbs
+  __device__ __forceinline__ uint32_t* hist() const { return at_smem<kLayV3.hist, uint32_t>(); }   // [3 * kV3Buckets] count, mass as low and high words
   __device__ __forceinline__ V3Member* members() const { return at_smem<kLayV3.members, V3Member>(); }  // [kV3ListCap] of a selection's deciding bucket
   __device__ __forceinline__ V3Entry* gbuf() const { return at_smem<kLayV3.members, V3Entry>(); }  // [kV3ListCap] top-N tokens (in the same place)
   __device__ __forceinline__ int* list() const { return at_smem<kLayV3.list, int>(); }             // [kV3TieCap] token ids
