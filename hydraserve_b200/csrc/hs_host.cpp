@@ -1062,10 +1062,45 @@ PyObject* mod_plan(PyObject*, PyObject* args) {
   return PyTuple_Pack(3, out_slots.p, resets.p, appends.p);
 }
 // samples(records, params, vocabulary) -> tuple of TokenSample; records: a buffer of hs_row_out
-PyObject* mod_samples(PyObject*, PyObject* args) {
-  PyObject *records, *params_in;
+// Samples without their numbers, made while the GPU is at work (for a caller that does not use a Stepper).
+// They stay in a capsule until there are records to fill them from: nobody sees them half made.
+struct Blank {
+  PyObject* samples;
+  std::vector<int8_t> logprobs;
   int vocab;
-  if (!PyArg_ParseTuple(args, "OOi", &records, &params_in, &vocab)) return nullptr;
+};
+constexpr const char* kBlank = "hydraserve_b200._host.blank";
+void blank_free(PyObject* capsule) {
+  auto* b = static_cast<Blank*>(PyCapsule_GetPointer(capsule, kBlank));
+  if (!b) return;
+  Py_XDECREF(b->samples);
+  delete b;
+}
+// blank(params, vocab) -> a capsule for samples()
+PyObject* mod_blank(PyObject*, PyObject* args) {
+  PyObject* params_in;
+  int vocab;
+  if (!PyArg_ParseTuple(args, "Oi", &params_in, &vocab)) return nullptr;
+  Ref params(PySequence_Tuple(params_in));
+  if (!params) return nullptr;
+  const Py_ssize_t n = PyTuple_GET_SIZE(params.p);
+  const BatchRef b = batch_of(reinterpret_cast<PyTupleObject*>(params.p)->ob_item, n);
+  if (!b) return nullptr;
+  Ref made(blank_samples(n, b->logprobs.data(), vocab));
+  if (!made) return nullptr;
+  auto* blank = new Blank{made.take(), b->logprobs, vocab};
+  PyObject* capsule = PyCapsule_New(blank, kBlank, blank_free);
+  if (!capsule) {
+    Py_DECREF(blank->samples);
+    delete blank;
+  }
+  return capsule;
+}
+// samples(records, params, vocab[, blank]) -> the samples, the blank ones (which are used up) if they are of this batch
+PyObject* mod_samples(PyObject*, PyObject* args) {
+  PyObject *records, *params_in, *capsule = Py_None;
+  int vocab;
+  if (!PyArg_ParseTuple(args, "OOi|O", &records, &params_in, &vocab, &capsule)) return nullptr;
   Ref params(PySequence_Tuple(params_in));
   if (!params) return nullptr;
   const Py_ssize_t n = PyTuple_GET_SIZE(params.p);
@@ -1075,7 +1110,17 @@ PyObject* mod_samples(PyObject*, PyObject* args) {
   if (PyObject_GetBuffer(records, &view, PyBUF_C_CONTIGUOUS) < 0) return nullptr;
   PyObject* out = nullptr;
   if (view.len != n * (Py_ssize_t)sizeof(hs_row_out)) PyErr_SetString(PyExc_ValueError, "one record per row");
-  else out = samples_of(static_cast<const hs_row_out*>(view.buf), *b, vocab);
+  else {
+    const auto* rec = static_cast<const hs_row_out*>(view.buf);
+    auto* blank = capsule == Py_None ? nullptr : static_cast<Blank*>(PyCapsule_GetPointer(capsule, kBlank));
+    if (blank && blank->samples && blank->vocab == vocab && blank->logprobs == b->logprobs) {
+      Ref made(blank->samples);
+      blank->samples = nullptr;
+      out = filled_samples(made, rec, *b, vocab);
+    } else if (!PyErr_Occurred()) {
+      out = samples_of(rec, *b, vocab);
+    }
+  }
   PyBuffer_Release(&view);
   return out;
 }
@@ -1102,6 +1147,7 @@ PyMethodDef module_methods[] = {
     {"survey", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(mod_survey)), METH_FASTCALL, "-1 for an all plain-greedy batch, else the longest penalised history."},
     {"pack", mod_pack, METH_VARARGS, "hs_row_params of a batch."},
     {"plan", mod_plan, METH_VARARGS, "Histogram slots of a batch."},
+    {"blank", mod_blank, METH_VARARGS, "Samples without their numbers, for samples()."},
     {"samples", mod_samples, METH_VARARGS, "Records to TokenSample objects."},
     {"logprob_codes", mod_codes, METH_O, "Log-probabilities asked for per row."},
     {nullptr, nullptr, 0, nullptr}};

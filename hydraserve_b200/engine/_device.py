@@ -489,8 +489,12 @@ def record_to_sample(rec, logprobs, vocab: int) -> TokenSample:
     return TokenSample(int(rec["token"]), float(rec["logprob"]), tuple(top))
 
 
-def records_to_samples(records, params, vocab: int):
-    return _host.samples(np.ascontiguousarray(records).view(np.uint8), params, vocab)
+def records_to_samples(records, params, vocab: int, blank=None):
+    return _host.samples(np.ascontiguousarray(records).view(np.uint8), params, vocab, blank)
+
+
+# blank_samples(params, vocab): what records_to_samples needs besides the numbers, made ahead of them
+blank_samples = _host.blank
 
 
 class PackedSamples:

@@ -95,8 +95,8 @@ def partial_records(sampler, local_logits, histories, params, steps, vocab_offse
     return recs, d_params
 
 
-def merge_records(sampler, all_recs, ranks: int, d_params, batch: int, vocab_total: int, *, noise=None):
-    """all_recs: [ranks, batch, 536] uint8 CUDA tensor.  Returns (records, full log-sum-exp)."""
+def launch_merge(sampler, all_recs, ranks: int, d_params, batch: int, vocab_total: int, *, noise=None):
+    """Starts the merge of all_recs, a [ranks, batch, 536] uint8 CUDA tensor; wait_merge has its result."""
     torch = sampler.torch
     host = sampler._pinned_records(batch)  # (the kernel writes the records straight into it)
     lse = torch.empty(batch, dtype=torch.float32, device=sampler.device)
@@ -106,8 +106,19 @@ def merge_records(sampler, all_recs, ranks: int, d_params, batch: int, vocab_tot
                                       d_noise.data_ptr() if d_noise is not None else None, lse.data_ptr(),
                                       sampler._stream())
     _lib.check(sampler.lib, sampler.handle, st, "hs_sharded_merge")
-    torch.cuda.current_stream(sampler.device).synchronize()
-    return host.numpy().view(_lib.ROW_OUT).reshape(batch).copy(), lse
+    return host, lse
+
+
+def wait_merge(sampler, pending):
+    """(records, full log-sum-exp) of the merge started last by this thread on this stream."""
+    host, lse = pending
+    sampler.torch.cuda.current_stream(sampler.device).synchronize()
+    return host.numpy().view(_lib.ROW_OUT).reshape(-1).copy(), lse
+
+
+def merge_records(sampler, all_recs, ranks: int, d_params, batch: int, vocab_total: int, *, noise=None):
+    """all_recs: [ranks, batch, 536] uint8 CUDA tensor.  Returns (records, full log-sum-exp)."""
+    return wait_merge(sampler, launch_merge(sampler, all_recs, ranks, d_params, batch, vocab_total, noise=noise))
 
 
 def check_records(records) -> None:
@@ -146,6 +157,9 @@ def sample_logits_sharded(local_logits, histories, params, *, steps, vocab_offse
             dist.all_gather_into_tensor(gathered, recs, group=group)
         else:
             gathered = recs.unsqueeze(0)
-        records, _ = merge_records(sampler, gathered, ranks, d_params, batch, vocab_total)
+        pending = launch_merge(sampler, gathered, ranks, d_params, batch, vocab_total)
+        # (the objects of the result are made while the GPU is at work: two thirds of what making it takes)
+        blank = _device.blank_samples(params, vocab_total)
+        records, _ = wait_merge(sampler, pending)
     check_records(records)
-    return _device.records_to_samples(records, params, vocab_total)
+    return _device.records_to_samples(records, params, vocab_total, blank)

@@ -189,8 +189,8 @@ int hs_sample_host(hs_sampler* h, const void* logits, int dtype, int64_t row_str
  * copies hs_sample_host makes.  The caller fills ONE pinned block that the sampler owns and hands
  * the step's description over; hs_step counts the new tokens into the histograms, samples, and points
  * *out at the records, in pinned memory of the sampler: they are there once hs_step_wait (or the
- * caller's own wait for `stream`) has returned.  hs_step_wait looks for the rows' last words, which the
- * kernel writes behind all else, and asks the stream only if they do not come; the stream's end may
+ * caller's own wait for `stream`) has returned.  hs_step_wait looks for the records' words as they
+ * arrive, each under the step's tag, and asks the stream only if they do not come; the stream's end may
  * be a few microseconds off when it returns.
  *   hs_step_block   the block, at least `bytes` long (grown as needed, kept, freed by hs_destroy)
  *   hs_step_desc    where in the block things are: hs_row_params[batch] at its start (slots filled
@@ -265,8 +265,8 @@ int hs_query(hs_sampler* h, int what, int vocab, int dtype);
  * row's work items started and ended, in ns of the global timer (slots 48..55: up to four
  * counting parts, 56..63: up to four candidate parts).  Copies batch x 64 counters to out_host (synchronises the device). */
 int hs_debug_phase_clocks(hs_sampler* h, int batch, unsigned long long* out_host);
-/* Tests and tuning.  what = 0: CTAs per candidate row, what = 1: CTAs per counting row; value 1, 2
- * or 4 (0 = chosen per call).  what = 3: near-flat counting rows draw by rejection on tokens
+/* Tests and tuning.  what = 0: CTAs per candidate row, 1, 2 or 4 (0 = chosen per call); what = 1:
+ * CTAs per counting row, 1 to 16 (0 likewise).  what = 3: near-flat counting rows draw by rejection on tokens
  * (1, the default) or always class by class (0).  what = 4: the tag of the last step's mail. */
 int hs_debug_set(hs_sampler* h, int what, int value);
 

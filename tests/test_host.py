@@ -297,3 +297,26 @@ def test_a_row_without_history_goes_without_a_slot_with_and_without_request_ids(
     # next step: both histories grew by one token; "a" now uses the slot that was reset for it
     assert plan([[5], [7, 7, 9, 4], [1, 2, 3]], params, 1000, request_ids=["a", "b", "c"]) == [held["a"], held["b"], -1]
     assert calls == [("reset", []), ("append", [held["a"], held["b"]], [[5], [4]])]
+
+
+@pytest.mark.parametrize("asked", [None, 0, 3, 20])
+def test_samples_made_ahead_are_those_made_at_once(asked):
+    """Blank samples are used up by the first records they are of, and by no other batch's."""
+    from hydraserve_b200 import _lib
+    from hydraserve_b200.engine import _device
+
+    params = tuple(SamplingParams(temperature=1.0, seed=i, logprobs=asked if i % 2 else None) for i in range(5))
+    records = np.zeros(5, _lib.ROW_OUT)
+    records["token"], records["logprob"], records["n_top"] = np.arange(5), -2.0, 2
+    records["top_ids"], records["top_logprobs"] = np.arange(20), -1.5
+    for vocab in (2, 1_000):
+        want = _device.records_to_samples(records, params, vocab)
+        blank = _device.blank_samples(params, vocab)
+        first = _device.records_to_samples(records, params, vocab, blank)
+        again = _device.records_to_samples(records, params, vocab, blank)
+        assert first == want and again == want and first is not again
+        other = _device.blank_samples(params[:2], vocab)
+        assert _device.records_to_samples(records, params, vocab, other) == want
+        _device.blank_samples(params, vocab)  # (dropped unused)
+    with pytest.raises(ValueError):
+        _device.records_to_samples(records, params, 1_000, object())
