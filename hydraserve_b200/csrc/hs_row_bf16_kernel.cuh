@@ -443,13 +443,15 @@ __device__ __forceinline__ bool cand_part(const RowV3Args& args, unsigned char* 
   __syncthreads();
   int n = c.hi > c.lo ? topk_candidates(c, L, min(P.top_k, c.hi - c.lo)) : 0;
   mark(1);
-  // a lone CTA cuts its list at the k-th highest score now; a part of a split row hands its
-  // candidates over as they are unless they would crowd the merged list
-  if (n > P.top_k && (split == 1 || n > kCandCap / split)) {
-    const uint32_t cut = cand_kth_key(*c.x(), L, n, P.top_k);
-    n = cand_compact(L, n, cut);
-  } else if (n > 0) {
-    n = cand_compact(L, n, 0u);  // drops entries the scoring pass voided
+  u64* mass = reinterpret_cast<u64*>(smem_raw + lay.mass);
+  // a lone CTA cuts its list at the k-th highest score now, and sorts it; a part of a split row hands
+  // its candidates over as they are unless they would crowd the merged list
+  if (n > 0) {
+    const bool cut = n > P.top_k && (split == 1 || n > kCandCap / split);
+    const uint32_t bound = cut ? cand_kth_key(*c.x(), L, n, P.top_k) : 0u;
+    mark(14);
+    // (without a cut the pass still drops the entries the scoring voided)
+    n = split == 1 ? cand_keep_sorted(L, mass, n, bound) : cand_compact(L, n, bound);
   }
   if (split > 1) {
     // hand this CTA's candidates over; the CTA that arrives last finishes the row
@@ -483,14 +485,13 @@ __device__ __forceinline__ bool cand_part(const RowV3Args& args, unsigned char* 
     }
     __syncthreads();
     mark(13);
-    if (n > kSortAll) {
-      const uint32_t cut = cand_kth_key(*c.x(), L, n, P.top_k);
-      n = cand_compact(L, n, cut);
+    if (n >= 0) {
+      const uint32_t bound = n > kSortAll ? cand_kth_key(*c.x(), L, n, P.top_k) : 0u;
+      mark(14);
+      n = cand_keep_sorted(L, mass, n, bound);
     }
   }
   if (n < 0) return true;  // more than a candidate list holds: the row is counted
-  mark(14);
-  cand_sort(L, n);
   mark(15);
   if (n > P.top_k) {
     // a list that was sorted whole: top-k keeps the first k entries and the ties of the k-th
@@ -502,7 +503,7 @@ __device__ __forceinline__ bool cand_part(const RowV3Args& args, unsigned char* 
   }
   mark(2);
   const float* noise_row = a.noise ? a.noise + (size_t)c.row * a.vocab : nullptr;
-  FinishOut r = finish_sorted(*c.x(), L.cand, reinterpret_cast<u64*>(smem_raw + lay.mass), n, P, noise_row, out, clocks);
+  FinishOut r = finish_sorted(*c.x(), L.cand, mass, n, P, noise_row, out, clocks);
   if (P.slot >= a.pool.slots_total) r.status |= 64;  // a slot this sampler does not have: no penalties
   if (a.scores_out) {
     float* dst = a.scores_out + (size_t)c.row * a.vocab;

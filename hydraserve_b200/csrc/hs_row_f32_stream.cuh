@@ -231,12 +231,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel_f32_stream(const __gri
   }
   int n = min(*L.n, kCandCap);
   score_pending(n_scored, n);
-  {
-    // (without a cut the pass still drops the entries the scoring voided)
-    const uint32_t cut = n > k && n > kSortAll ? cand_kth_key(*c.x(), L, n, k) : 0u;
-    n = cand_compact(L, n, cut);
-  }
-  cand_sort(L, n);
+  // (without a cut the pass still drops the entries the scoring voided)
+  n = cand_keep_sorted(L, reinterpret_cast<u64*>(smem_raw + lay.mass), n, n > k && n > kSortAll ? cand_kth_key(*c.x(), L, n, k) : 0u);
   if (n > k) {
     // a list that was sorted whole: top-k keeps the first k entries and the ties of the k-th
     const uint32_t cut = cand_key(L.cand[k - 1]);

@@ -701,8 +701,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
       int* small = reinterpret_cast<int*>(c.red_mass);
       CandCtx L{reinterpret_cast<u64*>(on_chip), small, small + 1, reinterpret_cast<uint32_t*>(c.hist), small + 2, nullptr};
       int n = total;
-      if (n > P.top_k && n > kSortAll) n = cand_compact(L, n, cand_kth_key(*c.x, L, n, P.top_k));
-      cand_sort(L, n);
+      u64* mass = reinterpret_cast<u64*>(on_chip) + kCandCap;
+      n = cand_keep_sorted(L, mass, n, n > P.top_k && n > kSortAll ? cand_kth_key(*c.x, L, n, P.top_k) : 0u);
       if (n > P.top_k) {
         // a list that was sorted whole: top-k keeps the first k entries and the ties of the k-th
         const uint32_t cut = cand_key(L.cand[P.top_k - 1]);
@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(const __grid_constant_
         n = (int)keep;
       }
       const float* noise_row = a.noise ? a.noise + (size_t)c.row * a.vocab : nullptr;
-      FinishOut r = finish_sorted(*c.x, L.cand, reinterpret_cast<u64*>(on_chip) + kCandCap, n, P, noise_row, &record);
+      FinishOut r = finish_sorted(*c.x, L.cand, mass, n, P, noise_row, &record);
       r.status |= status;
       if (a.scores_out) {
         float* dst = a.scores_out + (size_t)c.row * a.vocab;

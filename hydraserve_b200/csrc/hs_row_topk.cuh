@@ -548,6 +548,18 @@ __device__ int topk_candidates(Ctx3& c, CandCtx& L, int k) {
   return n;
 }
 
+// Entries of a list above `mine`.
+__device__ __forceinline__ int cand_rank(const u64* list, int n, u64 mine) {
+  int rank = 0;
+  const ulonglong2* two = reinterpret_cast<const ulonglong2*>(list);
+#pragma unroll 4
+  for (int j = 0; j < n / 2; ++j) {
+    const ulonglong2 o = two[j];
+    rank += (o.x > mine) + (o.y > mine);
+  }
+  if (n & 1) rank += list[n - 1] > mine;
+  return rank;
+}
 // Sorts the first n list entries descending (bitonic, n padded to a power of two with zeros).
 // A compare-exchange step of stride <= 32 stays inside the 64 entries one warp handles, so
 // only the wider steps (and the changes between the two kinds) need the block barrier.
@@ -557,16 +569,7 @@ __device__ void cand_sort(CandCtx& L, int n) {
     // end in the token id) and moves to that position
     const int i = threadIdx.x;
     const u64 mine = i < n ? L.cand[i] : 0ull;
-    int rank = 0;
-    if ((i & ~31) < n) {
-      const ulonglong2* two = reinterpret_cast<const ulonglong2*>(L.cand);
-#pragma unroll 4
-      for (int j = 0; j < n / 2; ++j) {
-        const ulonglong2 o = two[j];
-        rank += (o.x > mine) + (o.y > mine);
-      }
-      if (n & 1) rank += L.cand[n - 1] > mine;
-    }
+    const int rank = (i & ~31) < n ? cand_rank(L.cand, n, mine) : 0;
     __syncthreads();
     if (i < n) L.cand[rank] = mine;
     __syncthreads();
@@ -592,6 +595,35 @@ __device__ void cand_sort(CandCtx& L, int n) {
     }
   }
   __syncthreads();
+}
+
+// The entries at or above `bound` (void ones drop out in any case), sorted; returns how many.  `tmp` has room
+// for a list.  What cand_compact and cand_sort do, three barriers instead of five: one row of 151,936 44.3 -> 43.9 us a
+// call, 1,024 mixed rows 201.1 -> 200.0 us of GPU time.
+__device__ int cand_keep_sorted(CandCtx& L, u64* tmp, int n, uint32_t bound) {
+  const int tid = threadIdx.x;
+  __syncthreads();
+  if (tid == 0) *L.n = 0;
+  __syncthreads();
+  for (int i = tid; i < n; i += kThreads) {
+    const u64 e = L.cand[i];
+    if (e != 0ull && cand_key(e) >= bound) tmp[atomicAdd(L.n, 1)] = e;
+  }
+  __syncthreads();
+  const int m = *L.n;
+  if (m > kThreads) {
+    for (int i = tid; i < m; i += kThreads) L.cand[i] = tmp[i];
+    __syncthreads();
+    cand_sort(L, m);
+    return m;
+  }
+  if ((tid & ~31) < m) {
+    const u64 mine = tid < m ? tmp[tid] : 0ull;
+    const int rank = cand_rank(tmp, m, mine);
+    if (tid < m) L.cand[rank] = mine;
+  }
+  __syncthreads();
+  return m;
 }
 
 struct FinishOut {

@@ -70,13 +70,8 @@ __global__ void __launch_bounds__(kThreads, 2) shard_partial_kernel(const ShardA
   // list overflow: what is in the list is partly unscored, so the record carries no candidates
   // and the merge reports the row as failed
   if (n < 0) { status |= 16; n = 0; }
-  if (n > k) {
-    const uint32_t cut = cand_kth_key(*c.x(), L, n, k);
-    n = cand_compact(L, n, cut);
-  } else if (n > 0) {
-    n = cand_compact(L, n, 0u);  // drops entries the scoring pass voided
-  }
-  cand_sort(L, n);
+  // (without a cut the pass still drops the entries the scoring voided)
+  if (n > 0) n = cand_keep_sorted(L, reinterpret_cast<u64*>(smem_raw + lay.mass), n, n > k ? cand_kth_key(*c.x(), L, n, k) : 0u);
   if (n > HS_SHARD_CAND) { status |= 32; n = HS_SHARD_CAND; }  // more ties than the record holds
   __syncthreads();
   const float m = n > 0 ? score_of(cand_key(L.cand[0])) : 0.f;
@@ -175,11 +170,7 @@ __global__ void __launch_bounds__(kThreads, 2) shard_merge_kernel(const MergeArg
     return;
   }
   const int k = P.top_k > 0 ? P.top_k : n;
-  if (n > k) {
-    const uint32_t cut = cand_kth_key(*x, L, n, k);
-    n = cand_compact(L, n, cut);
-  }
-  cand_sort(L, n);
+  n = cand_keep_sorted(L, mass, n, n > k ? cand_kth_key(*x, L, n, k) : 0u);
   const float* noise_row = a.noise ? a.noise + (size_t)row * a.vocab_total : nullptr;
   FinishOut r = finish_sorted(*x, L.cand, mass, n, P, noise_row, &rec);
   r.status |= status;
