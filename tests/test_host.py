@@ -300,14 +300,16 @@ def test_a_row_without_history_goes_without_a_slot_with_and_without_request_ids(
 
 
 @pytest.mark.parametrize("asked", [None, 0, 3, 20])
-def test_samples_made_ahead_are_those_made_at_once(asked):
-    """Blank samples are used up by the first records they are of, and by no other batch's."""
+@pytest.mark.parametrize("rows", [5, 300])
+def test_samples_made_ahead_are_those_made_at_once(asked, rows):
+    """Blank samples are used up by the first records they are of, and by no other batch's; of a
+    large batch only the first ones are made ahead."""
     from hydraserve_b200 import _lib
     from hydraserve_b200.engine import _device
 
-    params = tuple(SamplingParams(temperature=1.0, seed=i, logprobs=asked if i % 2 else None) for i in range(5))
-    records = np.zeros(5, _lib.ROW_OUT)
-    records["token"], records["logprob"], records["n_top"] = np.arange(5), -2.0, 2
+    params = tuple(SamplingParams(temperature=1.0, seed=i, logprobs=asked if i % 2 else None) for i in range(rows))
+    records = np.zeros(rows, _lib.ROW_OUT)
+    records["token"], records["logprob"], records["n_top"] = np.arange(rows), -2.0, 2
     records["top_ids"], records["top_logprobs"] = np.arange(20), -1.5
     for vocab in (2, 1_000):
         want = _device.records_to_samples(records, params, vocab)
