@@ -4,8 +4,8 @@
 // and with two CTAs on an SM almost all of L1 is shared memory, so every spilled value was a round
 // trip to L2.  What bounds it now is the fetching of instructions a CTA goes through once, and the
 // barriers between the passes.  With its count table kept in shared memory and one histogram for all
-// cuts, 64 rows of 151,936 with 20 log-probabilities take 75 us (90), one row of 248,320 69 us (97),
-// 1,024 mixed rows of 151,936 199 us (231).
+// cuts, 64 rows of 151,936 with 20 log-probabilities took 75 us instead of 90 (71 now), 1,024 mixed rows of
+// 151,936 210 instead of 231 (203 now).
 #pragma once
 
 #include "hs_row_v3.cuh"

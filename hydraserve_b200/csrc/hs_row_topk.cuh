@@ -9,7 +9,7 @@
 // a valid bound for the whole row; whenever the candidate list grows past 2,048 entries
 // the bound is raised to the list's k-th highest score and the list is compacted.  Scores
 // grow with the raw value inside a history-count class, so the bound turns into one raw
-// threshold per class (binary search over the 65,536 bf16 values); a token whose history
+// threshold per class (a guess and its neighbours, else a search over the 65,536 bf16 values); a token whose history
 // count is 3 or more is always scored exactly.
 //
 // What is left, at most a few thousand (score key, token id) pairs in shared memory, is
