@@ -298,7 +298,7 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
     {
       // Warp w lists the w-th run of cells, 32 neighbours at a time, so that a list is in the order of
       // the cells: whoever adds it up finds neighbouring entries in different banks, and can look a
-      // class up in it (part_of_member).  A count that 17 bits do not hold takes several entries.
+      // class up in it (nth_in_parts).  A count that 17 bits do not hold takes several entries, side by side.
       const int lane = tid & 31, warp = tid >> 5;
       const int rows = (c.cls ? kCells : kV3Bins) / (32 * kWarps);  // (without penalties there is one count class)
       static_assert(kV3Bins % (32 * kWarps) == 0, "every warp has whole groups of 32 cells");
@@ -323,12 +323,25 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
       for (int u = 0; u < rows; ++u) {
         uint32_t v = run[32 * u];
         const uint32_t cell = (uint32_t)(first + 32 * u);
-        for (uint32_t who = __ballot_sync(0xffffffffu, v != 0u); who; who = __ballot_sync(0xffffffffu, v != 0u)) {
-          const uint32_t part_v = min(v, kMostHanded);
-          if (v) dst[at + __popc(who & ((1u << lane) - 1u))] = cell | (part_v << 15);
+        const uint32_t who = __ballot_sync(0xffffffffu, v != 0u);
+        if (!__any_sync(0xffffffffu, v > kMostHanded)) {
+          if (v) dst[at + __popc(who & ((1u << lane) - 1u))] = cell | (v << 15);
           at += __popc(who);
-          v -= part_v;
-          if (__all_sync(0xffffffffu, v == 0u)) break;  // (but for the largest counts)
+        } else {
+          const int entries = v ? 1 + (int)((v - 1u) / kMostHanded) : 0;
+          int incl = entries;
+#pragma unroll 1
+          for (int d = 1; d < 32; d <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += o;
+          }
+#pragma unroll 1
+          for (int to = at + incl - entries; v; ++to) {
+            const uint32_t part_v = min(v, kMostHanded);
+            dst[to] = cell | (part_v << 15);
+            v -= part_v;
+          }
+          at += __shfl_sync(0xffffffffu, incl, 31);
         }
       }
       __syncthreads();

@@ -106,6 +106,45 @@ def test_a_counted_row_is_the_same_in_any_number_of_parts(kind, vocab):
         s.close()
 
 
+@pytest.mark.parametrize("vocab, parts", [(300_000, 2), (600_000, 4)])
+def test_a_value_of_more_tokens_than_an_entry_holds(vocab, parts):
+    """One value fills most of the first part, more tokens than one entry of a hand-over counts (131,070), and
+    the 31 values above it, its neighbours in the count table, are drawn from: their members are looked up
+    in a list that holds several entries of the full class.  (With 991 values below them the list has 32 x 32
+    entries, and the search's first look goes to its last one.)"""
+    batch, full, each = 32, 140_000, 20
+    logits = torch.empty(batch, vocab, dtype=torch.bfloat16, device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(parts)
+    for i in range(batch):
+        low = torch.arange(vocab, device="cuda") % (991, 1_023, 1_055, 970 + i)[i % 4]  # (values from -1 down)
+        x = (-0x4080 + low).to(torch.int16).view(torch.bfloat16)
+        first = torch.randperm(vocab // parts, generator=gen, device="cuda")
+        rest = torch.randperm(vocab - vocab // parts, generator=gen, device="cuda") + vocab // parts
+        x[first[:full]] = 32.0
+        for k in range(1, 32):
+            x[first[full + each * k:full + each * (k + 1)]] = 32.0 + 0.25 * k
+            x[rest[4 * each * k:4 * each * (k + 1)]] = 32.0 + 0.25 * k
+        logits[i] = x
+    params = [SamplingParams(temperature=2.0, seed=3 * i + 1) for i in range(batch)]
+    s = _sampler(vocab, batch)
+    s.set_token_draw(False)
+    neighbours = 0
+    try:
+        with s.lock:
+            for step in range(8):
+                rec = _device.pack_params(params, [step] * batch, [-1] * batch)
+                s.set_count_split(1)
+                want, _ = s.run(logits, rec)
+                s.set_count_split(parts)
+                got, _ = s.run(logits, rec)
+                for name in (*COUNTS, "token"):
+                    np.testing.assert_array_equal(got[name], want[name], err_msg=name)
+                neighbours += int((logits.cpu()[range(batch), want["token"]] > 32).sum())
+    finally:
+        s.close()
+    assert neighbours > batch
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("vocab", [1, 9, 31, 5_003, 50_257])
 def test_greedy_rows_off_the_16_byte_grid(dtype, vocab):
