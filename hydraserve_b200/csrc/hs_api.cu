@@ -83,7 +83,7 @@ struct hs_sampler {
   int force_csplit = 0;   // CTAs per counting row (0 = chosen per call)
   int token_draw = 1;     // near-flat counting rows draw by rejection on tokens
   int ctab_tables = 0;    // parts of counting rows the hand-over scratch holds
-  uint32_t* ctab = nullptr;   // [ctab_tables, kCells]
+  uint32_t* ctab = nullptr;   // [ctab_tables, kHandedCap]
   int2* crare = nullptr;      // [ctab_tables, kV3RareCap]
   int2* crare_n = nullptr;    // [ctab_tables]
   int split_tables = 0;   // parts of candidate rows
@@ -569,7 +569,7 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
   // hand-over scratch of rows split over several CTAs: two parts per resident CTA
   h->ctab_tables = 2 * h->resident_bf16;
   h->split_tables = std::max(2 * h->resident_bf16, 2 * batch_max);
-  held.add(&h->ctab, (size_t)h->ctab_tables * hs::kCells * sizeof(uint32_t), false);
+  held.add(&h->ctab, (size_t)h->ctab_tables * hs::kHandedCap * sizeof(uint32_t), false);
   held.add(&h->crare, (size_t)h->ctab_tables * hs::kV3RareCap * sizeof(int2), false);
   held.add(&h->crare_n, (size_t)h->ctab_tables * sizeof(int2), false);
   held.add(&h->count_ticket, (size_t)batch_max * sizeof(int), true);

@@ -91,7 +91,7 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
     S.mail_row = mail_of(a, row_index);
     S.mail_tag = a.mail_tag;
     S.parts = part < 0 ? 1 : args.csplit;
-    S.lists = args.ctab + (size_t)row_index * args.csplit * kCells;
+    S.lists = args.ctab + (size_t)row_index * args.csplit * kHandedCap;
     S.lens = args.crare_n + (size_t)row_index * args.csplit;
     S.clocks = args.phase_clocks ? args.phase_clocks + (size_t)row_index * kV3PhaseSlots : nullptr;
     if (S.clocks) S.clocks[0] = clock64();
@@ -317,7 +317,7 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
       const int of_warp = lane < kWarps ? small[48 + lane] : 0;
       const int total = __reduce_add_sync(0xffffffffu, of_warp);
       int at = __reduce_add_sync(0xffffffffu, lane < warp ? of_warp : 0);
-      uint32_t* gtab = args.ctab + mine * kCells;
+      uint32_t* gtab = args.ctab + mine * kHandedCap;
       uint32_t* dst = total <= kV3Staged ? staged : gtab;
 #pragma unroll 1
       for (int u = 0; u < rows; ++u) {
@@ -360,7 +360,7 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
     // The other parts' lists, piece by piece of up to 4,096 entries, the next piece's on their way while this
     // one's are added.
     const int2* lens = args.crare_n + (size_t)c.row * parts;
-    const uint32_t* lists = args.ctab + (size_t)c.row * parts * kCells;
+    const uint32_t* lists = args.ctab + (size_t)c.row * parts * kHandedCap;
     int2* part_len = reinterpret_cast<int2*>(defer);  // (the staged list has left)
     if (tid < parts) part_len[tid] = __ldcg(lens + tid);
     __syncthreads();
@@ -369,7 +369,7 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
     auto fetch = [&](uint4 (&v)[kFlight]) {
       if (next.g >= parts) return;
       const int n = part_len[next.g].x, n4 = (n + 3) >> 2;
-      const uint4* src = reinterpret_cast<const uint4*>(lists + (size_t)next.g * kCells);
+      const uint4* src = reinterpret_cast<const uint4*>(lists + (size_t)next.g * kHandedCap);
 #pragma unroll
       for (int u = 0; u < kFlight; ++u) {
         const int i = next.at + tid + u * kThreads;

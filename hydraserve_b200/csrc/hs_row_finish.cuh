@@ -48,7 +48,7 @@ struct CountState {
   ulonglong2* mail_row;
   uint32_t mail_tag;
   int parts;              // CTAs that counted the row; of several, each left a list of its classes
-  const uint32_t* lists;  // [parts, kCells]
+  const uint32_t* lists;  // [parts, kHandedCap]
   const int2* lens;       // [parts]
   unsigned long long* clocks;
 };
@@ -688,7 +688,7 @@ __device__ __noinline__ int nth_in_parts(int cell, u64 n) {
   if (n <= (u64)__popc(ahead)) return (int)__fns(ahead, 0, (int)n);
   __syncthreads();
   if (warp < parts) {
-    const uint32_t* list = S.lists + (size_t)warp * kCells;
+    const uint32_t* list = S.lists + (size_t)warp * kHandedCap;
     const int len = __ldcg(S.lens + warp).x;
     int lo = 0, hi = len;
 #pragma unroll 1

@@ -48,6 +48,9 @@ constexpr int kV3TieCap = 1536;               // token ids ranked in shared memo
 constexpr int kV3Buckets = 1024;              // of a selection's histogram
 constexpr int kV3Staged = 7168;               // (class, count) entries of a hand-over staged in shared memory
 constexpr uint32_t kMostHanded = 0x1fffe;     // highest count of one such entry (17 bits beside a 15-bit class)
+// Room for a part's list: an entry for every cell, and those a part of the widest row (eight slices) adds by
+// counts above kMostHanded.
+constexpr int kHandedCap = (kCells + kMaxCluster * kMaxSliceElems / (int)kMostHanded + 3) & ~3;
 #ifndef HS_RARE_CAP
 #define HS_RARE_CAP 512
 #endif
@@ -81,7 +84,7 @@ struct RowV3Args {
   int* scratch_busy;   // [n_scratch] 1 while a CTA holds the set
   unsigned long long* phase_clocks;  // [batch, kV3PhaseSlots] or null
   int csplit;                        // CTAs per row on the counting path
-  uint32_t* ctab;                    // [batch, csplit, kCells] classes and counts handed over by the parts of a row
+  uint32_t* ctab;                    // [batch, csplit, kHandedCap] classes and counts handed over by the parts of a row
   int2* crare;                       // [batch, csplit, kV3RareCap] their rare lists
   int2* crare_n;                     // [batch, csplit] (classes, rare tokens)
   int* count_ticket;                 // [batch] arrival counter (returns to 0)

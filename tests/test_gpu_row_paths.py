@@ -145,6 +145,43 @@ def test_a_value_of_more_tokens_than_an_entry_holds(vocab, parts):
     assert neighbours > batch
 
 
+def test_a_part_with_every_class_and_a_full_one():
+    """Every value of the count table under every history count, and one of them more often than an entry
+    counts: the longest list a part can hand over."""
+    vocab, parts, batch = 600_000, 4, 6
+    lowest, highest = 113 << 7, (113 << 7) + 3_072  # (raw bits of 2^-14 and 2^10)
+    values = torch.arange(lowest, highest, dtype=torch.int16)
+    values = torch.cat([values, values | -0x8000]).repeat(3)  # not in the history; there once; there twice
+    gen = torch.Generator().manual_seed(3)
+    raw = torch.full((batch, vocab), 0x4000, dtype=torch.int16)
+    histories, per = [], vocab // parts
+    for i in range(batch):
+        here = torch.randperm(per, generator=gen)[:len(values)] + (0, parts - 1)[i % 2] * per
+        elsewhere = torch.ones(vocab, dtype=torch.bool)
+        elsewhere[(0, parts - 1)[i % 2] * per:][:per] = False
+        raw[i, elsewhere] = torch.randint(lowest, highest, (vocab - per,), generator=gen, dtype=torch.int16)
+        raw[i, here] = values
+        once, twice = here[len(values) // 3:2 * len(values) // 3], here[2 * len(values) // 3:]
+        histories.append(torch.cat([once, twice, twice]).tolist())
+    logits = raw.view(torch.bfloat16).cuda()
+    params = [SamplingParams(temperature=(1.0, 2.0)[i % 2], top_k=(3_000, 150_000, 400_000)[i // 2], seed=i + 1, frequency_penalty=0.01)
+              for i in range(batch)]
+    s = _sampler(vocab, batch)
+    try:
+        with s.lock:
+            slots = s.plan_slots(histories, params, vocab)
+            rec = _device.pack_params(params, [1] * batch, slots)
+            s.set_count_split(1)
+            want, _ = s.run(logits, rec)
+            s.set_count_split(parts)
+            for _ in range(3):
+                got, _ = s.run(logits, rec)
+                for name in (*COUNTS, "token"):
+                    np.testing.assert_array_equal(got[name], want[name], err_msg=name)
+    finally:
+        s.close()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("vocab", [1, 9, 31, 5_003, 50_257])
 def test_greedy_rows_off_the_16_byte_grid(dtype, vocab):
