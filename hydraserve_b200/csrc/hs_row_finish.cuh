@@ -453,10 +453,13 @@ __device__ __noinline__ void phase_cuts() {
       if (k >= cut_key && k < lowest && !(__fdiv_rn(expf(s - m), z1) < thr)) lowest = k;
     };
     // Of the cells, only those that come near the line: a token passes from m + log(min_p) on, give or
-    // take the roundings of exp and of the quotients (parts in a million).
+    // take the roundings of exp and of the quotients, parts in a million.  (All of them, when the threshold is
+    // no normal number: a subnormal one is off by any share of itself, everything passes 0, and a maximum of
+    // infinity leaves no line.)
     const float floor = __fadd_rd(__fadd_rd(m, logf(P.min_p)), -0.01f);
+    const bool line = thr >= 1.17549435e-38f && thr < INFINITY && floor > -3.0e38f;
     V3Map near_line;
-    near_line.by_key(floor > -3.0e38f ? key_of(floor) : 0u, 0xffffffffu);
+    near_line.by_key(line ? key_of(floor) : 0u, 0xffffffffu);
     locate_cells(c, near_line, 0);
     const Scorer sc = c;
 #pragma unroll 1

@@ -182,6 +182,35 @@ def test_a_part_with_every_class_and_a_full_one():
         s.close()
 
 
+@pytest.mark.parametrize("penalised", [False, True])
+@pytest.mark.parametrize("min_p", [1e-45, 1e-41, 3e-39, 1e-38, 5e-34, 2e-33, 1e-30, 0.05, 1.0])
+def test_min_p_down_to_the_smallest_number(min_p, penalised):
+    """Tens of thousands of tokens next to the maximum and as many far below it, every 0.002 of a score: where
+    the threshold is a subnormal number or 0, tokens far below the line pass."""
+    vocab, batch = 60_010, 6
+    gen = torch.Generator().manual_seed(5)
+    x = torch.randn(batch, vocab, generator=gen) * 0.01
+    x[:3, -30_000:] = -torch.linspace(60, 125, 30_000)
+    x[3:, -30_000:] = torch.tensor([-200.0, -99.0]).repeat(15_000)
+    logits = x[:, torch.randperm(vocab, generator=gen)].to(torch.bfloat16).cuda()
+    penalties = dict(repetition_penalty=1.2, frequency_penalty=0.3) if penalised else {}
+    params = [SamplingParams(temperature=(1.0, 0.9)[i % 2], top_k=(0, 50_000, 0)[i % 3], min_p=min_p, seed=i, **penalties)
+              for i in range(batch)]
+    histories = [[(31 * j * j + i) % vocab for j in range(500)] for i in range(batch)]
+    s = _sampler(vocab, batch)
+    try:
+        with s.lock:
+            rec = _device.pack_params(params, [1] * batch, s.plan_slots(histories, params, vocab))
+            want, _ = s.run(logits, rec, general=True)
+            for split in (1, 3):
+                s.set_count_split(split)
+                got, _ = s.run(logits, rec)
+                for name in COUNTS:
+                    np.testing.assert_array_equal(got[name], want[name], err_msg=name)
+    finally:
+        s.close()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("vocab", [1, 9, 31, 5_003, 50_257])
 def test_greedy_rows_off_the_16_byte_grid(dtype, vocab):
