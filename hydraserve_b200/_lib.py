@@ -71,6 +71,8 @@ EXPORTS = {
     "hs_step_block": (C.c_int, [C.c_void_p, C.c_size_t, C.POINTER(C.c_void_p)]),
     "hs_step": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int, C.c_int, C.c_void_p,
                           C.POINTER(C.c_void_p), C.c_void_p]),
+    "hs_step_awaited": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int, C.c_int, C.c_void_p,
+                                  C.POINTER(C.c_void_p), C.c_void_p]),
     "hs_step_wait": (C.c_int, [C.c_void_p, C.c_void_p]),
     "hs_step_greedy": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int, C.c_int,
                                  C.POINTER(C.c_void_p), C.c_void_p]),

@@ -817,14 +817,17 @@ int hs_step_block(hs_sampler* h, size_t bytes, void** block) {
   return HS_OK;
 }
 
-int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
-            const hs_step_desc* d, const hs_row_out** out, void* stream_) {
+namespace {
+
+// (awaited: the caller is going to call hs_step_wait, so the records go by mail alone)
+int step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
+         const hs_step_desc* d, const hs_row_out** out, bool awaited, void* stream_) {
   int rc = check_common(h, logits, dtype, batch, vocab);
   if (rc != HS_OK) return rc;
   if (!d || !out) return fail(h, HS_ERR_INVALID, "desc / out is null");
   *out = nullptr;
   nothing_awaited(h);
-  const bool repeats = (d->repeats & ~HS_STEP_WILL_WAIT) != 0;
+  const bool repeats = d->repeats != 0;
   if (batch == 0) return HS_OK;
   if (row_stride < vocab) return fail(h, HS_ERR_INVALID, "row_stride smaller than vocab");
   if (d->n_resets < 0 || d->n_appends < 0 || d->n_appends > 65535 || d->n_resets > 65535)
@@ -839,7 +842,7 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
   HS_CUDA(h, serial.status);
 
   *out = h->h_out;
-  h->mail_only = (d->repeats & HS_STEP_WILL_WAIT) != 0;
+  h->mail_only = awaited;
   if (++h->mail_tag == 0) {
     // (around once: no word may still stand under a tag that comes again)
     HS_CUDA(h, cudaStreamSynchronize(stream));
@@ -937,6 +940,18 @@ int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, in
   HS_CUDA(h, serial.done());
   h->awaited_records = batch;
   return HS_OK;
+}
+
+}  // namespace
+
+int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
+            const hs_step_desc* d, const hs_row_out** out, void* stream) {
+  return step(h, logits, dtype, row_stride, batch, vocab, d, out, false, stream);
+}
+
+int hs_step_awaited(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
+                    const hs_step_desc* d, const hs_row_out** out, void* stream) {
+  return step(h, logits, dtype, row_stride, batch, vocab, d, out, true, stream);
 }
 
 int hs_step_wait(hs_sampler* h, void* stream) {

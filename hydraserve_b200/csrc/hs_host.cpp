@@ -796,7 +796,7 @@ PyObject* stepper_step(PyObject* self, PyObject* const* args, Py_ssize_t n_args)
   d.n_resets = (int32_t)plan.resets.size();
   d.n_appends = (int32_t)plan.appends.size();
   d.max_tokens = (int32_t)longest;
-  d.repeats = (plan.repeats ? 1 : 0) | HS_STEP_WILL_WAIT;
+  d.repeats = plan.repeats ? 1 : 0;
   d.resets_at = at; at += up16(plan.resets.size() * 4);
   d.slots_at = at; at += up16(plan.appends.size() * 4);
   d.offsets_at = at; at += up16((plan.appends.size() + 1) * 4);

@@ -139,7 +139,7 @@ class DeviceSampler:
         self.book = SlotBook(self.resident_slots)
         address = lambda fn: C.cast(fn, C.c_void_p).value  # noqa: E731
         self.host = _host.Stepper(handle.value, self.book, self.scratch_base, _lib.SamplerError,
-                                  address(self.lib.hs_step_block), address(self.lib.hs_step),
+                                  address(self.lib.hs_step_block), address(self.lib.hs_step_awaited),
                                   address(self.lib.hs_step_greedy), address(self.lib.hs_step_wait),
                                   address(self.lib.hs_last_error))
         self.users = 0        # calls inside this sampler (guarded by _samplers_lock)

@@ -197,13 +197,12 @@ int hs_sample_host(hs_sampler* h, const void* logits, int dtype, int64_t row_str
  *                   in); int32 reset_slots[n_resets] at resets_at; and for the tokens to count
  *                   int32 slots[n_appends] at slots_at, int32 offsets[n_appends + 1] at offsets_at,
  *                   int32 tokens[] at tokens_at, as hs_slots_append takes them (sections 16-byte
- *                   aligned; bytes = end of the last one; repeats = 1 when a slot is listed twice, and
- *                   HS_STEP_WILL_WAIT beside it when the caller is going to call hs_step_wait: the
- *                   records are then written where that call looks for them and nowhere else)
+ *                   aligned; bytes = end of the last one; repeats not 0 when a slot is listed twice)
+ *   hs_step_awaited hs_step for a caller that is going to call hs_step_wait: the records are written where
+ *                   that call looks for them and nowhere else, so *out holds them only once it has returned
  * A record's top_ids / top_logprobs are written on rows with n_logprobs >= 0 only.
  * The block and the records belong to one step at a time: the caller serialises
  * hs_step_block .. hs_step .. hs_step_wait .. reading the records against other steps of the same sampler. */
-#define HS_STEP_WILL_WAIT (1 << 30)
 typedef struct hs_step_desc {
   size_t bytes, resets_at, slots_at, offsets_at, tokens_at;
   int32_t n_resets, n_appends, max_tokens, repeats;
@@ -211,6 +210,8 @@ typedef struct hs_step_desc {
 int hs_step_block(hs_sampler* h, size_t bytes, void** block);
 int hs_step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
             const hs_step_desc* desc, const hs_row_out** out, void* stream);
+int hs_step_awaited(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,
+                    const hs_step_desc* desc, const hs_row_out** out, void* stream);
 int hs_step_wait(hs_sampler* h, void* stream);
 /* The same for a batch of plain-greedy rows: hs_greedy with the ids in pinned memory. */
 int hs_step_greedy(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int batch, int vocab,

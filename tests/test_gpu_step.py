@@ -92,6 +92,39 @@ def test_a_wait_is_for_the_step_before_it(built_library):
         s.close()
 
 
+@pytest.mark.parametrize("repeats", [0, 1, -1])
+def test_records_of_a_step_its_caller_waits_for(built_library, repeats):
+    """hs_step without hs_step_wait: at the stream's end the records stand where *out points, whatever
+    number says that a slot is listed twice."""
+    from hydraserve_b200 import _lib
+    from hydraserve_b200.engine import _device
+
+    vocab, batch = 5_000, 6
+    params = [SamplingParams(temperature=1.0, top_k=(0, 40)[i % 2], seed=i, logprobs=(None, 5, None)[i % 3]) for i in range(batch)]
+    s = _device.DeviceSampler("cuda:0", vocab_max=vocab, batch_max=batch, resident_slots=1)
+    out = C.c_void_p()
+    try:
+        for step in range(3):
+            logits = torch.randn(batch, vocab, generator=torch.Generator().manual_seed(step)).cuda().bfloat16()
+            rec = _device.pack_params(params, [step] * batch, [-1] * batch)
+            want, _ = s.run(logits, rec)
+            if out.value:
+                C.memset(out.value, 0x55, batch * _lib.ROW_OUT.itemsize)  # (no record of an earlier step)
+            block = C.c_void_p()
+            assert s.lib.hs_step_block(s.handle, rec.nbytes, C.byref(block)) == 0
+            C.memmove(block.value, rec.ctypes.data, rec.nbytes)
+            d = _Desc(rec.nbytes, rec.nbytes, rec.nbytes, rec.nbytes, rec.nbytes, 0, 0, 0, repeats)
+            assert s.lib.hs_step(s.handle, logits.data_ptr(), 1, vocab, batch, vocab, C.byref(d), C.byref(out), s._stream()) == 0
+            torch.cuda.synchronize()
+            got = np.frombuffer((C.c_char * (batch * _lib.ROW_OUT.itemsize)).from_address(out.value), dtype=_lib.ROW_OUT)
+            for i in range(batch):
+                for name in _lib.ROW_OUT.names:
+                    if params[i].logprobs is not None or not name.startswith("top_"):
+                        np.testing.assert_array_equal(got[i][name], want[i][name], err_msg=f"{name} of row {i}")
+    finally:
+        s.close()
+
+
 def test_a_row_that_goes_again_is_counted_once(built_library):
     """HS_SAMPLE_APPEND_TOKEN and a row the bf16 kernel hands to the general one (more values outside
     its window than the side list holds): one token goes into the histogram, the one sampled."""
