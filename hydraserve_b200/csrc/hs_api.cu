@@ -123,8 +123,8 @@ struct hs_sampler {
   int32_t* h_tokens = nullptr;    // [batch_max]
   volatile u64* h_mail = nullptr;  // [batch_max, kRecordWords] a record's words as they arrive, each under its step's tag
   uint32_t mail_tag = 0;           // of the last hs_step
-  bool mail_only = false;          // its records are nowhere else
   std::vector<uint8_t> mail_words; // [batch_max] words of each row's record of that step
+  std::vector<int> pending;        // [batch_max] rows hs_step_wait still looks for
   std::atomic<int> awaited_ids{0}, awaited_records{0};  // on their way into h_tokens and h_mail
   std::mutex mu;         // the staging buffers of hs_sample_host
   // Every launching call takes launch_mu, and work of one call is ordered after the previous
@@ -606,6 +606,7 @@ int hs_create_ex(int device, int vocab_max, int slots_max, int hist_cap, int bat
       h->h_mail = reinterpret_cast<u64*>(base + at[4]);
       std::memset(base + at[4], 0, mail_bytes);
       h->mail_words.assign((size_t)batch_max, 0);
+      h->pending.assign((size_t)batch_max, 0);
       h->h_block = base + at[5];
       h->h_block_bytes = h->d_block_bytes = first_block;
     }
@@ -842,7 +843,6 @@ int step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int b
   HS_CUDA(h, serial.status);
 
   *out = h->h_out;
-  h->mail_only = awaited;
   if (++h->mail_tag == 0) {
     // (around once: no word may still stand under a tag that comes again)
     HS_CUDA(h, cudaStreamSynchronize(stream));
@@ -935,7 +935,7 @@ int step(hs_sampler* h, const void* logits, int dtype, int64_t row_stride, int b
   // (the records go straight to pinned memory: see write_record)
   rc = launch_rows(h, logits, dtype, row_stride, batch, vocab,
                    rows_inline ? nullptr : reinterpret_cast<const hs_row_params*>(h->d_block), rows_inline ? inl : kNoInlineRows,
-                   n_count_of(params, batch, vocab), h->mail_only ? nullptr : h->h_out, nullptr, nullptr, nullptr, 0u, behind, stream, true);
+                   n_count_of(params, batch, vocab), awaited ? nullptr : h->h_out, nullptr, nullptr, nullptr, 0u, behind, stream, true);
   if (rc != HS_OK) return rc;
   HS_CUDA(h, serial.done());
   h->awaited_records = batch;
@@ -958,35 +958,48 @@ int hs_step_wait(hs_sampler* h, void* stream) {
   if (!h) return HS_ERR_INVALID;
   // A greedy row's id is one word in pinned memory, any other row's record comes word by word (see
   // write_record) and is put together here: all are there some microseconds before the stream reports
-  // its end.  (For as long as a large step takes; then, or if something went wrong, the stream has
-  // the word, and the records stand where the kernel wrote them in one piece.)
+  // its end.  Rows are taken as they come: bound by the reads of memory the GPU has just written, about 10 ns
+  // a row, which in the order of the rows were left for the end whenever an early row was a late one (256 rows of
+  // 151,936: 20 counting rows among them 75.2 us a call in order, 72.6 this way, all counting 94.5 and 90.2,
+  // none 59.7 and 57.1).  (For as long as a large step takes; then, or if something went wrong, the stream
+  // has the word, and all mail is there.)
   const int ids = h->awaited_ids.exchange(0), records = h->awaited_records.exchange(0);
+  const uint32_t tag = h->mail_tag;
   auto there = [&](int row) {
     if (ids) return *reinterpret_cast<volatile int32_t*>(h->h_tokens + row) != kNoToken;
     const volatile u64* mail = h->h_mail + (size_t)row * hs::kRecordWords;
+    if ((uint32_t)(mail[0] >> 32) != tag) return false;
     const int n = h->mail_words[(size_t)row];
-    uint32_t words[hs::kRecordWords];
+    uint32_t words[hs::kRecordWords], other = 0;
     for (int i = 0; i < n; ++i) {
       const u64 w = mail[i];
-      if ((uint32_t)(w >> 32) != h->mail_tag) return false;
+      other |= (uint32_t)(w >> 32) ^ tag;
       words[i] = (uint32_t)w;
     }
+    if (other) return false;
     std::memcpy(h->h_out + row, words, (size_t)n * 4);
     return true;
   };
-  const int n = ids + records;
-  int seen = 0;
-  for (int turn = 0; turn < 200000 && seen < n; ++turn) {
-    while (seen < n && there(seen)) ++seen;
-    if (seen < n) hs_pause();
+  int* const pending = h->pending.data();
+  int left = ids + records;
+  for (int row = 0; row < left; ++row) pending[row] = row;
+  const bool awaited = left > 0;
+  auto look = [&] {
+    int kept = 0;
+    for (int i = 0; i < left; ++i)
+      if (!there(pending[i])) pending[kept++] = pending[i];
+    left = kept;
+  };
+  for (int looks = 0; looks < 200000 && left > 0; looks += 1 + left / 64) {
+    look();
+    if (left > 0) hs_pause();
   }
   std::atomic_thread_fence(std::memory_order_acquire);
-  if (n > 0 && seen == n) return HS_OK;
+  if (awaited && left == 0) return HS_OK;
   DeviceGuard guard(h->device);
   HS_CUDA(h, cudaStreamSynchronize((cudaStream_t)stream));
-  if (records && h->mail_only)
-    for (; seen < n; ++seen)
-      if (!there(seen)) return fail(h, HS_ERR_CUDA, "a step's records did not come");
+  look();
+  if (records && left > 0) return fail(h, HS_ERR_CUDA, "a step's records did not come");
   return HS_OK;
 }
 
