@@ -292,14 +292,18 @@ int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride
   if (dtype == HS_DTYPE_BF16 && !h->force_general && !(flags & HS_SAMPLE_GENERAL_KERNEL)) {
     // One launch: the parts of the counting rows, then the parts of the candidate rows, two CTAs
     // resident per SM.  How many rows take which path is known when the parameters come from the
-    // host (n_count >= 0).  Counting goes at the rate of an SM's shared atomics, so two counting CTAs on
-    // one gain nothing: the rows are cut into as many parts as give every SM one, eight at most and
-    // none below 32,768 tokens; and not at all when that makes less than four of them, because the
-    // hand-over then costs what the shorter count saves (us a call, whole rows / 2 / 4 parts: 64 rows of
-    // 151,936 82.3 / 91.2 / 81.7, 100 rows 93.5 / 104.3 / -, one row of 50,257 53.7 / 58.7 / 57.9; one
-    // row of 248,320 in 4 / 8 / 12 / 16 parts 89.2 / 85.5 / 88.7 / 93.5).  Candidate rows get what the wave
-    // has left, up to eight CTAs each (a second, partial wave costs more than idle SMs in the first), none
-    // below 16,384 tokens, its bound's sample.
+    // host (n_count >= 0).  Counting goes at the rate of an SM's shared atomics, so the rows are cut into as
+    // many parts as give every SM one, eight at most and none below 32,768 tokens (one row of 248,320 in 1 / 2 /
+    // 4 / 8 parts 58.2 / 54.5 / 51.1 / 50.5 us a call; whole or in four parts, one row and sixteen: of 98,304
+    // 47.3 / 47.3 and 47.4 / 48.1, of 128,256 48.5 / 47.8 and 50.9 / 48.9, of 151,936 51.5 / 49.4 and 53.7 / 50.3).
+    // Where that, or the hand-over scratch, makes less than four of them, the hand-over costs what the
+    // shorter count saves (64 rows of 151,936 whole or in two: 58.3 / 61.8), unless so many candidate rows
+    // share the SMs that whole counting rows wait for them and for each other: as many candidate rows as counting
+    // ones and more CTAs than SMs, or a quarter as many and a third more CTAs than SMs (whole or in two, 64 among 96
+    // rows 63.8 / 66.8, 80 among 100 63.6 / 67.9, but 64 among 128 70.8 / 69.4, 100 among 128 74.4 / 70.2), and rows of
+    // 131,072 on (64 among 256, of 65,536 64.9 / 66.8, of 131,072 77.8 / 73.5, of 248,320 100.8 / 87.4).
+    // Candidate rows get what the wave has left, up to eight CTAs each (a second, partial wave costs more
+    // than idle SMs in the first), none below 16,384 tokens, its bound's sample.
     // When the host does not know, every row may be either: four parts as far as the hand-over
     // scratch goes, else whole rows (256 rows of 248,320, half of them counting: 61.9 us a step, 66.0 in two
     // parts), and a wave of candidate parts.
@@ -308,8 +312,14 @@ int launch_rows(hs_sampler* h, const void* logits, int dtype, int64_t row_stride
     int csplit, split;
     if (known) {
       const int n_cand = batch - n_count;
-      csplit = std::min({h->sm_count / std::max(1, n_count), 8, vocab / 32768});
-      if (csplit < 4) csplit = 1;
+      const int most = h->ctab_tables / batch;
+      csplit = std::min({h->sm_count / std::max(1, n_count), 8, vocab / 32768, most});
+      if (csplit < 4) {
+        const int halves = 2 * n_count + n_cand;  // CTAs, the counting rows in two
+        const bool mixed = 2 * n_count <= resident && ((n_cand >= n_count && halves > h->sm_count) ||
+                                                       (4 * n_cand >= n_count && 3 * halves >= 4 * h->sm_count));
+        csplit = mixed && vocab >= 131072 ? std::max(1, std::min(std::max(csplit, 2), most)) : 1;
+      }
       split = (resident - std::min(resident, n_count * csplit)) / std::max(1, n_cand);
       split = std::max(1, std::min({split, kMaxSplit, vocab / hs::kSample}));
     } else {

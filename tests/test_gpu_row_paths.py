@@ -211,6 +211,26 @@ def test_min_p_down_to_the_smallest_number(min_p, penalised):
         s.close()
 
 
+@pytest.mark.parametrize("counting, batch, vocab", [(1, 1, 131_072), (1, 1, 248_320), (1, 1, 262_144), (37, 37, 131_072),  # four to eight parts
+                                                    (40, 120, 131_072), (20, 150, 151_936), (40, 160, 131_071),  # three; none
+                                                    (64, 128, 131_072), (60, 75, 131_072), (4, 300, 131_072)])  # two; none
+def test_the_parts_a_step_chooses(counting, batch, vocab):
+    """A step knows which of its rows count and cuts them as it sees fit: the same rows whole."""
+    logits = (torch.randn(batch, vocab, generator=torch.Generator(device="cuda").manual_seed(vocab), device="cuda") * 3).to(torch.bfloat16)
+    params = [SamplingParams(temperature=1.0, top_p=0.95, seed=i, logprobs=3) if i % (batch // counting) == 0 and i < counting * (batch // counting)
+              else SamplingParams(temperature=0.7, top_k=50, top_p=0.9, seed=i) for i in range(batch)]
+    assert sum(p.top_k == 0 for p in params) == counting
+    s = _sampler(vocab, batch)
+    try:
+        for step in range(3):
+            s.set_count_split(1)
+            want = s.step(logits, [[]] * batch, params, [step] * batch)
+            s.set_count_split(0)
+            assert s.step(logits, [[]] * batch, params, [step] * batch) == want
+    finally:
+        s.close()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("vocab", [1, 9, 31, 5_003, 50_257])
 def test_greedy_rows_off_the_16_byte_grid(dtype, vocab):
