@@ -721,15 +721,20 @@ __device__ __noinline__ int nth_in_parts(int cell, u64 n) {
   }
   if (g == parts) return -1;
   const int per = chunks_per_part(c.n8(), parts), first = min(g * per, c.n8());
+  // (the part as a row of its own, its ids counted from `from`; a last part without a chunk, which need not start
+  // on a whole word of classes, has the loose tokens alone)
   ScanArgs a = scan_args(c);
-  a.chunk0 = first;
   a.n8 = min(per, c.n8() - first);
+  const int from = a.n8 ? 8 * first : 0;
+  a.logits += from;
+  if (a.cls) a.cls += from / 16;
+  a.head += 8 * first - from;
+  a.vocab = g < parts - 1 ? a.head + 8 * a.n8 : c.vocab - from;
   a.front = 0;
-  if (g < parts - 1) a.back = c.vocab;
   scan_members<true>(a, raw, kNoRaw, kNoRaw, cc, (int)n - before, in_part);
   const u64 hit = c.x()->bcast[6];
   __syncthreads();
-  return (int)hit - 1;
+  return hit ? from + (int)hit - 1 : -1;
 }
 
 // Finds what a draw asks for: its own function, for the registers of the scan.

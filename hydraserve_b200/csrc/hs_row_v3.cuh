@@ -130,8 +130,9 @@ static_assert(sizeof(uint32_t) * (3 * kV3Buckets + kV3TieCap) + sizeof(V3Member)
               sizeof(int2) * kV3RareCap + sizeof(int) * kV3DeferCap <= sizeof(uint32_t) * kV3Staged,
               "the two uses fit the shared place");
 
-// Chunks of eight tokens a part of a counting row takes (the last one takes what is left).
-__device__ __forceinline__ int chunks_per_part(int n8, int parts) { return (n8 + parts - 1) / parts; }
+// Chunks of eight tokens a part of a counting row takes (the last one takes what is left): an even number, so
+// that the count classes of every part start on a whole word.
+__device__ __forceinline__ int chunks_per_part(int n8, int parts) { return ((n8 + parts - 1) / parts + 1) & ~1; }
 
 __device__ __forceinline__ int v3_bin_of_raw(uint32_t raw) {
   const uint32_t idx = (raw & 0x7fffu) - kV3Base;
@@ -496,13 +497,14 @@ __device__ __noinline__ int nth_in_large_group(Ctx3& c, const Group g, u64 n) {
 // a 248,320-token row).
 static_assert(kV3ScanCap <= kV3TieCap - 4, "scan ids fit the list of ids");
 // (Not inlined, and handed plain values instead of the row's context: the registers of the kernel's
-// main body are all taken.)
+// main body are all taken.  And no more of them than a whole row needs: with a range's first chunk as a value of
+// its own the walk of a row with penalties took 57.4 thousand cycles from the cuts to the token, 52.7 without; 200
+// such rows of 248,320 among 256 137.2 us a call and 132.0.)
 struct ScanArgs {
   const unsigned short* logits;
   const uint32_t* cls;
-  int vocab, head;
-  int chunk0, n8;   // the chunks to walk: chunk0 to chunk0 + n8 - 1,
-  int front, back;  // with the tokens ahead of `front` and those from `back` on
+  int vocab, head, n8;
+  int front;      // of the loose tokens ahead of the first chunk, how many are looked at: all (head) or none
   int* ids;       // [kV3TieCap]
   int* slot_n;    // ids in the list so far (the caller's own members first)
   int* step_n;    // [2]
@@ -527,8 +529,7 @@ __device__ __noinline__ void scan_members(const ScanArgs c, uint32_t raw0, uint3
   if (tid == 0) { c.step_n[0] = 0; c.step_n[1] = 0; *c.result = 0; }
   __syncthreads();
   const int n8 = c.n8;
-  const int first_id = c.head + 8 * c.chunk0;
-  const uint4* src4 = reinterpret_cast<const uint4*>(c.logits + first_id);
+  const uint4* src4 = reinterpret_cast<const uint4*>(c.logits + c.head);
   // Members found are counted in two counters that take turns from one look to the next:
   // after a look's barrier every thread reads that turn's counter, which nobody adds to before
   // the barrier after next, so all threads see the same running total and leave together.
@@ -542,7 +543,8 @@ __device__ __noinline__ void scan_members(const ScanArgs c, uint32_t raw0, uint3
     const int id = from + tid;
     if (id < to && member((uint32_t)c.logits[id], c.cls ? (int)((c.cls[id >> 4] >> ((id & 15) * 2)) & 3u) : 0)) note(id, parity);
   };
-  if (forward) loose(0, c.front, 0); else loose(c.back, c.vocab, 0);
+  const int tail_at = c.head + 8 * n8;
+  if (forward) loose(0, c.front, 0); else loose(tail_at, c.vocab, 0);
   constexpr int kBatch = 4;
   constexpr int kStep = kBatch * kThreads;  // chunks per step
   constexpr int kCheckShift = 1;            // the walk looks whether it may stop every 2^kCheckShift steps
@@ -557,9 +559,9 @@ __device__ __noinline__ void scan_members(const ScanArgs c, uint32_t raw0, uint3
     w[u] = __ldcg(src4 + i);
     if (!c.cls) return;
     if (c.head == 0) {
-      cl[u] = (uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(c.cls) + c.chunk0 + i);
+      cl[u] = (uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(c.cls) + i);
     } else {
-      const int id = first_id + 8 * i;
+      const int id = c.head + 8 * i;
       cl[u] = __funnelshift_r(__ldcg(c.cls + (id >> 4)), __ldcg(c.cls + (id >> 4) + 1), (uint32_t)(id & 15) * 2u);
     }
   };
@@ -588,7 +590,7 @@ __device__ __noinline__ void scan_members(const ScanArgs c, uint32_t raw0, uint3
           hits &= hits - 1;
           const uint32_t word = q < 2 ? cur.x : (q < 4 ? cur.y : (q < 6 ? cur.z : cur.w));
           if (member((word >> (16 * (q & 1))) & 0xffffu, (int)((cur_cl >> (2 * q)) & 3u)))
-            note(first_id + 8 * chunk_of(s, u) + q, (s >> kCheckShift) & 1);
+            note(c.head + 8 * chunk_of(s, u) + q, (s >> kCheckShift) & 1);
         }
       }
     }
@@ -603,7 +605,7 @@ __device__ __noinline__ void scan_members(const ScanArgs c, uint32_t raw0, uint3
       if (total >= need) { reached = true; break; }
     }
   }
-  if (!reached) { if (forward) loose(c.back, c.vocab, 0); else loose(0, c.front, 0); }
+  if (!reached) { if (forward) loose(tail_at, c.vocab, 0); else loose(0, c.front, 0); }
   __syncthreads();
   const int found = min(*c.slot_n, kV3ScanCap);
   if (tid < 4) ids[found + tid] = forward ? 0x7fffffff : -1;
@@ -623,7 +625,7 @@ __device__ __noinline__ void scan_members(const ScanArgs c, uint32_t raw0, uint3
   __syncthreads();
 }
 __device__ __forceinline__ ScanArgs scan_args(const Ctx3& c) {
-  return ScanArgs{c.logits, c.cls, c.vocab, c.head(), 0, c.n8(), c.head(), c.head() + 8 * c.n8(), c.list(), c.gbuf_n(), c.step_n(), &c.x()->bcast[6]};
+  return ScanArgs{c.logits, c.cls, c.vocab, c.head(), c.n8(), c.head(), c.list(), c.gbuf_n(), c.step_n(), &c.x()->bcast[6]};
 }
 // Token id of the n-th member of a group: by one scan when the group is small enough.
 __device__ int nth_in_group(Ctx3& c, const Group& g, u64 n) {

@@ -66,7 +66,8 @@ def test_small_top_k_rows_match_the_general_kernel(kind, vocab):
         s.close()
 
 
-@pytest.mark.parametrize("vocab", [8_192, 50_257, 65_543, 151_936])
+# (47 tokens: parts without a chunk, and one of those has the loose tokens)
+@pytest.mark.parametrize("vocab", [47, 8_192, 50_257, 65_543, 151_936])
 @pytest.mark.parametrize("kind", ["usual", "few values", "masked"])
 def test_a_counted_row_is_the_same_in_any_number_of_parts(kind, vocab):
     """The token too: it is the n-th member of a class whichever part holds it, and the same whether the
@@ -92,7 +93,7 @@ def test_a_counted_row_is_the_same_in_any_number_of_parts(kind, vocab):
                 general, _ = s.run(logits, rec, general=True)
                 for name in COUNTS:
                     np.testing.assert_array_equal(want[name], general[name], err_msg=f"{name}, against the general kernel")
-                for split in (2, 4, 0):
+                for split in (2, 3, 4, 5, 7, 8, 16, 0):
                     s.set_count_split(split)
                     for rows in (logits, odd):
                         got, _ = s.run(rows, rec)
