@@ -54,20 +54,29 @@ def test_a_wait_is_for_the_step_before_it(built_library):
     from hydraserve_b200 import _lib
     from hydraserve_b200.engine import _device
 
-    batch, unwritten = 8, 0x7fffffff
-    logits = torch.randn(batch, VOCAB, generator=torch.Generator().manual_seed(1)).cuda().bfloat16()
-    best = logits.argmax(1).tolist()
+    batch = 8
     s = _device.DeviceSampler("cuda:0", vocab_max=VOCAB, batch_max=batch, resident_slots=1)
     rec = _device.pack_params([SamplingParams(temperature=1.0, top_k=1, seed=i) for i in range(batch)], [0] * batch)
     stream = s._stream()
+    logits, records = None, None  # (of the step; where the sampler's records stand)
+
+    def rows(seed):  # and where each has its maximum
+        gen = torch.Generator().manual_seed(seed)
+        x, best = torch.randn(batch, VOCAB, generator=gen), torch.randint(0, VOCAB, (batch,), generator=gen)
+        x[range(batch), best] = 9.0
+        return x.cuda().bfloat16(), best.tolist()
 
     def sample():
+        nonlocal records
+        if records:  # (nothing of an earlier step is left there)
+            C.memset(records, 0x55, batch * 208)
         block, out = C.c_void_p(), C.c_void_p()
         assert s.lib.hs_step_block(s.handle, rec.nbytes, C.byref(block)) == 0
         C.memmove(block.value, rec.ctypes.data, rec.nbytes)
         d = _Desc(rec.nbytes, rec.nbytes, rec.nbytes, rec.nbytes, rec.nbytes, 0, 0, 0, 0)
         assert s.lib.hs_step(s.handle, logits.data_ptr(), 1, VOCAB, batch, VOCAB, C.byref(d), C.byref(out), stream) == 0
-        return lambda: np.frombuffer((C.c_char * (batch * 208)).from_address(out.value), dtype=_lib.ROW_OUT)
+        records = out.value
+        return lambda: np.frombuffer((C.c_char * (batch * 208)).from_address(records), dtype=_lib.ROW_OUT)
 
     def greedy():
         out = C.c_void_p()
@@ -75,16 +84,18 @@ def test_a_wait_is_for_the_step_before_it(built_library):
         return lambda: np.frombuffer((C.c_int32 * batch).from_address(out.value), dtype=np.int32)
 
     try:
-        for first in (greedy, sample, greedy, sample):
+        for step, first in enumerate((greedy, sample, greedy, sample, greedy)):
+            logits, _ = rows(2 * step)
             first()
             torch.cuda.synchronize()  # (the caller's own wait)
+            logits, best = rows(2 * step + 1)
             torch.cuda._sleep(2_000_000)  # a millisecond: the results cannot be there by themselves
             second = sample if first is greedy else greedy
             read = second()
             assert s.lib.hs_step_wait(s.handle, stream) == 0
             got = read().copy()
             if second is sample:
-                assert (got["status"] != unwritten).all() and got["token"].tolist() == best
+                assert not got["status"].any() and got["token"].tolist() == best
             else:
                 assert got.tolist() == best
             torch.cuda.synchronize()
