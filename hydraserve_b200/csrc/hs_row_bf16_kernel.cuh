@@ -289,9 +289,9 @@ __device__ __forceinline__ bool count_tokens(const RowV3Args& args, int row_inde
     // The part that draws the last ticket adds the other parts' lists to its own table and goes on;
     // the others are done.  Nobody waits for anybody.  (Lists instead of whole tables: about 16 KB a
     // part instead of 72.)  Bound by the banks when a list is added up, and by the round trips to L2: in the
-    // order of the cells, four entries a load and the next piece under way, the first token after a prompt
-    // of 8,192 takes 97.2 us a call, 107.6 before (248,320 tokens, sixteen parts; the look-up in
-    // nth_in_parts has its share in that).
+    // order of the cells, four entries a load and the next piece under way (by thread, one entry a load and list
+    // by list, and without the look-up in nth_in_parts, a call of one row of 248,320 took 107.6 us and 97.2 this way, when
+    // such a row was cut in sixteen; with the seven parts of now it takes 87.4).
     const size_t mine = (size_t)c.row * parts + my_part;
     const int nr = *rare_n;
     for (int t = tid; t < min(nr, kV3RareCap); t += kThreads) args.crare[mine * kV3RareCap + t] = rare[t];

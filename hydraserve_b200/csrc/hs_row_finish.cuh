@@ -4,8 +4,8 @@
 // and with two CTAs on an SM almost all of L1 is shared memory, so every spilled value was a round
 // trip to L2.  What bounds it now is the fetching of instructions a CTA goes through once, and the
 // barriers between the passes.  With its count table kept in shared memory and one histogram for all
-// cuts, 64 rows of 151,936 with 20 log-probabilities took 75 us instead of 90 (71 now), 1,024 mixed rows of
-// 151,936 210 instead of 231 (203 now).
+// cuts, 64 rows of 151,936 with 20 log-probabilities took 75 us instead of 90 (72 now), 1,024 mixed rows of
+// 151,936 210 instead of 231 (199 now).
 #pragma once
 
 #include "hs_row_v3.cuh"
@@ -552,8 +552,8 @@ __device__ __noinline__ void draw_by_classes(uint64_t seed) {
   // turn make a list, and its entries j, j + kThreads, ... are chunk j.  (Any fixed order
   // would do; the counts alone decide it.)  A thread adds its cells' masses to their chunks.
   // Only the cells above the cut weigh anything: the others are passed over by their number.  (Bound by the
-  // instructions per cell, of which scores and exponentials are most: this pass 14.9 -> 10.8 thousand cycles a
-  // row with top_p in a batch of 1,024 mixed rows, the one for min_p above 11.9 -> 9.0.)
+  // instructions per cell, of which scores and exponentials are most: over all cells this pass took 14.9 thousand
+  // cycles a row with top_p in a batch of 1,024 mixed rows, 10.8 this way, the one for min_p above 11.9 and 9.0.)
   const uint32_t* tab = c.tab();
   {
     V3Map at_cut;
@@ -676,8 +676,8 @@ __device__ __noinline__ void draw_by_classes(uint64_t seed) {
 // a list of its classes with their counts, in the order of the cells: a warp looks the class up in
 // each list, 32 entries at a time, the counts name the part, and that range alone is scanned.  (The loose
 // tokens belong to the last part, those ahead of the first chunk too.)  Bound by the latency of three or
-// four reads and of the range's: from the draw to the token, cold, 35.7 thousand cycles by a scan of the
-// row, 21.3 thousand this way (64 mixed rows of 151,936 in six parts each).
+// four reads and of the range's: from the cuts to the token 31.8 thousand cycles with a scan of the row, 26.7 this
+// way (one row of 248,320 in seven parts, a call 64.1 and 61.7 us), 29.3 and 26.2 (37 rows of 151,936 in four).
 __device__ __noinline__ int nth_in_parts(int cell, u64 n) {
   CountState& S = count_state();
   Ctx3& c = S.c;

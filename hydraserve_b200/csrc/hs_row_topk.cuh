@@ -65,9 +65,9 @@ struct CandCtx {
 // lie close together, so the 2,048 counters are laid over [lowest key, highest key] instead of
 // over fixed bit fields: one counting pass usually leaves a bucket with a handful of keys,
 // which are then ranked among themselves; a fuller bucket is counted again over its own range.
-// Bound by its barriers and the chains of shuffles between them: both ends in one exchange and counts
-// scanned in 32 bits, seven barriers instead of thirteen, one row of 151,936 46.7 -> 45.3 us a call, 1,024 mixed rows 208.8 ->
-// 206.8 us of GPU time.
+// Bound by its barriers and the chains of shuffles between them, of which it has seven (with an exchange for
+// either end and counts scanned in 64 bits there were thirteen: 1.4 us more of a call of one row of 151,936, 2.0 us more
+// GPU time of 1,024 mixed rows).
 __device__ uint32_t cand_kth_key(Exchange& x, CandCtx& L, int n, int k) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int kResolve = 64;  // in-bucket keys ranked directly
@@ -186,7 +186,8 @@ __device__ int cand_compact(CandCtx& L, int n, uint32_t bound) {
 // 65,536 values of class cc: undoing the score's steps in plain arithmetic gives the value to within a
 // few roundings, and when the 32 values around it hold both sides of the line, one evaluation per lane
 // and a ballot settle it; else they are searched 32 at a time, four such rounds.  Bound by the divisions of
-// one evaluation after another: one row of 151,936 45.8 -> 44.3 us a call, 1,024 mixed rows 206.1 -> 201.1 us of GPU time.
+// one evaluation after another: the search alone took 1.5 us more of a call of one row of 151,936, 5.0 us more GPU time of
+// 1,024 mixed rows.
 __device__ __noinline__ void class_thresholds(const Scorer sc, int* thr, uint32_t bound) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < 3) {
@@ -412,7 +413,7 @@ __device__ int topk_candidates(Ctx3& c, CandCtx& L, int k) {
   SampleRegs sample;
   sample_values(c, sample);
   // (the histograms are up to date from here on: the values do not depend on them, so their loads cross the
-  // end of the kernel that counts the new tokens; one row of 151,936 48.7 -> 47.9 us a call)
+  // end of the kernel that counts the new tokens: 0.8 us of a call of one row of 151,936)
   cudaGridDependencySynchronize();
   int n_heavy = 0, hv_q = -1;
   if (c.cls) {
@@ -598,8 +599,8 @@ __device__ void cand_sort(CandCtx& L, int n) {
 }
 
 // The entries at or above `bound` (void ones drop out in any case), sorted; returns how many.  `tmp` has room
-// for a list.  What cand_compact and cand_sort do, three barriers instead of five: one row of 151,936 44.3 -> 43.9 us a
-// call, 1,024 mixed rows 201.1 -> 200.0 us of GPU time.
+// for a list.  What cand_compact and cand_sort do, with three barriers instead of five: 0.4 us of a call of one row of
+// 151,936, 1.1 us of GPU time of 1,024 mixed rows.
 __device__ int cand_keep_sorted(CandCtx& L, u64* tmp, int n, uint32_t bound) {
   const int tid = threadIdx.x;
   __syncthreads();
